@@ -4,6 +4,7 @@
 
 #include "clique.cuh"
 #include "graph.cuh"
+#include "rows.cuh"
 #include "sched.cuh"
 #include "setprog.cuh"
 
@@ -19,6 +20,7 @@ struct Scalars {
   unsigned long long c4heads[2];
   int64_t n[8];  // task list sizes, copied back for the stats
   unsigned long long terms[6];  // motif-identity sums (launch_motif_terms)
+  OwnHeads own;                 // queue heads of the owner kernels (rows.cu)
 };
 
 struct Model;  // learned cost model (learned.cu)
@@ -108,6 +110,9 @@ void program_buffers_free(xgm_ctx* ctx);
 xgm_status schedule_into(TaskBuf& tb, const DevGraph& g, int k, const xgm_sched& sp,
                          cudaStream_t s, int k_feat = 0, bool hub = false);
 bool sched_may_bucket(const xgm_sched& sp);  // the policy can assign the BUCKET variant
+// The schedule leaves the choice of kernel to the engine: a default or learned policy with
+// no threshold, hub limit or membership test asked for.
+bool sched_is_open(const xgm_sched& sp);
 int ensure_clique_grid(xgm_ctx* ctx);
 int match_pattern(const xgm_plan_desc* d);  // builtin id, 0 unsupported, -1 malformed
 // Builtin id for a pattern name (0 if unknown); GLUMIN ids also set induced / scale.

@@ -58,6 +58,16 @@ bool sched_may_bucket(const xgm_sched& sp) {
   return sp.bucket_max > 0;
 }
 
+bool sched_is_open(const xgm_sched& sp) {
+  if (sp.policy == XGM_SCHED_LEARNED) {
+    if (!sp.model) return false;  // refused by schedule_into
+  } else if (sp.policy != XGM_SCHED_HEURISTIC || sp.warp_max > 0 || sp.cta_max > 0 ||
+             sp.wide_max != 0 || sp.search_max > 0 || sp.bucket_max > 0 || sp.group_max > 0) {
+    return false;
+  }
+  return sp.hub_max == 0 && !(sp.flags & XGM_SCHED_HASH_ONLY);
+}
+
 // Fills tb from the schedule policy for a k-clique style launch (k = 3 for the
 // participation and multi-pattern launches).  Builds the graph's bucket index first
 // when the policy can pick BUCKET (outside stream capture: callers that capture call
@@ -293,13 +303,18 @@ xgm_status count_dispatch(xgm_ctx* ctx, const DevGraph& g, int pattern, const xg
                           uint64_t* out, xgm_stats& st) {
   cudaStream_t s = ctx->stream;
   XGM_CUDA_TRY(cudaSetDevice(ctx->device));
-  XGM_CUDA_TRY(taskbuf_reserve(ctx->tb, g.nv, s));
+  const int k = clique_kind(pattern);
+  const bool owner = k == 3 && sched_is_open(sp);
+  if (!owner) XGM_CUDA_TRY(taskbuf_reserve(ctx->tb, g.nv, s));
   XGM_CUDA_TRY(cudaMemsetAsync(ctx->d_sc, 0, sizeof(Scalars), s));
   XGM_CUDA_TRY(cudaEventRecord(ctx->ev[0], s));
-  const int k = clique_kind(pattern);
   const GView view = g.view();
   int launches = 0;
-  if (k) {
+  if (owner) {
+    XGM_CUDA_TRY(cudaEventRecord(ctx->ev[1], s));
+    XGM_CUDA_TRY(launch_owner_count(g, &ctx->d_sc->own, &ctx->d_sc->count, ctx->num_sms, s));
+    launches = 1;
+  } else if (k) {
     xgm_status r = schedule_tasks(ctx, g, k, sp, true);
     if (r != XGM_OK) return r;
     XGM_CUDA_TRY(cudaEventRecord(ctx->ev[1], s));
@@ -344,7 +359,7 @@ xgm_status count_dispatch(xgm_ctx* ctx, const DevGraph& g, int pattern, const xg
     return XGM_ERR_INVALID;
   }
   XGM_CUDA_TRY(cudaEventRecord(ctx->ev[2], s));
-  if (k || pattern == XGM_PATTERN_DIAMOND || pattern == XGM_PATTERN_TAILED_TRIANGLE)
+  if ((k && !owner) || pattern == XGM_PATTERN_DIAMOND || pattern == XGM_PATTERN_TAILED_TRIANGLE)
     XGM_CUDA_TRY(cudaMemcpyAsync(ctx->d_sc->n, ctx->tb.n, sizeof(int64_t) * 8,
                                  cudaMemcpyDeviceToDevice, s));
   xgm_status r = ctx_sync_scalars(ctx);
@@ -365,6 +380,7 @@ xgm_status count_dispatch(xgm_ctx* ctx, const DevGraph& g, int pattern, const xg
   st.variant_tasks[XGM_VAR_GROUP] = ctx->h_sc->n[7];
   st.tasks = ctx->h_sc->n[1] + ctx->h_sc->n[2] + ctx->h_sc->n[3] + ctx->h_sc->n[4] +
              ctx->h_sc->n[5] + ctx->h_sc->n[6] + ctx->h_sc->n[7];
+  if (owner) st.tasks = g.n_roots[0];
   r = check_device_flag(ctx, ctx->h_sc->err);
   if (r != XGM_OK) return r;
   *out = ctx->h_sc->count;
@@ -382,6 +398,10 @@ xgm_status count_kernels(xgm_ctx* ctx, const DevGraph& g, int pattern, const xgm
   if (!k) {
     set_thread_error("kernel counting covers the triangle / clique plans");
     return XGM_ERR_UNSUPPORTED;
+  }
+  if (k == 3 && sched_is_open(sp)) {
+    *n_kernels = g.nv > 0 ? 1 : 0;
+    return XGM_OK;
   }
   ensure_clique_grid(ctx);
   if (sched_may_bucket(sp)) XGM_CUDA_TRY(ensure_bucket_index(g, s));

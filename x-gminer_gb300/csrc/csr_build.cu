@@ -15,6 +15,7 @@
 
 #include "graph.cuh"
 #include "prim.cuh"
+#include "rows.cuh"
 
 namespace xgm {
 
@@ -229,9 +230,11 @@ __global__ void k_extract_col(const uint64_t* keys, int64_t ne, int vb, int32_t*
 
 // dptr[r] = {first entry of row r with id > r, row end}; stats of the DAG.
 __global__ void k_dptr(const int64_t* rowptr, const int32_t* col, int64_t nv, longlong2* dptr,
-                       unsigned long long* max_out, unsigned long long* ne_dag) {
+                       unsigned long long* max_out, unsigned long long* ne_dag,
+                       unsigned long long* n_big, unsigned long long* n_roots) {
   int64_t mo = 0;
   unsigned long long sum = 0;
+  unsigned cnt[5] = {0, 0, 0, 0, 0};  // degree > kBigDeg; out-degree >= 2, 3, 4, 5
   for (int64_t r = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; r < nv;
        r += (int64_t)gridDim.x * blockDim.x) {
     int64_t lo = rowptr[r], hi = rowptr[r + 1];
@@ -244,6 +247,14 @@ __global__ void k_dptr(const int64_t* rowptr, const int32_t* col, int64_t nv, lo
     int64_t d = hi - a;
     mo = d > mo ? d : mo;
     sum += (unsigned long long)d;
+    cnt[0] += hi - lo > kBigDeg;
+#pragma unroll
+    for (int t = 1; t < 5; ++t) cnt[t] += d > t;
+  }
+#pragma unroll
+  for (int t = 0; t < 5; ++t) {
+    const unsigned c = __reduce_add_sync(kFull, cnt[t]);
+    if ((threadIdx.x & 31) == 0 && c) atomicAdd(t ? n_roots + t - 1 : n_big, (unsigned long long)c);
   }
 #pragma unroll
   for (int o = 16; o > 0; o >>= 1) {
@@ -399,16 +410,17 @@ cudaError_t finish_graph(DevGraph& g, const int32_t* group, int num_groups, cuda
   const int64_t nv = g.nv, ne = g.ne;
   const int vb = bits_for(nv);
   int32_t *deg = nullptr, *degp = nullptr;
-  unsigned long long* stats = nullptr;  // [0] max deg, [1] max out, [2] ne_dag, [3] long rows
+  // [0] max deg, [1] max out, [2] ne_dag, [3] long rows, [4] big vertices, [5..8] roots
+  unsigned long long* stats = nullptr;
   TRY(dalloc(&deg, nv, s));
   TRY(dalloc(&degp, nv, s));
-  TRY(dalloc(&stats, 4, s));
-  TRY(cudaMemsetAsync(stats, 0, 4 * sizeof(unsigned long long), s));
+  TRY(dalloc(&stats, 9, s));
+  TRY(cudaMemsetAsync(stats, 0, 9 * sizeof(unsigned long long), s));
   if (nv > 0) {
     k_degrees<<<grid_for(nv), kThreads, 0, s>>>(g.rowptr_o, nv, deg, stats);
     TRY(cudaGetLastError());
   }
-  unsigned long long h[3] = {0, 0, 0};
+  unsigned long long h[9] = {};
   TRY(cudaMemcpyAsync(h, stats, sizeof(h), cudaMemcpyDeviceToHost, s));
   TRY(cudaStreamSynchronize(s));
   g.max_deg = (int64_t)h[0];
@@ -463,13 +475,16 @@ cudaError_t finish_graph(DevGraph& g, const int32_t* group, int num_groups, cuda
     TRY(cudaGetLastError());
   }
   if (nv > 0) {
-    k_dptr<<<grid_for(nv), kThreads, 0, s>>>(g.rowptr, g.col, nv, g.dptr, stats + 1, stats + 2);
+    k_dptr<<<grid_for(nv), kThreads, 0, s>>>(g.rowptr, g.col, nv, g.dptr, stats + 1, stats + 2,
+                                             stats + 4, stats + 5);
     TRY(cudaGetLastError());
   }
   TRY(cudaMemcpyAsync(h, stats, sizeof(h), cudaMemcpyDeviceToHost, s));
   TRY(cudaStreamSynchronize(s));
   g.max_out = (int64_t)h[1];
   g.ne_dag = (int64_t)h[2];
+  g.n_big = group ? 0 : (int64_t)h[4];
+  for (int i = 0; i < 4; ++i) g.n_roots[i] = (int64_t)h[5 + i];
   cudaFreeAsync(keys, s);
   cudaFreeAsync(tmp, s);
   cudaFreeAsync(deg, s);

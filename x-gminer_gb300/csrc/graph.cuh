@@ -15,6 +15,9 @@ struct DevGraph {
   int64_t ne_dag = 0;      // entries kept by the orientation (= ne / 2)
   int64_t max_deg = 0;
   int64_t max_out = 0;     // max out-degree of the oriented DAG
+  int64_t n_big = 0;       // vertices of degree > kBigDeg: the top ranks (rows.cuh; 0 for
+                           // batched graphs, whose ranks are sorted by degree per graph)
+  int64_t n_roots[4] = {0, 0, 0, 0};  // vertices of out-degree >= 2, 3, 4, 5
   int64_t* rowptr_o = nullptr;
   int32_t* col_o = nullptr;
   int32_t* rank = nullptr;   // [nv] original -> rank
