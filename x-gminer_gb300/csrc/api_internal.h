@@ -64,6 +64,8 @@ struct xgm_ctx {
   int64_t* c4_ttab = nullptr;  // per group: tseg[m+1] then tcnt[m]
   int64_t c4_task_cap = 0;
   int clique_grid = 0;
+  uint32_t* rows = nullptr;  // row store (rows.cu)
+  int64_t rows_cap = 0;
   // set-operation programs (setprog.cu): per-warp slot scratch, split records, heads
   int32_t* prog_scratch = nullptr;
   int64_t prog_scratch_cap = 0;

@@ -58,6 +58,18 @@ bool sched_may_bucket(const xgm_sched& sp) {
   return sp.bucket_max > 0;
 }
 
+namespace {
+
+// The hub kernel counts up to 5-cliques, by default up to 4-cliques: at 5 the split
+// sub-tasks win (each works on the compressed rows of N+(v0) & N+(v1); R-MAT scale 23:
+// split 6.47 s, whole hubs 7.37 s; 4-cliques 1.08 s -> 0.25 s with whole hubs).
+int whole_hub_max(int k, int asked) {
+  if (k > 5 || asked < 0 || (asked == 0 && k > 4)) return 0;
+  return asked == 0 ? kHubCap : asked;
+}
+
+}  // namespace
+
 bool sched_is_open(const xgm_sched& sp) {
   if (sp.policy == XGM_SCHED_LEARNED) {
     if (!sp.model) return false;  // refused by schedule_into
@@ -122,13 +134,7 @@ xgm_status schedule_into(TaskBuf& tb, const DevGraph& g, int k, const xgm_sched&
     if (bmax > 0) XGM_CUDA_TRY(ensure_bucket_index(g, s));
     XGM_CUDA_TRY(classify_heuristic(g, k, wmax, dmax, cmax, tb, s, smax, bmax, gmax));
   }
-  // The hub kernel counts up to 5-cliques, by default up to 4-cliques: at 5 the split
-  // sub-tasks win (each works on the compressed rows of N+(v0) & N+(v1); R-MAT scale 23:
-  // split 6.47 s, whole hubs 7.37 s; 4-cliques 1.08 s -> 0.25 s with whole hubs).
-  const int hub_max = (!hub || k > 5 || sp.hub_max < 0 || (sp.hub_max == 0 && k > 4))
-                          ? 0
-                          : (sp.hub_max == 0 ? kHubCap : sp.hub_max);
-  XGM_CUDA_TRY(build_lists(g, tb, order, s, hub_max));
+  XGM_CUDA_TRY(build_lists(g, tb, order, s, hub ? whole_hub_max(k, sp.hub_max) : 0));
   tb.hash_only = (sp.flags & XGM_SCHED_HASH_ONLY) ? 1 : 0;
   return XGM_OK;
 }
@@ -138,6 +144,65 @@ namespace {
 xgm_status schedule_tasks(xgm_ctx* ctx, const DevGraph& g, int k, const xgm_sched& sp,
                           bool hub = false) {
   return schedule_into(ctx->tb, g, k, sp, ctx->stream, 0, hub);
+}
+
+// The row store holds a graph's rows up to 16 GB (R-MAT scale 22: 0.6 GB); larger graphs,
+// and a device without that much memory left, count with the task kernel.
+constexpr int64_t kRowStoreMax = int64_t(1) << 32;  // words
+
+// What a clique count launches: the owner kernel (triangles), the row kernels (k >= 4; the
+// task kernel then only runs the vertices above their capacity), or the task kernel.
+enum class CliqueRoute { kOwner, kRows, kTasks };
+
+// Chooses the route and gets its buffers and per-graph indexes (outside stream capture).
+xgm_status clique_route(xgm_ctx* ctx, const DevGraph& g, int k, const xgm_sched& sp,
+                        CliqueRoute* route) {
+  cudaStream_t s = ctx->stream;
+  *route = CliqueRoute::kTasks;
+  if (sched_is_open(sp)) {
+    if (k == 3) {
+      *route = CliqueRoute::kOwner;
+    } else if (g.nv > 0 && g.row_store_words <= kRowStoreMax) {
+      XGM_CUDA_TRY(ensure_rows_index(g, s));
+      const cudaError_t e = grow(&ctx->rows, &ctx->rows_cap, g.row_store_words + 4, s);
+      if (e == cudaSuccess) *route = CliqueRoute::kRows;
+      else if (e != cudaErrorMemoryAllocation) XGM_CUDA_TRY(e);
+      else cudaGetLastError();
+    }
+  }
+  if (*route == CliqueRoute::kTasks || (*route == CliqueRoute::kRows && g.max_out > kRowsCap))
+    XGM_CUDA_TRY(taskbuf_reserve(ctx->tb, g.nv, s));
+  if (*route == CliqueRoute::kTasks && sched_may_bucket(sp)) XGM_CUDA_TRY(ensure_bucket_index(g, s));
+  return XGM_OK;
+}
+
+// Enqueues the schedule (before `mark`, when given) and the counting kernels.
+xgm_status launch_route(xgm_ctx* ctx, const DevGraph& g, int k, const xgm_sched& sp,
+                        CliqueRoute route, cudaEvent_t mark, int* launches) {
+  cudaStream_t s = ctx->stream;
+  Scalars* sc = ctx->d_sc;
+  const bool hubs = route == CliqueRoute::kRows && g.max_out > kRowsCap;
+  if (route == CliqueRoute::kTasks) {
+    xgm_status r = schedule_tasks(ctx, g, k, sp, true);
+    if (r != XGM_OK) return r;
+  } else if (hubs) {  // only the vertices above the row capacity are tasks
+    XGM_CUDA_TRY(classify_heuristic(g, kRowsCap + 2, kWarpCap, kWideCap, kCtaCap, ctx->tb, s));
+    XGM_CUDA_TRY(build_lists(g, ctx->tb, false, s, whole_hub_max(k, 0)));
+  }
+  if (mark) XGM_CUDA_TRY(cudaEventRecord(mark, s));
+  if (launches) *launches = 1;
+  if (route == CliqueRoute::kOwner)
+    XGM_CUDA_TRY(launch_owner_count(g, &sc->own, &sc->count, ctx->num_sms, s));
+  if (route == CliqueRoute::kTasks || hubs) {
+    XGM_CUDA_TRY(launch_clique(k, g.view(), ctx->tb.lists(false), &sc->q, &sc->count, &sc->err,
+                               ensure_clique_grid(ctx), s));
+    if (launches && ctx->tb.hub_max > kCtaCap) *launches = 2;  // + the hub kernel
+  }
+  if (route == CliqueRoute::kRows) {
+    XGM_CUDA_TRY(launch_owner_rows(g, ctx->rows, &sc->own, ctx->num_sms, s));
+    XGM_CUDA_TRY(launch_rows_count(k, g, ctx->rows, &sc->own, &sc->count, ctx->num_sms, s));
+  }
+  return XGM_OK;
 }
 
 xgm_status ensure_c4(xgm_ctx* ctx, const DevGraph& g) {
@@ -294,7 +359,7 @@ void motif_buffers_free(xgm_ctx* ctx) {
   void* ps[] = {ctx->vpart, ctx->epart, ctx->c4_scratch, ctx->wedges, ctx->c4_flag_large,
                 ctx->c4_flag_small, ctx->c4_pos, ctx->c4_large, ctx->c4_small, ctx->c4_n,
                 ctx->c4_counters, ctx->c4_info, ctx->c4_seg_base, ctx->c4_seg_pre,
-                ctx->c4_seg_cnt, ctx->c4_tv0, ctx->c4_ttab};
+                ctx->c4_seg_cnt, ctx->c4_tv0, ctx->c4_ttab, ctx->rows};
   for (void* p : ps)
     if (p) cudaFreeAsync(p, s);
 }
@@ -304,23 +369,20 @@ xgm_status count_dispatch(xgm_ctx* ctx, const DevGraph& g, int pattern, const xg
   cudaStream_t s = ctx->stream;
   XGM_CUDA_TRY(cudaSetDevice(ctx->device));
   const int k = clique_kind(pattern);
-  const bool owner = k == 3 && sched_is_open(sp);
-  if (!owner) XGM_CUDA_TRY(taskbuf_reserve(ctx->tb, g.nv, s));
+  CliqueRoute route = CliqueRoute::kTasks;
+  if (k) {
+    xgm_status r = clique_route(ctx, g, k, sp, &route);
+    if (r != XGM_OK) return r;
+  } else {
+    XGM_CUDA_TRY(taskbuf_reserve(ctx->tb, g.nv, s));
+  }
   XGM_CUDA_TRY(cudaMemsetAsync(ctx->d_sc, 0, sizeof(Scalars), s));
   XGM_CUDA_TRY(cudaEventRecord(ctx->ev[0], s));
   const GView view = g.view();
   int launches = 0;
-  if (owner) {
-    XGM_CUDA_TRY(cudaEventRecord(ctx->ev[1], s));
-    XGM_CUDA_TRY(launch_owner_count(g, &ctx->d_sc->own, &ctx->d_sc->count, ctx->num_sms, s));
-    launches = 1;
-  } else if (k) {
-    xgm_status r = schedule_tasks(ctx, g, k, sp, true);
+  if (k) {
+    xgm_status r = launch_route(ctx, g, k, sp, route, ctx->ev[1], &launches);
     if (r != XGM_OK) return r;
-    XGM_CUDA_TRY(cudaEventRecord(ctx->ev[1], s));
-    XGM_CUDA_TRY(launch_clique(k, view, ctx->tb.lists(false), &ctx->d_sc->q, &ctx->d_sc->count,
-                               &ctx->d_sc->err, ensure_clique_grid(ctx), s));
-    launches = ctx->tb.hub_max > kCtaCap ? 2 : 1;  // + the hub kernel
   } else if (pattern == XGM_PATTERN_DIAMOND || pattern == XGM_PATTERN_TAILED_TRIANGLE) {
     xgm_sched tri = sp;
     if (tri.policy == XGM_SCHED_LEARNED && !tri.model) tri.policy = XGM_SCHED_HEURISTIC;
@@ -359,7 +421,7 @@ xgm_status count_dispatch(xgm_ctx* ctx, const DevGraph& g, int pattern, const xg
     return XGM_ERR_INVALID;
   }
   XGM_CUDA_TRY(cudaEventRecord(ctx->ev[2], s));
-  if ((k && !owner) || pattern == XGM_PATTERN_DIAMOND || pattern == XGM_PATTERN_TAILED_TRIANGLE)
+  if ((k && route == CliqueRoute::kTasks) || pattern == XGM_PATTERN_DIAMOND || pattern == XGM_PATTERN_TAILED_TRIANGLE)
     XGM_CUDA_TRY(cudaMemcpyAsync(ctx->d_sc->n, ctx->tb.n, sizeof(int64_t) * 8,
                                  cudaMemcpyDeviceToDevice, s));
   xgm_status r = ctx_sync_scalars(ctx);
@@ -380,7 +442,7 @@ xgm_status count_dispatch(xgm_ctx* ctx, const DevGraph& g, int pattern, const xg
   st.variant_tasks[XGM_VAR_GROUP] = ctx->h_sc->n[7];
   st.tasks = ctx->h_sc->n[1] + ctx->h_sc->n[2] + ctx->h_sc->n[3] + ctx->h_sc->n[4] +
              ctx->h_sc->n[5] + ctx->h_sc->n[6] + ctx->h_sc->n[7];
-  if (owner) st.tasks = g.n_roots[0];
+  if (k && route != CliqueRoute::kTasks) st.tasks = g.n_roots[k - 3];
   r = check_device_flag(ctx, ctx->h_sc->err);
   if (r != XGM_OK) return r;
   *out = ctx->h_sc->count;
@@ -393,35 +455,27 @@ xgm_status count_kernels(xgm_ctx* ctx, const DevGraph& g, int pattern, const xgm
                          int* n_kernels) {
   cudaStream_t s = ctx->stream;
   XGM_CUDA_TRY(cudaSetDevice(ctx->device));
-  XGM_CUDA_TRY(taskbuf_reserve(ctx->tb, g.nv, s));
   const int k = clique_kind(pattern);
   if (!k) {
     set_thread_error("kernel counting covers the triangle / clique plans");
     return XGM_ERR_UNSUPPORTED;
   }
-  if (k == 3 && sched_is_open(sp)) {
-    *n_kernels = g.nv > 0 ? 1 : 0;
-    return XGM_OK;
-  }
+  CliqueRoute route = CliqueRoute::kTasks;
+  xgm_status r = clique_route(ctx, g, k, sp, &route);
+  if (r != XGM_OK) return r;
   ensure_clique_grid(ctx);
-  if (sched_may_bucket(sp)) XGM_CUDA_TRY(ensure_bucket_index(g, s));
   XGM_CUDA_TRY(cudaStreamSynchronize(s));
   XGM_CUDA_TRY(cudaStreamBeginCapture(s, cudaStreamCaptureModeThreadLocal));
-  xgm_status r = schedule_tasks(ctx, g, k, sp, true);
-  cudaError_t e = cudaSuccess;
-  if (r == XGM_OK)
-    e = launch_clique(k, g.view(), ctx->tb.lists(false), &ctx->d_sc->q, &ctx->d_sc->count,
-                      &ctx->d_sc->err, ensure_clique_grid(ctx), s);
+  r = launch_route(ctx, g, k, sp, route, nullptr, nullptr);
   cudaGraph_t graph = nullptr;
   cudaError_t e2 = cudaStreamEndCapture(s, &graph);
   if (r != XGM_OK) {
     if (graph) cudaGraphDestroy(graph);
     return r;
   }
-  XGM_CUDA_TRY(e);
   XGM_CUDA_TRY(e2);
   size_t n = 0;
-  e = cudaGraphGetNodes(graph, nullptr, &n);
+  cudaError_t e = cudaGraphGetNodes(graph, nullptr, &n);
   std::vector<cudaGraphNode_t> nodes(n);
   if (e == cudaSuccess && n) e = cudaGraphGetNodes(graph, nodes.data(), &n);
   int kern = 0;

@@ -234,7 +234,8 @@ __global__ void k_dptr(const int64_t* rowptr, const int32_t* col, int64_t nv, lo
                        unsigned long long* n_big, unsigned long long* n_roots) {
   int64_t mo = 0;
   unsigned long long sum = 0;
-  unsigned cnt[5] = {0, 0, 0, 0, 0};  // degree > kBigDeg; out-degree >= 2, 3, 4, 5
+  unsigned cnt[6] = {0, 0, 0, 0, 0, 0};  // degree > kBigDeg; out-degree >= 2 .. 6
+  unsigned long long words = 0;       // of the row store
   for (int64_t r = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; r < nv;
        r += (int64_t)gridDim.x * blockDim.x) {
     int64_t lo = rowptr[r], hi = rowptr[r + 1];
@@ -247,12 +248,13 @@ __global__ void k_dptr(const int64_t* rowptr, const int32_t* col, int64_t nv, lo
     int64_t d = hi - a;
     mo = d > mo ? d : mo;
     sum += (unsigned long long)d;
+    words += row_words(d);
     cnt[0] += hi - lo > kBigDeg;
 #pragma unroll
-    for (int t = 1; t < 5; ++t) cnt[t] += d > t;
+    for (int t = 1; t < 6; ++t) cnt[t] += d > t;
   }
 #pragma unroll
-  for (int t = 0; t < 5; ++t) {
+  for (int t = 0; t < 6; ++t) {
     const unsigned c = __reduce_add_sync(kFull, cnt[t]);
     if ((threadIdx.x & 31) == 0 && c) atomicAdd(t ? n_roots + t - 1 : n_big, (unsigned long long)c);
   }
@@ -261,8 +263,10 @@ __global__ void k_dptr(const int64_t* rowptr, const int32_t* col, int64_t nv, lo
     int64_t y = __shfl_down_sync(kFull, mo, o);
     mo = y > mo ? y : mo;
     sum += __shfl_down_sync(kFull, sum, o);
+    words += __shfl_down_sync(kFull, words, o);
   }
   if ((threadIdx.x & 31) == 0) {
+    if (words) atomicAdd(n_roots + 5, words);
     if (mo > 0) atomicMax(max_out, (unsigned long long)mo);
     if (sum) atomicAdd(ne_dag, sum);
   }
@@ -341,7 +345,8 @@ cudaError_t dalloc(T** p, int64_t n, cudaStream_t s) {
 
 void free_graph(DevGraph& g, cudaStream_t s) {
   void* ps[] = {g.rowptr_o, g.col_o, g.rank, g.perm, g.rowptr, g.col, g.dptr, g.gid,
-                g.bcol, g.boff, g.bmask, g.lut_rows, g.lut_off, g.tsum, g.tmax};
+                g.bcol, g.boff, g.bmask, g.lut_rows, g.lut_off, g.tsum, g.tmax,
+                g.roff, g.rtask, g.rn};
   for (void* p : ps)
     if (p) cudaFreeAsync(p, s);
   g = DevGraph{};
@@ -410,17 +415,18 @@ cudaError_t finish_graph(DevGraph& g, const int32_t* group, int num_groups, cuda
   const int64_t nv = g.nv, ne = g.ne;
   const int vb = bits_for(nv);
   int32_t *deg = nullptr, *degp = nullptr;
-  // [0] max deg, [1] max out, [2] ne_dag, [3] long rows, [4] big vertices, [5..8] roots
+  // [0] max deg, [1] max out, [2] ne_dag, [3] long rows, [4] big vertices, [5..9] roots,
+  // [10] row store words
   unsigned long long* stats = nullptr;
   TRY(dalloc(&deg, nv, s));
   TRY(dalloc(&degp, nv, s));
-  TRY(dalloc(&stats, 9, s));
-  TRY(cudaMemsetAsync(stats, 0, 9 * sizeof(unsigned long long), s));
+  TRY(dalloc(&stats, 11, s));
+  TRY(cudaMemsetAsync(stats, 0, 11 * sizeof(unsigned long long), s));
   if (nv > 0) {
     k_degrees<<<grid_for(nv), kThreads, 0, s>>>(g.rowptr_o, nv, deg, stats);
     TRY(cudaGetLastError());
   }
-  unsigned long long h[9] = {};
+  unsigned long long h[11] = {};
   TRY(cudaMemcpyAsync(h, stats, sizeof(h), cudaMemcpyDeviceToHost, s));
   TRY(cudaStreamSynchronize(s));
   g.max_deg = (int64_t)h[0];
@@ -484,7 +490,8 @@ cudaError_t finish_graph(DevGraph& g, const int32_t* group, int num_groups, cuda
   g.max_out = (int64_t)h[1];
   g.ne_dag = (int64_t)h[2];
   g.n_big = group ? 0 : (int64_t)h[4];
-  for (int i = 0; i < 4; ++i) g.n_roots[i] = (int64_t)h[5 + i];
+  for (int i = 0; i < 5; ++i) g.n_roots[i] = (int64_t)h[5 + i];
+  g.row_store_words = (int64_t)h[10];
   cudaFreeAsync(keys, s);
   cudaFreeAsync(tmp, s);
   cudaFreeAsync(deg, s);

@@ -17,7 +17,7 @@ struct DevGraph {
   int64_t max_out = 0;     // max out-degree of the oriented DAG
   int64_t n_big = 0;       // vertices of degree > kBigDeg: the top ranks (rows.cuh; 0 for
                            // batched graphs, whose ranks are sorted by degree per graph)
-  int64_t n_roots[4] = {0, 0, 0, 0};  // vertices of out-degree >= 2, 3, 4, 5
+  int64_t n_roots[5] = {0, 0, 0, 0, 0};  // vertices of out-degree >= 2 .. 6
   int64_t* rowptr_o = nullptr;
   int32_t* col_o = nullptr;
   int32_t* rank = nullptr;   // [nv] original -> rank
@@ -36,6 +36,14 @@ struct DevGraph {
   mutable uint32_t* lut_rows = nullptr;
   mutable int64_t* lut_off = nullptr;
   mutable int lut_state = 0;
+  // row store offsets, row tasks by width and their numbers (rows.cu), built on first use
+  // by a clique count: rn = {words, tasks of <= 32 members, of <= kRowsMid, of more};
+  // rtask holds the first list from its start, the second from nv on, the third from its
+  // end down
+  int64_t row_store_words = 0;
+  mutable int64_t* roff = nullptr;
+  mutable int32_t* rtask = nullptr;
+  mutable unsigned long long* rn = nullptr;
   // out-neighbour degree sums / maxima (the learned schedule's task features), built on
   // first use by the learned schedule
   mutable int64_t* tsum = nullptr;

@@ -1,7 +1,9 @@
-// Triangles from the side of the later endpoint ("owner"), hand-written for sm_103a.
+// Triangles and k-cliques from the side of the later endpoint ("owner"), hand-written for
+// sm_103a.
 //
-// Reference kernel this replaces: warp_edge (TC),
-// codes/GraphMiner/src/triangle/gpu_kernels/bs_warp_edge.cuh:1-20.
+// Reference kernels this replaces (same counts, different schedule):
+//  - warp_edge (TC): codes/GraphMiner/src/triangle/gpu_kernels/bs_warp_edge.cuh:1-20
+//  - clique4_warp_edge / clique5_warp_edge and their LUT forms: as in clique.cu
 //
 // Every triangle v < u < x of the degree-oriented DAG is found at its edge (v, u): x lies
 // in N+(u) and in the part of N+(v) after u (its suffix).  Testing suffixes costs
@@ -12,17 +14,31 @@
 //  - big u (degree > kBigDeg): a CTA holds N+(u) as a bitmap over [u + 1, V) and takes up
 //    to kOwnChunk in-neighbours v of u.  A thread finds u's place in N+(v) by binary
 //    search (N+(v) is sorted); suffixes of up to kOwnShort elements are tested by that
-//    thread, longer ones go to a table in shared memory and are tested by whole warps,
-//    32 consecutive elements at a time.  A hub's in-neighbours are many units (u, chunk)
-//    that any CTA can take.
+//    thread, longer ones go to a table in shared memory, longest first, and are tested by
+//    eight lanes each, a 16-byte unit per lane and step.  A hub's in-neighbours are many
+//    units (u, chunk) that any CTA can take.
 //  - the other u: one lane per edge (v, u) merges the suffix with N+(u); both are short
 //    (deg v <= deg u <= kBigDeg).
-// Measured (GB300): triangles of R-MAT scale 20, ef 16: 8.45 -> 2.05 ms a call; of a
-// Barabasi-Albert graph of 3,312 vertices 115 -> 41 us (13 launches -> 1: no task lists).
-// Bound: instruction issue (74 % active, 27 of 32 threads per instruction, L2 hit 95 %).
 // Bitmaps are cleared by taking the inserted bits out again: a unit costs d+(u) stores,
 // not the bitmap's size.
+//
+// The tests of one pair (v, u), in order, are row i of v's local DAG (u = N+(v)[i]): bit j
+// iff N+(v)[j] is in N+(u).  The rows mode writes them to the row store, whole words from
+// one place, no atomics; the count kernels then read a vertex's rows as one contiguous
+// matrix (k = 4 .. 7).
+//
+// Measured (GB300, a call before -> now):
+//  triangles  R-MAT s20 ef16 8.45 -> 1.48 ms; Barabasi-Albert, 3,312 vertices, 106 -> 28 us
+//             (13 launches -> 1: no task lists)
+//  4-cliques  R-MAT s22 65.6 -> 23.0 ms (rows 12.3, counting 10.9); s20 12.4 -> 3.6 ms
+//  5-cliques  R-MAT s20 140 -> 33.5 ms; 6-cliques R-MAT s16 96 -> 18.5 ms
+// The tests with a warp per suffix, a ballot per 32 elements: 1.86 ms (s20 triangles), 15.2
+// ms (s22 rows): 145 instructions a pair, of which a third for the pair itself.
+// Bound: R-MAT s22 rows, L2 and DRAM latency (2.2 G sectors, 12 GB of DRAM reads: the lists
+// exceed L2) and instruction issue; counting, the ALU pipe (half rate: shifts, ANDs).
 #include <algorithm>
+#include <atomic>
+#include <type_traits>
 
 #include "rows.cuh"
 
@@ -35,19 +51,62 @@ constexpr int kOwnWarps = kOwnThreads / 32;
 constexpr int kOwnChunk = 512;   // in-neighbours of one unit (two per thread)
 constexpr int kOwnShort = 12;    // longest suffix one thread tests by itself
 constexpr int kOwnLevels = 512;  // most units of one owner (host: raises the chunk above it)
-constexpr int kSmallStep = 128;  // vertices per claim of the small phase
+constexpr int kSmallStep = 128;  // most vertices per claim of the small phase
 
 struct OwnArgs {
   GView g;
   int64_t big0;    // first big rank
   int64_t chunk;   // in-neighbours per unit: a multiple of kOwnChunk
   int levels;      // units of the vertex of the largest degree
-  int words;       // bitmap words
+  int wmask;       // bitmap words - 1 (a power of two of them)
+  int step;        // vertices per claim of the small phase
+  const int64_t* roff = nullptr;  // rows mode: row store offset per vertex (-1: no rows)
+  uint32_t* rows = nullptr;       // rows mode: the row store
 };
 
+enum { kOwnCount = 0, kOwnRows = 1 };
+
+// A suffix that eight lanes test: col[p .. p + len).  Rows mode: element e is bit
+// i + 1 + e of row i of v's local DAG, whose word i / 32 is rows[out].
+template <int MODE>
 struct OwnPair {
-  long long p;  // first element of the suffix
-  int len;      // its length
+  long long p;
+  int len;
+};
+template <>
+struct OwnPair<kOwnRows> {
+  long long p, out;
+  int len, i;
+};
+
+// 32-bit mask of the bits below r (r <= 0: none, r >= 32: all).
+__device__ __forceinline__ uint32_t mask_below(int r) {
+  uint32_t m;
+  asm("shl.b32 %0, %1, %2;" : "=r"(m) : "r"(0xFFFFFFFFu), "r"(r > 0 ? r : 0));  // clamps at 32
+  return ~m;
+}
+
+// Row i of an s-vertex local DAG, built one word after the other by one thread.
+struct RowWriter {
+  uint32_t* out;  // word i / 32 of the row
+  uint32_t bits = 0;
+  int w;
+  __device__ RowWriter(uint32_t* o, int i) : out(o), w(i >> 5) {}
+  __device__ void upto(int q) {
+    while (w < q) {
+      *out++ = bits;
+      bits = 0;
+      ++w;
+    }
+  }
+  __device__ void put(int j, uint32_t bit) {
+    upto(j >> 5);
+    bits |= bit << (j & 31);
+  }
+  __device__ void finish(int s) {
+    upto((s - 1) >> 5);
+    *out = bits;
+  }
 };
 
 // Elements two sorted ranges of col have in common.
@@ -67,6 +126,23 @@ __device__ __forceinline__ unsigned merge_count(const int32_t* col, long long a,
   }
 }
 
+// The same merge, a hit of the element a0 + k of the first range setting bit j0 + k.
+__device__ __forceinline__ void merge_row(const int32_t* col, long long a, long long ea,
+                                          long long b, long long eb, int j, RowWriter& row) {
+  if (a >= ea || b >= eb) return;
+  int32_t x = ldg_i32(col + a), y = ldg_i32(col + b);
+  for (;;) {
+    const bool le = x <= y, ge = x >= y;
+    if (le && ge) row.put(j, 1u);
+    a += le;
+    j += le;
+    b += ge;
+    if (a >= ea || b >= eb) return;
+    if (le) x = ldg_i32(col + a);
+    if (ge) y = ldg_i32(col + b);
+  }
+}
+
 __device__ __forceinline__ long long lower_at(const int32_t* col, long long lo, long long hi,
                                               int32_t x) {
   while (lo < hi) {
@@ -76,19 +152,21 @@ __device__ __forceinline__ long long lower_at(const int32_t* col, long long lo, 
   return lo;
 }
 
-__global__ void __launch_bounds__(kOwnThreads) k_owner_count(OwnArgs a, OwnHeads* heads,
-                                                             unsigned long long* count) {
+template <int MODE>
+__global__ void __launch_bounds__(kOwnThreads, 5) k_owner(OwnArgs a, OwnHeads* heads,
+                                                       unsigned long long* count) {
+  constexpr bool ROWS = MODE == kOwnRows;
   extern __shared__ uint32_t bm[];
-  __shared__ OwnPair tab[kOwnChunk];
+  __shared__ OwnPair<MODE> tab[kOwnChunk];
   __shared__ int lev[kOwnLevels + 1];  // lev[l]: units of levels above l (highest first)
-  __shared__ int n_long, claim;
+  __shared__ int hist[32];  // long suffixes of the chunk by length
   __shared__ long long unit_s;
   const GView& g = a.g;
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   unsigned long long acc = 0;
 
   if (a.big0 < g.nv) {
-    for (int w = tid; w < a.words; w += kOwnThreads) bm[w] = 0u;
+    for (int w = tid; w <= a.wmask; w += kOwnThreads) bm[w] = 0u;
     // Units: level l holds the chunk l of every big vertex of degree > l * chunk, a prefix
     // of the descending degree order.  Levels are taken from the highest down, so the
     // last units are the small ones.
@@ -100,7 +178,8 @@ __global__ void __launch_bounds__(kOwnThreads) k_owner_count(OwnArgs a, OwnHeads
       }
       lev[l] = (int)(g.nv - lo);
     }
-    if (tid == 0) n_long = 0, claim = 0, unit_s = (long long)atomicAdd(&heads->big, 1ull);
+    if (tid < 32) hist[tid] = 0;
+    if (tid == 0) unit_s = (long long)atomicAdd(&heads->big, 1ull);
     __syncthreads();
     if (warp == 0) {  // suffix sums over the levels
       int run = 0;
@@ -135,7 +214,8 @@ __global__ void __launch_bounds__(kOwnThreads) k_owner_count(OwnArgs a, OwnHeads
       const longlong2 du = ldg_ll2(g.dptr + u);
       const long long c0 = g.rowptr[u] + (long long)l * a.chunk;
       const long long c1 = c0 + a.chunk < du.x ? c0 + a.chunk : du.x;
-      const bool live = du.x < du.y && c0 < c1;  // uniform
+      // (rows mode: an owner without out-neighbours still writes its empty rows)
+      const bool live = (ROWS || du.x < du.y) && c0 < c1;  // uniform
       if (!live) __syncthreads();  // every thread has read unit_s
       for (long long cc = c0; live && cc < c1; cc += kOwnChunk) {
         // insert N+(u) (first pass) while the in-neighbours look u up in their lists
@@ -144,59 +224,125 @@ __global__ void __launch_bounds__(kOwnThreads) k_owner_count(OwnArgs a, OwnHeads
             const uint32_t off = (uint32_t)(ldg_i32(g.col + e) - (int32_t)u - 1);
             atomicOr(&bm[off >> 5], 1u << (off & 31));
           }
-        long long p[2];
-        int len[2];
+        long long p[2], row[2];  // list of v, row of the row store
+        int ii[2], ss[2];        // u's place in it, its length
+        int bin[2], slot[2];     // long suffixes: by length in words, longest first
 #pragma unroll
         for (int h = 0; h < 2; ++h) {
           const long long e = cc + h * kOwnThreads + tid;
-          len[h] = 0;
+          ii[h] = ss[h] = 0;
+          bin[h] = -1;
           if (e < c1) {
-            const longlong2 dv = ldg_ll2(g.dptr + ldg_i32(g.col + e));
-            const long long at = lower_at(g.col, dv.x, dv.y, (int32_t)u);
-            p[h] = at + 1;
-            len[h] = (int)(dv.y - at - 1);
-            if (len[h] > kOwnShort) {
-              const int k = atomicAdd(&n_long, 1);
-              tab[k].p = p[h];
-              tab[k].len = len[h];
-            }
-          }
-        }
-        __syncthreads();
-        unsigned part = 0;
-        const int32_t base = (int32_t)u + 1;
-#pragma unroll
-        for (int h = 0; h < 2; ++h)
-          if (len[h] <= kOwnShort)
-            for (int k = 0; k < len[h]; ++k) {
-              const uint32_t off = (uint32_t)(ldg_i32(g.col + p[h] + k) - base);
-              part += (bm[off >> 5] >> (off & 31)) & 1u;
-            }
-        const int nl = n_long;
-        for (;;) {
-          int k = 0;
-          if (lane == 0) k = atomicAdd(&claim, 2);
-          k = __shfl_sync(kFull, k, 0);
-          if (k >= nl) break;
-#pragma unroll 1
-          for (int k2 = k; k2 < k + 2 && k2 < nl; ++k2) {
-            const int32_t* q = g.col + tab[k2].p;
-            const int n = tab[k2].len;
-            for (int e = lane; e < n; e += 128) {  // four independent loads per pass
-              int32_t x[4];
-#pragma unroll
-              for (int h = 0; h < 4; ++h) x[h] = e + 32 * h < n ? ldg_i32(q + e + 32 * h) : -1;
-#pragma unroll
-              for (int h = 0; h < 4; ++h) {
-                const uint32_t off = (uint32_t)(x[h] - base);
-                if (x[h] >= 0) part += (bm[off >> 5] >> (off & 31)) & 1u;
+            const int32_t v = ldg_i32(g.col + e);
+            const long long ro = ROWS ? __ldg(a.roff + v) : 0;
+            if (ro >= 0) {
+              const longlong2 dv = ldg_ll2(g.dptr + v);
+              p[h] = dv.x;
+              ss[h] = (int)(dv.y - dv.x);
+              ii[h] = (int)(lower_at(g.col, dv.x, dv.y, (int32_t)u) - dv.x);
+              if (ROWS) row[h] = ro + tri_row_off(ii[h], (ss[h] + 31) >> 5);
+              const int len = ss[h] - ii[h] - 1;
+              if (len > kOwnShort) {
+                bin[h] = 31 - (len < 32 * 31 ? len >> 5 : 31);
+                slot[h] = atomicAdd(&hist[bin[h]], 1);
               }
             }
           }
         }
+        __syncthreads();
+        int nl;
+        {  // start of each bin (every warp for itself), then the table
+          const int c = hist[lane];
+          int inc = c;
+#pragma unroll
+          for (int o = 1; o < 32; o <<= 1) {
+            const int y = __shfl_up_sync(kFull, inc, o);
+            if (lane >= o) inc += y;
+          }
+          nl = __shfl_sync(kFull, inc, 31);
+#pragma unroll
+          for (int h = 0; h < 2; ++h) {
+            const int b0 = __shfl_sync(kFull, inc - c, bin[h] & 31);
+            if (bin[h] >= 0) {
+              OwnPair<MODE>& x = tab[b0 + slot[h]];
+              x.p = p[h] + ii[h] + 1;
+              x.len = ss[h] - ii[h] - 1;
+              if constexpr (ROWS) {
+                x.out = row[h];
+                x.i = ii[h];
+              }
+            }
+          }
+        }
+        unsigned part = 0;
+        const int32_t base = (int32_t)u + 1;
+#pragma unroll
+        for (int h = 0; h < 2; ++h)
+          if (bin[h] < 0 && ss[h] > 0) {
+            RowWriter w(ROWS ? a.rows + row[h] : nullptr, ii[h]);
+            for (int j = ii[h] + 1; j < ss[h]; ++j) {
+              const uint32_t off = (uint32_t)(ldg_i32(g.col + p[h] + j) - base);
+              const uint32_t bit = (bm[off >> 5] >> (off & 31)) & 1u;
+              if (ROWS) w.put(j, bit); else part += bit;
+            }
+            if (ROWS) w.finish(ss[h]);
+          }
+        __syncthreads();
+        // Eight lanes per suffix, one 16-byte unit each, from the unit its first element is
+        // in: 32 elements of four suffixes per step.  An element before or after the suffix
+        // reads some word of the bitmap (the index wraps) and is masked by its place.
+        const int l8 = lane & 7;
+        for (int k0 = 4 * warp; k0 < nl; k0 += 4 * kOwnWarps) {
+          const int k = k0 + (lane >> 3);
+          OwnPair<MODE> t{};
+          if (k < nl) t = tab[k];
+          const int ph = (int)(t.p & 3);
+          const int rem = t.len > 0 ? t.len + ph : 0;  // elements from the first unit on
+          const int4* q = reinterpret_cast<const int4*>(g.col + (t.p - ph)) + l8;
+          // rows mode: step n gives row bits from b0 + 32 n on
+          int b0 = 0, steps = (rem + 31) >> 5, w0 = 0;
+          uint32_t prev = 0;
+          uint32_t* out = nullptr;
+          if constexpr (ROWS) {
+            b0 = t.i + 1 - ph;
+            w0 = (b0 >> 5) - (t.i >> 5);  // of the first step, from the row's first word
+            out = a.rows + t.out + w0;
+            if (rem) steps = ((b0 + rem - 1) >> 5) - (b0 >> 5) + 1;
+            if (l8 == 0 && w0 == 1) out[-1] = 0u;  // bits up to i: none
+          }
+          const int most = __reduce_max_sync(kFull, steps);
+          int4 x = make_int4(0, 0, 0, 0);
+          if (4 * l8 < rem) x = __ldg(q);
+          for (int n = 0; n < most; ++n) {
+            int4 y = make_int4(0, 0, 0, 0);
+            if (32 * (n + 1) + 4 * l8 < rem) y = __ldg(q + 8 * (n + 1));
+            const int32_t xs[4] = {x.x, x.y, x.z, x.w};
+            uint32_t bits = 0;  // the four tests, in the top bits
+#pragma unroll
+            for (int h = 0; h < 4; ++h) {
+              const uint32_t off = (uint32_t)(xs[h] - base);
+              bits = __funnelshift_r(bits, bm[(off >> 5) & a.wmask] >> (off & 31), 1);
+            }
+            if constexpr (ROWS) {
+              uint32_t word = bits >> (28 - 4 * l8);
+              word |= __shfl_xor_sync(kFull, word, 1);
+              word |= __shfl_xor_sync(kFull, word, 2);
+              word |= __shfl_xor_sync(kFull, word, 4);
+              word &= mask_below(rem - 32 * n);
+              if (n == 0) word &= 0xFFFFFFFFu << ph;
+              if (l8 == 0 && n < steps && w0 + n >= 0) out[n] = __funnelshift_l(prev, word, b0 & 31);
+              prev = word;
+            } else {
+              uint32_t m = mask_below(rem - 32 * n - 4 * l8);
+              if (n == 0 && l8 == 0) m &= 0xFFFFFFFFu << ph;
+              part += __popc((bits >> 28) & m);
+            }
+            x = y;
+          }
+        }
         acc += part;
         __syncthreads();
-        if (tid == 0) n_long = 0, claim = 0;
+        if (tid < 32) hist[tid] = 0;
         if (cc + kOwnChunk < c1) __syncthreads();
       }
       if (tid == 0) unit_s = (long long)atomicAdd(&heads->big, 1ull);
@@ -211,16 +357,21 @@ __global__ void __launch_bounds__(kOwnThreads) k_owner_count(OwnArgs a, OwnHeads
   const long long nsm = a.big0;
   for (;;) {
     long long vb = 0;
-    if (lane == 0) vb = (long long)atomicAdd(&heads->small, (unsigned long long)kSmallStep);
+    if (lane == 0) vb = (long long)atomicAdd(&heads->small, (unsigned long long)a.step);
     vb = __shfl_sync(kFull, vb, 0);
     if (vb >= nsm) break;
-    const long long ve = vb + kSmallStep < nsm ? vb + kSmallStep : nsm;
+    const long long ve = vb + a.step < nsm ? vb + a.step : nsm;
     for (long long b = vb; b < ve; b += 32) {
       longlong2 d = make_longlong2(0, 0);
+      long long ro = 0;
       int cnt = 0;
       if (b + lane < ve) {
-        d = ldg_ll2(g.dptr + (nsm - 1 - (b + lane)));  // longest lists first
-        cnt = (int)(d.y - d.x) - 1;
+        const long long v = nsm - 1 - (b + lane);  // longest lists first
+        if (ROWS) ro = __ldg(a.roff + v);
+        if (ro >= 0) {
+          d = ldg_ll2(g.dptr + v);
+          cnt = (int)(d.y - d.x) - (ROWS ? 0 : 1);  // the last row is empty
+        }
         if (cnt > 0 && ldg_i32(g.col + d.x + cnt - 1) >= a.big0)
           cnt = (int)(lower_at(g.col, d.x, d.x + cnt, (int32_t)a.big0) - d.x);
         if (cnt < 0) cnt = 0;
@@ -243,42 +394,745 @@ __global__ void __launch_bounds__(kOwnThreads) k_owner_count(OwnArgs a, OwnHeads
         q &= 31;  // k >= total runs past the last lane
         const long long base = __shfl_sync(kFull, d.x, q), end = __shfl_sync(kFull, d.y, q);
         const int ex = __shfl_sync(kFull, inc - cnt, q);
+        const long long qro = ROWS ? __shfl_sync(kFull, ro, q) : 0;
         if (k < total) {
-          const long long at = base + (k - ex);
+          const int i = k - ex;
+          const long long at = base + i;
           const longlong2 du = ldg_ll2(g.dptr + ldg_i32(g.col + at));
-          acc += merge_count(g.col, at + 1, end, du.x, du.y);
+          if constexpr (ROWS) {
+            const int s = (int)(end - base);
+            RowWriter w(a.rows + qro + tri_row_off(i, (s + 31) >> 5), i);
+            merge_row(g.col, at + 1, end, du.x, du.y, i + 1, w);
+            w.finish(s);
+          } else {
+            acc += merge_count(g.col, at + 1, end, du.x, du.y);
+          }
         }
       }
     }
   }
-  acc = warp_sum_u64(acc);
-  if (lane == 0 && acc) atomicAdd(count, acc);
+  if constexpr (!ROWS) {
+    acc = warp_sum_u64(acc);
+    if (lane == 0 && acc) atomicAdd(count, acc);
+  }
 }
 
-}  // namespace
-
-cudaError_t launch_owner_count(const DevGraph& g, OwnHeads* heads, unsigned long long* count,
-                               int num_sms, cudaStream_t s) {
+template <int MODE>
+cudaError_t launch_owner(const DevGraph& g, OwnArgs a, OwnHeads* heads, unsigned long long* count,
+                         int num_sms, cudaStream_t s) {
   if (g.nv == 0) return cudaSuccess;
-  OwnArgs a;
   a.g = g.view();
   const int64_t nbig = std::min<int64_t>(g.n_big, kOwnBits);
   a.big0 = g.nv - nbig;
   const int64_t per = (g.max_deg + kOwnLevels - 1) / kOwnLevels;
   a.chunk = std::max<int64_t>(kOwnChunk, (per + kOwnChunk - 1) / kOwnChunk * kOwnChunk);
   a.levels = (int)std::max<int64_t>(1, (g.max_deg + a.chunk - 1) / a.chunk);
-  a.words = (int)((nbig + 31) / 32);
-  const int smem = 4 * std::max(a.words, 1);
+  int words = 32;
+  while (32 * (int64_t)words < nbig) words *= 2;
+  a.wmask = words - 1;
+  const int smem = 4 * words;
   int per_sm = 0;
   cudaError_t e =
-      cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_owner_count, kOwnThreads, smem);
+      cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_owner<MODE>, kOwnThreads, smem);
   if (e != cudaSuccess) return e;
-  // no more CTAs than there is work for: small graphs would only pay for starting them
-  const int64_t want = std::max<int64_t>(nbig, (g.nv + kSmallStep * kOwnWarps - 1) /
-                                                   (kSmallStep * kOwnWarps));
+  // no more CTAs than there is work for (small graphs would only pay for starting them),
+  // and claims small enough that every warp has a few
+  const int64_t want = std::max<int64_t>(nbig, (a.big0 + 4 * kOwnWarps - 1) / (4 * kOwnWarps));
   const int64_t grid = std::max<int64_t>(1, std::min<int64_t>((int64_t)per_sm * num_sms, want));
-  k_owner_count<<<(unsigned)grid, kOwnThreads, smem, s>>>(a, heads, count);
+  a.step = (int)std::max<int64_t>(4, std::min<int64_t>(kSmallStep, a.big0 / (4 * kOwnWarps * grid)));
+  k_owner<MODE><<<(unsigned)grid, kOwnThreads, smem, s>>>(a, heads, count);
   return cudaGetLastError();
+}
+
+// ------------------------------------------------------------------ row index
+// Offsets of the row store and the row tasks of a graph, by the width of their rows.
+__global__ void __launch_bounds__(256) k_rows_index(const longlong2* dptr, int64_t nv,
+                                                    int64_t* roff, int32_t* word_l,
+                                                    int32_t* team_l, unsigned long long* rn) {
+  __shared__ unsigned wsum[8], lcnt[3];
+  __shared__ unsigned long long wbase, lbase[3];
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  for (int64_t b = (int64_t)blockIdx.x * 256; b < nv; b += (int64_t)gridDim.x * 256) {
+    const int64_t v = b + tid;
+    int s = 0;
+    if (v < nv) {
+      const longlong2 d = ldg_ll2(dptr + v);
+      s = d.y - d.x <= kRowsCap ? (int)(d.y - d.x) : 0;
+    }
+    const unsigned words = row_words(s);
+    const int cls = words == 0 ? 3 : (s <= 32 ? 0 : (s <= kRowsMid ? 1 : 2));
+    if (tid < 3) lcnt[tid] = 0;
+    unsigned inc = words;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const unsigned y = __shfl_up_sync(kFull, inc, o);
+      if (lane >= o) inc += y;
+    }
+    if (lane == 31) wsum[warp] = inc;
+    __syncthreads();
+    unsigned slot = 0;
+    if (cls < 3) slot = atomicAdd(&lcnt[cls], 1u);
+    unsigned off = inc - words, tot = 0;
+    for (int w = 0; w < 8; ++w) {
+      if (w < warp) off += wsum[w];
+      tot += wsum[w];
+    }
+    __syncthreads();
+    if (tid == 0) wbase = atomicAdd(&rn[0], (unsigned long long)tot);
+    if (tid < 3) lbase[tid] = atomicAdd(&rn[1 + tid], (unsigned long long)lcnt[tid]);
+    __syncthreads();
+    if (v < nv) {
+      roff[v] = words ? (int64_t)(wbase + off) : -1;
+      if (cls == 0) word_l[lbase[0] + slot] = (int32_t)v;
+      else if (cls == 1) team_l[lbase[1] + slot] = (int32_t)v;
+      else if (cls == 2) team_l[nv - 1 - (int64_t)(lbase[2] + slot)] = (int32_t)v;
+    }
+    __syncthreads();
+  }
+}
+
+// ------------------------------------------------------------------ counting
+// A task's rows are the strict upper triangle of a 0/1 matrix A (row i: words i/32 .. W-1).
+// Its triangles are the sum over edges (j, l) of (A A^T)_jl, a contraction: 32 x 32 blocks
+// of A A^T on the tensor cores, fp8 (e4m3) operands and fp32 accumulators, masked by the
+// block of A itself.  An operand element is 2^-6 or 0, so a sum of n products is n 2^-12,
+// exact (n <= 1024).  The fragments come straight from the bit rows: the k index of an
+// m16n8k32 step may be permuted if both operands agree, and with thread t of a quad taking
+// bits 8 b + t and 8 b + t + 4 (b = 0..3) of a row's word, a fragment register is one shift
+// and one AND.
+// popc over row words issues 4.3 words per clock and SM partition (measured; FLO for the
+// walk over members costs as much), the e4m3 step 824 multiply-adds = 26 words' worth; the
+// 1-bit mma.sync is emulated on this chip (525 cycles a step against 5).  A tcgen05 tile
+// has 128 rows: most matrices here are 60 to 300 wide and triangular, so its doubled rate
+// would go into padding.
+__device__ __forceinline__ void mma_e4m3(float (&d)[4], uint32_t a0, uint32_t a1, uint32_t a2,
+                                         uint32_t a3, uint32_t b0, uint32_t b1) {
+  asm("mma.sync.aligned.m16n8k32.row.col.f32.e4m3.e4m3.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, "
+      "{%8,%9}, {%0,%1,%2,%3};"
+      : "+f"(d[0]), "+f"(d[1]), "+f"(d[2]), "+f"(d[3])
+      : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
+}
+constexpr float kUnit = 4096.0f;  // 1 / (2^-6)^2
+
+// First word of block q's rows; a row of the block spans W - q words.
+__device__ __forceinline__ int blk_off(int q, int W) { return 16 * q * (2 * W - q + 1); }
+
+// Fragment registers of the words w[r] of rows 8 r + lane / 4.
+__device__ __forceinline__ void frag(const uint32_t (&w)[4], int t, uint32_t (&lo)[4],
+                                     uint32_t (&hi)[4]) {
+#pragma unroll
+  for (int r = 0; r < 4; ++r) {
+    lo[r] = (w[r] << (3 - t)) & 0x08080808u;
+    hi[r] = (w[r] >> (t + 1)) & 0x08080808u;
+  }
+}
+
+// One step (32 k) of a 32 x 32 block, or of its first 16 MT rows and 8 NT columns.
+template <int MT, int NT>
+__device__ __forceinline__ void block_mma(float (&c)[2][4][4], const uint32_t (&al)[4],
+                                          const uint32_t (&ah)[4], const uint32_t (&bl)[4],
+                                          const uint32_t (&bh)[4]) {
+#pragma unroll
+  for (int m = 0; m < MT; ++m)
+#pragma unroll
+    for (int n = 0; n < NT; ++n)
+      mma_e4m3(c[m][n], al[2 * m], al[2 * m + 1], ah[2 * m], ah[2 * m + 1], bl[n], bh[n]);
+}
+
+// Sum of c over the set bits of the block of A (mk[r]: its row 8 r + lane / 4).
+template <int MT, int NT>
+__device__ __forceinline__ uint32_t block_sum(const float (&c)[2][4][4], const uint32_t (&mk)[4],
+                                              int t) {
+  float sum = 0.0f;
+#pragma unroll
+  for (int m = 0; m < MT; ++m) {
+    const uint32_t w0 = mk[2 * m] >> (2 * t), w1 = mk[2 * m + 1] >> (2 * t);
+#pragma unroll
+    for (int n = 0; n < NT; ++n)
+#pragma unroll
+      for (int e = 0; e < 2; ++e) {
+        if (w0 & (1u << (8 * n + e))) sum += c[m][n][e];
+        if (w1 & (1u << (8 * n + e))) sum += c[m][n][2 + e];
+      }
+  }
+  return (uint32_t)(sum * kUnit);  // <= 32 x 1024 per thread: exact
+}
+
+// Edges (j, l), j in block J, l in block L >= J: the sum of |R_j & R_l|, and with MASK (m: a
+// row's words, read from J on) of |R_j & R_l & m| over j, l in m.  This lane's part.  (Two
+// blocks of j sharing the fragments of l take 3 instead of 4 shifts and ANDs per step of the
+// tensor cores, but 168 registers instead of 128: a CTA fewer per SM, and no gain.)
+template <bool MASK>
+__device__ __forceinline__ uint32_t tri_block(const uint32_t* M, int W, int J, int L,
+                                              const uint32_t* m) {
+  const int lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
+  const int sa = W - J, sb = W - L;
+  const uint32_t* A = M + blk_off(J, W) - J + g * sa;
+  const uint32_t* B = M + blk_off(L, W) - L + g * sb;
+  uint32_t mk[4];
+#pragma unroll
+  for (int r = 0; r < 4; ++r) {
+    mk[r] = A[8 * r * sa + L];
+    if (MASK) mk[r] = (m[J] >> (8 * r + g)) & 1u ? mk[r] & m[L] : 0u;
+  }
+  if (!__any_sync(kFull, (mk[0] | mk[1] | mk[2] | mk[3]) != 0u)) return 0u;
+  float c[2][4][4] = {};
+  for (int w = L; w < W; ++w) {
+    uint32_t a[4], b[4], al[4], ah[4], bl[4], bh[4];
+#pragma unroll
+    for (int r = 0; r < 4; ++r) {
+      a[r] = A[8 * r * sa + w];
+      if (MASK) a[r] &= m[w];
+      b[r] = B[8 * r * sb + w];
+    }
+    frag(a, t, al, ah);
+    frag(b, t, bl, bh);
+    block_mma<2, 4>(c, al, ah, bl, bh);
+  }
+  return block_sum<2, 4>(c, mk, t);
+}
+
+// Blocks of a matrix from block q on, dealt to nw warps (this one is wi), longest sums first.
+template <bool MASK>
+__device__ uint64_t tri_blocks(const uint32_t* M, int W, int q, const uint32_t* m, int wi, int nw) {
+  uint64_t acc = 0;
+  int L = 0, J = wi;  // block (q + J, q + L), J <= L, in the order L, J
+  for (;;) {
+    while (J > L) J -= ++L;
+    if (q + L >= W) return acc;
+    acc += tri_block<MASK>(M, W, q + J, q + L, m);
+    J += nw;
+  }
+}
+
+// Triangles of a matrix of at most 32 vertices, row i in lane i: the operands by shuffle.
+__device__ __forceinline__ uint32_t tri_word(uint32_t row, int n) {
+  const int lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
+  uint32_t a[4], al[4], ah[4];
+#pragma unroll
+  for (int r = 0; r < 4; ++r) a[r] = __shfl_sync(kFull, row, 8 * r + g);
+  frag(a, t, al, ah);
+  float c[2][4][4] = {};
+  if (n <= 16) {
+    block_mma<1, 2>(c, al, ah, al, ah);
+    return block_sum<1, 2>(c, a, t);
+  }
+  block_mma<2, 4>(c, al, ah, al, ah);
+  return block_sum<2, 4>(c, a, t);
+}
+
+// The matrix induced on a set of n <= 32 vertices (lane w holds word w of the set), row r in
+// lane r: lane b holds member b and one ballot gives a row.  ids: 32 entries of this warp.
+__device__ uint32_t small_matrix(const uint32_t* M, int W, uint32_t word, int n, uint16_t* ids) {
+  const int lane = threadIdx.x & 31;
+  const int cnt = __popc(word);
+  int inc = cnt;
+#pragma unroll
+  for (int o = 1; o < 32; o <<= 1) {
+    const int y = __shfl_up_sync(kFull, inc, o);
+    if (lane >= o) inc += y;
+  }
+  for (unsigned nz = __ballot_sync(kFull, word != 0u); nz; nz &= nz - 1) {
+    const int w = __ffs(nz) - 1;
+    const uint32_t x = __shfl_sync(kFull, word, w);
+    const int e = __shfl_sync(kFull, inc - cnt, w);
+    if ((x >> lane) & 1u) ids[e + __popc(x & lanemask_lt())] = (uint16_t)(32 * w + lane);
+  }
+  __syncwarp();
+  const int id = lane < n ? (int)ids[lane] : 0;
+  const uint32_t bit = lane < n ? 1u << (id & 31) : 0u;
+  const int base = tri_row_off(id, W) - (id >> 5);
+  const uint32_t* Mw = M + (id >> 5);
+  uint32_t mine = 0;
+  for (int r = 0; r < n; ++r) {
+    // a word below the row's own block belongs to an earlier row: masked out below
+    const uint32_t y = __ballot_sync(kFull, (Mw[__shfl_sync(kFull, base, r)] & bit) != 0u);
+    if (lane == r) mine = y;
+  }
+  __syncwarp();
+  return mine & (0xFFFFFFFEu << lane);  // members after r
+}
+
+// How the members of a row (R_i) are taken out of another row's words: per word of R_i, the
+// word, the five move masks of a bit compress (Hacker's Delight, 7-4: each step moves the
+// bits of its mask down by 1, 2, 4, 8, 16), and the number of members before it and in it.
+struct PickWord {
+  uint32_t m, mv[5];
+  int pos, cnt;
+};
+static_assert(sizeof(PickWord) == 32, "read as two uint4");
+
+// Prepares the members of row i: the picks (one warp of the team) and the ids (idx, by nw
+// warps).  Returns |R_i|.
+__device__ int row_members(const uint32_t* M, int W, int i, uint16_t* idx, PickWord* pick, int wi,
+                           int nw) {
+  const int lane = threadIdx.x & 31, q = i >> 5;
+  const uint32_t word = lane >= q && lane < W ? M[tri_row_off(i, W) + lane - q] : 0u;
+  const int cnt = __popc(word);
+  int inc = cnt;
+#pragma unroll
+  for (int o = 1; o < 32; o <<= 1) {
+    const int y = __shfl_up_sync(kFull, inc, o);
+    if (lane >= o) inc += y;
+  }
+  if (wi == 0 && lane < W) {
+    PickWord p;
+    p.m = word;
+    p.pos = inc - cnt;
+    p.cnt = cnt;
+    uint32_t mk = ~word << 1, m = word;
+#pragma unroll
+    for (int k = 0; k < 5; ++k) {
+      uint32_t mp = mk ^ (mk << 1);
+      mp ^= mp << 2;
+      mp ^= mp << 4;
+      mp ^= mp << 8;
+      mp ^= mp << 16;
+      p.mv[k] = mp & m;
+      m = (m ^ p.mv[k]) | (p.mv[k] >> (1 << k));
+      mk &= ~mp;
+    }
+    pick[lane] = p;
+  }
+  for (int w = q + wi; w < W; w += nw) {
+    const uint32_t x = __shfl_sync(kFull, word, w);
+    const int e = __shfl_sync(kFull, inc - cnt, w);
+    if ((x >> lane) & 1u) idx[e + __popc(x & lanemask_lt())] = (uint16_t)(32 * w + lane);
+  }
+  return __shfl_sync(kFull, inc, 31);
+}
+
+// The matrix induced on R_i, in the same triangular form (C, W2 = ceil(n / 32) words), by
+// nw warps: lane r of a warp takes row 32 J + r of it, compresses the words of that
+// member's row by the picks and appends the bits.  (One ballot per 32 members and row, the
+// lanes holding the members, cost 2.5 to 4 times as many instructions.)
+__device__ void compress(const uint32_t* M, int W, const uint16_t* idx, const PickWord* pick,
+                         int n, uint32_t* C, int wi, int nw) {
+  const int lane = threadIdx.x & 31, W2 = (n + 31) >> 5;
+  for (int J = wi; J < W2; J += nw) {
+    const bool live = 32 * J + lane < n;
+    const int id = live ? (int)idx[32 * J + lane] : 0;
+    const int q = live ? id >> 5 : 32;  // words of the row from q on (bits after id only)
+    const uint32_t* row = M + tri_row_off(id, W) - (id >> 5);
+    uint32_t* out = C + blk_off(J, W2) + lane * (W2 - J);  // words J .. W2 - 1 of the row
+    int w = (int)idx[32 * J] >> 5;  // the first word that holds a member of block J or later
+    uint32_t bits = 0;
+    int sh = pick[w].pos - 32 * J;  // < 0: members of earlier blocks, no bits of these rows
+    for (; w < W; ++w) {
+      const uint4 p0 = reinterpret_cast<const uint4*>(pick + w)[0];
+      const uint4 p1 = reinterpret_cast<const uint4*>(pick + w)[1];
+      if (p0.x == 0u) continue;
+      uint32_t x = w >= q ? row[w] & p0.x : 0u, t;
+      t = x & p0.y; x = (x ^ t) | (t >> 1);
+      t = x & p0.z; x = (x ^ t) | (t >> 2);
+      t = x & p0.w; x = (x ^ t) | (t >> 4);
+      t = x & p1.x; x = (x ^ t) | (t >> 8);
+      t = x & p1.y; x = (x ^ t) | (t >> 16);
+      const int cnt = (int)p1.w;
+      if (sh < 0) {  // first word: drop the bits before block J (all zero)
+        x >>= -sh;
+        sh += cnt;
+        bits = x;
+        continue;
+      }
+      bits |= x << sh;
+      sh += cnt;
+      if (sh >= 32) {
+        *out++ = bits;
+        sh -= 32;
+        bits = sh ? x >> (cnt - sh) : 0u;
+      }
+    }
+    if (sh > 0) *out = bits;
+  }
+}
+
+// Cliques of D vertices in the rows' subset m of a one-word matrix.
+template <int D>
+__device__ uint64_t word_cliques(const uint32_t* rows, uint32_t m) {
+  if constexpr (D == 1) {
+    return (uint64_t)__popc(m);
+  } else {
+    uint64_t acc = 0;
+    while (m) {
+      const int l = __ffs(m) - 1;
+      m &= m - 1;
+      acc += word_cliques<D - 1>(rows, m & rows[l]);
+    }
+    return acc;
+  }
+}
+
+// D-cliques (D = 3, 4, 5) among a set of n <= 32 vertices of a matrix, by one warp; tmp: 32
+// words, ids: 32 entries of this warp.
+template <int D>
+__device__ __forceinline__ uint64_t set_cliques(const uint32_t* M, int W, uint32_t word, int n,
+                                                uint16_t* ids, uint32_t* tmp) {
+  const uint32_t row = small_matrix(M, W, word, n, ids);
+  if constexpr (D == 3) {
+    return tri_word(row, n);
+  } else {
+    tmp[threadIdx.x & 31] = row;
+    __syncwarp();
+    const uint64_t r = word_cliques<D - 1>(tmp, row);
+    __syncwarp();
+    return r;
+  }
+}
+
+// D-cliques (D = 3, 4, 5) of the matrix C of n vertices, by nw warps; ids / tmp as above.
+// D = 4: for each row j the triangles inside it; D = 5: for each edge (j, l) the triangles
+// inside R_j & R_l; sets of up to 32 as a matrix of their own, longer ones as a mask.
+template <int D>
+__device__ uint64_t matrix_cliques(const uint32_t* C, int n, int wi, int nw, uint16_t* ids,
+                                   uint32_t* tmp) {
+  const int lane = threadIdx.x & 31, W = (n + 31) >> 5;
+  if constexpr (D == 3) {
+    return tri_blocks<false>(C, W, 0, nullptr, wi, nw);
+  } else {
+    uint64_t acc = 0;
+    for (int j = wi; j + D - 1 < n; j += nw) {
+      const int q = j >> 5;
+      const uint32_t* row = C + tri_row_off(j, W) - q;  // word w of row j (w >= q)
+      const uint32_t word = lane >= q && lane < W ? row[lane] : 0u;
+      const int nj = (int)__reduce_add_sync(kFull, (unsigned)__popc(word));
+      if (nj < D - 1) continue;
+      if (nj <= 32) {
+        acc += set_cliques<D - 1>(C, W, word, nj, ids, tmp);
+      } else if constexpr (D == 4) {
+        acc += tri_blocks<true>(C, W, q, row, 0, 1);
+      } else {
+        for (unsigned nz = __ballot_sync(kFull, word != 0u); nz; nz &= nz - 1) {
+          const int ql = __ffs(nz) - 1;
+          for (uint32_t bits = __shfl_sync(kFull, word, ql); bits; bits &= bits - 1) {
+            const int l = 32 * ql + __ffs(bits) - 1;
+            const uint32_t m2 =
+                lane >= ql && lane < W ? word & C[tri_row_off(l, W) - ql + lane] : 0u;
+            const int nl = (int)__reduce_add_sync(kFull, (unsigned)__popc(m2));
+            if (nl < 3) continue;
+            if (nl <= 32) {
+              acc += set_cliques<3>(C, W, m2, nl, ids, tmp);
+            } else {
+              __syncwarp();
+              tmp[lane] = m2;
+              __syncwarp();
+              acc += tri_blocks<true>(C, W, ql, tmp, 0, 1);
+            }
+          }
+        }
+      }
+    }
+    return acc;
+  }
+}
+
+struct RowTasks {
+  const longlong2* dptr;
+  const int64_t* roff;
+  const uint32_t* rows;
+  const int32_t* list;  // task t: list[t], or list[-t] when `down`
+  const unsigned long long* n;
+  int down;
+  int wcap;  // words of a row the CTA's shared memory is laid out for (word tasks: tasks
+             // per claim, at most 32)
+};
+
+constexpr int kOwnN = 128;                // longest row one warp takes by itself
+constexpr int kOwnWords = 16 * 4 * 5;     // its matrix
+constexpr int kTeam = 4;                  // warps of a team
+constexpr int kTeamN = 512;               // longest row a team takes
+// Scratch of a warp, in words: picks, matrix, 32 words of masks, ids, ids of a small set.
+constexpr int kWarpScratch = 8 * 32 + kOwnWords + 32 + kOwnN / 2 + 16;
+
+// Words of shared memory of a CTA of row tasks: the task's matrix; K >= 5: per team a
+// matrix and ids for rows up to kTeamN (together one for the longest row) and picks, the
+// list of rows too long for a warp, and each warp's scratch.
+__host__ __device__ constexpr int matrix_words(int W) { return 16 * W * (W + 1); }
+__host__ __device__ constexpr int team_matrix_words(int W) {
+  return matrix_words(W < kTeamN / 32 ? W : kTeamN / 32);
+}
+template <int K>
+constexpr int team_words(int W, int warps) {
+  return K == 4 ? matrix_words(W)
+                : matrix_words(W) + warps / kTeam * (team_matrix_words(W) + 8 * 32 + kTeamN / 2) +
+                      16 * W + warps * kWarpScratch;
+}
+
+__device__ __forceinline__ void team_sync(int team) {  // barrier 0 is __syncthreads
+  asm volatile("bar.sync %0, %1;" ::"r"(team + 1), "r"(32 * kTeam) : "memory");
+}
+
+// CTAs per SM the registers are cut for (K = 4: 8-warp CTAs, K >= 6 spills below 168).
+constexpr int team_ctas(int K, int NT) {
+  return NT == 128 ? (K >= 6 ? 3 : 4) : (K == 4 ? 2 : 1);
+}
+
+// Tasks of more than 32 out-neighbours, one CTA each: the (K - 1)-cliques of the task's
+// matrix.  K >= 5: the (K - 2)-cliques of the matrix induced on each row, a row of up to
+// kOwnN members by one warp, of up to kTeamN by a team of four, longer ones by the CTA.
+template <int K, int NT>
+__global__ void __launch_bounds__(NT, team_ctas(K, NT)) k_rows_team(RowTasks t, unsigned long long* head,
+                                                  unsigned long long* count) {
+  extern __shared__ __align__(16) uint32_t M[];
+  __shared__ long long task_s;
+  __shared__ int next_i, n_long, next_long, n_huge, team_x[NT / 32 / kTeam];
+  constexpr int kWarps = NT / 32, kTeams = kWarps / kTeam;
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const long long nt = (long long)*t.n;
+  uint64_t acc = 0;
+  if (tid == 0) task_s = (long long)atomicAdd(head, 1ull);
+  __syncthreads();
+  for (;;) {
+    const long long ti = task_s;
+    if (ti >= nt) break;
+    const int32_t v = t.down ? t.list[-ti] : t.list[ti];
+    const longlong2 d = ldg_ll2(t.dptr + v);
+    const int s = (int)(d.y - d.x), W = (s + 31) >> 5;
+    const int used = tri_words(s), all = matrix_words(W);  // the last block padded to 32 rows
+    const uint4* src = reinterpret_cast<const uint4*>(t.rows + t.roff[v]);
+    for (int x = tid; 4 * x < all; x += NT) {
+      uint4 y = make_uint4(0, 0, 0, 0);
+      if (4 * x < used) y = __ldcs(src + x);
+      if (4 * x + 1 >= used) y.y = 0;
+      if (4 * x + 2 >= used) y.z = 0;
+      if (4 * x + 3 >= used) y.w = 0;
+      reinterpret_cast<uint4*>(M)[x] = y;
+    }
+    if (tid == 0) next_i = 0, n_long = 0, next_long = 0, n_huge = 0;
+    __syncthreads();
+    if (tid == 0) task_s = (long long)atomicAdd(head, 1ull);
+    if constexpr (K == 4) {
+      acc += tri_blocks<false>(M, W, 0, nullptr, warp, kWarps);
+    } else {
+      const int tm = team_matrix_words(t.wcap), team = warp / kTeam, tw = warp % kTeam;
+      uint32_t* Cs = M + matrix_words(t.wcap);  // the teams' matrices, then their picks, ids
+      PickWord* picks = reinterpret_cast<PickWord*>(Cs + kTeams * tm);
+      uint16_t* idxs = reinterpret_cast<uint16_t*>(picks + kTeams * 32);
+      uint16_t* longs = idxs + kTeams * kTeamN;  // rows of <= kTeamN from the front, others
+      const int lcap = 32 * t.wcap;              // from the back
+      uint32_t* own = reinterpret_cast<uint32_t*>(longs + lcap) + warp * kWarpScratch;
+      PickWord* opick = reinterpret_cast<PickWord*>(own);
+      uint32_t* oC = own + 8 * 32;
+      uint32_t* otmp = oC + kOwnWords;
+      uint16_t* oidx = reinterpret_cast<uint16_t*>(otmp + 32);
+      uint16_t* oids = oidx + kOwnN;
+      for (;;) {
+        int i = 0;
+        if (lane == 0) i = atomicAdd(&next_i, 1);
+        i = __shfl_sync(kFull, i, 0);
+        if (i + K - 2 >= s) break;
+        const uint32_t word = lane >= (i >> 5) && lane < W
+                                  ? M[tri_row_off(i, W) + lane - (i >> 5)] : 0u;
+        const int n = (int)__reduce_add_sync(kFull, (unsigned)__popc(word));
+        if (n < K - 2) continue;
+        if (n <= 32) {
+          acc += set_cliques<K - 2>(M, W, word, n, oidx, otmp);
+          continue;
+        }
+        if (n > kOwnN) {
+          if (lane == 0) {
+            if (n <= kTeamN) longs[atomicAdd(&n_long, 1)] = (uint16_t)i;
+            else longs[lcap - 1 - atomicAdd(&n_huge, 1)] = (uint16_t)i;
+          }
+          continue;
+        }
+        row_members(M, W, i, oidx, opick, 0, 1);
+        __syncwarp();
+        compress(M, W, oidx, opick, n, oC, 0, 1);
+        __syncwarp();
+        acc += matrix_cliques<K - 2>(oC, n, 0, 1, oids, otmp);
+        __syncwarp();
+      }
+      __syncthreads();
+      for (;;) {
+        team_sync(team);  // the team is done with its last row
+        if (tw == 0 && lane == 0) team_x[team] = atomicAdd(&next_long, 1);
+        team_sync(team);
+        const int x = team_x[team];
+        if (x >= n_long) break;
+        uint32_t* C = Cs + team * tm;
+        const int n = row_members(M, W, longs[x], idxs + team * kTeamN, picks + 32 * team, tw, kTeam);
+        team_sync(team);
+        compress(M, W, idxs + team * kTeamN, picks + 32 * team, n, C, tw, kTeam);
+        team_sync(team);
+        acc += matrix_cliques<K - 2>(C, n, tw, kTeam, oids, otmp);
+      }
+      if constexpr (kTeams * team_matrix_words(32) >= matrix_words(32)) {
+        const int nh = n_huge;
+        if (nh) __syncthreads();  // every team is done
+        for (int x = 0; x < nh; ++x) {
+          const int n = row_members(M, W, longs[lcap - 1 - x], idxs, picks, warp, kWarps);
+          __syncthreads();
+          compress(M, W, idxs, picks, n, Cs, warp, kWarps);
+          __syncthreads();
+          acc += matrix_cliques<K - 2>(Cs, n, warp, kWarps, oids, otmp);
+          __syncthreads();
+        }
+      }
+    }
+    __syncthreads();
+  }
+  acc = warp_sum_u64(acc);
+  if (lane == 0 && acc) atomicAdd(count, (unsigned long long)acc);
+}
+
+// Tasks of up to 32 out-neighbours, a warp each, lane i holding row i.  K = 4: one block on
+// the tensor cores, its operands by shuffle.
+constexpr int kWordThreads = 256;
+template <int K>
+__global__ void __launch_bounds__(kWordThreads) k_rows_word(RowTasks t, unsigned long long* head,
+                                                            unsigned long long* count) {
+  __shared__ uint32_t rows_s[kWordThreads / 32][32];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const long long nt = (long long)*t.n;
+  uint64_t acc = 0;
+  for (;;) {
+    long long base = 0;
+    if (lane == 0) base = (long long)atomicAdd(head, (unsigned long long)t.wcap);
+    base = __shfl_sync(kFull, base, 0);
+    if (base >= nt) break;
+    const int n = nt - base < t.wcap ? (int)(nt - base) : t.wcap;
+    int s = 0;
+    long long off = 0;
+    if (lane < n) {
+      const int32_t v = t.list[base + lane];
+      const longlong2 d = ldg_ll2(t.dptr + v);
+      s = (int)(d.y - d.x);
+      off = t.roff[v];
+    }
+    int sx = __shfl_sync(kFull, s, 0);
+    long long ox = __shfl_sync(kFull, off, 0);
+    uint32_t next = lane < sx ? __ldcs(t.rows + ox + lane) : 0u;
+    for (int x = 0; x < n; ++x) {
+      const uint32_t r = next;
+      const int sc = sx;
+      if (x + 1 < n) {  // the next task's rows are in flight while this one is counted
+        sx = __shfl_sync(kFull, s, x + 1);
+        ox = __shfl_sync(kFull, off, x + 1);
+        next = lane < sx ? __ldcs(t.rows + ox + lane) : 0u;
+      }
+      if (sc < K - 1) continue;
+      if constexpr (K == 4) {
+        acc += tri_word(r, sc);
+      } else {
+        rows_s[warp][lane] = r;
+        __syncwarp();
+        acc += word_cliques<K - 2>(rows_s[warp], r);
+        __syncwarp();
+      }
+    }
+  }
+  acc = warp_sum_u64(acc);
+  if (lane == 0 && acc) atomicAdd(count, (unsigned long long)acc);
+}
+
+// Grid of a persistent kernel: every CTA the chip holds.
+template <class F>
+cudaError_t full_grid(F fn, int threads, int smem, int num_sms, int* grid) {
+  int per_sm = 0;
+  cudaError_t e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, fn, threads, smem);
+  *grid = std::max(per_sm, 1) * num_sms;
+  return e;
+}
+
+template <int K, int NT>
+cudaError_t launch_team(const DevGraph& g, RowTasks t, int cap, unsigned long long* head,
+                        unsigned long long* count, int num_sms, cudaStream_t s) {
+  t.wcap = (int)((std::min<int64_t>(g.max_out, cap) + 31) / 32);
+  const int smem = 4 * team_words<K>(t.wcap, NT / 32);
+  int grid = 0, dev = 0;
+  // the shared-memory opt-in of the widest layout, once per device
+  static std::atomic<unsigned long long> opted{0};
+  cudaError_t e = cudaGetDevice(&dev);
+  const unsigned long long bit = dev < 64 ? 1ull << dev : 0ull;
+  if (e == cudaSuccess && !(opted.load(std::memory_order_acquire) & bit)) {
+    e = cudaFuncSetAttribute(k_rows_team<K, NT>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                             4 * team_words<K>(cap / 32, NT / 32));
+    if (e == cudaSuccess) opted.fetch_or(bit, std::memory_order_acq_rel);
+  }
+  if (e == cudaSuccess) e = full_grid(k_rows_team<K, NT>, NT, smem, num_sms, &grid);
+  if (e != cudaSuccess) return e;
+  grid = (int)std::min<int64_t>(grid, g.nv);
+  k_rows_team<K, NT><<<grid, NT, smem, s>>>(t, head, count);
+  return cudaGetLastError();
+}
+
+template <int K>
+cudaError_t launch_rows_k(const DevGraph& g, const uint32_t* rows, OwnHeads* heads,
+                          unsigned long long* count, int num_sms, cudaStream_t s) {
+  const unsigned long long* rn = g.rn;
+  cudaError_t e = cudaSuccess;
+  if (g.max_out > kRowsMid) {
+    const RowTasks t{g.dptr, g.roff, rows, g.rtask + 2 * g.nv - 1, rn + 3, 1, 0};
+    e = launch_team<K, K == 4 ? 256 : 512>(g, t, kRowsCap, &heads->wide, count, num_sms, s);
+  }
+  if (e == cudaSuccess && g.max_out > 32) {
+    const RowTasks t{g.dptr, g.roff, rows, g.rtask + g.nv, rn + 2, 0, 0};
+    e = launch_team<K, 128>(g, t, kRowsMid, &heads->team, count, num_sms, s);
+  }
+  if (e != cudaSuccess) return e;
+  RowTasks t{g.dptr, g.roff, rows, g.rtask, rn + 1, 0, 32};
+  int grid = 0;
+  e = full_grid(k_rows_word<K>, kWordThreads, 0, num_sms, &grid);
+  if (e != cudaSuccess) return e;
+  const int64_t roots = std::max<int64_t>(g.n_roots[1], 1);  // at most this many word tasks
+  grid = (int)std::min<int64_t>(grid, (4 * roots + kWordThreads - 1) / kWordThreads);
+  t.wcap = (int)std::max<int64_t>(1, std::min<int64_t>(32, roots / (kWordThreads / 8 * (int64_t)grid)));
+  k_rows_word<K><<<grid, kWordThreads, 0, s>>>(t, &heads->word, count);
+  return cudaGetLastError();
+}
+
+}  // namespace
+
+cudaError_t launch_owner_count(const DevGraph& g, OwnHeads* heads, unsigned long long* count,
+                               int num_sms, cudaStream_t s) {
+  return launch_owner<kOwnCount>(g, OwnArgs{}, heads, count, num_sms, s);
+}
+
+cudaError_t ensure_rows_index(const DevGraph& g, cudaStream_t s) {
+  if (g.roff || g.nv == 0) return cudaSuccess;
+  int64_t* roff = nullptr;
+  int32_t* rtask = nullptr;
+  unsigned long long* rn = nullptr;
+  cudaError_t e = cudaMallocAsync((void**)&roff, sizeof(int64_t) * (size_t)g.nv, s);
+  if (e == cudaSuccess) e = cudaMallocAsync((void**)&rtask, sizeof(int32_t) * 2 * (size_t)g.nv, s);
+  if (e == cudaSuccess) e = cudaMallocAsync((void**)&rn, sizeof(*rn) * 4, s);
+  if (e == cudaSuccess) e = cudaMemsetAsync(rn, 0, sizeof(*rn) * 4, s);
+  if (e == cudaSuccess) {
+    const int64_t blocks = std::min<int64_t>((g.nv + 255) / 256, 65536);
+    k_rows_index<<<(unsigned)blocks, 256, 0, s>>>(g.dptr, g.nv, roff, rtask, rtask + g.nv, rn);
+    e = cudaGetLastError();
+  }
+  if (e != cudaSuccess) {
+    if (roff) cudaFreeAsync(roff, s);
+    if (rtask) cudaFreeAsync(rtask, s);
+    if (rn) cudaFreeAsync(rn, s);
+    return e;
+  }
+  g.roff = roff;
+  g.rtask = rtask;
+  g.rn = rn;
+  return cudaSuccess;
+}
+
+cudaError_t launch_owner_rows(const DevGraph& g, uint32_t* rows, OwnHeads* heads, int num_sms,
+                              cudaStream_t s) {
+  OwnArgs a{};
+  a.roff = g.roff;
+  a.rows = rows;
+  return launch_owner<kOwnRows>(g, a, heads, nullptr, num_sms, s);
+}
+
+cudaError_t launch_rows_count(int k, const DevGraph& g, const uint32_t* rows, OwnHeads* heads,
+                              unsigned long long* count, int num_sms, cudaStream_t s) {
+  if (g.nv == 0) return cudaSuccess;
+  switch (k) {
+    case 4: return launch_rows_k<4>(g, rows, heads, count, num_sms, s);
+    case 5: return launch_rows_k<5>(g, rows, heads, count, num_sms, s);
+    case 6: return launch_rows_k<6>(g, rows, heads, count, num_sms, s);
+    case 7: return launch_rows_k<7>(g, rows, heads, count, num_sms, s);
+    default: return cudaErrorInvalidValue;
+  }
 }
 
 }  // namespace xgm

@@ -12,13 +12,35 @@ namespace xgm {
 constexpr int kBigDeg = 64;
 constexpr int64_t kOwnBits = int64_t(1) << 18;
 
+constexpr int kRowsCap = 1024;  // largest out-degree whose rows are stored
+constexpr int kRowsMid = 512;   // largest one of the four-warp tasks
+
+// Row store words of a task of out-degree s (the triangular bitmap, rounded to 16 bytes).
+__host__ __device__ __forceinline__ unsigned row_words(int64_t s) {
+  return s < 3 || s > kRowsCap ? 0u : ((unsigned)tri_words((int)s) + 3u) & ~3u;
+}
+
 // Queue heads of one call (zeroed before it).
 struct OwnHeads {
-  unsigned long long big, small;
+  unsigned long long big, small;        // owner kernel: units, vertices
+  unsigned long long wide, team, word;  // row tasks by width
 };
 
 // Adds the triangle count of g to *count.
 cudaError_t launch_owner_count(const DevGraph& g, OwnHeads* heads, unsigned long long* count,
                                int num_sms, cudaStream_t s);
+
+// Clique counts from stored rows.  Row i of vertex v's local DAG (the DAG induced on N+(v))
+// holds bit j iff N+(v)[j] is an out-neighbour of N+(v)[i]; the rows of a vertex of
+// out-degree 3 .. kRowsCap are kept in the triangular layout (tri_row_off) at word roff[v]
+// of the row store, DevGraph::row_store_words words in all.
+//  ensure_rows_index: offsets and task lists by row width, once per graph.
+//  launch_owner_rows: fills the row store.
+//  launch_rows_count: adds the k-cliques (k = 4 .. 7) of all stored tasks to *count.
+cudaError_t ensure_rows_index(const DevGraph& g, cudaStream_t s);
+cudaError_t launch_owner_rows(const DevGraph& g, uint32_t* rows, OwnHeads* heads, int num_sms,
+                              cudaStream_t s);
+cudaError_t launch_rows_count(int k, const DevGraph& g, const uint32_t* rows, OwnHeads* heads,
+                              unsigned long long* count, int num_sms, cudaStream_t s);
 
 }  // namespace xgm
