@@ -4,6 +4,7 @@
 
 #include "clique.cuh"
 #include "graph.cuh"
+#include "motif.cuh"
 #include "rows.cuh"
 #include "sched.cuh"
 #include "setprog.cuh"
@@ -17,7 +18,7 @@ struct Scalars {
   uint32_t err;
   uint32_t pad;
   QueueHeads q;
-  unsigned long long c4heads[2];
+  C4Queue c4;
   int64_t n[8];  // task list sizes, copied back for the stats
   unsigned long long terms[6];  // motif-identity sums (launch_motif_terms)
   OwnHeads own;                 // queue heads of the owner kernels (rows.cu)
@@ -41,28 +42,10 @@ struct xgm_ctx {
   int64_t vpart_cap = 0;
   unsigned* epart = nullptr;
   int64_t epart_cap = 0;
-  uint32_t* c4_scratch = nullptr;
-  int64_t c4_scratch_cap = 0;
   long long* wedges = nullptr;
-  uint8_t* c4_flag_large = nullptr;
-  uint8_t* c4_flag_small = nullptr;
-  int64_t* c4_pos = nullptr;
-  int32_t* c4_large = nullptr;
-  int32_t* c4_small = nullptr;
-  int64_t* c4_n = nullptr;
-  int64_t c4_vcap = 0;
-  // grouped dense 4-cycle tasks (motif.cu): counters (kept zeroed), task info,
-  // segment arrays and the groups' task tables
-  uint32_t* c4_counters = nullptr;
-  int64_t* c4_info = nullptr;
-  int64_t c4_info_cap = 0;
-  int64_t* c4_seg_base = nullptr;
-  int64_t* c4_seg_pre = nullptr;
-  int32_t* c4_seg_cnt = nullptr;
-  int64_t c4_seg_cap = 0;
-  int32_t* c4_tv0 = nullptr;
-  int64_t* c4_ttab = nullptr;  // per group: tseg[m+1] then tcnt[m]
-  int64_t c4_task_cap = 0;
+  int64_t wedges_cap = 0;
+  int32_t* c4_lists = nullptr;  // the three task lists of the 4-cycle kernels
+  int64_t c4_lists_cap = 0;
   int clique_grid = 0;
   uint32_t* rows = nullptr;  // row store (rows.cu)
   int64_t rows_cap = 0;

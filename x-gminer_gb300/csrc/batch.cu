@@ -46,15 +46,7 @@ struct xgm_batch {
   xgm::TaskBuf tb;
   unsigned long long* vpart = nullptr;
   unsigned* epart = nullptr;
-  // 4-cycle buffers
-  uint32_t* c4_scratch = nullptr;
-  long long* wedges = nullptr;
-  uint8_t* fl_large = nullptr;
-  uint8_t* fl_small = nullptr;
-  int64_t* c4_pos = nullptr;
-  int32_t* c4_large = nullptr;
-  int32_t* c4_small = nullptr;
-  int64_t* c4_n = nullptr;
+  int32_t* c4_lists = nullptr;  // task lists of the 4-cycle kernels
   std::vector<xgm::CachedExec> cache;
 };
 
@@ -99,8 +91,7 @@ void batch_free(xgm_batch* b) {
     if (c.exec) cudaGraphExecDestroy(c.exec);
   b->cache.clear();
   taskbuf_free(b->tb, s);
-  void* ps[] = {b->d_out, b->vpart, b->epart, b->c4_scratch, b->wedges, b->fl_large,
-                b->fl_small, b->c4_pos, b->c4_large, b->c4_small, b->c4_n};
+  void* ps[] = {b->d_out, b->vpart, b->epart, b->c4_lists};
   for (void* p : ps)
     if (p) cudaFreeAsync(p, s);
   free_graph(b->graph.g, s);
@@ -203,16 +194,7 @@ xgm_status batch_prepare(xgm_ctx* ctx, xgm_batch* b, const Slots& sl, int P,
     XGM_CUDA_TRY(alloc_once(&b->vpart, g.nv, s));
     XGM_CUDA_TRY(alloc_once(&b->epart, g.ne, s));
   }
-  if (sl.c4 >= 0) {
-    XGM_CUDA_TRY(alloc_once(&b->c4_scratch, (int64_t)cycle4_grid(ctx->num_sms) * g.nv, s, true));
-    XGM_CUDA_TRY(alloc_once(&b->wedges, g.nv, s));
-    XGM_CUDA_TRY(alloc_once(&b->fl_large, g.nv, s));
-    XGM_CUDA_TRY(alloc_once(&b->fl_small, g.nv, s));
-    XGM_CUDA_TRY(alloc_once(&b->c4_pos, g.nv, s));
-    XGM_CUDA_TRY(alloc_once(&b->c4_large, g.nv, s));
-    XGM_CUDA_TRY(alloc_once(&b->c4_small, g.nv, s));
-    XGM_CUDA_TRY(alloc_once(&b->c4_n, 2, s));
-  }
+  if (sl.c4 >= 0) XGM_CUDA_TRY(alloc_once(&b->c4_lists, 3 * g.nv, s));
   ensure_clique_grid(ctx);
   if (sched_may_bucket(sp)) XGM_CUDA_TRY(ensure_bucket_index(g, s));  // before any capture
   if (sp.policy == XGM_SCHED_LEARNED) XGM_CUDA_TRY(ensure_task_stats(g, s));
@@ -265,15 +247,9 @@ xgm_status batch_sequence(xgm_ctx* ctx, xgm_batch* b, const Slots& sl, int P,
                                grid, s, o));
   }
   if (sl.c4 >= 0) {
-    XGM_CUDA_TRY(launch_wedge_count(view, b->wedges, b->fl_large, b->fl_small, s));
-    XGM_CUDA_TRY(scan_excl(b->fl_large, b->c4_pos, g.nv, b->c4_n + 0, s));
-    XGM_CUDA_TRY(launch_scatter_flags(b->fl_large, b->c4_pos, g.nv, b->c4_large, s));
-    XGM_CUDA_TRY(scan_excl(b->fl_small, b->c4_pos, g.nv, b->c4_n + 1, s));
-    XGM_CUDA_TRY(launch_scatter_flags(b->fl_small, b->c4_pos, g.nv, b->c4_small, s));
-    GOut o{g.gid, b->d_out, P, sl.c4, -1};
-    XGM_CUDA_TRY(launch_cycle4(view, b->c4_large, b->c4_small, b->c4_n, b->d_sc->c4heads,
-                               b->c4_scratch, nullptr, &b->d_sc->err, cycle4_grid(ctx->num_sms), s,
-                               o));
+    const C4Lists lists{b->c4_lists, b->c4_lists + g.nv, b->c4_lists + 2 * g.nv};
+    const GOut o{g.gid, b->d_out, P, sl.c4, -1};
+    XGM_CUDA_TRY(launch_cycle4(g, &b->d_sc->c4, lists, nullptr, ctx->num_sms, s, o));
   }
   XGM_CUDA_TRY(cudaMemcpyAsync(b->h_out, b->d_out, sizeof(unsigned long long) * nout,
                                cudaMemcpyDeviceToHost, s));

@@ -205,161 +205,11 @@ xgm_status launch_route(xgm_ctx* ctx, const DevGraph& g, int k, const xgm_sched&
   return XGM_OK;
 }
 
-xgm_status ensure_c4(xgm_ctx* ctx, const DevGraph& g) {
-  cudaStream_t s = ctx->stream;
-  if (ctx->c4_vcap < g.nv || !ctx->wedges) {
-    void* ps[] = {ctx->wedges, ctx->c4_flag_large, ctx->c4_flag_small, ctx->c4_pos,
-                  ctx->c4_large, ctx->c4_small, ctx->c4_n};
-    for (void* p : ps)
-      if (p) cudaFreeAsync(p, s);
-    const int64_t c = g.nv > 0 ? g.nv : 1;
-    XGM_CUDA_TRY(cudaMallocAsync(&ctx->wedges, sizeof(long long) * c, s));
-    XGM_CUDA_TRY(cudaMallocAsync(&ctx->c4_flag_large, c, s));
-    XGM_CUDA_TRY(cudaMallocAsync(&ctx->c4_flag_small, c, s));
-    XGM_CUDA_TRY(cudaMallocAsync(&ctx->c4_pos, sizeof(int64_t) * c, s));
-    XGM_CUDA_TRY(cudaMallocAsync(&ctx->c4_large, sizeof(int32_t) * c, s));
-    XGM_CUDA_TRY(cudaMallocAsync(&ctx->c4_small, sizeof(int32_t) * c, s));
-    XGM_CUDA_TRY(cudaMallocAsync(&ctx->c4_n, sizeof(int64_t) * 2, s));
-    ctx->c4_vcap = c;
-  }
-  const int64_t need = (int64_t)cycle4_grid(ctx->num_sms) * (g.nv > 0 ? g.nv : 1);
-  if (ctx->c4_scratch_cap < need) {
-    XGM_CUDA_TRY(grow(&ctx->c4_scratch, &ctx->c4_scratch_cap, need, s));
-    XGM_CUDA_TRY(cudaMemsetAsync(ctx->c4_scratch, 0, sizeof(uint32_t) * need, s));
-  }
-  return XGM_OK;
-}
-
-}  // namespace
-
-namespace {
-
-// Large 4-cycle tasks with at least 1/16 wedge per id of their range (v2 < v0) and
-// numerous wedges are counted a group at a time with L2-resident counters
-// (launch_c4_dense_walk); the others stay in the persistent kernel's list, whose large
-// tasks pay two DRAM atomics per wedge.  A group's counters are reset by a memset of
-// its ranges when they hold fewer than 8 counters per wedge, else by a second walk.
-// Reads the large list back, rewrites it without the grouped tasks, and launches them.
-constexpr int64_t kC4DenseMinWedges = int64_t(1) << 16;
-constexpr int64_t kC4DenseRangePerWedge = 16;
-
-xgm_status cycle4_dense_groups(xgm_ctx* ctx, const DevGraph& g, int* launches) {
-  cudaStream_t s = ctx->stream;
-  int64_t nls[2] = {0, 0};
-  XGM_CUDA_TRY(cudaMemcpyAsync(nls, ctx->c4_n, sizeof(nls), cudaMemcpyDeviceToHost, s));
-  XGM_CUDA_TRY(cudaStreamSynchronize(s));
-  const int64_t nl = nls[0];
-  if (nl == 0) return XGM_OK;
-  XGM_CUDA_TRY(grow(&ctx->c4_info, &ctx->c4_info_cap, 2 * nl, s));
-  XGM_CUDA_TRY(launch_c4_task_info(g.view(), ctx->c4_large, nl, ctx->wedges, ctx->c4_info, s));
-  std::vector<int32_t> list(nl);
-  std::vector<int64_t> info(2 * nl);
-  XGM_CUDA_TRY(cudaMemcpyAsync(list.data(), ctx->c4_large, sizeof(int32_t) * nl,
-                               cudaMemcpyDeviceToHost, s));
-  XGM_CUDA_TRY(cudaMemcpyAsync(info.data(), ctx->c4_info, sizeof(int64_t) * 2 * nl,
-                               cudaMemcpyDeviceToHost, s));
-  XGM_CUDA_TRY(cudaStreamSynchronize(s));
-  std::vector<int32_t> sparse, dense;
-  for (int64_t t = 0; t < nl; ++t) {
-    const int64_t w = info[2 * t], v0 = list[t];
-    if (w >= kC4DenseMinWedges && kC4DenseRangePerWedge * w >= v0 && v0 <= kC4GroupCounters)
-      dense.push_back((int32_t)t);
-    else sparse.push_back(list[t]);
-  }
-  if (dense.empty()) return XGM_OK;
-  std::sort(dense.begin(), dense.end(), [&](int32_t a, int32_t b) { return list[a] > list[b]; });
-  // groups: consecutive dense tasks whose ranges fit the counter array
-  std::vector<int32_t> tv0;
-  std::vector<int64_t> ttab;
-  struct Group { int64_t t0, m, tab, nseg, ncnt, wedges; };
-  // groups: consecutive tasks whose ranges fit the counter array.  Segments (one per
-  // task and lower neighbour) are numbered across all groups, so one segment launch and
-  // one scan serve every group; a group is a segment range.
-  std::vector<Group> groups;
-  std::vector<int64_t> tseg{0}, tcnt;
-  for (size_t i = 0; i < dense.size();) {
-    Group gr{(int64_t)tv0.size(), 0, tseg.back(), 0, 0, 0};
-    while (i < dense.size() && (gr.m == 0 || gr.ncnt + list[dense[i]] <= kC4GroupCounters)) {
-      const int32_t t = dense[i++];
-      tv0.push_back(list[t]);
-      tcnt.push_back(gr.ncnt);
-      gr.ncnt += list[t];
-      gr.wedges += info[2 * t];
-      tseg.push_back(tseg.back() + info[2 * t + 1]);
-      ++gr.m;
-    }
-    gr.nseg = tseg.back() - gr.tab;  // tab: first segment of the group
-    groups.push_back(gr);
-  }
-  const int64_t nseg_all = tseg.back();
-  const int64_t m_all = (int64_t)tv0.size();
-  ttab = tseg;
-  ttab.insert(ttab.end(), tcnt.begin(), tcnt.end());
-  if (!ctx->c4_counters) {
-    XGM_CUDA_TRY(cudaMallocAsync(&ctx->c4_counters, sizeof(uint32_t) * kC4GroupCounters, s));
-    XGM_CUDA_TRY(cudaMemsetAsync(ctx->c4_counters, 0, sizeof(uint32_t) * kC4GroupCounters, s));
-  }
-  if (ctx->c4_seg_cap < nseg_all) {
-    void* ps[] = {ctx->c4_seg_base, ctx->c4_seg_pre, ctx->c4_seg_cnt};
-    for (void* p : ps)
-      if (p) cudaFreeAsync(p, s);
-    ctx->c4_seg_cap = 0;
-    XGM_CUDA_TRY(cudaMallocAsync(&ctx->c4_seg_base, sizeof(int64_t) * nseg_all, s));
-    XGM_CUDA_TRY(cudaMallocAsync(&ctx->c4_seg_pre, sizeof(int64_t) * (nseg_all + 1), s));
-    XGM_CUDA_TRY(cudaMallocAsync(&ctx->c4_seg_cnt, sizeof(int32_t) * nseg_all, s));
-    ctx->c4_seg_cap = nseg_all;
-  }
-  const int64_t need = std::max<int64_t>(m_all, (int64_t)ttab.size());
-  if (ctx->c4_task_cap < need) {
-    if (ctx->c4_tv0) cudaFreeAsync(ctx->c4_tv0, s);
-    if (ctx->c4_ttab) cudaFreeAsync(ctx->c4_ttab, s);
-    ctx->c4_task_cap = 0;
-    XGM_CUDA_TRY(cudaMallocAsync(&ctx->c4_tv0, sizeof(int32_t) * need, s));
-    XGM_CUDA_TRY(cudaMallocAsync(&ctx->c4_ttab, sizeof(int64_t) * need, s));
-    ctx->c4_task_cap = need;
-  }
-  // the sparse large tasks stay with the persistent kernel; all tables go up at once
-  const int64_t ns = (int64_t)sparse.size();
-  if (ns) XGM_CUDA_TRY(cudaMemcpyAsync(ctx->c4_large, sparse.data(), sizeof(int32_t) * ns,
-                                      cudaMemcpyHostToDevice, s));
-  XGM_CUDA_TRY(cudaMemcpyAsync(ctx->c4_n, &ns, sizeof(int64_t), cudaMemcpyHostToDevice, s));
-  XGM_CUDA_TRY(cudaMemcpyAsync(ctx->c4_tv0, tv0.data(), sizeof(int32_t) * m_all,
-                               cudaMemcpyHostToDevice, s));
-  XGM_CUDA_TRY(cudaMemcpyAsync(ctx->c4_ttab, ttab.data(), sizeof(int64_t) * ttab.size(),
-                               cudaMemcpyHostToDevice, s));
-  XGM_CUDA_TRY(cudaStreamSynchronize(s));  // host tables are freed on return
-  const GView view = g.view();
-  const int grid = 4 * ctx->num_sms;
-  XGM_CUDA_TRY(launch_c4_segments(view, ctx->c4_tv0, ctx->c4_ttab, ctx->c4_ttab + m_all + 1,
-                                  (int)m_all, nseg_all, ctx->c4_seg_base, ctx->c4_seg_pre,
-                                  ctx->c4_seg_cnt, s));
-  XGM_CUDA_TRY(scan_excl(ctx->c4_seg_pre, ctx->c4_seg_pre, nseg_all, ctx->c4_seg_pre + nseg_all,
-                         s));
-  *launches += 2;
-  for (const Group& gr : groups) {
-    const int64_t e0 = gr.tab;
-    XGM_CUDA_TRY(launch_c4_dense_walk(g.col, ctx->c4_seg_pre + e0, ctx->c4_seg_base + e0,
-                                      ctx->c4_seg_cnt + e0, gr.nseg, ctx->c4_counters,
-                                      &ctx->d_sc->count, grid, s));
-    if (gr.ncnt <= 8 * gr.wedges)
-      XGM_CUDA_TRY(cudaMemsetAsync(ctx->c4_counters, 0, sizeof(uint32_t) * gr.ncnt, s));
-    else
-      XGM_CUDA_TRY(launch_c4_dense_walk(g.col, ctx->c4_seg_pre + e0, ctx->c4_seg_base + e0,
-                                        ctx->c4_seg_cnt + e0, gr.nseg, ctx->c4_counters, nullptr,
-                                        grid, s, true));
-    *launches += 2;
-  }
-  return XGM_OK;
-}
-
 }  // namespace
 
 void motif_buffers_free(xgm_ctx* ctx) {
   cudaStream_t s = ctx->stream;
-  void* ps[] = {ctx->vpart, ctx->epart, ctx->c4_scratch, ctx->wedges, ctx->c4_flag_large,
-                ctx->c4_flag_small, ctx->c4_pos, ctx->c4_large, ctx->c4_small, ctx->c4_n,
-                ctx->c4_counters, ctx->c4_info, ctx->c4_seg_base, ctx->c4_seg_pre,
-                ctx->c4_seg_cnt, ctx->c4_tv0, ctx->c4_ttab, ctx->rows};
+  void* ps[] = {ctx->vpart, ctx->epart, ctx->wedges, ctx->c4_lists, ctx->rows};
   for (void* p : ps)
     if (p) cudaFreeAsync(p, s);
 }
@@ -373,7 +223,7 @@ xgm_status count_dispatch(xgm_ctx* ctx, const DevGraph& g, int pattern, const xg
   if (k) {
     xgm_status r = clique_route(ctx, g, k, sp, &route);
     if (r != XGM_OK) return r;
-  } else {
+  } else if (pattern != XGM_PATTERN_CYCLE4) {
     XGM_CUDA_TRY(taskbuf_reserve(ctx->tb, g.nv, s));
   }
   XGM_CUDA_TRY(cudaMemsetAsync(ctx->d_sc, 0, sizeof(Scalars), s));
@@ -402,20 +252,11 @@ xgm_status count_dispatch(xgm_ctx* ctx, const DevGraph& g, int pattern, const xg
       XGM_CUDA_TRY(launch_tailed_reduce(ctx->vpart, g.rowptr, g.nv, &ctx->d_sc->count, s));
     launches = 2;
   } else if (pattern == XGM_PATTERN_CYCLE4) {
-    xgm_status r = ensure_c4(ctx, g);
-    if (r != XGM_OK) return r;
-    XGM_CUDA_TRY(launch_wedge_count(view, ctx->wedges, ctx->c4_flag_large, ctx->c4_flag_small, s));
-    XGM_CUDA_TRY(scan_excl(ctx->c4_flag_large, ctx->c4_pos, g.nv, ctx->c4_n + 0, s));
-    XGM_CUDA_TRY(launch_scatter_flags(ctx->c4_flag_large, ctx->c4_pos, g.nv, ctx->c4_large, s));
-    XGM_CUDA_TRY(scan_excl(ctx->c4_flag_small, ctx->c4_pos, g.nv, ctx->c4_n + 1, s));
-    XGM_CUDA_TRY(launch_scatter_flags(ctx->c4_flag_small, ctx->c4_pos, g.nv, ctx->c4_small, s));
+    XGM_CUDA_TRY(grow(&ctx->c4_lists, &ctx->c4_lists_cap, 3 * g.nv, s));
     XGM_CUDA_TRY(cudaEventRecord(ctx->ev[1], s));
+    const C4Lists lists{ctx->c4_lists, ctx->c4_lists + g.nv, ctx->c4_lists + 2 * g.nv};
+    XGM_CUDA_TRY(launch_cycle4(g, &ctx->d_sc->c4, lists, &ctx->d_sc->count, ctx->num_sms, s));
     launches = 1;
-    r = cycle4_dense_groups(ctx, g, &launches);
-    if (r != XGM_OK) return r;
-    XGM_CUDA_TRY(launch_cycle4(view, ctx->c4_large, ctx->c4_small, ctx->c4_n, ctx->d_sc->c4heads,
-                               ctx->c4_scratch, &ctx->d_sc->count, &ctx->d_sc->err,
-                               cycle4_grid(ctx->num_sms), s));
   } else {
     set_thread_error("unknown pattern");
     return XGM_ERR_INVALID;
@@ -524,10 +365,9 @@ xgm_status algo_bytes_dispatch(xgm_ctx* ctx, const DevGraph& g, int pattern, uin
   } else if (pattern == XGM_PATTERN_TAILED_TRIANGLE) {
     XGM_CUDA_TRY(launch_bytes_basic(view, 2, acc, s));
   } else if (pattern == XGM_PATTERN_CYCLE4) {
-    xgm_status r = ensure_c4(ctx, g);
-    if (r != XGM_OK) return r;
+    XGM_CUDA_TRY(grow(&ctx->wedges, &ctx->wedges_cap, g.nv, s));
     XGM_CUDA_TRY(launch_bytes_basic(view, 3, acc, s));
-    XGM_CUDA_TRY(launch_wedge_count(view, ctx->wedges, ctx->c4_flag_large, ctx->c4_flag_small, s));
+    XGM_CUDA_TRY(launch_wedge_count(view, ctx->wedges, s));
     XGM_CUDA_TRY(launch_sum_ll(ctx->wedges, g.nv, &ctx->d_sc->aux, s));
     xgm_status r2 = ctx_sync_scalars(ctx);
     if (r2 != XGM_OK) return r2;
