@@ -64,3 +64,35 @@ def test_no_edges_and_batched_ranks(xgm, ctx):
     g = ctx.graph_from_edges(7, none, none)
     assert ctx.count(g, "triangle") == 0
     g.close()
+
+
+@pytest.mark.parametrize("core,leaves,per", [(66, 0, 0), (70, 441, 70), (70, 443, 3),
+                                             (20, 1600, 13), (140, 5000, 14), (3, 70000, 2)])
+def test_participation_of_hubs(ctx, core, leaves, per):
+    """Diamonds and tailed triangles from triangles per edge, at the same edges of the tiers:
+    every pair of the core is an edge of core - 2 triangles inside it, and of `leaves` more
+    when both are joined to them."""
+    g = ctx.graph_from_edges(*_join(core, leaves, per))
+    t_core = [core - 2 + (leaves if j < per else 0) for j in range(core) for _ in range(j)]
+    diamonds = sum(math.comb(t, 2) for t in t_core) + leaves * per * math.comb(max(per - 1, 0), 2)
+    assert ctx.count(g, "diamond") == diamonds
+    # per vertex: triangles x (degree - 2)
+    t_in = math.comb(core - 1, 2) + leaves * max(per - 1, 0)
+    tailed = per * t_in * (core - 1 + leaves - 2) + (core - per) * math.comb(core - 1, 2) * (core - 3)
+    tailed += leaves * math.comb(per, 2) * (per - 2) if per > 2 else 0
+    assert ctx.count(g, "tailedtriangle") == tailed
+    g.close()
+
+
+@pytest.mark.parametrize("gen,args", [("rmat", (11, 16)), ("er", (500, 60000)),
+                                      ("er", (20001, 160000)),
+                                      ("chung_lu", (20001, 2.1, 3000.0, 20.0))])
+def test_participation_oracle_and_task_tiers(xgm, orc, ctx, gen, args):
+    nv, src, dst = getattr(xgm, "gen_" + gen)(*args, seed=43)
+    rowptr, col = orc.build_csr(nv, src, dst)
+    g = ctx.graph_from_edges(nv, src, dst)
+    for kind, pattern in (("diamond", "diamond"), ("tailed", "tailedtriangle")):
+        want = orc.count(kind, rowptr, col)
+        assert ctx.count(g, pattern) == want
+        assert ctx.count(g, pattern, policy=xgm.SCHED_FIXED, variant=xgm.VAR_WARP) == want
+    g.close()

@@ -20,7 +20,7 @@ struct Scalars {
   QueueHeads q;
   C4Queue c4;
   int64_t n[8];  // task list sizes, copied back for the stats
-  unsigned long long terms[6];  // motif-identity sums (launch_motif_terms)
+  unsigned long long terms[7];  // motif-identity sums (launch_motif_terms)
   OwnHeads own;                 // queue heads of the owner kernels (rows.cu)
 };
 

@@ -205,6 +205,32 @@ xgm_status launch_route(xgm_ctx* ctx, const DevGraph& g, int k, const xgm_sched&
   return XGM_OK;
 }
 
+// Triangles per edge into ctx->epart; *tasks: the task kernel ran (explicit schedules).
+// Records ev[1] between the preparation and the counting.
+xgm_status launch_participation(xgm_ctx* ctx, const DevGraph& g, const xgm_sched& sp, bool* tasks) {
+  cudaStream_t s = ctx->stream;
+  xgm_sched tri = sp;
+  if (tri.policy == XGM_SCHED_LEARNED && !tri.model) tri.policy = XGM_SCHED_HEURISTIC;
+  *tasks = !sched_is_open(tri) || g.max_out > kOwnPartMaxOut;
+  XGM_CUDA_TRY(grow(&ctx->epart, &ctx->epart_cap, g.ne, s));
+  XGM_CUDA_TRY(cudaMemsetAsync(ctx->epart, 0, sizeof(unsigned) * (g.ne > 0 ? g.ne : 1), s));
+  if (!*tasks) {
+    XGM_CUDA_TRY(cudaEventRecord(ctx->ev[1], s));
+    XGM_CUDA_TRY(launch_owner_part(g, &ctx->d_sc->own, ctx->epart, ctx->num_sms, s));
+    return XGM_OK;
+  }
+  XGM_CUDA_TRY(taskbuf_reserve(ctx->tb, g.nv, s));
+  xgm_status r = schedule_tasks(ctx, g, 3, tri);
+  if (r != XGM_OK) return r;
+  XGM_CUDA_TRY(grow(&ctx->vpart, &ctx->vpart_cap, g.nv, s));
+  XGM_CUDA_TRY(cudaMemsetAsync(ctx->vpart, 0, sizeof(unsigned long long) * (g.nv > 0 ? g.nv : 1), s));
+  XGM_CUDA_TRY(cudaEventRecord(ctx->ev[1], s));
+  XGM_CUDA_TRY(launch_triangle_participation(g.view(), ctx->tb.lists(false), &ctx->d_sc->q,
+                                             ctx->vpart, ctx->epart, &ctx->d_sc->err,
+                                             ensure_clique_grid(ctx), s));
+  return XGM_OK;
+}
+
 }  // namespace
 
 void motif_buffers_free(xgm_ctx* ctx) {
@@ -223,33 +249,22 @@ xgm_status count_dispatch(xgm_ctx* ctx, const DevGraph& g, int pattern, const xg
   if (k) {
     xgm_status r = clique_route(ctx, g, k, sp, &route);
     if (r != XGM_OK) return r;
-  } else if (pattern != XGM_PATTERN_CYCLE4) {
-    XGM_CUDA_TRY(taskbuf_reserve(ctx->tb, g.nv, s));
   }
   XGM_CUDA_TRY(cudaMemsetAsync(ctx->d_sc, 0, sizeof(Scalars), s));
   XGM_CUDA_TRY(cudaEventRecord(ctx->ev[0], s));
   const GView view = g.view();
   int launches = 0;
+  bool tasks = k && route == CliqueRoute::kTasks;  // the task kernel ran
   if (k) {
     xgm_status r = launch_route(ctx, g, k, sp, route, ctx->ev[1], &launches);
     if (r != XGM_OK) return r;
   } else if (pattern == XGM_PATTERN_DIAMOND || pattern == XGM_PATTERN_TAILED_TRIANGLE) {
-    xgm_sched tri = sp;
-    if (tri.policy == XGM_SCHED_LEARNED && !tri.model) tri.policy = XGM_SCHED_HEURISTIC;
-    xgm_status r = schedule_tasks(ctx, g, 3, tri);
+    xgm_status r = launch_participation(ctx, g, sp, &tasks);
     if (r != XGM_OK) return r;
-    XGM_CUDA_TRY(grow(&ctx->vpart, &ctx->vpart_cap, g.nv, s));
-    XGM_CUDA_TRY(grow(&ctx->epart, &ctx->epart_cap, g.ne, s));
-    XGM_CUDA_TRY(cudaMemsetAsync(ctx->vpart, 0, sizeof(unsigned long long) * (g.nv > 0 ? g.nv : 1), s));
-    XGM_CUDA_TRY(cudaMemsetAsync(ctx->epart, 0, sizeof(unsigned) * (g.ne > 0 ? g.ne : 1), s));
-    XGM_CUDA_TRY(cudaEventRecord(ctx->ev[1], s));
-    XGM_CUDA_TRY(launch_triangle_participation(view, ctx->tb.lists(false), &ctx->d_sc->q,
-                                               ctx->vpart, ctx->epart, &ctx->d_sc->err,
-                                               ensure_clique_grid(ctx), s));
     if (pattern == XGM_PATTERN_DIAMOND)
       XGM_CUDA_TRY(launch_diamond_reduce(ctx->epart, g.ne, &ctx->d_sc->count, s));
     else
-      XGM_CUDA_TRY(launch_tailed_reduce(ctx->vpart, g.rowptr, g.nv, &ctx->d_sc->count, s));
+      XGM_CUDA_TRY(launch_motif_terms(view, ctx->epart, ctx->d_sc->terms, s));
     launches = 2;
   } else if (pattern == XGM_PATTERN_CYCLE4) {
     XGM_CUDA_TRY(grow(&ctx->c4_lists, &ctx->c4_lists_cap, 3 * g.nv, s));
@@ -262,7 +277,7 @@ xgm_status count_dispatch(xgm_ctx* ctx, const DevGraph& g, int pattern, const xg
     return XGM_ERR_INVALID;
   }
   XGM_CUDA_TRY(cudaEventRecord(ctx->ev[2], s));
-  if ((k && route == CliqueRoute::kTasks) || pattern == XGM_PATTERN_DIAMOND || pattern == XGM_PATTERN_TAILED_TRIANGLE)
+  if (tasks)
     XGM_CUDA_TRY(cudaMemcpyAsync(ctx->d_sc->n, ctx->tb.n, sizeof(int64_t) * 8,
                                  cudaMemcpyDeviceToDevice, s));
   xgm_status r = ctx_sync_scalars(ctx);
@@ -283,10 +298,12 @@ xgm_status count_dispatch(xgm_ctx* ctx, const DevGraph& g, int pattern, const xg
   st.variant_tasks[XGM_VAR_GROUP] = ctx->h_sc->n[7];
   st.tasks = ctx->h_sc->n[1] + ctx->h_sc->n[2] + ctx->h_sc->n[3] + ctx->h_sc->n[4] +
              ctx->h_sc->n[5] + ctx->h_sc->n[6] + ctx->h_sc->n[7];
-  if (k && route != CliqueRoute::kTasks) st.tasks = g.n_roots[k - 3];
+  if (k && !tasks) st.tasks = g.n_roots[k - 3];
+  else if (!k && !tasks && pattern != XGM_PATTERN_CYCLE4) st.tasks = g.n_roots[0];
   r = check_device_flag(ctx, ctx->h_sc->err);
   if (r != XGM_OK) return r;
-  *out = ctx->h_sc->count;
+  *out = pattern == XGM_PATTERN_TAILED_TRIANGLE ? tailed_from_terms(ctx->h_sc->terms)
+                                                : ctx->h_sc->count;
   return XGM_OK;
 }
 
@@ -389,30 +406,19 @@ xgm_status motif_terms(xgm_ctx* ctx, const DevGraph& g, const xgm_sched& sp, boo
                        uint64_t terms[6], xgm_stats& st) {
   cudaStream_t s = ctx->stream;
   XGM_CUDA_TRY(cudaSetDevice(ctx->device));
-  XGM_CUDA_TRY(taskbuf_reserve(ctx->tb, g.nv, s));
   XGM_CUDA_TRY(cudaMemsetAsync(ctx->d_sc, 0, sizeof(Scalars), s));
   XGM_CUDA_TRY(cudaEventRecord(ctx->ev[0], s));
   const GView view = g.view();
+  bool tasks = false;  // the task kernel ran
   if (part) {
-    xgm_sched tri = sp;
-    if (tri.policy == XGM_SCHED_LEARNED && !tri.model) tri.policy = XGM_SCHED_HEURISTIC;
-    xgm_status r = schedule_tasks(ctx, g, 3, tri);
+    xgm_status r = launch_participation(ctx, g, sp, &tasks);
     if (r != XGM_OK) return r;
-    XGM_CUDA_TRY(grow(&ctx->vpart, &ctx->vpart_cap, g.nv, s));
-    XGM_CUDA_TRY(grow(&ctx->epart, &ctx->epart_cap, g.ne, s));
-    XGM_CUDA_TRY(cudaMemsetAsync(ctx->vpart, 0, sizeof(unsigned long long) * (g.nv > 0 ? g.nv : 1), s));
-    XGM_CUDA_TRY(cudaMemsetAsync(ctx->epart, 0, sizeof(unsigned) * (g.ne > 0 ? g.ne : 1), s));
-    XGM_CUDA_TRY(cudaEventRecord(ctx->ev[1], s));
-    XGM_CUDA_TRY(launch_triangle_participation(view, ctx->tb.lists(false), &ctx->d_sc->q,
-                                               ctx->vpart, ctx->epart, &ctx->d_sc->err,
-                                               ensure_clique_grid(ctx), s));
   } else {
     XGM_CUDA_TRY(cudaEventRecord(ctx->ev[1], s));
   }
-  XGM_CUDA_TRY(launch_motif_terms(view, part ? ctx->vpart : nullptr, part ? ctx->epart : nullptr,
-                                  ctx->d_sc->terms, s));
+  XGM_CUDA_TRY(launch_motif_terms(view, part ? ctx->epart : nullptr, ctx->d_sc->terms, s));
   XGM_CUDA_TRY(cudaEventRecord(ctx->ev[2], s));
-  if (part)
+  if (tasks)
     XGM_CUDA_TRY(cudaMemcpyAsync(ctx->d_sc->n, ctx->tb.n, sizeof(int64_t) * 8,
                                  cudaMemcpyDeviceToDevice, s));
   xgm_status r = ctx_sync_scalars(ctx);
@@ -425,7 +431,8 @@ xgm_status motif_terms(xgm_ctx* ctx, const DevGraph& g, const xgm_sched& sp, boo
   st.kernel_ms = kern;
   st.device_error = ctx->h_sc->err;
   st.launches = part ? 2 : 1;
-  if (part) {
+  if (part) st.tasks = g.n_roots[0];
+  if (tasks) {
     st.variant_tasks[XGM_VAR_WARP] = ctx->h_sc->n[2];
     st.variant_tasks[XGM_VAR_CTA] = ctx->h_sc->n[1];
     st.variant_tasks[XGM_VAR_SPLIT] = ctx->h_sc->n[0];
@@ -439,6 +446,7 @@ xgm_status motif_terms(xgm_ctx* ctx, const DevGraph& g, const xgm_sched& sp, boo
   r = check_device_flag(ctx, ctx->h_sc->err);
   if (r != XGM_OK) return r;
   for (int i = 0; i < 6; ++i) terms[i] = ctx->h_sc->terms[i];
+  terms[3] = tailed_from_terms(ctx->h_sc->terms);
   return XGM_OK;
 }
 

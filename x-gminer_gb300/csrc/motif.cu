@@ -7,7 +7,7 @@
 //  diamond        = sum over undirected edges e of C(n_e, 2), n_e = |N(u) & N(v)| =
 //                   number of triangles containing e.
 //  tailed triangle = sum over v with deg(v) > 2 of t(v) * (deg(v) - 2), t(v) = number
-//                   of triangles containing v.
+//                   of triangles containing v = half the sum of n_e over v's edges.
 //  4-cycle        = for every v0, wedges v0-v1-v2 with v1 < v0 and v2 < v0 grouped by
 //                   v2; a group of c wedges closes C(c, 2) cycles.
 // n_e and t(v) come from one triangle-participation pass of the DAG kernels
@@ -20,25 +20,27 @@ namespace xgm {
 namespace {
 
 constexpr int kThreads = 256;
+constexpr unsigned kReduceBlocks = 152 * 8;  // of a reduction: every SM full, once
 
-__global__ void k_diamond_reduce(const unsigned* epart, int64_t ne, unsigned long long* out) {
+// Sum of C(n, 2) over all entries (16 bytes a load; entries of lower neighbours are zero).
+__global__ void __launch_bounds__(kThreads) k_diamond_reduce(const unsigned* epart, int64_t ne,
+                                                             unsigned long long* out) {
   unsigned long long acc = 0;
-  for (int64_t e = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; e < ne;
-       e += (int64_t)gridDim.x * blockDim.x) {
-    unsigned long long n = epart[e];
-    acc += n * (n - (n > 0)) / 2;
+  const int64_t stride = (int64_t)gridDim.x * blockDim.x;
+  const int64_t n4 = ne >> 2;
+  for (int64_t e = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; e < n4; e += stride) {
+    const uint4 c = __ldcs(reinterpret_cast<const uint4*>(epart) + e);
+    if (!(c.x | c.y | c.z | c.w)) continue;
+    const unsigned cs[4] = {c.x, c.y, c.z, c.w};
+#pragma unroll
+    for (int h = 0; h < 4; ++h) {
+      const unsigned long long n = cs[h];
+      acc += n * (n - (n > 0)) / 2;
+    }
   }
-  acc = warp_sum_u64(acc);
-  if ((threadIdx.x & 31) == 0 && acc) atomicAdd(out, acc);
-}
-
-__global__ void k_tailed_reduce(const unsigned long long* vpart, const int64_t* rowptr, int64_t nv,
-                                unsigned long long* out) {
-  unsigned long long acc = 0;
-  for (int64_t r = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; r < nv;
-       r += (int64_t)gridDim.x * blockDim.x) {
-    int64_t d = rowptr[r + 1] - rowptr[r];
-    if (d > 2) acc += vpart[r] * (unsigned long long)(d - 2);
+  for (int64_t e = 4 * n4 + blockIdx.x * (int64_t)blockDim.x + threadIdx.x; e < ne; e += stride) {
+    const unsigned long long n = epart[e];
+    acc += n * (n - (n > 0)) / 2;
   }
   acc = warp_sum_u64(acc);
   if ((threadIdx.x & 31) == 0 && acc) atomicAdd(out, acc);
@@ -57,27 +59,23 @@ __device__ __forceinline__ unsigned long long choose3(unsigned long long d) {
 //   out[0] = sum_v C(d_v, 2)                 edge-induced wedges
 //   out[1] = sum_v C(d_v, 3)                 edge-induced 3-stars
 //   out[2] = sum_{uv in E} (d_u-1)(d_v-1)    3-edge walks x-u-v-y, x != v, y != u
-//   out[3] = sum_v t_v (d_v - 2)             edge-induced tailed triangles
+//   out[3] = 2 sum_v t_v (d_v - 2)           twice the edge-induced tailed triangles, as
+//   out[6]                                   the sum of low and of high 32-bit halves
 //   out[4] = sum_{uv in E} C(t_uv, 2)        edge-induced diamonds
-//   out[5] = sum_v t_v                       3 x triangles
-// t_v / t_uv are the triangle-participation counters (vpart / epart, null for the
-// 3-vertex census: out[3..5] stay 0).
-__global__ void __launch_bounds__(kThreads) k_motif_terms(GView g, const unsigned long long* vpart,
-                                                          const unsigned* epart,
+//   out[5] = sum_{uv in E} t_uv              3 x triangles
+// t_uv are the triangle-participation counters (epart, null for the 3-vertex census: out[3..6]
+// stay 0); t_v is half the sum of t over v's edges, so out[3] is sum t_uv (d_u + d_v - 4).
+// Few blocks: a sum costs one atomic per warp and term.
+__global__ void __launch_bounds__(kThreads) k_motif_terms(GView g, const unsigned* epart,
                                                           unsigned long long* out) {
   const int lane = threadIdx.x & 31;
-  unsigned long long acc[6] = {0, 0, 0, 0, 0, 0};
+  unsigned long long acc[7] = {0, 0, 0, 0, 0, 0, 0};
   const int64_t nwarps = (int64_t)gridDim.x * (kThreads / 32);
   for (int64_t r = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) >> 5; r < g.nv; r += nwarps) {
     const unsigned long long d = (unsigned long long)(g.rowptr[r + 1] - g.rowptr[r]);
     if (lane == 0) {
       acc[0] += d * (d - (d > 0)) / 2;
       acc[1] += choose3(d);
-      if (vpart) {
-        const unsigned long long t = vpart[r];
-        if (d > 2) acc[3] += t * (d - 2);
-        acc[5] += t;
-      }
     }
     const longlong2 p = g.dptr[r];
     for (long long j = p.x + lane; j < p.y; j += 32) {
@@ -86,12 +84,18 @@ __global__ void __launch_bounds__(kThreads) k_motif_terms(GView g, const unsigne
       acc[2] += (d - 1) * (dv - 1);
       if (epart) {
         const unsigned long long n = epart[j];
-        acc[4] += n * (n - (n > 0)) / 2;
+        if (n) {  // both ends have degree >= 2; n < 2^31, degrees < 2^31
+          acc[4] += n * (n - 1) / 2;
+          acc[5] += n;
+          const unsigned long long t = n * (d + dv - 4);
+          acc[3] += t & 0xFFFFFFFFull;
+          acc[6] += t >> 32;
+        }
       }
     }
   }
 #pragma unroll
-  for (int i = 0; i < 6; ++i) {
+  for (int i = 0; i < 7; ++i) {
     const unsigned long long w = warp_sum_u64(acc[i]);
     if (lane == 0 && w) atomicAdd(out + i, w);
   }
@@ -170,21 +174,21 @@ inline unsigned grid_for(int64_t n) {
 
 cudaError_t launch_diamond_reduce(const unsigned* epart, int64_t ne, unsigned long long* out,
                                   cudaStream_t s) {
-  k_diamond_reduce<<<grid_for(ne), kThreads, 0, s>>>(epart, ne, out);
+  k_diamond_reduce<<<std::min(grid_for((ne + 3) / 4), kReduceBlocks), kThreads, 0, s>>>(epart, ne,
+                                                                                       out);
   return cudaGetLastError();
 }
 
-cudaError_t launch_tailed_reduce(const unsigned long long* vpart, const int64_t* rowptr, int64_t nv,
-                                 unsigned long long* out, cudaStream_t s) {
-  k_tailed_reduce<<<grid_for(nv), kThreads, 0, s>>>(vpart, rowptr, nv, out);
-  return cudaGetLastError();
-}
-
-cudaError_t launch_motif_terms(const GView& g, const unsigned long long* vpart,
-                               const unsigned* epart, unsigned long long* out, cudaStream_t s) {
+cudaError_t launch_motif_terms(const GView& g, const unsigned* epart, unsigned long long* out,
+                               cudaStream_t s) {
   if (g.nv == 0) return cudaSuccess;
-  k_motif_terms<<<grid_for(g.nv * 32), kThreads, 0, s>>>(g, vpart, epart, out);
+  k_motif_terms<<<std::min(grid_for(g.nv * 32), kReduceBlocks), kThreads, 0, s>>>(g, epart, out);
   return cudaGetLastError();
+}
+
+uint64_t tailed_from_terms(const unsigned long long* terms) {
+  const unsigned __int128 twice = ((unsigned __int128)terms[6] << 32) + terms[3];
+  return (uint64_t)(twice >> 1);
 }
 
 cudaError_t launch_wedge_count(const GView& g, long long* wedges, cudaStream_t s) {

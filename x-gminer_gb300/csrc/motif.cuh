@@ -10,13 +10,13 @@ namespace xgm {
 
 cudaError_t launch_diamond_reduce(const unsigned* epart, int64_t ne, unsigned long long* out,
                                   cudaStream_t s);
-cudaError_t launch_tailed_reduce(const unsigned long long* vpart, const int64_t* rowptr, int64_t nv,
-                                 unsigned long long* out, cudaStream_t s);
 
-// out[0..5] += wedge / 3-star / 3-walk / tailed-triangle / diamond / 3 x triangle sums
-// (edge-induced; vpart/epart null for the 3-vertex census).
-cudaError_t launch_motif_terms(const GView& g, const unsigned long long* vpart,
-                               const unsigned* epart, unsigned long long* out, cudaStream_t s);
+// out[0..6] += the wedge / 3-star / 3-walk / tailed-triangle / diamond / 3 x triangle sums
+// (edge-induced; see motif.cu; epart null for the 3-vertex census).
+cudaError_t launch_motif_terms(const GView& g, const unsigned* epart, unsigned long long* out,
+                               cudaStream_t s);
+// Edge-induced tailed triangles from the seven sums.
+uint64_t tailed_from_terms(const unsigned long long* terms);
 
 // wedges[r] = wedges r-v1-v2 with v1, v2 < r (the 4-cycle plan's algorithmic bytes).
 cudaError_t launch_wedge_count(const GView& g, long long* wedges, cudaStream_t s);

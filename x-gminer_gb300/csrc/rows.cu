@@ -32,6 +32,9 @@
 //             (13 launches -> 1: no task lists)
 //  4-cliques  R-MAT s22 65.6 -> 23.0 ms (rows 12.3, counting 10.9); s20 12.4 -> 3.6 ms
 //  5-cliques  R-MAT s20 140 -> 33.5 ms; 6-cliques R-MAT s16 96 -> 18.5 ms
+//  triangles per edge (diamonds), Chung-Lu 1.5 M vertices, degree 32: 9.9 -> 3.5 ms; R-MAT
+//             s19 3.76 -> 1.47 ms (the hits' rank look-ups and counters: the bare count of
+//             the same suffixes is 2.5 times faster)
 // The tests with a warp per suffix, a ballot per 32 elements: 1.86 ms (s20 triangles), 15.2
 // ms (s22 rows): 145 instructions a pair, of which a third for the pair itself.
 // Bound: R-MAT s22 rows, L2 and DRAM latency (2.2 G sectors, 12 GB of DRAM reads: the lists
@@ -62,9 +65,15 @@ struct OwnArgs {
   int step;        // vertices per claim of the small phase
   const int64_t* roff = nullptr;  // rows mode: row store offset per vertex (-1: no rows)
   uint32_t* rows = nullptr;       // rows mode: the row store
+  unsigned* epart = nullptr;      // participation mode: triangles per col entry
+  int ranks = 0;                  // and its counters per out-neighbour of the owner
 };
 
-enum { kOwnCount = 0, kOwnRows = 1 };
+// kOwnPart credits every triangle (v, u, x) to its three edges, each at its lower end's col
+// entry: (v, u) once per pair, (v, x) at the tested element itself, (u, x) in a shared
+// counter of x's rank in N+(u), flushed once per unit.
+enum { kOwnCount = 0, kOwnRows = 1, kOwnPart = 2 };
+constexpr int kOwnRanks = 4096;  // most shared counters; longer out-lists credit epart itself
 
 // A suffix that eight lanes test: col[p .. p + len).  Rows mode: element e is bit
 // i + 1 + e of row i of v's local DAG, whose word i / 32 is rows[out].
@@ -126,6 +135,27 @@ __device__ __forceinline__ unsigned merge_count(const int32_t* col, long long a,
   }
 }
 
+// The same merge, crediting the hits' entries of both ranges.
+__device__ __forceinline__ unsigned merge_part(const int32_t* col, long long a, long long ea,
+                                               long long b, long long eb, unsigned* epart) {
+  if (a >= ea || b >= eb) return 0u;
+  unsigned acc = 0;
+  int32_t x = ldg_i32(col + a), y = ldg_i32(col + b);
+  for (;;) {
+    const bool le = x <= y, ge = x >= y;
+    if (le && ge) {
+      ++acc;
+      atomicAdd(&epart[a], 1u);
+      atomicAdd(&epart[b], 1u);
+    }
+    a += le;
+    b += ge;
+    if (a >= ea || b >= eb) return acc;
+    if (le) x = ldg_i32(col + a);
+    if (ge) y = ldg_i32(col + b);
+  }
+}
+
 // The same merge, a hit of the element a0 + k of the first range setting bit j0 + k.
 __device__ __forceinline__ void merge_row(const int32_t* col, long long a, long long ea,
                                           long long b, long long eb, int j, RowWriter& row) {
@@ -155,18 +185,24 @@ __device__ __forceinline__ long long lower_at(const int32_t* col, long long lo, 
 template <int MODE>
 __global__ void __launch_bounds__(kOwnThreads, 5) k_owner(OwnArgs a, OwnHeads* heads,
                                                        unsigned long long* count) {
-  constexpr bool ROWS = MODE == kOwnRows;
+  constexpr bool ROWS = MODE == kOwnRows, PART = MODE == kOwnPart;
   extern __shared__ uint32_t bm[];
+  // participation mode: counters per rank in N+(u), members before each bitmap word
+  uint32_t* rcnt = bm + a.wmask + 1;
+  uint16_t* wpre = reinterpret_cast<uint16_t*>(rcnt + a.ranks);
   __shared__ OwnPair<MODE> tab[kOwnChunk];
   __shared__ int lev[kOwnLevels + 1];  // lev[l]: units of levels above l (highest first)
   __shared__ int hist[32];  // long suffixes of the chunk by length
   __shared__ long long unit_s;
+  __shared__ int wsum[2][kOwnWarps];
   const GView& g = a.g;
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   unsigned long long acc = 0;
 
   if (a.big0 < g.nv) {
     for (int w = tid; w <= a.wmask; w += kOwnThreads) bm[w] = 0u;
+    if (PART)
+      for (int w = tid; w < a.ranks; w += kOwnThreads) rcnt[w] = 0u;
     // Units: level l holds the chunk l of every big vertex of degree > l * chunk, a prefix
     // of the descending degree order.  Levels are taken from the highest down, so the
     // last units are the small ones.
@@ -276,16 +312,53 @@ __global__ void __launch_bounds__(kOwnThreads, 5) k_owner(OwnArgs a, OwnHeads* h
         }
         unsigned part = 0;
         const int32_t base = (int32_t)u + 1;
+        // participation mode: x is the bit `off` of N+(u)
+        auto credit = [&](uint32_t off) {
+          const uint32_t word = bm[off >> 5];
+          const int r = wpre[off >> 5] + __popc(word & ((1u << (off & 31)) - 1u));
+          if (r < a.ranks) atomicAdd(&rcnt[r], 1u);
+          else atomicAdd(&a.epart[du.x + r], 1u);
+        };
+        if (PART && cc == c0) {
+          // members before each word (whole bitmap words of this owner), by a scan of 32
+          // words per warp and step; the totals of the steps before in wsum
+          const int words = (int)((g.nv - u + 30) >> 5);  // bits [0, V - u - 1)
+          int run = 0;
+          for (int w0 = 0; w0 < words; w0 += kOwnThreads) {
+            const int w = w0 + tid;
+            const int c = w < words ? __popc(bm[w]) : 0;
+            int inc = c;
+#pragma unroll
+            for (int o = 1; o < 32; o <<= 1) {
+              const int y = __shfl_up_sync(kFull, inc, o);
+              if (lane >= o) inc += y;
+            }
+            if (lane == 31) wsum[(w0 / kOwnThreads) & 1][warp] = inc;
+            __syncthreads();
+            const int ws = lane < kOwnWarps ? wsum[(w0 / kOwnThreads) & 1][lane] : 0;
+            const int before = (int)__reduce_add_sync(kFull, (unsigned)(lane < warp ? ws : 0));
+            if (w < words) wpre[w] = (uint16_t)(run + before + inc - c);
+            run += (int)__reduce_add_sync(kFull, (unsigned)ws);
+          }
+          __syncthreads();
+        }
 #pragma unroll
         for (int h = 0; h < 2; ++h)
           if (bin[h] < 0 && ss[h] > 0) {
             RowWriter w(ROWS ? a.rows + row[h] : nullptr, ii[h]);
+            unsigned hits = 0;
             for (int j = ii[h] + 1; j < ss[h]; ++j) {
               const uint32_t off = (uint32_t)(ldg_i32(g.col + p[h] + j) - base);
               const uint32_t bit = (bm[off >> 5] >> (off & 31)) & 1u;
-              if (ROWS) w.put(j, bit); else part += bit;
+              if (ROWS) w.put(j, bit); else hits += bit;
+              if (PART && bit) {
+                atomicAdd(&a.epart[p[h] + j], 1u);
+                credit(off);
+              }
             }
             if (ROWS) w.finish(ss[h]);
+            if (PART && hits) atomicAdd(&a.epart[p[h] + ii[h]], hits);
+            part += hits;
           }
         __syncthreads();
         // Eight lanes per suffix, one 16-byte unit each, from the unit its first element is
@@ -311,6 +384,7 @@ __global__ void __launch_bounds__(kOwnThreads, 5) k_owner(OwnArgs a, OwnHeads* h
             if (l8 == 0 && w0 == 1) out[-1] = 0u;  // bits up to i: none
           }
           const int most = __reduce_max_sync(kFull, steps);
+          unsigned hits = 0;
           int4 x = make_int4(0, 0, 0, 0);
           if (4 * l8 < rem) x = __ldg(q);
           for (int n = 0; n < most; ++n) {
@@ -321,7 +395,17 @@ __global__ void __launch_bounds__(kOwnThreads, 5) k_owner(OwnArgs a, OwnHeads* h
 #pragma unroll
             for (int h = 0; h < 4; ++h) {
               const uint32_t off = (uint32_t)(xs[h] - base);
-              bits = __funnelshift_r(bits, bm[(off >> 5) & a.wmask] >> (off & 31), 1);
+              const uint32_t word = bm[(off >> 5) & a.wmask] >> (off & 31);
+              if constexpr (PART) {
+                const int e = 32 * n + 4 * l8 + h;
+                if ((word & 1u) && e >= ph && e < rem) {
+                  ++hits;
+                  atomicAdd(&a.epart[t.p - ph + e], 1u);
+                  credit(off);
+                }
+              } else {
+                bits = __funnelshift_r(bits, word, 1);
+              }
             }
             if constexpr (ROWS) {
               uint32_t word = bits >> (28 - 4 * l8);
@@ -332,12 +416,18 @@ __global__ void __launch_bounds__(kOwnThreads, 5) k_owner(OwnArgs a, OwnHeads* h
               if (n == 0) word &= 0xFFFFFFFFu << ph;
               if (l8 == 0 && n < steps && w0 + n >= 0) out[n] = __funnelshift_l(prev, word, b0 & 31);
               prev = word;
-            } else {
+            } else if constexpr (!PART) {
               uint32_t m = mask_below(rem - 32 * n - 4 * l8);
               if (n == 0 && l8 == 0) m &= 0xFFFFFFFFu << ph;
               part += __popc((bits >> 28) & m);
             }
             x = y;
+          }
+          if constexpr (PART) {
+            hits += __shfl_xor_sync(kFull, hits, 1);
+            hits += __shfl_xor_sync(kFull, hits, 2);
+            hits += __shfl_xor_sync(kFull, hits, 4);
+            if (l8 == 0 && hits) atomicAdd(&a.epart[t.p - 1], hits);
           }
         }
         acc += part;
@@ -347,8 +437,16 @@ __global__ void __launch_bounds__(kOwnThreads, 5) k_owner(OwnArgs a, OwnHeads* h
       }
       if (tid == 0) unit_s = (long long)atomicAdd(&heads->big, 1ull);
       if (live)
-        for (long long e = du.x + tid; e < du.y; e += kOwnThreads)
+        for (long long e = du.x + tid; e < du.y; e += kOwnThreads) {
           bm[(uint32_t)(ldg_i32(g.col + e) - (int32_t)u - 1) >> 5] = 0u;
+          if (PART && e - du.x < a.ranks) {
+            const uint32_t c = rcnt[e - du.x];
+            if (c) {
+              atomicAdd(&a.epart[e], c);
+              rcnt[e - du.x] = 0u;
+            }
+          }
+        }
       __syncthreads();
     }
   }
@@ -404,6 +502,9 @@ __global__ void __launch_bounds__(kOwnThreads, 5) k_owner(OwnArgs a, OwnHeads* h
             RowWriter w(a.rows + qro + tri_row_off(i, (s + 31) >> 5), i);
             merge_row(g.col, at + 1, end, du.x, du.y, i + 1, w);
             w.finish(s);
+          } else if constexpr (PART) {
+            const unsigned n = merge_part(g.col, at + 1, end, du.x, du.y, a.epart);
+            if (n) atomicAdd(&a.epart[at], n);
           } else {
             acc += merge_count(g.col, at + 1, end, du.x, du.y);
           }
@@ -411,7 +512,7 @@ __global__ void __launch_bounds__(kOwnThreads, 5) k_owner(OwnArgs a, OwnHeads* h
       }
     }
   }
-  if constexpr (!ROWS) {
+  if constexpr (MODE == kOwnCount) {
     acc = warp_sum_u64(acc);
     if (lane == 0 && acc) atomicAdd(count, acc);
   }
@@ -430,10 +531,25 @@ cudaError_t launch_owner(const DevGraph& g, OwnArgs a, OwnHeads* heads, unsigned
   int words = 32;
   while (32 * (int64_t)words < nbig) words *= 2;
   a.wmask = words - 1;
-  const int smem = 4 * words;
+  int smem = 4 * words;
+  cudaError_t e = cudaSuccess;
+  if constexpr (MODE == kOwnPart) {
+    a.ranks = (int)std::min<int64_t>(g.max_out, kOwnRanks);
+    smem += 4 * a.ranks + 2 * words;
+    // the shared-memory opt-in of the largest layout, once per device
+    static std::atomic<unsigned long long> opted{0};
+    int dev = 0;
+    e = cudaGetDevice(&dev);
+    const unsigned long long bit = dev < 64 ? 1ull << dev : 0ull;
+    if (e == cudaSuccess && !(opted.load(std::memory_order_acquire) & bit)) {
+      e = cudaFuncSetAttribute(k_owner<MODE>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                               (int)(kOwnBits / 32) * 6 + 4 * kOwnRanks);
+      if (e == cudaSuccess) opted.fetch_or(bit, std::memory_order_acq_rel);
+    }
+    if (e != cudaSuccess) return e;
+  }
   int per_sm = 0;
-  cudaError_t e =
-      cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_owner<MODE>, kOwnThreads, smem);
+  e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_owner<MODE>, kOwnThreads, smem);
   if (e != cudaSuccess) return e;
   // no more CTAs than there is work for (small graphs would only pay for starting them),
   // and claims small enough that every warp has a few
@@ -1087,6 +1203,13 @@ cudaError_t launch_rows_k(const DevGraph& g, const uint32_t* rows, OwnHeads* hea
 cudaError_t launch_owner_count(const DevGraph& g, OwnHeads* heads, unsigned long long* count,
                                int num_sms, cudaStream_t s) {
   return launch_owner<kOwnCount>(g, OwnArgs{}, heads, count, num_sms, s);
+}
+
+cudaError_t launch_owner_part(const DevGraph& g, OwnHeads* heads, unsigned* epart, int num_sms,
+                              cudaStream_t s) {
+  OwnArgs a{};
+  a.epart = epart;
+  return launch_owner<kOwnPart>(g, a, heads, nullptr, num_sms, s);
 }
 
 cudaError_t ensure_rows_index(const DevGraph& g, cudaStream_t s) {

@@ -30,6 +30,12 @@ struct OwnHeads {
 cudaError_t launch_owner_count(const DevGraph& g, OwnHeads* heads, unsigned long long* count,
                                int num_sms, cudaStream_t s);
 
+// Adds to epart[e] the number of triangles that contain the edge of every col entry e of the
+// out-lists (the edge at its lower end).  For out-degrees up to kOwnPartMaxOut (16-bit ranks).
+constexpr int64_t kOwnPartMaxOut = 0xFFFF;
+cudaError_t launch_owner_part(const DevGraph& g, OwnHeads* heads, unsigned* epart, int num_sms,
+                              cudaStream_t s);
+
 // Clique counts from stored rows.  Row i of vertex v's local DAG (the DAG induced on N+(v))
 // holds bit j iff N+(v)[j] is an out-neighbour of N+(v)[i]; the rows of a vertex of
 // out-degree 3 .. kRowsCap are kept in the triangular layout (tri_row_off) at word roff[v]
