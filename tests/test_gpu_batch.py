@@ -96,3 +96,36 @@ def test_full_batch_config_matches_oracle(xgm, ctx, orc):
         want = (orc.count("tc", drow, dcol), orc.count("clique4", drow, dcol),
                 orc.count("diamond", rowptr, col))
         assert tuple(int(x) for x in got[g]) == want, g
+
+
+def test_batches_of_mixed_graphs(xgm, ctx, orc):
+    """Graphs at the edges of the row kernels' tiers side by side: out-degrees around 8, 32 and
+    above, empty graphs, graphs smaller than the 32 ranks that one warp sums."""
+    sizes = [3, 9, 10, 11, 33, 34, 35, 70, 1, 5, 140]
+    parts, off = [], [0]
+    for n in sizes:
+        iu = np.triu_indices(n, 1)
+        parts.append((iu[0] + off[-1], iu[1] + off[-1]))
+        off.append(off[-1] + n)
+    for seed, (n, m) in enumerate([(400, 3000), (37, 60), (1200, 60000)]):
+        _, s, d = xgm.gen_er(n, m, seed=seed + 3)
+        parts.append((s + off[-1], d + off[-1]))
+        off.append(off[-1] + n)
+    src = np.concatenate([p[0] for p in parts]).astype(np.int32)
+    dst = np.concatenate([p[1] for p in parts]).astype(np.int32)
+    b = ctx.batch_from_edges(np.array(off, dtype=np.int64), src, dst)
+    got = ctx.count_batched(b, PATTERNS)
+    for g, p in enumerate(parts):
+        rowptr, col = orc.build_csr(off[g + 1] - off[g], (p[0] - off[g]).astype(np.int32),
+                                    (p[1] - off[g]).astype(np.int32))
+        drow, dcol = orc.orient(rowptr, col)
+        for i, name in enumerate(PATTERNS):
+            k = KIND[name]
+            want = orc.count(k, drow, dcol) if k in ("tc", "clique4", "clique5") \
+                else orc.count(k, rowptr, col)
+            assert int(got[g, i]) == want, (g, name)
+    # every subset of the plans takes its own mix of kernels; explicit schedules the task kernel
+    for sub in (["triangle"], ["4-clique"], ["5-clique", "tailedtriangle"], ["diamond"]):
+        cols = [PATTERNS.index(x) for x in sub]
+        assert np.array_equal(ctx.count_batched(b, sub), got[:, cols]), sub
+    assert np.array_equal(ctx.count_batched(b, PATTERNS, group_max=8), got)

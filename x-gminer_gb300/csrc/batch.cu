@@ -47,6 +47,8 @@ struct xgm_batch {
   unsigned long long* vpart = nullptr;
   unsigned* epart = nullptr;
   int32_t* c4_lists = nullptr;  // task lists of the 4-cycle kernels
+  uint32_t* rows = nullptr;     // row store (rows.cu)
+  unsigned long long* sums = nullptr;  // per-graph sums of launch_graph_terms
   std::vector<xgm::CachedExec> cache;
 };
 
@@ -91,7 +93,7 @@ void batch_free(xgm_batch* b) {
     if (c.exec) cudaGraphExecDestroy(c.exec);
   b->cache.clear();
   taskbuf_free(b->tb, s);
-  void* ps[] = {b->d_out, b->vpart, b->epart, b->c4_lists};
+  void* ps[] = {b->d_out, b->vpart, b->epart, b->c4_lists, b->rows, b->sums};
   for (void* p : ps)
     if (p) cudaFreeAsync(p, s);
   free_graph(b->graph.g, s);
@@ -172,6 +174,12 @@ cudaError_t alloc_once(T** p, int64_t n, cudaStream_t s, bool zero = false) {
   return e;
 }
 
+// Triangles, cliques and participation plans from the owner and row kernels; explicit
+// schedules, and graphs above the row capacity, run the task kernel.
+bool batch_from_rows(const DevGraph& g, const xgm_sched& sp) {
+  return sched_is_open(sp) && g.max_out <= kRowsCap && g.row_store_words <= kRowStoreMax;
+}
+
 // Allocations a sequence needs, made before any capture.
 xgm_status batch_prepare(xgm_ctx* ctx, xgm_batch* b, const Slots& sl, int P,
                          const xgm_sched& sp) {
@@ -190,14 +198,23 @@ xgm_status batch_prepare(xgm_ctx* ctx, xgm_batch* b, const Slots& sl, int P,
       if (c.exec) cudaGraphExecDestroy(c.exec);
     b->cache.clear();
   }
-  if (sl.dia >= 0 || sl.tail >= 0) {
+  const bool rows = batch_from_rows(g, sp);
+  if (rows && (sl.tri >= 0 || sl.dia >= 0 || sl.tail >= 0)) {
+    XGM_CUDA_TRY(alloc_once(&b->epart, g.ne + 3, s));  // whole 16-byte units
+    XGM_CUDA_TRY(alloc_once(&b->sums, 3 * (int64_t)b->num_graphs, s));
+  }
+  if (rows && (sl.k4 >= 0 || sl.k5 >= 0)) {
+    XGM_CUDA_TRY(ensure_rows_index(g, s));
+    XGM_CUDA_TRY(alloc_once(&b->rows, g.row_store_words + 4, s));
+  }
+  if (!rows && (sl.dia >= 0 || sl.tail >= 0)) {
     XGM_CUDA_TRY(alloc_once(&b->vpart, g.nv, s));
-    XGM_CUDA_TRY(alloc_once(&b->epart, g.ne, s));
+    XGM_CUDA_TRY(alloc_once(&b->epart, g.ne + 3, s));
   }
   if (sl.c4 >= 0) XGM_CUDA_TRY(alloc_once(&b->c4_lists, 3 * g.nv, s));
   ensure_clique_grid(ctx);
-  if (sched_may_bucket(sp)) XGM_CUDA_TRY(ensure_bucket_index(g, s));  // before any capture
-  if (sp.policy == XGM_SCHED_LEARNED) XGM_CUDA_TRY(ensure_task_stats(g, s));
+  if (!rows && sched_may_bucket(sp)) XGM_CUDA_TRY(ensure_bucket_index(g, s));  // before any capture
+  if (!rows && sp.policy == XGM_SCHED_LEARNED) XGM_CUDA_TRY(ensure_task_stats(g, s));
   XGM_CUDA_TRY(cudaStreamSynchronize(s));
   return XGM_OK;
 }
@@ -212,7 +229,29 @@ xgm_status batch_sequence(xgm_ctx* ctx, xgm_batch* b, const Slots& sl, int P,
   const int grid = ensure_clique_grid(ctx);
   XGM_CUDA_TRY(cudaMemsetAsync(b->d_out, 0, sizeof(unsigned long long) * nout, s));
   XGM_CUDA_TRY(cudaMemsetAsync(b->d_sc, 0, sizeof(Scalars), s));
-  if (sl.tri >= 0 || sl.k4 >= 0 || sl.dia >= 0 || sl.tail >= 0) {
+  const bool rows = batch_from_rows(g, sp);
+  if (rows) {
+    const bool part = sl.tri >= 0 || sl.dia >= 0 || sl.tail >= 0, k = sl.k4 >= 0 || sl.k5 >= 0;
+    OwnHeads* heads = &b->d_sc->own;
+    if (part) {
+      XGM_CUDA_TRY(cudaMemsetAsync(b->epart, 0, sizeof(unsigned) * (g.ne + 3), s));
+      XGM_CUDA_TRY(cudaMemsetAsync(b->sums, 0, sizeof(unsigned long long) * 3 * b->num_graphs, s));
+    }
+    if (part && k) XGM_CUDA_TRY(launch_owner_multi(g, b->rows, b->epart, heads, ctx->num_sms, s));
+    else if (part) XGM_CUDA_TRY(launch_owner_part(g, heads, b->epart, ctx->num_sms, s));
+    else if (k) XGM_CUDA_TRY(launch_owner_rows(g, b->rows, heads, ctx->num_sms, s));
+    if (sl.k4 >= 0)
+      XGM_CUDA_TRY(launch_rows_count(4, g, b->rows, heads, nullptr, ctx->num_sms, s,
+                                     GOut{g.gid, b->d_out, P, sl.k4, -1}));
+    if (sl.k5 >= 0) {
+      XGM_CUDA_TRY(cudaMemsetAsync(heads, 0, sizeof(OwnHeads), s));
+      XGM_CUDA_TRY(launch_rows_count(5, g, b->rows, heads, nullptr, ctx->num_sms, s,
+                                     GOut{g.gid, b->d_out, P, sl.k5, -1}));
+    }
+    if (part)
+      XGM_CUDA_TRY(launch_graph_terms(view, g.gid, b->num_graphs, b->epart, b->sums, b->d_out, P,
+                                      sl.tri, sl.dia, sl.tail, s));
+  } else if (sl.tri >= 0 || sl.k4 >= 0 || sl.dia >= 0 || sl.tail >= 0) {
     const bool part = sl.dia >= 0 || sl.tail >= 0;
     if (part) {
       XGM_CUDA_TRY(cudaMemsetAsync(b->vpart, 0, sizeof(unsigned long long) * (g.nv > 0 ? g.nv : 1), s));
@@ -226,7 +265,7 @@ xgm_status batch_sequence(xgm_ctx* ctx, xgm_batch* b, const Slots& sl, int P,
     // kernel always credits participation, so give it real buffers
     if (!part) {
       XGM_CUDA_TRY(alloc_once(&b->vpart, g.nv, s));
-      XGM_CUDA_TRY(alloc_once(&b->epart, g.ne, s));
+      XGM_CUDA_TRY(alloc_once(&b->epart, g.ne + 3, s));
     }
     GOut o{g.gid, b->d_out, P, sl.tri, sl.k4};
     XGM_CUDA_TRY(launch_multi(view, b->tb.lists(false), &b->d_sc->q, b->vpart, b->epart,
@@ -238,7 +277,7 @@ xgm_status batch_sequence(xgm_ctx* ctx, xgm_batch* b, const Slots& sl, int P,
       XGM_CUDA_TRY(launch_part_reduce_graphs(view, g.gid, b->vpart, b->epart, b->d_out, P, sl.dia,
                                              sl.tail, s));
   }
-  if (sl.k5 >= 0) {
+  if (!rows && sl.k5 >= 0) {
     XGM_CUDA_TRY(cudaMemsetAsync(&b->d_sc->q, 0, sizeof(QueueHeads), s));
     xgm_status r = schedule_into(b->tb, g, 5, sp, s, 0, true);
     if (r != XGM_OK) return r;
@@ -262,7 +301,7 @@ std::string sched_key(const Slots& sl, const xgm_sched& sp) {
   k.append(reinterpret_cast<const char*>(&sp.policy), sizeof(int) * 2);
   k.append(reinterpret_cast<const char*>(&sp.model), sizeof(void*));
   k.append(reinterpret_cast<const char*>(&sp.warp_max), sizeof(int) * 3);
-  const int more[4] = {sp.wide_max, sp.search_max, sp.bucket_max, sp.group_max};
+  const int more[5] = {sp.wide_max, sp.search_max, sp.bucket_max, sp.group_max, sp.hub_max};
   k.append(reinterpret_cast<const char*>(more), sizeof(more));
   k.append(reinterpret_cast<const char*>(&sp.margin), sizeof(float));
   const int hash_only = sp.flags & XGM_SCHED_HASH_ONLY;

@@ -146,10 +146,6 @@ xgm_status schedule_tasks(xgm_ctx* ctx, const DevGraph& g, int k, const xgm_sche
   return schedule_into(ctx->tb, g, k, sp, ctx->stream, 0, hub);
 }
 
-// The row store holds a graph's rows up to 16 GB (R-MAT scale 22: 0.6 GB); larger graphs,
-// and a device without that much memory left, count with the task kernel.
-constexpr int64_t kRowStoreMax = int64_t(1) << 32;  // words
-
 // What a clique count launches: the owner kernel (triangles), the row kernels (k >= 4; the
 // task kernel then only runs the vertices above their capacity), or the task kernel.
 enum class CliqueRoute { kOwner, kRows, kTasks };

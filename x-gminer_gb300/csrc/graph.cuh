@@ -37,9 +37,9 @@ struct DevGraph {
   mutable int64_t* lut_off = nullptr;
   mutable int lut_state = 0;
   // row store offsets, row tasks by width and their numbers (rows.cu), built on first use
-  // by a clique count: rn = {words, tasks of <= 32 members, of <= kRowsMid, of more};
-  // rtask holds the first list from its start, the second from nv on, the third from its
-  // end down
+  // by a clique count: rn = {words, tasks of <= 8 members, <= 32, <= kRowsMid, more}; rtask
+  // holds the first list from its start, the second from nv - 1 down, the third from nv on,
+  // the fourth from its end down
   int64_t row_store_words = 0;
   mutable int64_t* roff = nullptr;
   mutable int32_t* rtask = nullptr;

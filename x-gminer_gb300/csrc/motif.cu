@@ -165,6 +165,101 @@ __global__ void k_part_reduce_graphs(GView g, const int32_t* gid,
   }
 }
 
+// Per-graph sums from the triangles per edge (batched graphs): diamonds to out, three times
+// the triangles and (TAIL) twice the tailed triangles (low and high 32-bit halves) to
+// sums[3 gid].  A warp streams the rows of 32 consecutive ranks, 16 bytes a lane (entries of
+// lower neighbours are zero); graphs are contiguous in rank order, so most blocks belong to
+// one graph and end in one atomic per sum.  (A thread per vertex walking its out-list: 368
+// us on 5.2 M vertices.)
+template <bool TAIL>
+__global__ void __launch_bounds__(kThreads) k_graph_terms(GView g, const int32_t* gid,
+                                                          const unsigned* epart,
+                                                          unsigned long long* out, int stride,
+                                                          int slot_d, unsigned long long* sums) {
+  __shared__ int64_t row_s[kThreads / 32][33];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  int64_t* row = row_s[warp];
+  const int64_t nwarps = (int64_t)gridDim.x * (kThreads / 32);
+  for (int64_t r0 = 32 * ((blockIdx.x * (int64_t)blockDim.x + threadIdx.x) >> 5); r0 < g.nv;
+       r0 += 32 * nwarps) {
+    const int64_t r1 = r0 + 32 < g.nv ? r0 + 32 : g.nv;
+    __syncwarp();
+    row[lane] = g.rowptr[r0 + lane < r1 ? r0 + lane : r1];
+    if (lane == 0) row[32] = g.rowptr[r1];
+    __syncwarp();
+    const int64_t e0 = row[0], e1 = row[32];
+    const int32_t first = gid[r0];
+    const bool one = gid[r1 - 1] == first;  // one graph
+    unsigned long long dia = 0, tri = 0, lo = 0, hi = 0;
+    for (int64_t q = (e0 >> 2) + lane; 4 * q < e1; q += 32) {
+      // (epart holds whole 16-byte units; a unit may begin or end in a neighbouring row)
+      const uint4 c4 = __ldcs(reinterpret_cast<const uint4*>(epart) + q);
+      if (!(c4.x | c4.y | c4.z | c4.w)) continue;
+      const unsigned cs[4] = {c4.x, c4.y, c4.z, c4.w};
+#pragma unroll
+      for (int h = 0; h < 4; ++h) {
+        const int64_t e = 4 * q + h;
+        const unsigned long long n = cs[h];
+        if (!n || e < e0 || e >= e1) continue;
+        if (!TAIL && one) {
+          dia += n * (n - 1) / 2;
+          tri += n;
+          continue;
+        }
+        int r = 0;  // the entry's row: largest with row[r] <= e
+#pragma unroll
+        for (int d = 16; d > 0; d >>= 1)
+          if (row[r + d] <= e) r += d;
+        unsigned long long t = 0;
+        if (TAIL) {
+          const int32_t v = ldg_i32(g.col + e);
+          t = n * (unsigned long long)(row[r + 1] - row[r] + (g.dptr[v].y - g.rowptr[v]) - 4);
+        }
+        if (one) {
+          dia += n * (n - 1) / 2;
+          tri += n;
+          lo += t & 0xFFFFFFFFull;
+          hi += t >> 32;
+        } else {
+          const int64_t gg = gid[r0 + r];
+          if (slot_d >= 0 && n > 1) atomicAdd(&out[gg * stride + slot_d], n * (n - 1) / 2);
+          atomicAdd(&sums[3 * gg], n);
+          if (TAIL) {
+            atomicAdd(&sums[3 * gg + 1], t & 0xFFFFFFFFull);
+            if (t >> 32) atomicAdd(&sums[3 * gg + 2], t >> 32);
+          }
+        }
+      }
+    }
+    if (!one) continue;
+    dia = warp_sum_u64(dia);
+    tri = warp_sum_u64(tri);
+    if (TAIL) lo = warp_sum_u64(lo), hi = warp_sum_u64(hi);
+    if (lane == 0 && tri) {
+      if (slot_d >= 0 && dia) atomicAdd(&out[(int64_t)first * stride + slot_d], dia);
+      atomicAdd(&sums[3 * (int64_t)first], tri);
+      if (TAIL) {
+        atomicAdd(&sums[3 * (int64_t)first + 1], lo);
+        if (hi) atomicAdd(&sums[3 * (int64_t)first + 2], hi);
+      }
+    }
+  }
+}
+
+// Triangles and tailed triangles per graph from the sums (a slot < 0 is skipped).
+__global__ void k_graph_finish(const unsigned long long* sums, int graphs, unsigned long long* out,
+                               int stride, int slot_tri, int slot_t) {
+  for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < graphs;
+       i += (int64_t)gridDim.x * blockDim.x) {
+    if (slot_tri >= 0) out[i * stride + slot_tri] = sums[3 * i] / 3;
+    if (slot_t >= 0) {  // (high half << 32 + low half) / 2
+      const unsigned long long lo = sums[3 * i + 1], hi = sums[3 * i + 2];
+      const unsigned long long low = lo + (hi << 32), carry = low < lo;
+      out[i * stride + slot_t] = (low >> 1) | (((hi >> 32) + carry) << 63);
+    }
+  }
+}
+
 inline unsigned grid_for(int64_t n) {
   int64_t b = (n + kThreads - 1) / kThreads;
   return (unsigned)std::max<int64_t>(1, std::min<int64_t>(b, int64_t(1) << 20));
@@ -194,6 +289,20 @@ uint64_t tailed_from_terms(const unsigned long long* terms) {
 cudaError_t launch_wedge_count(const GView& g, long long* wedges, cudaStream_t s) {
   if (g.nv == 0) return cudaSuccess;
   k_wedge_count<<<grid_for(g.nv * 32), kThreads, 0, s>>>(g, wedges);
+  return cudaGetLastError();
+}
+
+cudaError_t launch_graph_terms(const GView& g, const int32_t* gid, int graphs,
+                               const unsigned* epart, unsigned long long* sums,
+                               unsigned long long* out, int stride, int slot_tri, int slot_d,
+                               int slot_t, cudaStream_t s) {
+  if (g.nv == 0) return cudaSuccess;
+  const unsigned grid = std::min(grid_for(g.nv), kReduceBlocks);
+  if (slot_t >= 0)
+    k_graph_terms<true><<<grid, kThreads, 0, s>>>(g, gid, epart, out, stride, slot_d, sums);
+  else
+    k_graph_terms<false><<<grid, kThreads, 0, s>>>(g, gid, epart, out, stride, slot_d, sums);
+  k_graph_finish<<<grid_for(graphs), kThreads, 0, s>>>(sums, graphs, out, stride, slot_tri, slot_t);
   return cudaGetLastError();
 }
 

@@ -42,4 +42,11 @@ cudaError_t launch_part_reduce_graphs(const GView& g, const int32_t* gid,
                                       unsigned long long* out, int stride, int slot_d, int slot_t,
                                       cudaStream_t s);
 
+// Batched graphs: per-graph triangles, diamonds and tailed triangles from the triangles per
+// edge (a slot < 0 is skipped); sums: 3 values per graph, zeroed.
+cudaError_t launch_graph_terms(const GView& g, const int32_t* gid, int graphs,
+                               const unsigned* epart, unsigned long long* sums,
+                               unsigned long long* out, int stride, int slot_tri, int slot_d,
+                               int slot_t, cudaStream_t s);
+
 }  // namespace xgm

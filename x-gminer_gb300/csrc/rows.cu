@@ -35,6 +35,7 @@
 //  triangles per edge (diamonds), Chung-Lu 1.5 M vertices, degree 32: 9.9 -> 3.5 ms; R-MAT
 //             s19 3.76 -> 1.47 ms (the hits' rank look-ups and counters: the bare count of
 //             the same suffixes is 2.5 times faster)
+//  4,096 Barabasi-Albert graphs, triangles + 4-cliques + diamonds each: 3.44 -> 1.54 ms
 // The tests with a warp per suffix, a ballot per 32 elements: 1.86 ms (s20 triangles), 15.2
 // ms (s22 rows): 145 instructions a pair, of which a third for the pair itself.
 // Bound: R-MAT s22 rows, L2 and DRAM latency (2.2 G sectors, 12 GB of DRAM reads: the lists
@@ -72,7 +73,8 @@ struct OwnArgs {
 // kOwnPart credits every triangle (v, u, x) to its three edges, each at its lower end's col
 // entry: (v, u) once per pair, (v, x) at the tested element itself, (u, x) in a shared
 // counter of x's rank in N+(u), flushed once per unit.
-enum { kOwnCount = 0, kOwnRows = 1, kOwnPart = 2 };
+// kOwnMulti does what kOwnRows and kOwnPart do.
+enum { kOwnCount = 0, kOwnRows = 1, kOwnPart = 2, kOwnMulti = 3 };
 constexpr int kOwnRanks = 4096;  // most shared counters; longer out-lists credit epart itself
 
 // A suffix that eight lanes test: col[p .. p + len).  Rows mode: element e is bit
@@ -87,6 +89,8 @@ struct OwnPair<kOwnRows> {
   long long p, out;
   int len, i;
 };
+template <>
+struct OwnPair<kOwnMulti> : OwnPair<kOwnRows> {};
 
 // 32-bit mask of the bits below r (r <= 0: none, r >= 32: all).
 __device__ __forceinline__ uint32_t mask_below(int r) {
@@ -118,54 +122,17 @@ struct RowWriter {
   }
 };
 
-// Elements two sorted ranges of col have in common.
-__device__ __forceinline__ unsigned merge_count(const int32_t* col, long long a, long long ea,
-                                                long long b, long long eb) {
-  if (a >= ea || b >= eb) return 0u;
-  unsigned acc = 0;
-  int32_t x = ldg_i32(col + a), y = ldg_i32(col + b);
-  for (;;) {
-    const bool le = x <= y, ge = x >= y;
-    acc += (le && ge) ? 1u : 0u;
-    a += le;
-    b += ge;
-    if (a >= ea || b >= eb) return acc;
-    if (le) x = ldg_i32(col + a);
-    if (ge) y = ldg_i32(col + b);
-  }
-}
-
-// The same merge, crediting the hits' entries of both ranges.
-__device__ __forceinline__ unsigned merge_part(const int32_t* col, long long a, long long ea,
-                                               long long b, long long eb, unsigned* epart) {
-  if (a >= ea || b >= eb) return 0u;
-  unsigned acc = 0;
-  int32_t x = ldg_i32(col + a), y = ldg_i32(col + b);
-  for (;;) {
-    const bool le = x <= y, ge = x >= y;
-    if (le && ge) {
-      ++acc;
-      atomicAdd(&epart[a], 1u);
-      atomicAdd(&epart[b], 1u);
-    }
-    a += le;
-    b += ge;
-    if (a >= ea || b >= eb) return acc;
-    if (le) x = ldg_i32(col + a);
-    if (ge) y = ldg_i32(col + b);
-  }
-}
-
-// The same merge, a hit of the element a0 + k of the first range setting bit j0 + k.
-__device__ __forceinline__ void merge_row(const int32_t* col, long long a, long long ea,
-                                          long long b, long long eb, int j, RowWriter& row) {
+// Calls f(k, l) for every element the sorted ranges [a, ea) and [b, eb) of col have in common,
+// at col[k] and col[l].
+template <class F>
+__device__ __forceinline__ void merge_lists(const int32_t* col, long long a, long long ea,
+                                            long long b, long long eb, F f) {
   if (a >= ea || b >= eb) return;
   int32_t x = ldg_i32(col + a), y = ldg_i32(col + b);
   for (;;) {
     const bool le = x <= y, ge = x >= y;
-    if (le && ge) row.put(j, 1u);
+    if (le && ge) f(a, b);
     a += le;
-    j += le;
     b += ge;
     if (a >= ea || b >= eb) return;
     if (le) x = ldg_i32(col + a);
@@ -182,10 +149,18 @@ __device__ __forceinline__ long long lower_at(const int32_t* col, long long lo, 
   return lo;
 }
 
+// CTAs per SM the registers are cut for, measured per mode (the bitmap allows 5 at R-MAT s22):
+// triangles s20 1.52 / 1.49 / 1.43 ms with 4 / 5 / 6, rows s22 11.9 / 13.9 / 13.5,
+// participation of a 1.5 M vertex Chung-Lu graph 3.72 / 3.53 / 4.23, rows and participation
+// of 4,096 small graphs 1.26 / 1.13 / 1.04.
+constexpr int own_ctas(int mode) {
+  return mode == kOwnRows ? 4 : (mode == kOwnPart ? 5 : 6);
+}
+
 template <int MODE>
-__global__ void __launch_bounds__(kOwnThreads, 5) k_owner(OwnArgs a, OwnHeads* heads,
+__global__ void __launch_bounds__(kOwnThreads, own_ctas(MODE)) k_owner(OwnArgs a, OwnHeads* heads,
                                                        unsigned long long* count) {
-  constexpr bool ROWS = MODE == kOwnRows, PART = MODE == kOwnPart;
+  constexpr bool ROWS = (MODE & kOwnRows) != 0, PART = (MODE & kOwnPart) != 0;
   extern __shared__ uint32_t bm[];
   // participation mode: counters per rank in N+(u), members before each bitmap word
   uint32_t* rcnt = bm + a.wmask + 1;
@@ -271,8 +246,8 @@ __global__ void __launch_bounds__(kOwnThreads, 5) k_owner(OwnArgs a, OwnHeads* h
           if (e < c1) {
             const int32_t v = ldg_i32(g.col + e);
             const long long ro = ROWS ? __ldg(a.roff + v) : 0;
-            if (ro >= 0) {
-              const longlong2 dv = ldg_ll2(g.dptr + v);
+            const longlong2 dv = ro >= 0 ? ldg_ll2(g.dptr + v) : make_longlong2(0, 0);
+            if (dv.y - dv.x >= (MODE == kOwnRows ? 3 : 2)) {
               p[h] = dv.x;
               ss[h] = (int)(dv.y - dv.x);
               ii[h] = (int)(lower_at(g.col, dv.x, dv.y, (int32_t)u) - dv.x);
@@ -350,7 +325,8 @@ __global__ void __launch_bounds__(kOwnThreads, 5) k_owner(OwnArgs a, OwnHeads* h
             for (int j = ii[h] + 1; j < ss[h]; ++j) {
               const uint32_t off = (uint32_t)(ldg_i32(g.col + p[h] + j) - base);
               const uint32_t bit = (bm[off >> 5] >> (off & 31)) & 1u;
-              if (ROWS) w.put(j, bit); else hits += bit;
+              if (ROWS) w.put(j, bit);
+              hits += bit;
               if (PART && bit) {
                 atomicAdd(&a.epart[p[h] + j], 1u);
                 credit(off);
@@ -403,9 +379,8 @@ __global__ void __launch_bounds__(kOwnThreads, 5) k_owner(OwnArgs a, OwnHeads* h
                   atomicAdd(&a.epart[t.p - ph + e], 1u);
                   credit(off);
                 }
-              } else {
-                bits = __funnelshift_r(bits, word, 1);
               }
+              if constexpr (MODE != kOwnPart) bits = __funnelshift_r(bits, word, 1);
             }
             if constexpr (ROWS) {
               uint32_t word = bits >> (28 - 4 * l8);
@@ -466,10 +441,9 @@ __global__ void __launch_bounds__(kOwnThreads, 5) k_owner(OwnArgs a, OwnHeads* h
       if (b + lane < ve) {
         const long long v = nsm - 1 - (b + lane);  // longest lists first
         if (ROWS) ro = __ldg(a.roff + v);
-        if (ro >= 0) {
-          d = ldg_ll2(g.dptr + v);
-          cnt = (int)(d.y - d.x) - (ROWS ? 0 : 1);  // the last row is empty
-        }
+        if (ro >= 0) d = ldg_ll2(g.dptr + v);
+        cnt = (int)(d.y - d.x) - (ROWS ? 0 : 1);  // the last row is empty
+        if (d.y - d.x < (MODE == kOwnRows ? 3 : 2)) cnt = 0;
         if (cnt > 0 && ldg_i32(g.col + d.x + cnt - 1) >= a.big0)
           cnt = (int)(lower_at(g.col, d.x, d.x + cnt, (int32_t)a.big0) - d.x);
         if (cnt < 0) cnt = 0;
@@ -497,17 +471,30 @@ __global__ void __launch_bounds__(kOwnThreads, 5) k_owner(OwnArgs a, OwnHeads* h
           const int i = k - ex;
           const long long at = base + i;
           const longlong2 du = ldg_ll2(g.dptr + ldg_i32(g.col + at));
+          unsigned hits = 0;
           if constexpr (ROWS) {
             const int s = (int)(end - base);
             RowWriter w(a.rows + qro + tri_row_off(i, (s + 31) >> 5), i);
-            merge_row(g.col, at + 1, end, du.x, du.y, i + 1, w);
+            merge_lists(g.col, at + 1, end, du.x, du.y, [&](long long k, long long l) {
+              w.put((int)(k - base), 1u);
+              if (PART) {
+                ++hits;
+                atomicAdd(&a.epart[k], 1u);
+                atomicAdd(&a.epart[l], 1u);
+              }
+            });
             w.finish(s);
-          } else if constexpr (PART) {
-            const unsigned n = merge_part(g.col, at + 1, end, du.x, du.y, a.epart);
-            if (n) atomicAdd(&a.epart[at], n);
           } else {
-            acc += merge_count(g.col, at + 1, end, du.x, du.y);
+            merge_lists(g.col, at + 1, end, du.x, du.y, [&](long long k, long long l) {
+              ++hits;
+              if (PART) {
+                atomicAdd(&a.epart[k], 1u);
+                atomicAdd(&a.epart[l], 1u);
+              }
+            });
+            if (!PART) acc += hits;
           }
+          if (PART && hits) atomicAdd(&a.epart[at], hits);
         }
       }
     }
@@ -533,7 +520,7 @@ cudaError_t launch_owner(const DevGraph& g, OwnArgs a, OwnHeads* heads, unsigned
   a.wmask = words - 1;
   int smem = 4 * words;
   cudaError_t e = cudaSuccess;
-  if constexpr (MODE == kOwnPart) {
+  if constexpr ((MODE & kOwnPart) != 0) {
     a.ranks = (int)std::min<int64_t>(g.max_out, kOwnRanks);
     smem += 4 * a.ranks + 2 * words;
     // the shared-memory opt-in of the largest layout, once per device
@@ -565,8 +552,8 @@ cudaError_t launch_owner(const DevGraph& g, OwnArgs a, OwnHeads* heads, unsigned
 __global__ void __launch_bounds__(256) k_rows_index(const longlong2* dptr, int64_t nv,
                                                     int64_t* roff, int32_t* word_l,
                                                     int32_t* team_l, unsigned long long* rn) {
-  __shared__ unsigned wsum[8], lcnt[3];
-  __shared__ unsigned long long wbase, lbase[3];
+  __shared__ unsigned wsum[8], lcnt[4];
+  __shared__ unsigned long long wbase, lbase[4];
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   for (int64_t b = (int64_t)blockIdx.x * 256; b < nv; b += (int64_t)gridDim.x * 256) {
     const int64_t v = b + tid;
@@ -576,8 +563,8 @@ __global__ void __launch_bounds__(256) k_rows_index(const longlong2* dptr, int64
       s = d.y - d.x <= kRowsCap ? (int)(d.y - d.x) : 0;
     }
     const unsigned words = row_words(s);
-    const int cls = words == 0 ? 3 : (s <= 32 ? 0 : (s <= kRowsMid ? 1 : 2));
-    if (tid < 3) lcnt[tid] = 0;
+    const int cls = s < 3 ? 4 : (s <= 8 ? 0 : (s <= 32 ? 1 : (s <= kRowsMid ? 2 : 3)));
+    if (tid < 4) lcnt[tid] = 0;
     unsigned inc = words;
 #pragma unroll
     for (int o = 1; o < 32; o <<= 1) {
@@ -587,7 +574,7 @@ __global__ void __launch_bounds__(256) k_rows_index(const longlong2* dptr, int64
     if (lane == 31) wsum[warp] = inc;
     __syncthreads();
     unsigned slot = 0;
-    if (cls < 3) slot = atomicAdd(&lcnt[cls], 1u);
+    if (cls < 4) slot = atomicAdd(&lcnt[cls], 1u);
     unsigned off = inc - words, tot = 0;
     for (int w = 0; w < 8; ++w) {
       if (w < warp) off += wsum[w];
@@ -595,13 +582,14 @@ __global__ void __launch_bounds__(256) k_rows_index(const longlong2* dptr, int64
     }
     __syncthreads();
     if (tid == 0) wbase = atomicAdd(&rn[0], (unsigned long long)tot);
-    if (tid < 3) lbase[tid] = atomicAdd(&rn[1 + tid], (unsigned long long)lcnt[tid]);
+    if (tid < 4) lbase[tid] = atomicAdd(&rn[1 + tid], (unsigned long long)lcnt[tid]);
     __syncthreads();
     if (v < nv) {
       roff[v] = words ? (int64_t)(wbase + off) : -1;
       if (cls == 0) word_l[lbase[0] + slot] = (int32_t)v;
-      else if (cls == 1) team_l[lbase[1] + slot] = (int32_t)v;
-      else if (cls == 2) team_l[nv - 1 - (int64_t)(lbase[2] + slot)] = (int32_t)v;
+      else if (cls == 1) word_l[nv - 1 - (int64_t)(lbase[1] + slot)] = (int32_t)v;
+      else if (cls == 2) team_l[lbase[2] + slot] = (int32_t)v;
+      else if (cls == 3) team_l[nv - 1 - (int64_t)(lbase[3] + slot)] = (int32_t)v;
     }
     __syncthreads();
   }
@@ -942,6 +930,18 @@ __device__ uint64_t matrix_cliques(const uint32_t* C, int n, int wi, int nw, uin
   }
 }
 
+// Totals: one sum per thread, or (o.gid) a task's total to its graph's output.  Called by all
+// lanes of a warp.
+__device__ __forceinline__ void emit_rows(const GOut& o, int32_t v, uint64_t part, uint64_t& acc) {
+  if (!o.gid) {
+    acc += part;
+    return;
+  }
+  const uint64_t w = warp_sum_u64(part);
+  if ((threadIdx.x & 31) == 0 && w)
+    atomicAdd(&o.out[(long long)o.gid[v] * o.stride + o.slot], (unsigned long long)w);
+}
+
 struct RowTasks {
   const longlong2* dptr;
   const int64_t* roff;
@@ -988,20 +988,21 @@ constexpr int team_ctas(int K, int NT) {
 // kOwnN members by one warp, of up to kTeamN by a team of four, longer ones by the CTA.
 template <int K, int NT>
 __global__ void __launch_bounds__(NT, team_ctas(K, NT)) k_rows_team(RowTasks t, unsigned long long* head,
-                                                  unsigned long long* count) {
+                                                  unsigned long long* count, GOut o) {
   extern __shared__ __align__(16) uint32_t M[];
   __shared__ long long task_s;
   __shared__ int next_i, n_long, next_long, n_huge, team_x[NT / 32 / kTeam];
   constexpr int kWarps = NT / 32, kTeams = kWarps / kTeam;
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const long long nt = (long long)*t.n;
-  uint64_t acc = 0;
+  uint64_t total = 0;
   if (tid == 0) task_s = (long long)atomicAdd(head, 1ull);
   __syncthreads();
   for (;;) {
     const long long ti = task_s;
     if (ti >= nt) break;
     const int32_t v = t.down ? t.list[-ti] : t.list[ti];
+    uint64_t acc = 0;
     const longlong2 d = ldg_ll2(t.dptr + v);
     const int s = (int)(d.y - d.x), W = (s + 31) >> 5;
     const int used = tri_words(s), all = matrix_words(W);  // the last block padded to 32 rows
@@ -1086,10 +1087,11 @@ __global__ void __launch_bounds__(NT, team_ctas(K, NT)) k_rows_team(RowTasks t, 
         }
       }
     }
+    emit_rows(o, v, acc, total);
     __syncthreads();
   }
-  acc = warp_sum_u64(acc);
-  if (lane == 0 && acc) atomicAdd(count, (unsigned long long)acc);
+  total = warp_sum_u64(total);
+  if (lane == 0 && total) atomicAdd(count, (unsigned long long)total);
 }
 
 // Tasks of up to 32 out-neighbours, a warp each, lane i holding row i.  K = 4: one block on
@@ -1097,7 +1099,7 @@ __global__ void __launch_bounds__(NT, team_ctas(K, NT)) k_rows_team(RowTasks t, 
 constexpr int kWordThreads = 256;
 template <int K>
 __global__ void __launch_bounds__(kWordThreads) k_rows_word(RowTasks t, unsigned long long* head,
-                                                            unsigned long long* count) {
+                                                            unsigned long long* count, GOut o) {
   __shared__ uint32_t rows_s[kWordThreads / 32][32];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const long long nt = (long long)*t.n;
@@ -1109,9 +1111,10 @@ __global__ void __launch_bounds__(kWordThreads) k_rows_word(RowTasks t, unsigned
     if (base >= nt) break;
     const int n = nt - base < t.wcap ? (int)(nt - base) : t.wcap;
     int s = 0;
+    int32_t v = 0;
     long long off = 0;
     if (lane < n) {
-      const int32_t v = t.list[base + lane];
+      v = t.down ? t.list[-(base + lane)] : t.list[base + lane];
       const longlong2 d = ldg_ll2(t.dptr + v);
       s = (int)(d.y - d.x);
       off = t.roff[v];
@@ -1129,12 +1132,71 @@ __global__ void __launch_bounds__(kWordThreads) k_rows_word(RowTasks t, unsigned
       }
       if (sc < K - 1) continue;
       if constexpr (K == 4) {
-        acc += tri_word(r, sc);
+        emit_rows(o, __shfl_sync(kFull, v, x), tri_word(r, sc), acc);
       } else {
         rows_s[warp][lane] = r;
         __syncwarp();
-        acc += word_cliques<K - 2>(rows_s[warp], r);
+        const uint64_t c = word_cliques<K - 2>(rows_s[warp], r);
         __syncwarp();
+        emit_rows(o, __shfl_sync(kFull, v, x), c, acc);
+      }
+    }
+  }
+  acc = warp_sum_u64(acc);
+  if (lane == 0 && acc) atomicAdd(count, (unsigned long long)acc);
+}
+
+// Tasks of up to 8 out-neighbours, four to a warp, lane l of a group holding row l.
+template <int K>
+__global__ void __launch_bounds__(kWordThreads) k_rows_group(RowTasks t, unsigned long long* head,
+                                                             unsigned long long* count, GOut o) {
+  __shared__ uint32_t rows_s[kWordThreads];
+  const int lane = threadIdx.x & 31, l8 = lane & 7, g0 = lane & 24;
+  const uint32_t* mine = rows_s + (threadIdx.x & ~7);
+  const long long nt = (long long)*t.n;
+  uint64_t acc = 0;
+  for (;;) {
+    long long base = 0;
+    if (lane == 0) base = (long long)atomicAdd(head, (unsigned long long)t.wcap);
+    base = __shfl_sync(kFull, base, 0);
+    if (base >= nt) break;
+    const int n = nt - base < t.wcap ? (int)(nt - base) : t.wcap;
+    int s = 0;
+    int32_t v = 0;
+    long long off = 0;
+    if (lane < n) {
+      v = t.list[base + lane];
+      const longlong2 d = ldg_ll2(t.dptr + v);
+      s = (int)(d.y - d.x);
+      off = t.roff[v];
+    }
+    for (int x = 0; x < n; x += 4) {
+      const int src = x + (lane >> 3);  // (lanes past n hold s = 0)
+      const int sc = __shfl_sync(kFull, s, src);
+      const long long ro = __shfl_sync(kFull, off, src);
+      const uint32_t r = l8 < sc ? __ldcs(t.rows + ro + l8) : 0u;
+      uint32_t c = 0;
+      if constexpr (K == 4) {
+#pragma unroll
+        for (int j = 1; j < 7; ++j) {  // the last two rows hold no pair
+          const uint32_t rj = __shfl_sync(kFull, r, g0 + j);
+          if ((r >> j) & 1u) c += __popc(r & rj);
+        }
+      } else {
+        rows_s[threadIdx.x] = r;
+        __syncwarp();
+        c = (uint32_t)word_cliques<K - 2>(mine, r);
+        __syncwarp();
+      }
+      if (o.gid) {
+        c += __shfl_xor_sync(kFull, c, 1);
+        c += __shfl_xor_sync(kFull, c, 2);
+        c += __shfl_xor_sync(kFull, c, 4);
+        const int32_t vx = __shfl_sync(kFull, v, src);
+        if (l8 == 0 && c)
+          atomicAdd(&o.out[(long long)o.gid[vx] * o.stride + o.slot], (unsigned long long)c);
+      } else {
+        acc += c;
       }
     }
   }
@@ -1153,7 +1215,7 @@ cudaError_t full_grid(F fn, int threads, int smem, int num_sms, int* grid) {
 
 template <int K, int NT>
 cudaError_t launch_team(const DevGraph& g, RowTasks t, int cap, unsigned long long* head,
-                        unsigned long long* count, int num_sms, cudaStream_t s) {
+                        unsigned long long* count, int num_sms, cudaStream_t s, const GOut& o) {
   t.wcap = (int)((std::min<int64_t>(g.max_out, cap) + 31) / 32);
   const int smem = 4 * team_words<K>(t.wcap, NT / 32);
   int grid = 0, dev = 0;
@@ -1169,33 +1231,43 @@ cudaError_t launch_team(const DevGraph& g, RowTasks t, int cap, unsigned long lo
   if (e == cudaSuccess) e = full_grid(k_rows_team<K, NT>, NT, smem, num_sms, &grid);
   if (e != cudaSuccess) return e;
   grid = (int)std::min<int64_t>(grid, g.nv);
-  k_rows_team<K, NT><<<grid, NT, smem, s>>>(t, head, count);
+  k_rows_team<K, NT><<<grid, NT, smem, s>>>(t, head, count, o);
   return cudaGetLastError();
 }
 
 template <int K>
 cudaError_t launch_rows_k(const DevGraph& g, const uint32_t* rows, OwnHeads* heads,
-                          unsigned long long* count, int num_sms, cudaStream_t s) {
+                          unsigned long long* count, int num_sms, cudaStream_t s, const GOut& o) {
   const unsigned long long* rn = g.rn;
   cudaError_t e = cudaSuccess;
   if (g.max_out > kRowsMid) {
-    const RowTasks t{g.dptr, g.roff, rows, g.rtask + 2 * g.nv - 1, rn + 3, 1, 0};
-    e = launch_team<K, K == 4 ? 256 : 512>(g, t, kRowsCap, &heads->wide, count, num_sms, s);
+    const RowTasks t{g.dptr, g.roff, rows, g.rtask + 2 * g.nv - 1, rn + 4, 1, 0};
+    e = launch_team<K, K == 4 ? 256 : 512>(g, t, kRowsCap, &heads->wide, count, num_sms, s, o);
   }
   if (e == cudaSuccess && g.max_out > 32) {
-    const RowTasks t{g.dptr, g.roff, rows, g.rtask + g.nv, rn + 2, 0, 0};
-    e = launch_team<K, 128>(g, t, kRowsMid, &heads->team, count, num_sms, s);
+    const RowTasks t{g.dptr, g.roff, rows, g.rtask + g.nv, rn + 3, 0, 0};
+    e = launch_team<K, 128>(g, t, kRowsMid, &heads->team, count, num_sms, s, o);
   }
-  if (e != cudaSuccess) return e;
-  RowTasks t{g.dptr, g.roff, rows, g.rtask, rn + 1, 0, 32};
-  int grid = 0;
-  e = full_grid(k_rows_word<K>, kWordThreads, 0, num_sms, &grid);
-  if (e != cudaSuccess) return e;
-  const int64_t roots = std::max<int64_t>(g.n_roots[1], 1);  // at most this many word tasks
-  grid = (int)std::min<int64_t>(grid, (4 * roots + kWordThreads - 1) / kWordThreads);
-  t.wcap = (int)std::max<int64_t>(1, std::min<int64_t>(32, roots / (kWordThreads / 8 * (int64_t)grid)));
-  k_rows_word<K><<<grid, kWordThreads, 0, s>>>(t, &heads->word, count);
-  return cudaGetLastError();
+  // the word and group kernels: at most `roots` tasks; claims small enough that every warp
+  // has a few
+  const int64_t roots = std::max<int64_t>(g.n_roots[1], 1);
+  auto narrow = [&](auto kernel, const int32_t* list, int down, const unsigned long long* n,
+                    unsigned long long* head, int per_warp) -> cudaError_t {
+    int grid = 0;
+    const cudaError_t r = full_grid(kernel, kWordThreads, 0, num_sms, &grid);
+    if (r != cudaSuccess) return r;
+    constexpr int kWarps = kWordThreads / 32;
+    grid = (int)std::min<int64_t>(grid, (roots + kWarps * per_warp - 1) / (kWarps * per_warp));
+    const int claim = (int)std::max<int64_t>(
+        per_warp, std::min<int64_t>(32, roots / (4 * kWarps * (int64_t)grid)));
+    const RowTasks t{g.dptr, g.roff, rows, list, n, down, claim};
+    kernel<<<grid, kWordThreads, 0, s>>>(t, head, count, o);
+    return cudaGetLastError();
+  };
+  if (e == cudaSuccess && g.max_out > 8)
+    e = narrow(k_rows_word<K>, g.rtask + g.nv - 1, 1, rn + 2, &heads->word, 1);
+  if (e == cudaSuccess) e = narrow(k_rows_group<K>, g.rtask, 0, rn + 1, &heads->group, 4);
+  return e;
 }
 
 }  // namespace
@@ -1203,6 +1275,15 @@ cudaError_t launch_rows_k(const DevGraph& g, const uint32_t* rows, OwnHeads* hea
 cudaError_t launch_owner_count(const DevGraph& g, OwnHeads* heads, unsigned long long* count,
                                int num_sms, cudaStream_t s) {
   return launch_owner<kOwnCount>(g, OwnArgs{}, heads, count, num_sms, s);
+}
+
+cudaError_t launch_owner_multi(const DevGraph& g, uint32_t* rows, unsigned* epart,
+                               OwnHeads* heads, int num_sms, cudaStream_t s) {
+  OwnArgs a{};
+  a.roff = g.roff;
+  a.rows = rows;
+  a.epart = epart;
+  return launch_owner<kOwnMulti>(g, a, heads, nullptr, num_sms, s);
 }
 
 cudaError_t launch_owner_part(const DevGraph& g, OwnHeads* heads, unsigned* epart, int num_sms,
@@ -1219,8 +1300,8 @@ cudaError_t ensure_rows_index(const DevGraph& g, cudaStream_t s) {
   unsigned long long* rn = nullptr;
   cudaError_t e = cudaMallocAsync((void**)&roff, sizeof(int64_t) * (size_t)g.nv, s);
   if (e == cudaSuccess) e = cudaMallocAsync((void**)&rtask, sizeof(int32_t) * 2 * (size_t)g.nv, s);
-  if (e == cudaSuccess) e = cudaMallocAsync((void**)&rn, sizeof(*rn) * 4, s);
-  if (e == cudaSuccess) e = cudaMemsetAsync(rn, 0, sizeof(*rn) * 4, s);
+  if (e == cudaSuccess) e = cudaMallocAsync((void**)&rn, sizeof(*rn) * 5, s);
+  if (e == cudaSuccess) e = cudaMemsetAsync(rn, 0, sizeof(*rn) * 5, s);
   if (e == cudaSuccess) {
     const int64_t blocks = std::min<int64_t>((g.nv + 255) / 256, 65536);
     k_rows_index<<<(unsigned)blocks, 256, 0, s>>>(g.dptr, g.nv, roff, rtask, rtask + g.nv, rn);
@@ -1247,13 +1328,14 @@ cudaError_t launch_owner_rows(const DevGraph& g, uint32_t* rows, OwnHeads* heads
 }
 
 cudaError_t launch_rows_count(int k, const DevGraph& g, const uint32_t* rows, OwnHeads* heads,
-                              unsigned long long* count, int num_sms, cudaStream_t s) {
+                              unsigned long long* count, int num_sms, cudaStream_t s,
+                              const GOut& o) {
   if (g.nv == 0) return cudaSuccess;
   switch (k) {
-    case 4: return launch_rows_k<4>(g, rows, heads, count, num_sms, s);
-    case 5: return launch_rows_k<5>(g, rows, heads, count, num_sms, s);
-    case 6: return launch_rows_k<6>(g, rows, heads, count, num_sms, s);
-    case 7: return launch_rows_k<7>(g, rows, heads, count, num_sms, s);
+    case 4: return launch_rows_k<4>(g, rows, heads, count, num_sms, s, o);
+    case 5: return launch_rows_k<5>(g, rows, heads, count, num_sms, s, o);
+    case 6: return launch_rows_k<6>(g, rows, heads, count, num_sms, s, o);
+    case 7: return launch_rows_k<7>(g, rows, heads, count, num_sms, s, o);
     default: return cudaErrorInvalidValue;
   }
 }

@@ -12,18 +12,21 @@ namespace xgm {
 constexpr int kBigDeg = 64;
 constexpr int64_t kOwnBits = int64_t(1) << 18;
 
+// Row store up to 16 GB (R-MAT scale 22: 0.6 GB); larger graphs, and a device without that
+// much memory left, count with the task kernel.
+constexpr int64_t kRowStoreMax = int64_t(1) << 32;  // words
 constexpr int kRowsCap = 1024;  // largest out-degree whose rows are stored
 constexpr int kRowsMid = 512;   // largest one of the four-warp tasks
 
 // Row store words of a task of out-degree s (the triangular bitmap, rounded to 16 bytes).
 __host__ __device__ __forceinline__ unsigned row_words(int64_t s) {
-  return s < 3 || s > kRowsCap ? 0u : ((unsigned)tri_words((int)s) + 3u) & ~3u;
+  return s < 2 || s > kRowsCap ? 0u : ((unsigned)tri_words((int)s) + 3u) & ~3u;
 }
 
 // Queue heads of one call (zeroed before it).
 struct OwnHeads {
   unsigned long long big, small;        // owner kernel: units, vertices
-  unsigned long long wide, team, word;  // row tasks by width
+  unsigned long long wide, team, word, group;  // row tasks by width
 };
 
 // Adds the triangle count of g to *count.
@@ -38,7 +41,7 @@ cudaError_t launch_owner_part(const DevGraph& g, OwnHeads* heads, unsigned* epar
 
 // Clique counts from stored rows.  Row i of vertex v's local DAG (the DAG induced on N+(v))
 // holds bit j iff N+(v)[j] is an out-neighbour of N+(v)[i]; the rows of a vertex of
-// out-degree 3 .. kRowsCap are kept in the triangular layout (tri_row_off) at word roff[v]
+// out-degree 2 .. kRowsCap are kept in the triangular layout (tri_row_off) at word roff[v]
 // of the row store, DevGraph::row_store_words words in all.
 //  ensure_rows_index: offsets and task lists by row width, once per graph.
 //  launch_owner_rows: fills the row store.
@@ -46,7 +49,12 @@ cudaError_t launch_owner_part(const DevGraph& g, OwnHeads* heads, unsigned* epar
 cudaError_t ensure_rows_index(const DevGraph& g, cudaStream_t s);
 cudaError_t launch_owner_rows(const DevGraph& g, uint32_t* rows, OwnHeads* heads, int num_sms,
                               cudaStream_t s);
+//  launch_owner_multi: fills the row store and credits epart (launch_owner_part) in one pass.
+cudaError_t launch_owner_multi(const DevGraph& g, uint32_t* rows, unsigned* epart,
+                               OwnHeads* heads, int num_sms, cudaStream_t s);
+//  (o: per-graph totals of batched graphs instead)
 cudaError_t launch_rows_count(int k, const DevGraph& g, const uint32_t* rows, OwnHeads* heads,
-                              unsigned long long* count, int num_sms, cudaStream_t s);
+                              unsigned long long* count, int num_sms, cudaStream_t s,
+                              const GOut& o = GOut{});
 
 }  // namespace xgm
