@@ -597,132 +597,169 @@ __global__ void __launch_bounds__(256) k_rows_index(const longlong2* dptr, int64
 
 // ------------------------------------------------------------------ counting
 // A task's rows are the strict upper triangle of a 0/1 matrix A (row i: words i/32 .. W-1).
-// Its triangles are the sum over edges (j, l) of (A A^T)_jl, a contraction: 32 x 32 blocks
-// of A A^T on the tensor cores, fp8 (e4m3) operands and fp32 accumulators, masked by the
-// block of A itself.  An operand element is 2^-6 or 0, so a sum of n products is n 2^-12,
-// exact (n <= 1024).  The fragments come straight from the bit rows: the k index of an
-// m16n8k32 step may be permuted if both operands agree, and with thread t of a quad taking
-// bits 8 b + t and 8 b + t + 4 (b = 0..3) of a row's word, a fragment register is one shift
-// and one AND.
-// popc over row words issues 4.3 words per clock and SM partition (measured; FLO for the
-// walk over members costs as much), the e4m3 step 824 multiply-adds = 26 words' worth; the
-// 1-bit mma.sync is emulated on this chip (525 cycles a step against 5).  A tcgen05 tile
-// has 128 rows: most matrices here are 60 to 300 wide and triangular, so its doubled rate
-// would go into padding.
-__device__ __forceinline__ void mma_e4m3(float (&d)[4], uint32_t a0, uint32_t a1, uint32_t a2,
-                                         uint32_t a3, uint32_t b0, uint32_t b1) {
-  asm("mma.sync.aligned.m16n8k32.row.col.f32.e4m3.e4m3.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, "
-      "{%8,%9}, {%0,%1,%2,%3};"
-      : "+f"(d[0]), "+f"(d[1]), "+f"(d[2]), "+f"(d[3])
+// Its triangles are the sum over edges (j, l) of C_jl = (A A^T)_jl, a contraction: 32 x 32
+// blocks of C on the tensor cores, f16 operands and accumulators, masked by the block of A.
+//  - The operands come straight from the bit rows: the k index of a step may be permuted if
+//    both operands agree, so thread t of a quad takes the bits p, p + 16 of a row's word for
+//    p = t, t + 4, t + 8, t + 12.  A bit p <= 11 of a 16-bit half is an f16 power of two by
+//    itself, 2^(p-24), so j's fragments are the word ANDed with a mask; l's carry 2^(14-p).
+//    A product is 2^-10, and a sum of n <= 1024 of them is exact in f16.
+//  - The masked sum of a block is one more contraction: C's accumulator layout is the layout
+//    of a k x n operand (C^T), so the diagonal of mask x C^T gathers sum_l A_jl C_jl per row
+//    j in f32.  For that the columns of a block are taken in the order that puts l and
+//    l + 16 into one accumulator register, as the mask's bits lie.  Only the diagonals of
+//    two accumulators count; they are read once per matrix.
+// popc over row words issues 4.3 words per clock and SM partition (measured; FLO for a walk
+// over members costs as much), an f16 m16n8k16 7.5 words' worth in 8.5 clocks.  e4m3
+// m16n8k32 is converted to f16 on this chip (12 conversions, 2 f16 steps and 4 additions
+// each; R-MAT s20 5-clique 33.5 ms with it), the 1-bit form emulated (525 clocks), u8 65
+// clocks.  A tcgen05 tile has 128 rows: most matrices here are 60 to 300 wide and
+// triangular, and bits would have to be spread to bytes in shared memory first.
+__device__ __forceinline__ void mma_f16(uint32_t (&d)[2], uint32_t a0, uint32_t a1, uint32_t a2,
+                                        uint32_t a3, uint32_t b0, uint32_t b1) {
+  asm("mma.sync.aligned.m16n8k16.row.col.f16.f16.f16.f16 {%0,%1}, {%2,%3,%4,%5}, {%6,%7}, {%0,%1};"
+      : "+r"(d[0]), "+r"(d[1])
       : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
 }
-constexpr float kUnit = 4096.0f;  // 1 / (2^-6)^2
+// Rows 8 .. 15 of the left operand are zero.
+__device__ __forceinline__ void mma_f32(float (&d)[4], uint32_t a0, uint32_t a2, uint32_t b0,
+                                        uint32_t b1) {
+  asm("mma.sync.aligned.m16n8k16.row.col.f32.f16.f16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, "
+      "{%0,%1,%2,%3};"
+      : "+f"(d[0]), "+f"(d[1]), "+f"(d[2]), "+f"(d[3])
+      : "r"(a0), "r"(0u), "r"(a2), "r"(0u), "r"(b0), "r"(b1));
+}
+constexpr float kUnit = 17179869184.0f;  // 2^34: a mask bit is 2^-24, a common neighbour 2^-10
+constexpr uint32_t kPair = 0x00010001u;  // bits p, p + 16 of a word
 
 // First word of block q's rows; a row of the block spans W - q words.
 __device__ __forceinline__ int blk_off(int q, int W) { return 16 * q * (2 * W - q + 1); }
 
-// Fragment registers of the words w[r] of rows 8 r + lane / 4.
-__device__ __forceinline__ void frag(const uint32_t (&w)[4], int t, uint32_t (&lo)[4],
-                                     uint32_t (&hi)[4]) {
+// Row of a block that column c of its n-tile nt takes (+ 4 nt).
+__device__ __forceinline__ int col_row(int c) { return (c >> 1) + 16 * (c & 1); }
+
+// Fragments of j's words w[r] (rows 8 r + lane / 4) and of l's (rows 4 r + col_row(lane / 4)):
+// four registers per word, two per k step.
+__device__ __forceinline__ void frag_j(uint32_t w, int t, uint32_t (&f)[4]) {
+  f[0] = w & (kPair << t);
+  f[1] = w & (kPair << (t + 4));
+  f[2] = w & (kPair << (t + 8));
+  f[3] = (w >> 4) & (kPair << (t + 8));
+}
+__device__ __forceinline__ void frag_l(uint32_t w, int t, uint32_t (&f)[4]) {
+  // f16 2^(14 - p) is (29 - p) << 10; the last pair is at t + 12 but j's has weight t + 8
+  f[0] = ((w >> t) & kPair) * ((29u - t) << 10);
+  f[1] = ((w >> (t + 4)) & kPair) * ((25u - t) << 10);
+  f[2] = ((w >> (t + 8)) & kPair) * ((21u - t) << 10);
+  f[3] = ((w >> (t + 12)) & kPair) * ((21u - t) << 10);
+}
+
+// One step (32 k) of the first MT x 16 rows of a block.
+template <int MT>
+__device__ __forceinline__ void block_mma(uint32_t (&c)[2][4][2], const uint32_t (&a)[4],
+                                          const uint32_t (&b)[4], int t) {
+  uint32_t fa[4][4];
 #pragma unroll
-  for (int r = 0; r < 4; ++r) {
-    lo[r] = (w[r] << (3 - t)) & 0x08080808u;
-    hi[r] = (w[r] >> (t + 1)) & 0x08080808u;
+  for (int r = 0; r < 2 * MT; ++r) frag_j(a[r], t, fa[r]);
+#pragma unroll
+  for (int n = 0; n < 4; ++n) {
+    uint32_t fb[4];
+    frag_l(b[n], t, fb);
+#pragma unroll
+    for (int m = 0; m < MT; ++m) {
+      mma_f16(c[m][n], fa[2 * m][0], fa[2 * m + 1][0], fa[2 * m][1], fa[2 * m + 1][1], fb[0], fb[1]);
+      mma_f16(c[m][n], fa[2 * m][2], fa[2 * m + 1][2], fa[2 * m][3], fa[2 * m + 1][3], fb[2], fb[3]);
+    }
   }
 }
 
-// One step (32 k) of a 32 x 32 block, or of its first 16 MT rows and 8 NT columns.
-template <int MT, int NT>
-__device__ __forceinline__ void block_mma(float (&c)[2][4][4], const uint32_t (&al)[4],
-                                          const uint32_t (&ah)[4], const uint32_t (&bl)[4],
-                                          const uint32_t (&bh)[4]) {
+// Adds the masked sums of a block to the diagonal of d (mk[r]: the block's row 8 r + lane / 4).
+template <int MT>
+__device__ __forceinline__ void block_sum(float (&d)[4], const uint32_t (&c)[2][4][2],
+                                          const uint32_t (&mk)[4], int t) {
 #pragma unroll
-  for (int m = 0; m < MT; ++m)
+  for (int r = 0; r < 2 * MT; ++r) {
+    const uint32_t w = mk[r] >> t;
 #pragma unroll
-    for (int n = 0; n < NT; ++n)
-      mma_e4m3(c[m][n], al[2 * m], al[2 * m + 1], ah[2 * m], ah[2 * m + 1], bl[n], bh[n]);
-}
-
-// Sum of c over the set bits of the block of A (mk[r]: its row 8 r + lane / 4).
-template <int MT, int NT>
-__device__ __forceinline__ uint32_t block_sum(const float (&c)[2][4][4], const uint32_t (&mk)[4],
-                                              int t) {
-  float sum = 0.0f;
-#pragma unroll
-  for (int m = 0; m < MT; ++m) {
-    const uint32_t w0 = mk[2 * m] >> (2 * t), w1 = mk[2 * m + 1] >> (2 * t);
-#pragma unroll
-    for (int n = 0; n < NT; ++n)
-#pragma unroll
-      for (int e = 0; e < 2; ++e) {
-        if (w0 & (1u << (8 * n + e))) sum += c[m][n][e];
-        if (w1 & (1u << (8 * n + e))) sum += c[m][n][2 + e];
-      }
+    for (int h = 0; h < 2; ++h)
+      mma_f32(d, (w >> (8 * h)) & kPair, (w >> (8 * h + 4)) & kPair, c[r >> 1][2 * h][r & 1],
+              c[r >> 1][2 * h + 1][r & 1]);
   }
-  return (uint32_t)(sum * kUnit);  // <= 32 x 1024 per thread: exact
 }
 
-// Edges (j, l), j in block J, l in block L >= J: the sum of |R_j & R_l|, and with MASK (m: a
-// row's words, read from J on) of |R_j & R_l & m| over j, l in m.  This lane's part.  (Two
-// blocks of j sharing the fragments of l take 3 instead of 4 shifts and ANDs per step of the
-// tensor cores, but 168 registers instead of 128: a CTA fewer per SM, and no gain.)
+// The sums gathered in d, each diagonal element once (this lane's part), and d cleared.
+__device__ __forceinline__ uint32_t take_diag(float (&d)[4]) {
+  const int lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
+  const float v = (g >> 1) == t ? ((g & 1) ? d[1] : d[0]) : 0.0f;
+  d[0] = d[1] = d[2] = d[3] = 0.0f;
+  return (uint32_t)(v * kUnit);
+}
+
+// Edges (j, l), j in block J, l in block L >= J: adds |R_j & R_l|, and with MASK (m: a row's
+// words, read from J on) |R_j & R_l & m| over j, l in m, to the diagonal of d.
 template <bool MASK>
-__device__ __forceinline__ uint32_t tri_block(const uint32_t* M, int W, int J, int L,
-                                              const uint32_t* m) {
+__device__ __forceinline__ void tri_block(const uint32_t* M, int W, int J, int L,
+                                          const uint32_t* m, float (&d)[4]) {
   const int lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
   const int sa = W - J, sb = W - L;
   const uint32_t* A = M + blk_off(J, W) - J + g * sa;
-  const uint32_t* B = M + blk_off(L, W) - L + g * sb;
+  const uint32_t* B = M + blk_off(L, W) - L + col_row(g) * sb;
   uint32_t mk[4];
 #pragma unroll
   for (int r = 0; r < 4; ++r) {
     mk[r] = A[8 * r * sa + L];
     if (MASK) mk[r] = (m[J] >> (8 * r + g)) & 1u ? mk[r] & m[L] : 0u;
   }
-  if (!__any_sync(kFull, (mk[0] | mk[1] | mk[2] | mk[3]) != 0u)) return 0u;
-  float c[2][4][4] = {};
+  if (!__any_sync(kFull, (mk[0] | mk[1] | mk[2] | mk[3]) != 0u)) return;
+  uint32_t c[2][4][2] = {};
   for (int w = L; w < W; ++w) {
-    uint32_t a[4], b[4], al[4], ah[4], bl[4], bh[4];
+    uint32_t a[4], b[4];
 #pragma unroll
     for (int r = 0; r < 4; ++r) {
       a[r] = A[8 * r * sa + w];
       if (MASK) a[r] &= m[w];
-      b[r] = B[8 * r * sb + w];
+      b[r] = B[4 * r * sb + w];
     }
-    frag(a, t, al, ah);
-    frag(b, t, bl, bh);
-    block_mma<2, 4>(c, al, ah, bl, bh);
+    block_mma<2>(c, a, b, t);
   }
-  return block_sum<2, 4>(c, mk, t);
+  block_sum<2>(d, c, mk, t);
 }
 
 // Blocks of a matrix from block q on, dealt to nw warps (this one is wi), longest sums first.
 template <bool MASK>
 __device__ uint64_t tri_blocks(const uint32_t* M, int W, int q, const uint32_t* m, int wi, int nw) {
   uint64_t acc = 0;
+  float d[4] = {};
   int L = 0, J = wi;  // block (q + J, q + L), J <= L, in the order L, J
-  for (;;) {
+  for (int done = 0;;) {
     while (J > L) J -= ++L;
-    if (q + L >= W) return acc;
-    acc += tri_block<MASK>(M, W, q + J, q + L, m);
+    if (q + L >= W) return acc + take_diag(d);
+    tri_block<MASK>(M, W, q + J, q + L, m, d);
     J += nw;
+    // a block adds at most 4 rows x 32 x 1024 to an element: exact below 2^24
+    if (++done % 64 == 0) acc += take_diag(d);
   }
 }
 
 // Triangles of a matrix of at most 32 vertices, row i in lane i: the operands by shuffle.
 __device__ __forceinline__ uint32_t tri_word(uint32_t row, int n) {
   const int lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
-  uint32_t a[4], al[4], ah[4];
+  uint32_t a[4], b[4];
 #pragma unroll
-  for (int r = 0; r < 4; ++r) a[r] = __shfl_sync(kFull, row, 8 * r + g);
-  frag(a, t, al, ah);
-  float c[2][4][4] = {};
-  if (n <= 16) {
-    block_mma<1, 2>(c, al, ah, al, ah);
-    return block_sum<1, 2>(c, a, t);
+  for (int r = 0; r < 4; ++r) {
+    a[r] = __shfl_sync(kFull, row, 8 * r + g);
+    b[r] = __shfl_sync(kFull, row, 4 * r + col_row(g));
   }
-  block_mma<2, 4>(c, al, ah, al, ah);
-  return block_sum<2, 4>(c, a, t);
+  uint32_t c[2][4][2] = {};
+  float d[4] = {};
+  if (n <= 16) {
+    block_mma<1>(c, a, b, t);
+    block_sum<1>(d, c, a, t);
+  } else {
+    block_mma<2>(c, a, b, t);
+    block_sum<2>(d, c, a, t);
+  }
+  return take_diag(d);
 }
 
 // The matrix induced on a set of n <= 32 vertices (lane w holds word w of the set), row r in
@@ -980,7 +1017,7 @@ __device__ __forceinline__ void team_sync(int team) {  // barrier 0 is __syncthr
 
 // CTAs per SM the registers are cut for (K = 4: 8-warp CTAs, K >= 6 spills below 168).
 constexpr int team_ctas(int K, int NT) {
-  return NT == 128 ? (K >= 6 ? 3 : 4) : (K == 4 ? 2 : 1);
+  return NT == 128 ? (K == 5 ? 5 : (K == 4 ? 4 : 3)) : (K == 4 ? 2 : 1);
 }
 
 // Tasks of more than 32 out-neighbours, one CTA each: the (K - 1)-cliques of the task's
