@@ -291,8 +291,9 @@ class Context:
                          group_max=group_max, margin=margin, hub_max=hub_max)
         out = C.c_uint64()
         st = Stats()
+        # without statistics the call records no timing events
         _check(lib().xgm_count(self._h, graph._h, plan._h, C.byref(sp), C.byref(out),
-                               C.byref(st)), self)
+                               C.byref(st) if with_stats else None), self)
         return (int(out.value), st.as_dict()) if with_stats else int(out.value)
 
     def motif_count(self, graph: "Graph", k: int, policy: int = SCHED_HEURISTIC,
@@ -302,8 +303,8 @@ class Context:
         sp = self._sched(policy, variant, model)
         out = (C.c_uint64 * 6)()
         st = Stats()
-        _check(lib().xgm_motif_count(self._h, graph._h, k, C.byref(sp), out, 6, C.byref(st)),
-               self)
+        _check(lib().xgm_motif_count(self._h, graph._h, k, C.byref(sp), out, 6,
+                                     C.byref(st) if with_stats else None), self)
         res = [int(x) for x in out[: 2 if k == 3 else 6]]
         return (res, st.as_dict()) if with_stats else res
 
@@ -354,7 +355,8 @@ class Context:
         out = np.empty(batch.num_graphs * len(plans), dtype=np.uint64)
         st = Stats()
         _check(lib().xgm_count_batched(self._h, batch._h, C.cast(arr, C.c_void_p), len(plans),
-                                       C.byref(sp), _ptr(out), C.byref(st)), self)
+                                       C.byref(sp), _ptr(out),
+                                       C.byref(st) if with_stats else None), self)
         res = out.reshape(batch.num_graphs, len(plans))
         return (res, st.as_dict()) if with_stats else res
 

@@ -478,6 +478,7 @@ xgm_status xgm_count(xgm_ctx* ctx, const xgm_graph* g, const xgm_plan* plan, con
   xgm_stats st_local;
   xgm_stats& st = stats ? *stats : st_local;
   std::memset(&st, 0, sizeof(st));
+  ctx->timed = stats != nullptr;
   xgm_status r = plan->pattern == XGM_PATTERN_PROGRAM
                      ? count_program(ctx, g->g, plan->prog, out_count, st)
                      : count_plan(ctx, g->g, plan->pattern, plan->induced, sp, out_count, st);
@@ -497,6 +498,7 @@ xgm_status xgm_motif_count(xgm_ctx* ctx, const xgm_graph* g, int k, const xgm_sc
   xgm_stats st_local;
   xgm_stats& st = stats ? *stats : st_local;
   std::memset(&st, 0, sizeof(st));
+  ctx->timed = stats != nullptr;
   return finish_status(ctx, count_motifs(ctx, g->g, k, sched ? *sched : def, counts, st));
 }
 

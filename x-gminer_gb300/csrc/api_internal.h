@@ -36,6 +36,8 @@ struct xgm_ctx {
   xgm::Scalars* d_sc = nullptr;
   xgm::Scalars* h_sc = nullptr;  // pinned
   cudaEvent_t ev[4] = {nullptr, nullptr, nullptr, nullptr};
+  // the call wants its times (statistics asked for): three event records cost a call 12 us
+  bool timed = true;
   xgm::TaskBuf tb;
   // motif buffers (grown on demand)
   unsigned long long* vpart = nullptr;
@@ -69,6 +71,16 @@ struct xgm_plan {
 };
 
 namespace xgm {
+
+// Records timing event i of the call, and the time between two of them (0 when not asked for).
+inline cudaError_t ctx_mark(xgm_ctx* ctx, int i) {
+  return ctx->timed ? cudaEventRecord(ctx->ev[i], ctx->stream) : cudaSuccess;
+}
+inline float ctx_ms(xgm_ctx* ctx, int from, int to) {
+  float ms = 0;
+  if (ctx->timed) cudaEventElapsedTime(&ms, ctx->ev[from], ctx->ev[to]);
+  return ms;
+}
 
 xgm_status finish_status(xgm_ctx* ctx, xgm_status st);
 xgm_status check_device_flag(xgm_ctx* ctx, uint32_t flag);

@@ -320,7 +320,7 @@ xgm_status count_batched_impl(xgm_ctx* ctx, xgm_batch* b, const xgm_plan* const*
   r = batch_prepare(ctx, b, sl, P, sp);
   if (r != XGM_OK) return r;
   const bool use_graph = !(sp.flags & XGM_SCHED_NO_GRAPH);
-  XGM_CUDA_TRY(cudaEventRecord(ctx->ev[0], s));
+  XGM_CUDA_TRY(ctx_mark(ctx, 0));
   if (use_graph) {
     const std::string key = sched_key(sl, sp);
     cudaGraphExec_t exec = nullptr;
@@ -355,17 +355,16 @@ xgm_status count_batched_impl(xgm_ctx* ctx, xgm_batch* b, const xgm_plan* const*
       XGM_CUDA_TRY(e2);
       b->cache.push_back(CachedExec{key, exec, kern});
       st.launches = kern;
-      XGM_CUDA_TRY(cudaEventRecord(ctx->ev[0], s));
+      XGM_CUDA_TRY(ctx_mark(ctx, 0));
     }
     XGM_CUDA_TRY(cudaGraphLaunch(exec, s));
   } else {
     r = batch_sequence(ctx, b, sl, P, sp);
     if (r != XGM_OK) return r;
   }
-  XGM_CUDA_TRY(cudaEventRecord(ctx->ev[1], s));
+  XGM_CUDA_TRY(ctx_mark(ctx, 1));
   XGM_CUDA_TRY(cudaStreamSynchronize(s));
-  float ms = 0;
-  cudaEventElapsedTime(&ms, ctx->ev[0], ctx->ev[1]);
+  const float ms = ctx_ms(ctx, 0, 1);
   st.kernel_ms = ms;
   st.device_error = b->h_sc->err;
   st.tasks = b->graph.g.nv;
@@ -501,6 +500,7 @@ xgm_status xgm_count_batched(xgm_ctx* ctx, xgm_batch* b, const xgm_plan* const* 
   xgm_stats local;
   xgm_stats& st = stats ? *stats : local;
   std::memset(&st, 0, sizeof(st));
+  ctx->timed = stats != nullptr;
   return finish_status(ctx, count_batched_impl(ctx, b, plans, n_plans, sched ? *sched : def, out, st));
 }
 
@@ -526,6 +526,7 @@ xgm_status xgm_autotune(xgm_ctx* ctx, const xgm_graph* g, xgm_batch* b, const xg
     for (int i = 0; i < reps + 1; ++i) {
       xgm_stats st;
       std::memset(&st, 0, sizeof(st));
+      ctx->timed = true;
       xgm_status r = b ? count_batched_impl(ctx, b, plans, n_plans, sp, res.data(), st)
                        : count_dispatch(ctx, g->g, plans[0]->pattern, sp, res.data(), st);
       if (r != XGM_OK) return r;

@@ -172,9 +172,9 @@ xgm_status clique_route(xgm_ctx* ctx, const DevGraph& g, int k, const xgm_sched&
   return XGM_OK;
 }
 
-// Enqueues the schedule (before `mark`, when given) and the counting kernels.
+// Enqueues the schedule, timing event 1 and the counting kernels.
 xgm_status launch_route(xgm_ctx* ctx, const DevGraph& g, int k, const xgm_sched& sp,
-                        CliqueRoute route, cudaEvent_t mark, int* launches) {
+                        CliqueRoute route, int* launches) {
   cudaStream_t s = ctx->stream;
   Scalars* sc = ctx->d_sc;
   const bool hubs = route == CliqueRoute::kRows && g.max_out > kRowsCap;
@@ -185,7 +185,7 @@ xgm_status launch_route(xgm_ctx* ctx, const DevGraph& g, int k, const xgm_sched&
     XGM_CUDA_TRY(classify_heuristic(g, kRowsCap + 2, kWarpCap, kWideCap, kCtaCap, ctx->tb, s));
     XGM_CUDA_TRY(build_lists(g, ctx->tb, false, s, whole_hub_max(k, 0)));
   }
-  if (mark) XGM_CUDA_TRY(cudaEventRecord(mark, s));
+  XGM_CUDA_TRY(ctx_mark(ctx, 1));
   if (launches) *launches = 1;
   if (route == CliqueRoute::kOwner)
     XGM_CUDA_TRY(launch_owner_count(g, &sc->own, &sc->count, ctx->num_sms, s));
@@ -211,7 +211,7 @@ xgm_status launch_participation(xgm_ctx* ctx, const DevGraph& g, const xgm_sched
   XGM_CUDA_TRY(grow(&ctx->epart, &ctx->epart_cap, g.ne, s));
   XGM_CUDA_TRY(cudaMemsetAsync(ctx->epart, 0, sizeof(unsigned) * (g.ne > 0 ? g.ne : 1), s));
   if (!*tasks) {
-    XGM_CUDA_TRY(cudaEventRecord(ctx->ev[1], s));
+    XGM_CUDA_TRY(ctx_mark(ctx, 1));
     XGM_CUDA_TRY(launch_owner_part(g, &ctx->d_sc->own, ctx->epart, ctx->num_sms, s));
     return XGM_OK;
   }
@@ -220,7 +220,7 @@ xgm_status launch_participation(xgm_ctx* ctx, const DevGraph& g, const xgm_sched
   if (r != XGM_OK) return r;
   XGM_CUDA_TRY(grow(&ctx->vpart, &ctx->vpart_cap, g.nv, s));
   XGM_CUDA_TRY(cudaMemsetAsync(ctx->vpart, 0, sizeof(unsigned long long) * (g.nv > 0 ? g.nv : 1), s));
-  XGM_CUDA_TRY(cudaEventRecord(ctx->ev[1], s));
+  XGM_CUDA_TRY(ctx_mark(ctx, 1));
   XGM_CUDA_TRY(launch_triangle_participation(g.view(), ctx->tb.lists(false), &ctx->d_sc->q,
                                              ctx->vpart, ctx->epart, &ctx->d_sc->err,
                                              ensure_clique_grid(ctx), s));
@@ -247,12 +247,12 @@ xgm_status count_dispatch(xgm_ctx* ctx, const DevGraph& g, int pattern, const xg
     if (r != XGM_OK) return r;
   }
   XGM_CUDA_TRY(cudaMemsetAsync(ctx->d_sc, 0, sizeof(Scalars), s));
-  XGM_CUDA_TRY(cudaEventRecord(ctx->ev[0], s));
+  XGM_CUDA_TRY(ctx_mark(ctx, 0));
   const GView view = g.view();
   int launches = 0;
   bool tasks = k && route == CliqueRoute::kTasks;  // the task kernel ran
   if (k) {
-    xgm_status r = launch_route(ctx, g, k, sp, route, ctx->ev[1], &launches);
+    xgm_status r = launch_route(ctx, g, k, sp, route, &launches);
     if (r != XGM_OK) return r;
   } else if (pattern == XGM_PATTERN_DIAMOND || pattern == XGM_PATTERN_TAILED_TRIANGLE) {
     xgm_status r = launch_participation(ctx, g, sp, &tasks);
@@ -264,7 +264,7 @@ xgm_status count_dispatch(xgm_ctx* ctx, const DevGraph& g, int pattern, const xg
     launches = 2;
   } else if (pattern == XGM_PATTERN_CYCLE4) {
     XGM_CUDA_TRY(grow(&ctx->c4_lists, &ctx->c4_lists_cap, 3 * g.nv, s));
-    XGM_CUDA_TRY(cudaEventRecord(ctx->ev[1], s));
+    XGM_CUDA_TRY(ctx_mark(ctx, 1));
     const C4Lists lists{ctx->c4_lists, ctx->c4_lists + g.nv, ctx->c4_lists + 2 * g.nv};
     XGM_CUDA_TRY(launch_cycle4(g, &ctx->d_sc->c4, lists, &ctx->d_sc->count, ctx->num_sms, s));
     launches = 1;
@@ -272,15 +272,13 @@ xgm_status count_dispatch(xgm_ctx* ctx, const DevGraph& g, int pattern, const xg
     set_thread_error("unknown pattern");
     return XGM_ERR_INVALID;
   }
-  XGM_CUDA_TRY(cudaEventRecord(ctx->ev[2], s));
+  XGM_CUDA_TRY(ctx_mark(ctx, 2));
   if (tasks)
     XGM_CUDA_TRY(cudaMemcpyAsync(ctx->d_sc->n, ctx->tb.n, sizeof(int64_t) * 8,
                                  cudaMemcpyDeviceToDevice, s));
   xgm_status r = ctx_sync_scalars(ctx);
   if (r != XGM_OK) return r;
-  float prep = 0, kern = 0;
-  cudaEventElapsedTime(&prep, ctx->ev[0], ctx->ev[1]);
-  cudaEventElapsedTime(&kern, ctx->ev[1], ctx->ev[2]);
+  const float prep = ctx_ms(ctx, 0, 1), kern = ctx_ms(ctx, 1, 2);
   st.prep_ms = prep;
   st.kernel_ms = kern;
   st.device_error = ctx->h_sc->err;
@@ -320,7 +318,8 @@ xgm_status count_kernels(xgm_ctx* ctx, const DevGraph& g, int pattern, const xgm
   ensure_clique_grid(ctx);
   XGM_CUDA_TRY(cudaStreamSynchronize(s));
   XGM_CUDA_TRY(cudaStreamBeginCapture(s, cudaStreamCaptureModeThreadLocal));
-  r = launch_route(ctx, g, k, sp, route, nullptr, nullptr);
+  ctx->timed = false;
+  r = launch_route(ctx, g, k, sp, route, nullptr);
   cudaGraph_t graph = nullptr;
   cudaError_t e2 = cudaStreamEndCapture(s, &graph);
   if (r != XGM_OK) {
@@ -403,25 +402,23 @@ xgm_status motif_terms(xgm_ctx* ctx, const DevGraph& g, const xgm_sched& sp, boo
   cudaStream_t s = ctx->stream;
   XGM_CUDA_TRY(cudaSetDevice(ctx->device));
   XGM_CUDA_TRY(cudaMemsetAsync(ctx->d_sc, 0, sizeof(Scalars), s));
-  XGM_CUDA_TRY(cudaEventRecord(ctx->ev[0], s));
+  XGM_CUDA_TRY(ctx_mark(ctx, 0));
   const GView view = g.view();
   bool tasks = false;  // the task kernel ran
   if (part) {
     xgm_status r = launch_participation(ctx, g, sp, &tasks);
     if (r != XGM_OK) return r;
   } else {
-    XGM_CUDA_TRY(cudaEventRecord(ctx->ev[1], s));
+    XGM_CUDA_TRY(ctx_mark(ctx, 1));
   }
   XGM_CUDA_TRY(launch_motif_terms(view, part ? ctx->epart : nullptr, ctx->d_sc->terms, s));
-  XGM_CUDA_TRY(cudaEventRecord(ctx->ev[2], s));
+  XGM_CUDA_TRY(ctx_mark(ctx, 2));
   if (tasks)
     XGM_CUDA_TRY(cudaMemcpyAsync(ctx->d_sc->n, ctx->tb.n, sizeof(int64_t) * 8,
                                  cudaMemcpyDeviceToDevice, s));
   xgm_status r = ctx_sync_scalars(ctx);
   if (r != XGM_OK) return r;
-  float prep = 0, kern = 0;
-  cudaEventElapsedTime(&prep, ctx->ev[0], ctx->ev[1]);
-  cudaEventElapsedTime(&kern, ctx->ev[1], ctx->ev[2]);
+  const float prep = ctx_ms(ctx, 0, 1), kern = ctx_ms(ctx, 1, 2);
   std::memset(&st, 0, sizeof(st));
   st.prep_ms = prep;
   st.kernel_ms = kern;
@@ -465,6 +462,44 @@ struct Motif4Parts {
 xgm_status motif4_parts(xgm_ctx* ctx, const DevGraph& g, const xgm_sched& sp, bool need_c4,
                         Motif4Parts& m, xgm_stats& st) {
   xgm_stats x;
+  // open schedules, every vertex within the row capacity: rows and triangles per edge from
+  // one owner pass, all parts behind one read-back
+  CliqueRoute route = CliqueRoute::kTasks;
+  if (sched_is_open(sp) && g.max_out <= kRowsCap) {
+    XGM_CUDA_TRY(cudaSetDevice(ctx->device));
+    xgm_status q = clique_route(ctx, g, 4, sp, &route);
+    if (q != XGM_OK) return q;
+  }
+  if (route == CliqueRoute::kRows) {
+    cudaStream_t s = ctx->stream;
+    Scalars* sc = ctx->d_sc;
+    XGM_CUDA_TRY(grow(&ctx->epart, &ctx->epart_cap, g.ne, s));
+    if (need_c4) XGM_CUDA_TRY(grow(&ctx->c4_lists, &ctx->c4_lists_cap, 3 * g.nv, s));
+    XGM_CUDA_TRY(cudaMemsetAsync(sc, 0, sizeof(Scalars), s));
+    XGM_CUDA_TRY(ctx_mark(ctx, 0));
+    XGM_CUDA_TRY(cudaMemsetAsync(ctx->epart, 0, sizeof(unsigned) * (g.ne > 0 ? g.ne : 1), s));
+    XGM_CUDA_TRY(ctx_mark(ctx, 1));
+    XGM_CUDA_TRY(launch_owner_multi(g, ctx->rows, ctx->epart, &sc->own, ctx->num_sms, s));
+    XGM_CUDA_TRY(launch_rows_count(4, g, ctx->rows, &sc->own, &sc->count, ctx->num_sms, s));
+    XGM_CUDA_TRY(launch_motif_terms(g.view(), ctx->epart, sc->terms, s));
+    if (need_c4) {
+      const C4Lists lists{ctx->c4_lists, ctx->c4_lists + g.nv, ctx->c4_lists + 2 * g.nv};
+      XGM_CUDA_TRY(launch_cycle4(g, &sc->c4, lists, &sc->aux, ctx->num_sms, s));
+    }
+    XGM_CUDA_TRY(ctx_mark(ctx, 2));
+    xgm_status q = ctx_sync_scalars(ctx);
+    if (q != XGM_OK) return q;
+    st.prep_ms = ctx_ms(ctx, 0, 1);
+    st.kernel_ms = ctx_ms(ctx, 1, 2);
+    st.launches = need_c4 ? 4 : 3;
+    st.tasks = g.n_roots[0] + g.n_roots[1];
+    st.device_error = ctx->h_sc->err;
+    for (int i = 0; i < 6; ++i) m.t[i] = ctx->h_sc->terms[i];
+    m.t[3] = tailed_from_terms(ctx->h_sc->terms);
+    m.k4 = ctx->h_sc->count;
+    m.c4e = ctx->h_sc->aux;
+    return check_device_flag(ctx, ctx->h_sc->err);
+  }
   xgm_status r = motif_terms(ctx, g, sp, true, m.t, x);
   if (r != XGM_OK) return r;
   add_stats(st, x);
@@ -519,6 +554,26 @@ xgm_status count_motifs(xgm_ctx* ctx, const DevGraph& g, int k, const xgm_sched&
   if (k == 3) {
     uint64_t t[6], tri = 0;
     xgm_stats x;
+    if (sched_is_open(sp)) {  // both parts behind one read-back
+      cudaStream_t s = ctx->stream;
+      Scalars* sc = ctx->d_sc;
+      XGM_CUDA_TRY(cudaSetDevice(ctx->device));
+      XGM_CUDA_TRY(cudaMemsetAsync(sc, 0, sizeof(Scalars), s));
+      XGM_CUDA_TRY(ctx_mark(ctx, 0));
+      XGM_CUDA_TRY(ctx_mark(ctx, 1));
+      XGM_CUDA_TRY(launch_motif_terms(g.view(), nullptr, sc->terms, s));
+      XGM_CUDA_TRY(launch_owner_count(g, &sc->own, &sc->count, ctx->num_sms, s));
+      XGM_CUDA_TRY(ctx_mark(ctx, 2));
+      xgm_status q = ctx_sync_scalars(ctx);
+      if (q != XGM_OK) return q;
+      st.prep_ms = ctx_ms(ctx, 0, 1);
+      st.kernel_ms = ctx_ms(ctx, 1, 2);
+      st.launches = 2;
+      st.tasks = g.n_roots[0];
+      out[1] = ctx->h_sc->count;
+      out[0] = ctx->h_sc->terms[0] - 3 * out[1];
+      return XGM_OK;
+    }
     xgm_status r = motif_terms(ctx, g, sp, false, t, x);
     if (r != XGM_OK) return r;
     add_stats(st, x);

@@ -30,8 +30,8 @@
 // Measured (GB300, a call before -> now):
 //  triangles  R-MAT s20 ef16 8.45 -> 1.48 ms; Barabasi-Albert, 3,312 vertices, 106 -> 28 us
 //             (13 launches -> 1: no task lists)
-//  4-cliques  R-MAT s22 65.6 -> 23.0 ms (rows 12.3, counting 10.9); s20 12.4 -> 3.6 ms
-//  5-cliques  R-MAT s20 140 -> 33.5 ms; 6-cliques R-MAT s16 96 -> 18.5 ms
+//  4-cliques  R-MAT s22 65.6 -> 22.1 ms (rows 11.9, counting 9.6); s20 12.4 -> 3.5 ms
+//  5-cliques  R-MAT s20 140 -> 29 ms; 6-cliques R-MAT s16 96 -> 10.6 ms
 //  triangles per edge (diamonds), Chung-Lu 1.5 M vertices, degree 32: 9.9 -> 3.5 ms; R-MAT
 //             s19 3.76 -> 1.47 ms (the hits' rank look-ups and counters: the bare count of
 //             the same suffixes is 2.5 times faster)
@@ -39,7 +39,8 @@
 // The tests with a warp per suffix, a ballot per 32 elements: 1.86 ms (s20 triangles), 15.2
 // ms (s22 rows): 145 instructions a pair, of which a third for the pair itself.
 // Bound: R-MAT s22 rows, L2 and DRAM latency (2.2 G sectors, 12 GB of DRAM reads: the lists
-// exceed L2) and instruction issue; counting, the ALU pipe (half rate: shifts, ANDs).
+// exceed L2) and instruction issue; counting, the tensor pipe (8.5 clocks a step: 9 of the
+// 29 ms of the s20 5-clique) and the shifts and ANDs that feed it at 16 warps per SM.
 #include <algorithm>
 #include <atomic>
 #include <type_traits>
@@ -654,19 +655,18 @@ __device__ __forceinline__ void frag_l(uint32_t w, int t, uint32_t (&f)[4]) {
   f[3] = ((w >> (t + 12)) & kPair) * ((21u - t) << 10);
 }
 
-// One step (32 k) of the first MT x 16 rows of a block.
-template <int MT>
+// One step (32 k) of a block.
 __device__ __forceinline__ void block_mma(uint32_t (&c)[2][4][2], const uint32_t (&a)[4],
                                           const uint32_t (&b)[4], int t) {
   uint32_t fa[4][4];
 #pragma unroll
-  for (int r = 0; r < 2 * MT; ++r) frag_j(a[r], t, fa[r]);
+  for (int r = 0; r < 4; ++r) frag_j(a[r], t, fa[r]);
 #pragma unroll
   for (int n = 0; n < 4; ++n) {
     uint32_t fb[4];
     frag_l(b[n], t, fb);
 #pragma unroll
-    for (int m = 0; m < MT; ++m) {
+    for (int m = 0; m < 2; ++m) {
       mma_f16(c[m][n], fa[2 * m][0], fa[2 * m + 1][0], fa[2 * m][1], fa[2 * m + 1][1], fb[0], fb[1]);
       mma_f16(c[m][n], fa[2 * m][2], fa[2 * m + 1][2], fa[2 * m][3], fa[2 * m + 1][3], fb[2], fb[3]);
     }
@@ -674,11 +674,10 @@ __device__ __forceinline__ void block_mma(uint32_t (&c)[2][4][2], const uint32_t
 }
 
 // Adds the masked sums of a block to the diagonal of d (mk[r]: the block's row 8 r + lane / 4).
-template <int MT>
 __device__ __forceinline__ void block_sum(float (&d)[4], const uint32_t (&c)[2][4][2],
                                           const uint32_t (&mk)[4], int t) {
 #pragma unroll
-  for (int r = 0; r < 2 * MT; ++r) {
+  for (int r = 0; r < 4; ++r) {
     const uint32_t w = mk[r] >> t;
 #pragma unroll
     for (int h = 0; h < 2; ++h)
@@ -720,9 +719,9 @@ __device__ __forceinline__ void tri_block(const uint32_t* M, int W, int J, int L
       if (MASK) a[r] &= m[w];
       b[r] = B[4 * r * sb + w];
     }
-    block_mma<2>(c, a, b, t);
+    block_mma(c, a, b, t);
   }
-  block_sum<2>(d, c, mk, t);
+  block_sum(d, c, mk, t);
 }
 
 // Blocks of a matrix from block q on, dealt to nw warps (this one is wi), longest sums first.
@@ -741,8 +740,22 @@ __device__ uint64_t tri_blocks(const uint32_t* M, int W, int q, const uint32_t* 
   }
 }
 
-// Triangles of a matrix of at most 32 vertices, row i in lane i: the operands by shuffle.
+// Triangles of a matrix of at most 32 vertices, row i in lane i.  Up to kPopcN vertices row by
+// row (8 clocks of popc each), above that one block, its operands by shuffle (24 steps of 8.5
+// clocks and as many again of fragments).
+constexpr int kPopcN = 16;
 __device__ __forceinline__ uint32_t tri_word(uint32_t row, int n) {
+  if (n <= kPopcN) {
+    uint32_t c = 0;
+    for (int j = 1; j < n - 1; j += 4) {  // (rows from n on are empty)
+#pragma unroll
+      for (int h = 0; h < 4; ++h) {
+        const uint32_t r = __shfl_sync(kFull, row, j + h);
+        if ((row >> (j + h)) & 1u) c += __popc(row & r);
+      }
+    }
+    return c;
+  }
   const int lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
   uint32_t a[4], b[4];
 #pragma unroll
@@ -752,13 +765,8 @@ __device__ __forceinline__ uint32_t tri_word(uint32_t row, int n) {
   }
   uint32_t c[2][4][2] = {};
   float d[4] = {};
-  if (n <= 16) {
-    block_mma<1>(c, a, b, t);
-    block_sum<1>(d, c, a, t);
-  } else {
-    block_mma<2>(c, a, b, t);
-    block_sum<2>(d, c, a, t);
-  }
+  block_mma(c, a, b, t);
+  block_sum(d, c, a, t);
   return take_diag(d);
 }
 
@@ -803,12 +811,16 @@ struct PickWord {
 };
 static_assert(sizeof(PickWord) == 32, "read as two uint4");
 
-// Prepares the members of row i: the picks (one warp of the team) and the ids (idx, by nw
-// warps).  Returns |R_i|.
-__device__ int row_members(const uint32_t* M, int W, int i, uint16_t* idx, PickWord* pick, int wi,
-                           int nw) {
+// Word `lane` of row i of a matrix (0 outside the row).
+__device__ __forceinline__ uint32_t row_word(const uint32_t* M, int W, int i) {
   const int lane = threadIdx.x & 31, q = i >> 5;
-  const uint32_t word = lane >= q && lane < W ? M[tri_row_off(i, W) + lane - q] : 0u;
+  return lane >= q && lane < W ? M[tri_row_off(i, W) + lane - q] : 0u;
+}
+
+// Prepares the members of a set of rows (lane w: word w of it): the picks (one warp of the
+// team) and the ids (idx, by nw warps).  Returns their number.
+__device__ int set_members(int W, uint32_t word, uint16_t* idx, PickWord* pick, int wi, int nw) {
+  const int lane = threadIdx.x & 31;
   const int cnt = __popc(word);
   int inc = cnt;
 #pragma unroll
@@ -835,7 +847,7 @@ __device__ int row_members(const uint32_t* M, int W, int i, uint16_t* idx, PickW
     }
     pick[lane] = p;
   }
-  for (int w = q + wi; w < W; w += nw) {
+  for (int w = wi; w < W; w += nw) {
     const uint32_t x = __shfl_sync(kFull, word, w);
     const int e = __shfl_sync(kFull, inc - cnt, w);
     if ((x >> lane) & 1u) idx[e + __popc(x & lanemask_lt())] = (uint16_t)(32 * w + lane);
@@ -921,12 +933,32 @@ __device__ __forceinline__ uint64_t set_cliques(const uint32_t* M, int W, uint32
   }
 }
 
-// D-cliques (D = 3, 4, 5) of the matrix C of n vertices, by nw warps; ids / tmp as above.
-// D = 4: for each row j the triangles inside it; D = 5: for each edge (j, l) the triangles
-// inside R_j & R_l; sets of up to 32 as a matrix of their own, longer ones as a mask.
+constexpr int kOwnN = 128;             // longest row one warp takes by itself
+constexpr int kOwnWords = 16 * 4 * 5;  // its matrix
+
+// Scratch of a warp: the matrix induced on a row of up to kOwnN members and what building it
+// takes, 32 words of masks, ids of a small set; K >= 6: the same for a row of that matrix.
+struct InduceScratch {
+  PickWord pick[32];
+  uint32_t mat[kOwnWords];
+  uint16_t idx[kOwnN];
+};
+template <int LEVELS>
+struct WarpScratch {
+  InduceScratch level[LEVELS];
+  uint32_t tmp[32];
+  uint16_t ids[32];
+};
+static_assert(sizeof(WarpScratch<1>) % 32 == 0 && sizeof(WarpScratch<2>) % 32 == 0,
+              "picks are read 16 bytes at a time");
+
+// D-cliques (D = 3, 4, 5) of the matrix C of n vertices, by nw warps.  D = 4: for each row j
+// the triangles inside it: of up to 32 members as a matrix in registers, of up to kOwnN as
+// one in `in` (null: none), else as a mask over C.  D = 5: for each row j the 4-cliques
+// inside it, or for each edge (j, l) the triangles inside R_j & R_l.
 template <int D>
-__device__ uint64_t matrix_cliques(const uint32_t* C, int n, int wi, int nw, uint16_t* ids,
-                                   uint32_t* tmp) {
+__device__ uint64_t matrix_cliques(const uint32_t* C, int n, int wi, int nw, InduceScratch* in,
+                                   uint16_t* ids, uint32_t* tmp) {
   const int lane = threadIdx.x & 31, W = (n + 31) >> 5;
   if constexpr (D == 3) {
     return tri_blocks<false>(C, W, 0, nullptr, wi, nw);
@@ -934,21 +966,26 @@ __device__ uint64_t matrix_cliques(const uint32_t* C, int n, int wi, int nw, uin
     uint64_t acc = 0;
     for (int j = wi; j + D - 1 < n; j += nw) {
       const int q = j >> 5;
-      const uint32_t* row = C + tri_row_off(j, W) - q;  // word w of row j (w >= q)
-      const uint32_t word = lane >= q && lane < W ? row[lane] : 0u;
+      const uint32_t word = row_word(C, W, j);
       const int nj = (int)__reduce_add_sync(kFull, (unsigned)__popc(word));
       if (nj < D - 1) continue;
       if (nj <= 32) {
         acc += set_cliques<D - 1>(C, W, word, nj, ids, tmp);
+      } else if (in && nj <= kOwnN) {
+        set_members(W, word, in->idx, in->pick, 0, 1);
+        __syncwarp();
+        compress(C, W, in->idx, in->pick, nj, in->mat, 0, 1);
+        __syncwarp();
+        acc += matrix_cliques<D - 1>(in->mat, nj, 0, 1, nullptr, ids, tmp);
+        __syncwarp();
       } else if constexpr (D == 4) {
-        acc += tri_blocks<true>(C, W, q, row, 0, 1);
+        acc += tri_blocks<true>(C, W, q, C + tri_row_off(j, W) - q, 0, 1);
       } else {
         for (unsigned nz = __ballot_sync(kFull, word != 0u); nz; nz &= nz - 1) {
           const int ql = __ffs(nz) - 1;
           for (uint32_t bits = __shfl_sync(kFull, word, ql); bits; bits &= bits - 1) {
             const int l = 32 * ql + __ffs(bits) - 1;
-            const uint32_t m2 =
-                lane >= ql && lane < W ? word & C[tri_row_off(l, W) - ql + lane] : 0u;
+            const uint32_t m2 = word & row_word(C, W, l);
             const int nl = (int)__reduce_add_sync(kFull, (unsigned)__popc(m2));
             if (nl < 3) continue;
             if (nl <= 32) {
@@ -990,12 +1027,11 @@ struct RowTasks {
              // per claim, at most 32)
 };
 
-constexpr int kOwnN = 128;                // longest row one warp takes by itself
-constexpr int kOwnWords = 16 * 4 * 5;     // its matrix
 constexpr int kTeam = 4;                  // warps of a team
 constexpr int kTeamN = 512;               // longest row a team takes
-// Scratch of a warp, in words: picks, matrix, 32 words of masks, ids, ids of a small set.
-constexpr int kWarpScratch = 8 * 32 + kOwnWords + 32 + kOwnN / 2 + 16;
+// (the 16-warp CTAs of wide tasks have no room for a second level: masks)
+template <int K, int WARPS>
+using TaskScratch = WarpScratch<(K >= 6 && WARPS == kTeam ? 2 : 1)>;
 
 // Words of shared memory of a CTA of row tasks: the task's matrix; K >= 5: per team a
 // matrix and ids for rows up to kTeamN (together one for the longest row) and picks, the
@@ -1004,15 +1040,22 @@ __host__ __device__ constexpr int matrix_words(int W) { return 16 * W * (W + 1);
 __host__ __device__ constexpr int team_matrix_words(int W) {
   return matrix_words(W < kTeamN / 32 ? W : kTeamN / 32);
 }
-template <int K>
-constexpr int team_words(int W, int warps) {
+template <int K, int WARPS>
+constexpr int team_words(int W) {
   return K == 4 ? matrix_words(W)
-                : matrix_words(W) + warps / kTeam * (team_matrix_words(W) + 8 * 32 + kTeamN / 2) +
-                      16 * W + warps * kWarpScratch;
+                : matrix_words(W) + WARPS / kTeam * (team_matrix_words(W) + 8 * 32 + kTeamN / 2) +
+                      16 * W + WARPS * (int)sizeof(TaskScratch<K, WARPS>) / 4;
 }
 
 __device__ __forceinline__ void team_sync(int team) {  // barrier 0 is __syncthreads
   asm volatile("bar.sync %0, %1;" ::"r"(team + 1), "r"(32 * kTeam) : "memory");
+}
+
+// Parts a task's rows are dealt to (k >= 5): a task of 256 members takes one CTA milliseconds
+// at k = 6, and a graph has few of the largest.  R-MAT s16 6-clique 16.8 / 9.9 / 10.2 ms with
+// 1 / 4 / 8 parts, the 16-warp tasks of the s20 5-clique 7.4 / 5.9 / 6.2 ms with 1 / 4 / 8.
+constexpr int team_parts(int K, int NT) {
+  return K == 4 ? 1 : (K == 5 ? (NT == 128 ? 2 : 4) : (K == 6 ? 4 : 8));
 }
 
 // CTAs per SM the registers are cut for (K = 4: 8-warp CTAs, K >= 6 spills below 168).
@@ -1031,14 +1074,18 @@ __global__ void __launch_bounds__(NT, team_ctas(K, NT)) k_rows_team(RowTasks t, 
   __shared__ int next_i, n_long, next_long, n_huge, team_x[NT / 32 / kTeam];
   constexpr int kWarps = NT / 32, kTeams = kWarps / kTeam;
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  constexpr int kParts = team_parts(K, NT);
   const long long nt = (long long)*t.n;
   uint64_t total = 0;
   if (tid == 0) task_s = (long long)atomicAdd(head, 1ull);
   __syncthreads();
   for (;;) {
     const long long ti = task_s;
-    if (ti >= nt) break;
-    const int32_t v = t.down ? t.list[-ti] : t.list[ti];
+    if (ti >= nt * kParts) break;
+    // from the list's end: its start holds the low ranks, the smallest tasks
+    const long long at = nt - 1 - ti / kParts;
+    const int part = (int)(ti % kParts);  // of the task's rows: part, part + kParts, ..
+    const int32_t v = t.down ? t.list[-at] : t.list[at];
     uint64_t acc = 0;
     const longlong2 d = ldg_ll2(t.dptr + v);
     const int s = (int)(d.y - d.x), W = (s + 31) >> 5;
@@ -1064,23 +1111,21 @@ __global__ void __launch_bounds__(NT, team_ctas(K, NT)) k_rows_team(RowTasks t, 
       uint16_t* idxs = reinterpret_cast<uint16_t*>(picks + kTeams * 32);
       uint16_t* longs = idxs + kTeams * kTeamN;  // rows of <= kTeamN from the front, others
       const int lcap = 32 * t.wcap;              // from the back
-      uint32_t* own = reinterpret_cast<uint32_t*>(longs + lcap) + warp * kWarpScratch;
-      PickWord* opick = reinterpret_cast<PickWord*>(own);
-      uint32_t* oC = own + 8 * 32;
-      uint32_t* otmp = oC + kOwnWords;
-      uint16_t* oidx = reinterpret_cast<uint16_t*>(otmp + 32);
-      uint16_t* oids = oidx + kOwnN;
+      using Scratch = TaskScratch<K, kWarps>;
+      Scratch& ws = reinterpret_cast<Scratch*>(longs + lcap)[warp];
+      InduceScratch& own = ws.level[0];
+      constexpr bool kDeep = sizeof(Scratch) == sizeof(WarpScratch<2>);
+      InduceScratch* deep = kDeep ? &ws.level[kDeep ? 1 : 0] : nullptr;
       for (;;) {
         int i = 0;
-        if (lane == 0) i = atomicAdd(&next_i, 1);
-        i = __shfl_sync(kFull, i, 0);
+        if (lane == 0) i = atomicAdd(&next_i, kParts);
+        i = __shfl_sync(kFull, i, 0) + part;
         if (i + K - 2 >= s) break;
-        const uint32_t word = lane >= (i >> 5) && lane < W
-                                  ? M[tri_row_off(i, W) + lane - (i >> 5)] : 0u;
+        const uint32_t word = row_word(M, W, i);
         const int n = (int)__reduce_add_sync(kFull, (unsigned)__popc(word));
         if (n < K - 2) continue;
         if (n <= 32) {
-          acc += set_cliques<K - 2>(M, W, word, n, oidx, otmp);
+          acc += set_cliques<K - 2>(M, W, word, n, ws.ids, ws.tmp);
           continue;
         }
         if (n > kOwnN) {
@@ -1090,11 +1135,11 @@ __global__ void __launch_bounds__(NT, team_ctas(K, NT)) k_rows_team(RowTasks t, 
           }
           continue;
         }
-        row_members(M, W, i, oidx, opick, 0, 1);
+        set_members(W, word, own.idx, own.pick, 0, 1);
         __syncwarp();
-        compress(M, W, oidx, opick, n, oC, 0, 1);
+        compress(M, W, own.idx, own.pick, n, own.mat, 0, 1);
         __syncwarp();
-        acc += matrix_cliques<K - 2>(oC, n, 0, 1, oids, otmp);
+        acc += matrix_cliques<K - 2>(own.mat, n, 0, 1, deep, ws.ids, ws.tmp);
         __syncwarp();
       }
       __syncthreads();
@@ -1105,21 +1150,23 @@ __global__ void __launch_bounds__(NT, team_ctas(K, NT)) k_rows_team(RowTasks t, 
         const int x = team_x[team];
         if (x >= n_long) break;
         uint32_t* C = Cs + team * tm;
-        const int n = row_members(M, W, longs[x], idxs + team * kTeamN, picks + 32 * team, tw, kTeam);
+        const int n = set_members(W, row_word(M, W, longs[x]), idxs + team * kTeamN,
+                                  picks + 32 * team, tw, kTeam);
         team_sync(team);
         compress(M, W, idxs + team * kTeamN, picks + 32 * team, n, C, tw, kTeam);
         team_sync(team);
-        acc += matrix_cliques<K - 2>(C, n, tw, kTeam, oids, otmp);
+        acc += matrix_cliques<K - 2>(C, n, tw, kTeam, deep, ws.ids, ws.tmp);
       }
       if constexpr (kTeams * team_matrix_words(32) >= matrix_words(32)) {
         const int nh = n_huge;
         if (nh) __syncthreads();  // every team is done
         for (int x = 0; x < nh; ++x) {
-          const int n = row_members(M, W, longs[lcap - 1 - x], idxs, picks, warp, kWarps);
+          const int n = set_members(W, row_word(M, W, longs[lcap - 1 - x]), idxs, picks, warp,
+                                    kWarps);
           __syncthreads();
           compress(M, W, idxs, picks, n, Cs, warp, kWarps);
           __syncthreads();
-          acc += matrix_cliques<K - 2>(Cs, n, warp, kWarps, oids, otmp);
+          acc += matrix_cliques<K - 2>(Cs, n, warp, kWarps, deep, ws.ids, ws.tmp);
           __syncthreads();
         }
       }
@@ -1135,10 +1182,10 @@ __global__ void __launch_bounds__(NT, team_ctas(K, NT)) k_rows_team(RowTasks t, 
 // the tensor cores, its operands by shuffle.
 constexpr int kWordThreads = 256;
 template <int K>
-__global__ void __launch_bounds__(kWordThreads) k_rows_word(RowTasks t, unsigned long long* head,
-                                                            unsigned long long* count, GOut o) {
-  __shared__ uint32_t rows_s[kWordThreads / 32][32];
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+__device__ uint64_t word_tasks(const RowTasks& t, unsigned long long* head, const GOut& o,
+                               uint32_t* rows_s) {
+  const int lane = threadIdx.x & 31;
+  uint32_t* mine = rows_s + (threadIdx.x & ~31);
   const long long nt = (long long)*t.n;
   uint64_t acc = 0;
   for (;;) {
@@ -1171,23 +1218,21 @@ __global__ void __launch_bounds__(kWordThreads) k_rows_word(RowTasks t, unsigned
       if constexpr (K == 4) {
         emit_rows(o, __shfl_sync(kFull, v, x), tri_word(r, sc), acc);
       } else {
-        rows_s[warp][lane] = r;
+        mine[lane] = r;
         __syncwarp();
-        const uint64_t c = word_cliques<K - 2>(rows_s[warp], r);
+        const uint64_t c = word_cliques<K - 2>(mine, r);
         __syncwarp();
         emit_rows(o, __shfl_sync(kFull, v, x), c, acc);
       }
     }
   }
-  acc = warp_sum_u64(acc);
-  if (lane == 0 && acc) atomicAdd(count, (unsigned long long)acc);
+  return acc;
 }
 
 // Tasks of up to 8 out-neighbours, four to a warp, lane l of a group holding row l.
 template <int K>
-__global__ void __launch_bounds__(kWordThreads) k_rows_group(RowTasks t, unsigned long long* head,
-                                                             unsigned long long* count, GOut o) {
-  __shared__ uint32_t rows_s[kWordThreads];
+__device__ uint64_t group_tasks(const RowTasks& t, unsigned long long* head, const GOut& o,
+                                uint32_t* rows_s) {
   const int lane = threadIdx.x & 31, l8 = lane & 7, g0 = lane & 24;
   const uint32_t* mine = rows_s + (threadIdx.x & ~7);
   const long long nt = (long long)*t.n;
@@ -1237,9 +1282,24 @@ __global__ void __launch_bounds__(kWordThreads) k_rows_group(RowTasks t, unsigne
       }
     }
   }
-  acc = warp_sum_u64(acc);
-  if (lane == 0 && acc) atomicAdd(count, (unsigned long long)acc);
+  return acc;
 }
+
+// The narrow tasks: KIND 1 word tasks, 2 group tasks, 3 both in one launch.  A launch costs a
+// call 3 us; with many tasks the group tasks' own 32 registers (64 warps per SM against 32)
+// are worth more: 4,096 Barabasi-Albert graphs 1.52 against 1.59 ms.
+template <int K, int KIND>
+__global__ void __launch_bounds__(kWordThreads, KIND == 3 ? 4 : 1)
+    k_rows_narrow(RowTasks word, RowTasks group, OwnHeads* heads, unsigned long long* count,
+                  GOut o) {
+  __shared__ uint32_t rows_s[kWordThreads];
+  uint64_t acc = 0;
+  if (KIND & 1) acc += word_tasks<K>(word, &heads->word, o, rows_s);
+  if (KIND & 2) acc += group_tasks<K>(group, &heads->group, o, rows_s);
+  acc = warp_sum_u64(acc);
+  if ((threadIdx.x & 31) == 0 && acc) atomicAdd(count, (unsigned long long)acc);
+}
+constexpr int64_t kOneNarrow = int64_t(1) << 17;  // tasks up to which both kinds share a launch
 
 // Grid of a persistent kernel: every CTA the chip holds.
 template <class F>
@@ -1250,11 +1310,13 @@ cudaError_t full_grid(F fn, int threads, int smem, int num_sms, int* grid) {
   return e;
 }
 
+static_assert(4 * team_words<7, 16>(kRowsCap / 32) <= 226 * 1024, "wide tasks fit an SM");
+
 template <int K, int NT>
 cudaError_t launch_team(const DevGraph& g, RowTasks t, int cap, unsigned long long* head,
                         unsigned long long* count, int num_sms, cudaStream_t s, const GOut& o) {
   t.wcap = (int)((std::min<int64_t>(g.max_out, cap) + 31) / 32);
-  const int smem = 4 * team_words<K>(t.wcap, NT / 32);
+  const int smem = 4 * team_words<K, NT / 32>(t.wcap);
   int grid = 0, dev = 0;
   // the shared-memory opt-in of the widest layout, once per device
   static std::atomic<unsigned long long> opted{0};
@@ -1262,12 +1324,12 @@ cudaError_t launch_team(const DevGraph& g, RowTasks t, int cap, unsigned long lo
   const unsigned long long bit = dev < 64 ? 1ull << dev : 0ull;
   if (e == cudaSuccess && !(opted.load(std::memory_order_acquire) & bit)) {
     e = cudaFuncSetAttribute(k_rows_team<K, NT>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                             4 * team_words<K>(cap / 32, NT / 32));
+                             4 * team_words<K, NT / 32>(cap / 32));
     if (e == cudaSuccess) opted.fetch_or(bit, std::memory_order_acq_rel);
   }
   if (e == cudaSuccess) e = full_grid(k_rows_team<K, NT>, NT, smem, num_sms, &grid);
   if (e != cudaSuccess) return e;
-  grid = (int)std::min<int64_t>(grid, g.nv);
+  grid = (int)std::min<int64_t>(grid, g.nv * team_parts(K, NT));
   k_rows_team<K, NT><<<grid, NT, smem, s>>>(t, head, count, o);
   return cudaGetLastError();
 }
@@ -1285,26 +1347,26 @@ cudaError_t launch_rows_k(const DevGraph& g, const uint32_t* rows, OwnHeads* hea
     const RowTasks t{g.dptr, g.roff, rows, g.rtask + g.nv, rn + 3, 0, 0};
     e = launch_team<K, 128>(g, t, kRowsMid, &heads->team, count, num_sms, s, o);
   }
-  // the word and group kernels: at most `roots` tasks; claims small enough that every warp
-  // has a few
+  if (e != cudaSuccess) return e;
+  // at most `roots` word and group tasks; claims small enough that every warp has a few
   const int64_t roots = std::max<int64_t>(g.n_roots[1], 1);
-  auto narrow = [&](auto kernel, const int32_t* list, int down, const unsigned long long* n,
-                    unsigned long long* head, int per_warp) -> cudaError_t {
+  auto narrow = [&](auto kernel, int per_warp) -> cudaError_t {
     int grid = 0;
     const cudaError_t r = full_grid(kernel, kWordThreads, 0, num_sms, &grid);
     if (r != cudaSuccess) return r;
     constexpr int kWarps = kWordThreads / 32;
     grid = (int)std::min<int64_t>(grid, (roots + kWarps * per_warp - 1) / (kWarps * per_warp));
-    const int claim = (int)std::max<int64_t>(
-        per_warp, std::min<int64_t>(32, roots / (4 * kWarps * (int64_t)grid)));
-    const RowTasks t{g.dptr, g.roff, rows, list, n, down, claim};
-    kernel<<<grid, kWordThreads, 0, s>>>(t, head, count, o);
+    const int64_t claim = std::min<int64_t>(32, roots / (4 * kWarps * (int64_t)grid));
+    const RowTasks word{g.dptr, g.roff, rows, g.rtask + g.nv - 1, rn + 2, 1,
+                        (int)std::max<int64_t>(claim, 1)};
+    const RowTasks group{g.dptr, g.roff, rows, g.rtask, rn + 1, 0, (int)std::max<int64_t>(claim, 4)};
+    kernel<<<grid, kWordThreads, 0, s>>>(word, group, heads, count, o);
     return cudaGetLastError();
   };
-  if (e == cudaSuccess && g.max_out > 8)
-    e = narrow(k_rows_word<K>, g.rtask + g.nv - 1, 1, rn + 2, &heads->word, 1);
-  if (e == cudaSuccess) e = narrow(k_rows_group<K>, g.rtask, 0, rn + 1, &heads->group, 4);
-  return e;
+  if (g.max_out <= 8) return narrow(k_rows_narrow<K, 2>, 4);
+  if (roots <= kOneNarrow) return narrow(k_rows_narrow<K, 3>, 1);
+  e = narrow(k_rows_narrow<K, 1>, 1);
+  return e == cudaSuccess ? narrow(k_rows_narrow<K, 2>, 4) : e;
 }
 
 }  // namespace

@@ -1379,7 +1379,7 @@ xgm_status count_program(xgm_ctx* ctx, const DevGraph& g, const Prog& p, uint64_
   cudaStream_t s = ctx->stream;
   XGM_CUDA_TRY(cudaSetDevice(ctx->device));
   XGM_CUDA_TRY(cudaMemsetAsync(ctx->d_sc, 0, sizeof(Scalars), s));
-  XGM_CUDA_TRY(cudaEventRecord(ctx->ev[0], s));
+  XGM_CUDA_TRY(ctx_mark(ctx, 0));
   const int nslots = p.nslots > 0 ? p.nslots : 1;
   const int64_t slot_cap = g.max_deg > 0 ? g.max_deg : 1;
   // resident warps, fewer when the scratch would pass 8 GB
@@ -1406,7 +1406,7 @@ xgm_status count_program(xgm_ctx* ctx, const DevGraph& g, const Prog& p, uint64_
   ProgLut lut;
   const bool lut_ok = prog_lut(p, &lut);
   if (lut_ok && p.k >= 4) XGM_CUDA_TRY(ensure_lut_rows(g, s));  // once per graph
-  XGM_CUDA_TRY(cudaEventRecord(ctx->ev[1], s));
+  XGM_CUDA_TRY(ctx_mark(ctx, 1));
   ProgArgs a;
   a.rowptr = g.rowptr_o;
   a.col = g.col_o;
@@ -1444,14 +1444,12 @@ xgm_status count_program(xgm_ctx* ctx, const DevGraph& g, const Prog& p, uint64_
     if (e != cudaSuccess) return cuda_fail(e, "k_setprog", __FILE__, __LINE__);
     launches = p.k == 3 ? 1 : (a.lut_ok ? (a.lut_stream >= 0 ? 4 : 3) : 2);
   }
-  XGM_CUDA_TRY(cudaEventRecord(ctx->ev[2], s));
+  XGM_CUDA_TRY(ctx_mark(ctx, 2));
   XGM_CUDA_TRY(cudaMemcpyAsync(ctx->d_sc->n, ctx->prog_heads + 1, sizeof(int64_t),
                                cudaMemcpyDeviceToDevice, s));
   xgm_status r = ctx_sync_scalars(ctx);
   if (r != XGM_OK) return r;
-  float prep = 0, kern = 0;
-  cudaEventElapsedTime(&prep, ctx->ev[0], ctx->ev[1]);
-  cudaEventElapsedTime(&kern, ctx->ev[1], ctx->ev[2]);
+  const float prep = ctx_ms(ctx, 0, 1), kern = ctx_ms(ctx, 1, 2);
   std::memset(&st, 0, sizeof(st));
   st.prep_ms = prep;
   st.kernel_ms = kern;
