@@ -505,12 +505,8 @@ xgm_status xgm_motif_count(xgm_ctx* ctx, const xgm_graph* g, int k, const xgm_sc
 xgm_status xgm_count_kernels(xgm_ctx* ctx, const xgm_graph* g, const xgm_plan* plan,
                              const xgm_sched* sched, int* n_kernels) {
   if (!ctx || !g || !plan || !n_kernels) return XGM_ERR_INVALID;
-  if (plan->pattern == XGM_PATTERN_PROGRAM) {  // bitmap launch (where eligible), tasks, splits
-    ProgLut lut;
-    *n_kernels = plan->prog.k == 3 ? 1
-                                   : (prog_lut(plan->prog, &lut) ? (lut.stream >= 0 ? 4 : 3) : 2);
-    return XGM_OK;
-  }
+  if (plan->pattern == XGM_PATTERN_PROGRAM)
+    return finish_status(ctx, program_kernels(ctx, g->g, plan->prog, n_kernels));
   xgm_sched def;
   std::memset(&def, 0, sizeof(def));
   return finish_status(ctx, count_kernels(ctx, g->g, plan->pattern, sched ? *sched : def, n_kernels));

@@ -22,6 +22,9 @@ struct Scalars {
   int64_t n[8];  // task list sizes, copied back for the stats
   unsigned long long terms[7];  // motif-identity sums (launch_motif_terms)
   OwnHeads own;                 // queue heads of the owner kernels (rows.cu)
+  // set-operation programs: unit heads of the bitmap form by class, then the list form's
+  // entry head, split tail and split head
+  unsigned long long prog[6];
 };
 
 struct Model;  // learned cost model (learned.cu)
@@ -55,7 +58,6 @@ struct xgm_ctx {
   int32_t* prog_scratch = nullptr;
   int64_t prog_scratch_cap = 0;
   void* prog_split = nullptr;
-  unsigned long long* prog_heads = nullptr;
 };
 
 struct xgm_graph {
@@ -99,6 +101,8 @@ xgm_status count_kernels(xgm_ctx* ctx, const DevGraph& g, int pattern, const xgm
                          int* n_kernels);
 void motif_buffers_free(xgm_ctx* ctx);
 // setprog.cu
+// Kernels a count of the program launches on g.
+xgm_status program_kernels(xgm_ctx* ctx, const DevGraph& g, const Prog& p, int* n);
 xgm_status count_program(xgm_ctx* ctx, const DevGraph& g, const Prog& p, uint64_t* out,
                          xgm_stats& st);
 void program_buffers_free(xgm_ctx* ctx);

@@ -30,12 +30,16 @@ struct DevGraph {
   mutable int32_t* bcol = nullptr;
   mutable uint32_t* boff = nullptr;
   mutable uint16_t* bmask = nullptr;
-  // adjacency rows among N(v) for v of degree 33..1024 (setprog.cu), built on first use
-  // by a set-operation program: lut_off[v] words into lut_rows; lut_state 1 built,
-  // -1 not built (too large)
+  // set-operation programs (setbits.cu), built on first use: plan_deg is the largest
+  // degree whose tasks run in the bitmap form (-1 none, 0 not built); its units {v0, part,
+  // parts} by class from plan_off[class], their numbers in plan_un; adjacency rows among
+  // N(v) for v of degree 33..1024, lut_off[v] words into lut_rows
+  mutable int plan_deg = 0;
+  mutable int4* plan_units = nullptr;
+  mutable int64_t plan_off[3] = {0, 0, 0};
+  mutable unsigned long long* plan_un = nullptr;
   mutable uint32_t* lut_rows = nullptr;
   mutable int64_t* lut_off = nullptr;
-  mutable int lut_state = 0;
   // row store offsets, row tasks by width and their numbers (rows.cu), built on first use
   // by a clique count: rn = {words, tasks of <= 8 members, <= 32, <= kRowsMid, more}; rtask
   // holds the first list from its start, the second from nv - 1 down, the third from nv on,

@@ -22,6 +22,8 @@
 
 namespace xgm {
 
+struct DevGraph;
+
 constexpr int kProgMaxK = 6;
 constexpr int kProgLevels = kProgMaxK - 2;  // level l runs after v_{l+1} is matched
 constexpr int kProgMaxOps = 6;              // per level
@@ -68,14 +70,39 @@ bool prog_check(const Prog& p, std::string* why);
 // Bitmap (LUT) form: whether the program runs in the index space of N(v0) — every
 // operand read after level 0, the v3 candidates and the counted operand descend from
 // N(v0); the v2 candidates may instead be the stream N(v1) \ N(v0) (one level-0
-// difference, `stream`), whose vertices get their rows built on the fly.  The bitmap
-// kernels hold kLutSlots slots per task (4- and 5-vertex programs use at most 5).
-constexpr int kLutSlots = 8;
+// difference, `stream`).
 struct ProgLut {
   int8_t ok = 0;
   int8_t stream = -1;  // index of the level-0 operation giving cand[2] from N(v1), or -1
 };
 bool prog_lut(const Prog& p, ProgLut* out);
+
+// A set of such a program, flattened through its slots: the elements of N(v0) in N(v_j)
+// for every j of `pos`, in no N(v_j) of `neg`, below every v_j of `bound` and none of the
+// v_j of `excl` (bit masks over j; bit 0 of pos and neg is resolved when it is built).
+struct BitTerm {
+  uint8_t pos = 0, neg = 0, bound = 0, excl = 0;
+};
+struct BitPlan {
+  int8_t k = 0;
+  int8_t v1lt = 0;
+  int8_t stream = 0;  // v2 runs over N(v1) \ N(v0): c2 holds that list's bound and excl only
+  int8_t bound2 = 0;  // a bound reads v2's place in N(v0)
+  BitTerm c2, c3, fin;  // v2's and (k = 5) v3's candidates, the counted set
+};
+BitPlan prog_terms(const Prog& p, const ProgLut& lut);
+
+#ifdef __CUDACC__
+// Builds g's units and stored rows once (setbits.cu); later calls return at once.
+cudaError_t ensure_plan_index(const DevGraph& g, int num_sms, cudaStream_t s);
+// Kernels launch_bits launches.
+int bits_launches(const DevGraph& g);
+// Adds the program's count over the v0 of degree <= g.plan_deg to *total.  heads: three
+// zeroed unit heads; split_out (or null) receives the units of v0s dealt to several.
+cudaError_t launch_bits(const DevGraph& g, const BitPlan& p, unsigned long long* heads,
+                        unsigned long long* total, int64_t* split_out, int num_sms,
+                        cudaStream_t s, int* launches);
+#endif
 
 // GLUMIN's P6..P22 (vertex-induced 5-vertex plans), exactly as generated.
 bool prog_glumin(int pid, Prog* p);
