@@ -38,6 +38,17 @@ def test_dense_graphs(xgm, ctx, orc, nv, p):
     g.close()
 
 
+@pytest.mark.parametrize("nv,deg", [(1200, 13), (1200, 21), (1500, 24), (900, 40), (3000, 100)])
+def test_sparse_graphs(xgm, ctx, orc, nv, deg):
+    # few steps share a v2: the tables of two-hop vertices are filled to the limit and past
+    # it (a pass that does not fit is halved); at degree 24 some vertices have over 32
+    rowptr, col = _random_graph(nv, deg / nv, nv + deg)
+    g = ctx.graph_from_csr(rowptr, col)
+    for pid in (7, 8, 11, 12, 15, 16) if deg < 50 else (7, 8, 12):
+        assert ctx.count(g, f"P{pid}") == orc.glumin5(pid, rowptr, col), pid
+    g.close()
+
+
 @pytest.mark.parametrize("edges", [
     [(0, 1), (0, 2), (1, 2), (1, 3), (0, 4)],                  # bull
     [(0, 1), (1, 2), (1, 3), (2, 3), (0, 4)],

@@ -38,6 +38,7 @@ struct DevGraph {
   mutable int4* plan_units = nullptr;
   mutable int64_t plan_off[3] = {0, 0, 0};
   mutable unsigned long long* plan_un = nullptr;
+  mutable int plan_items = 0;  // list entries a block takes to a table at a time (0: no tables)
   mutable uint32_t* lut_rows = nullptr;
   mutable int64_t* lut_off = nullptr;
   // row store offsets, row tasks by width and their numbers (rows.cu), built on first use

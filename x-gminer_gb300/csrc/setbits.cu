@@ -22,13 +22,20 @@
 //   a lane for the count.  Blocks of 256 threads up to 256 neighbours, of 1,024 above, where
 //   the rows leave room for one block an SM (the line at 384: 2.00 against 1.93 ms).
 //
-// The row of a v2 outside N(v0) is found by looking N(v2) up in a hash table of N(v0) in
-// shared memory.
+// - k_bits_map, a stream program's v0 of 33 to 256 neighbours in place of k_bits_cta, on
+//   graphs with enough of them.
 //
-// What bounds them: instruction issue (70-80 %, the integer pipe).  P7 on R-MAT scale 12
-// (5.9 M steps, 119 M v3 candidates, 400 M look-ups): 6.40 ms when k_setlut and k_setprog
-// interpreted the operations with binary searches in lists, 1.95 ms; R-MAT scale 9 1.84 ms
-// -> 0.14, where a few heavy tasks were the time; P10 on Erdos-Renyi 2^16 0.83 -> 0.24 ms.
+// The row of a v2 outside N(v0): up to 256 neighbours the rows of all two-hop vertices are
+// built at once, by streaming the lists of N(v0)'s members into a table, whose set bits are
+// the steps.  Above, where the table would not fit, or where few tasks have steps, N(v2) is
+// looked up in a hash table of N(v0), a step at a time.
+//
+// What bounds them: instruction issue (60-80 %, the integer pipe).  P7 on R-MAT scale 12
+// (5.9 M steps, 119 M v3 candidates): 6.40 ms when k_setlut and k_setprog interpreted the
+// operations with binary searches in lists, 1.97 ms with a look-up of every v2's list (400 M
+// look-ups), 1.32 ms with the tables; P15 on Erdos-Renyi 2^16 2.25, 1.25, 0.67 ms.
+// R-MAT scale 9 P7 1.84 ms -> 0.12, where a few heavy tasks were the time; P10 on
+// Erdos-Renyi 2^16 0.83 -> 0.24 ms.
 #include <algorithm>
 
 #include "api_internal.h"
@@ -70,6 +77,7 @@ struct BitArgs {
   int64_t* split_out;               // statistics: un[3] (or null)
   BitPlan p;
   int cls;
+  int items;  // list entries a block of k_bits_map takes at a time
   CtaLayout lay;
 };
 
@@ -201,11 +209,14 @@ __device__ __forceinline__ uint32_t term(const BitTerm& t, uint32_t r1, uint32_t
 
 template <int NW>
 __device__ __forceinline__ void load_row(uint32_t (&x)[NW], const uint32_t* r) {
-  if constexpr (NW == 4) {
-    const uint4 q = *(const uint4*)r;
-    x[0] = q.x, x[1] = q.y, x[2] = q.z, x[3] = q.w;
-  } else {
+  if constexpr (NW == 1) {
     x[0] = r[0];
+  } else {
+#pragma unroll
+    for (int k = 0; k < NW; k += 4) {
+      const uint4 q = ((const uint4*)r)[k / 4];
+      x[k] = q.x, x[k + 1] = q.y, x[k + 2] = q.z, x[k + 3] = q.w;
+    }
   }
 }
 
@@ -352,66 +363,169 @@ __device__ __forceinline__ Item decode(const BitArgs& a, const Local& w, const i
   return s;
 }
 
+// The count of one step: v1 = N(v0)[i1], v2 with its row and places.
+template <int K, int NW>
+__device__ __forceinline__ unsigned count_step(const BitPlan& p, const Local& w, int i1, int i2,
+                                               int pre2, const uint32_t (&r2)[NW]) {
+  unsigned c = 0;
+  uint32_t r1[NW], fk[NW];
+  load_row<NW>(r1, w.rows + i1 * w.ld);
+  uint32_t any = 0;
+#pragma unroll
+  for (int q = 0; q < NW; ++q) {
+    fk[q] = term(p.fin, r1[q], r2[q], i1, i2, w.pre0, pre2, q, w.d0, true);
+    any |= fk[q];
+    if (K == 4) c += __popc(fk[q]);
+  }
+  if (K == 4 || !any) return c;
+  const bool f_ub = (p.fin.bound >> 3) & 1, f_ux = (p.fin.excl >> 3) & 1;
+  const bool f_row = ((p.fin.pos | p.fin.neg) >> 3) & 1;
+  const uint32_t flip = (p.fin.neg >> 3) & 1 ? 0xffffffffu : 0u;
+#pragma unroll
+  for (int q = 0; q < NW; ++q) {
+    for (uint32_t m = term(p.c3, r1[q], r2[q], i1, i2, w.pre0, pre2, q, w.d0, true); m;
+         m &= m - 1) {
+      const int b = __ffs(m) - 1;
+      uint32_t r3[NW];
+      if (f_row) {
+        load_row<NW>(r3, w.rows + (32 * q + b) * w.ld);
+      } else {
+#pragma unroll
+        for (int k = 0; k < NW; ++k) r3[k] = fk[k];
+      }
+      const uint32_t upto = f_ub ? (1u << b) - 1u : (f_ux ? ~(1u << b) : 0xffffffffu);
+#pragma unroll
+      for (int k = 0; k < NW; ++k) {
+        uint32_t x = fk[k] & (r3[k] ^ flip);
+        if (k == q) x &= upto;
+        if (k > q && f_ub) x = 0u;
+        c += __popc(x);
+      }
+    }
+  }
+  return c;
+}
+
 // A lane a step: 32 items from `base`.
 template <int K, int NW>
-__device__ __forceinline__ unsigned long long lane_steps(const BitArgs& a, const Local& w,
-                                                         const int32_t* rel, const int32_t* off,
-                                                         uint32_t* out, int base, int total,
-                                                         int lane) {
-  const BitPlan& p = a.p;
+__device__ __forceinline__ unsigned lane_steps(const BitArgs& a, const Local& w,
+                                               const int32_t* rel, const int32_t* off,
+                                               uint32_t* out, int base, int total, int lane) {
   const Item s = decode(a, w, rel, off, NW, base + lane < total, base + lane);
   uint32_t r2[NW];
-  if (p.stream) {
+  if (a.p.stream) {
     list_rows<NW>(w, out, a.col, s.on, s.by, s.dy, r2, lane);
   } else if (s.on) {
     load_row<NW>(r2, w.rows + s.i2 * w.ld);
   }
-  unsigned c = 0;
-  unsigned long long sum = 0;
-  if (s.on) {
-    uint32_t r1[NW], fk[NW];
-    load_row<NW>(r1, w.rows + s.i1 * w.ld);
-    uint32_t any = 0;
-#pragma unroll
-    for (int q = 0; q < NW; ++q) {
-      fk[q] = term(p.fin, r1[q], r2[q], s.i1, s.i2, w.pre0, s.pre2, q, w.d0, true);
-      any |= fk[q];
-      if (K == 4) c += __popc(fk[q]);
+  return s.on ? count_step<K, NW>(a.p, w, s.i1, s.i2, s.pre2, r2) : 0u;
+}
+
+// Rows over N(v0) of the vertices y outside it, by streaming the lists of N(v0)'s members
+// (the graph is symmetric): y's bit i is set where y is in N(N(v0)[i]).  Every set bit of a
+// finished table is a step (v0, v1, y).  Open addressing; a table takes the y whose hash_part
+// lies in a range, and a range that does not fit is halved (one value of hash_part is one y).
+struct YTable {
+  int32_t* key;
+  uint32_t* val;  // NW words a slot
+  int mask, shift;
+};
+
+__device__ __forceinline__ uint32_t hash_part(int y) {
+  uint32_t h = (uint32_t)y * 0x85ebca6bu;
+  return h ^ (h >> 16);
+}
+
+template <int NW>
+__device__ __forceinline__ bool put(const YTable& t, int y, int i) {
+  uint32_t h = ((uint32_t)y * 2654435761u) >> t.shift;
+  for (int k = 0; k < 64; ++k, h = (h + 1) & t.mask) {
+    int at = ((volatile int32_t*)t.key)[h];
+    if (at == -1) {
+      at = atomicCAS(&t.key[h], -1, y);
+      if (at == -1) at = y;
     }
-    if (K == 5 && any) {
-      const bool f_ub = (p.fin.bound >> 3) & 1, f_ux = (p.fin.excl >> 3) & 1;
-      const bool f_row = ((p.fin.pos | p.fin.neg) >> 3) & 1;
-      const uint32_t flip = (p.fin.neg >> 3) & 1 ? 0xffffffffu : 0u;
+    if (at == y) {
+      atomicOr(&t.val[h * NW + (NW == 1 ? 0 : i >> 5)], 1u << (i & 31));
+      return true;
+    }
+  }
+  return false;
+}
+
+// The steps of the table's slots, 32 slots a warp at a time (from *next for a block's warps).
+// queue: 64 words of the warp; steps gather there until a lane each.  live: the tasks with
+// steps.
+template <int K, int NW>
+__device__ __forceinline__ unsigned long long table_steps(const BitPlan& p, const Local& w,
+                                                          const YTable& t, const uint32_t* live,
+                                                          uint32_t* queue, int* next, int lane) {
+  unsigned long long c = 0;
+  int qn = 0;
+  auto step = [&](uint32_t e) {
+    const int slot = e >> 16;
+    uint32_t r2[NW];
+    load_row<NW>(r2, t.val + slot * NW);
+    const int pre2 = p.bound2 ? lower_index(w.n0, w.d0, t.key[slot]) : 0;
+    c += count_step<K, NW>(p, w, e & 0xffff, -1, pre2, r2);
+  };
+  for (int base = 0;; base += 32) {
+    if (next) {
+      if (lane == 0) base = atomicAdd(next, 32);
+      base = __shfl_sync(0xffffffffu, base, 0);
+    }
+    if (base > t.mask) break;
+    const int slot = base + lane;
+    const int y = t.key[slot];
+    uint32_t m[NW];
 #pragma unroll
-      for (int q = 0; q < NW; ++q) {
-        for (uint32_t m = term(p.c3, r1[q], r2[q], s.i1, s.i2, w.pre0, s.pre2, q, w.d0, true); m;
-             m &= m - 1) {
-          const int b = __ffs(m) - 1;
-          uint32_t r3[NW];
-          if (f_row) {
-            load_row<NW>(r3, w.rows + (32 * q + b) * w.ld);
-          } else {
+    for (int q = 0; q < NW; ++q) m[q] = 0u;
+    // the stream's bound and exclusion: y below v0, v1; not v0
+    if (y >= 0 && !((p.c2.bound & 1) && y >= w.v0) && !((p.c2.excl & 1) && y == w.v0)) {
+      load_row<NW>(m, t.val + slot * NW);
+      const int pre = p.c2.bound & 2 ? lower_index(w.n0, w.d0, y) : 0;
 #pragma unroll
-            for (int k = 0; k < NW; ++k) r3[k] = fk[k];
-          }
-          const uint32_t upto = f_ub ? (1u << b) - 1u : (f_ux ? ~(1u << b) : 0xffffffffu);
+      for (int q = 0; q < NW; ++q) m[q] &= live[q] & ~below(pre, 32 * q);
+    }
+    for (;;) {
+      int i1 = -1;
 #pragma unroll
-          for (int k = 0; k < NW; ++k) {
-            uint32_t x = fk[k] & (r3[k] ^ flip);
-            if (k == q) x &= upto;
-            if (k > q && f_ub) x = 0u;
-            c += __popc(x);
-          }
+      for (int q = 0; q < NW; ++q)
+        if (i1 < 0 && m[q]) {
+          i1 = 32 * q + __ffs(m[q]) - 1;
+          m[q] &= m[q] - 1;
         }
+      const unsigned b = __ballot_sync(0xffffffffu, i1 >= 0);
+      if (!b) break;
+      if (i1 >= 0) queue[qn + __popc(b & ((1u << lane) - 1u))] = (uint32_t)slot << 16 | i1;
+      qn += __popc(b);
+      __syncwarp();
+      if (qn >= 32) {
+        step(queue[lane]);
+        const uint32_t rest = queue[32 + lane];
+        __syncwarp();
+        queue[lane] = rest;
+        qn -= 32;
+        __syncwarp();
       }
     }
   }
-  sum = c;
-  return sum;
+  if (lane < qn) step(queue[lane]);
+  __syncwarp();
+  return c;
 }
 
 // ---------------------------------------------------------------- d(v0) <= 32
 constexpr int kSmallBuckets = 64;
+
+constexpr int kSmallTable = 512;  // slots of a warp's table of two-hop vertices
+constexpr int kSmallItems = 448;  // list entries taken to one table at first
+
+struct SmallMap {
+  int32_t key[kSmallTable];
+  uint32_t val[kSmallTable];
+  uint32_t queue[64];
+};
 
 struct SmallWarp {
   int32_t key[4 * kSmallBuckets];
@@ -422,11 +536,75 @@ struct SmallWarp {
   int32_t rel[32], off[32];
 };
 
+// The unit's share, by hash_part, of the steps whose v2 are the two-hop vertices of the lists
+// [b1, b1 + d1) (a lane a list, `lists` entries in all).
 template <int K>
-__global__ void __launch_bounds__(kThreads, 5) k_bits_warp(BitArgs a) {
-  __shared__ __align__(16) SmallWarp ws[kWarps];
+__device__ __forceinline__ unsigned long long small_map(const BitArgs& a, const Local& w,
+                                                        SmallMap& map, const int4& unit,
+                                                        int64_t b1, int d1, int lists,
+                                                        uint32_t live, int lane) {
+  const YTable t{map.key, map.val, kSmallTable - 1, __clz(kSmallTable) + 1};
+  int incl = (d1 + 15) >> 4;  // pieces of 16 entries, as in list_rows
+#pragma unroll
+  for (int k = 1; k < 32; k <<= 1) {
+    const int y = __shfl_up_sync(0xffffffffu, incl, k);
+    if (lane >= k) incl += y;
+  }
+  const int total = __shfl_sync(0xffffffffu, incl, 31);
+  const int first = incl - ((d1 + 15) >> 4);
+  const int g = lane >> 3, sub = lane & 7;
+  const long long end = share(1LL << 32, unit.y + 1, unit.z);
+  long long lo = share(1LL << 32, unit.y, unit.z);
+  const int per = lists / unit.z + 1;
+  long long span = (end - lo + (per + kSmallItems - 1) / kSmallItems - 1) /
+                   ((per + kSmallItems - 1) / kSmallItems);
+  unsigned long long c = 0;
+  while (lo < end) {
+    const long long hi = min(lo + span, end);
+#pragma unroll
+    for (int k = lane; k < kSmallTable / 4; k += 32) {
+      ((int4*)map.key)[k] = make_int4(-1, -1, -1, -1);
+      ((int4*)map.val)[k] = make_int4(0, 0, 0, 0);
+    }
+    __syncwarp();
+    bool fits = true;
+    for (int base = 0; base < total; base += 4) {
+      const int item = base + g;
+      int i = 0;  // the list of this piece
+#pragma unroll
+      for (int h = 16; h > 0; h >>= 1)
+        if (__shfl_sync(0xffffffffu, incl, i + h - 1) <= item) i += h;
+      i &= 31;
+      const int at = 16 * (item - __shfl_sync(0xffffffffu, first, i)) + sub;
+      const int len = __shfl_sync(0xffffffffu, d1, i);
+      const int ln = item < total ? len : 0;
+      const int32_t* l = a.col + __shfl_sync(0xffffffffu, b1, i);
+      const int y0 = at < ln ? l[at] : -1, y1 = at + 8 < ln ? l[at + 8] : -1;
+#pragma unroll
+      for (int k = 0; k < 2; ++k) {
+        const int y = k ? y1 : y0;
+        const uint32_t h = hash_part(y);
+        if (y >= 0 && h >= lo && h < hi && look_up(w.t, w.probes, y) < 0) fits &= put<1>(t, y, i);
+      }
+      __syncwarp();
+    }
+    if (!__all_sync(0xffffffffu, fits)) {
+      span = (span + 1) / 2;
+      continue;
+    }
+    c += table_steps<K, 1>(a.p, w, t, &live, map.queue, nullptr, lane);
+    lo = hi;
+  }
+  return c;
+}
+
+template <int K>
+__global__ void __launch_bounds__(kThreads, 4) k_bits_warp(BitArgs a) {
+  extern __shared__ __align__(16) unsigned char sm[];
   const int lane = threadIdx.x & 31;
-  SmallWarp& w = ws[threadIdx.x >> 5];
+  SmallWarp& w = ((SmallWarp*)sm)[threadIdx.x >> 5];
+  // (a stream program's launch only)
+  SmallMap& map = ((SmallMap*)(sm + kWarps * sizeof(SmallWarp)))[threadIdx.x >> 5];
   if (blockIdx.x == 0 && threadIdx.x == 0 && a.split_out) *a.split_out = (int64_t)a.un[3];
   const int64_t n_units = (int64_t)a.un[a.cls];
   // one unit a claim, up to eight when every warp takes 64 and more
@@ -477,6 +655,20 @@ __global__ void __launch_bounds__(kThreads, 5) k_bits_warp(BitArgs a) {
         if (lane >= k) incl += y;
       }
       const long long all = __shfl_sync(0xffffffffu, incl, 31);
+      __syncwarp();
+      if (all == 0) continue;
+      if (a.p.stream) {
+        long long lists = d1;
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) lists += __shfl_xor_sync(0xffffffffu, lists, o);
+        // from a table unless few tasks have steps (a table takes every list's entries, a
+        // look-up form only theirs) or a pass over the lists would keep under a sixteenth
+        if (2 * all >= lists && lists <= 16 * kSmallItems) {
+          c += small_map<K>(a, l, map, unit, b1, d1, (int)lists,
+                            __ballot_sync(0xffffffffu, n > 0), lane);
+          continue;
+        }
+      }
       const long long lo = share(all, unit.y, unit.z), hi = share(all, unit.y + 1, unit.z);
       const int total = (int)(hi - lo);
       w.rel[lane] = (int)max(0LL, min(incl - lo, (long long)total));
@@ -615,6 +807,37 @@ __device__ __forceinline__ unsigned long long warp_step(const BitArgs& a, const 
   return c;
 }
 
+// N(v0), its rows and its hash table into shared memory; the row words.  A block, which
+// synchronises before it reads *probes.
+template <int NT>
+__device__ __forceinline__ int load_v0(const BitArgs& a, Local& w, int v0, int32_t* n0,
+                                       uint32_t* rows, int max_buckets, int* probes, int tid) {
+  w.v0 = v0;
+  const int64_t rb = a.rowptr[v0];
+  const int d0 = (int)(a.rowptr[v0 + 1] - rb);
+  w.d0 = d0;
+  const int W = (d0 + 31) >> 5;
+  w.ld = row_stride(W);
+  int nb = 64;
+  while (nb < 2 * d0 && nb < max_buckets) nb <<= 1;
+  w.t.mask = nb - 1;
+  w.t.shift = __clz(nb) + 1;
+  for (int i = tid; i < nb; i += NT) ((int4*)w.t.key)[i] = make_int4(-1, -1, -1, -1);
+  for (int i = tid; i < d0; i += NT) n0[i] = a.col[rb + i];
+  const uint32_t* g = a.rows + a.roff[v0];
+  for (int i = tid; i < d0 * w.ld; i += NT) {
+    const int r = i / w.ld, wi = i - r * w.ld;
+    rows[i] = wi < W ? g[(int64_t)r * W + wi] : 0u;
+  }
+  __syncthreads();
+  for (int i = tid; i < d0; i += NT) {
+    const int k = insert(w.t, n0[i], i);
+    if (k > 1) atomicMax(probes, k);
+  }
+  w.pre0 = lower_index(n0, d0, v0);
+  return W;
+}
+
 template <int K, int NT>
 __global__ void __launch_bounds__(NT, NT == kThreads ? 4 : 1) k_bits_cta(BitArgs a) {
   extern __shared__ __align__(16) unsigned char sm[];
@@ -645,29 +868,8 @@ __global__ void __launch_bounds__(NT, NT == kThreads ? 4 : 1) k_bits_cta(BitArgs
     const int64_t u = s_unit;
     if (u >= n_units) break;
     const int4 unit = a.units[u];
-    w.v0 = unit.x;
-    const int64_t rb = a.rowptr[w.v0];
-    const int d0 = (int)(a.rowptr[w.v0 + 1] - rb);
-    w.d0 = d0;
-    const int W = (d0 + 31) >> 5;
-    w.ld = row_stride(W);
-    int nb = 64;
-    while (nb < 2 * d0 && nb < L.buckets) nb <<= 1;
-    w.t.mask = nb - 1;
-    w.t.shift = __clz(nb) + 1;
-    for (int i = tid; i < nb; i += NT) ((int4*)w.t.key)[i] = make_int4(-1, -1, -1, -1);
-    for (int i = tid; i < d0; i += NT) n0[i] = a.col[rb + i];
-    const uint32_t* g = a.rows + a.roff[w.v0];
-    for (int i = tid; i < d0 * w.ld; i += NT) {
-      const int r = i / w.ld, wi = i - r * w.ld;
-      rows[i] = wi < W ? g[(int64_t)r * W + wi] : 0u;
-    }
-    __syncthreads();
-    for (int i = tid; i < d0; i += NT) {
-      const int k = insert(w.t, n0[i], i);
-      if (k > 1) atomicMax(&s_probes, k);
-    }
-    w.pre0 = lower_index(n0, d0, w.v0);
+    const int W = load_v0<NT>(a, w, unit.x, n0, rows, L.buckets, &s_probes, tid);
+    const int d0 = w.d0;
     // the steps of each task (v0, N(v0)[i]), this thread's run of tasks
     const int per = (d0 + NT - 1) / NT;
     const int t0 = min(tid * per, d0), t1 = min(t0 + per, d0);
@@ -722,6 +924,171 @@ __global__ void __launch_bounds__(NT, NT == kThreads ? 4 : 1) k_bits_cta(BitArgs
         t.dy = __shfl_sync(0xffffffffu, s.dy, src);
         c += warp_step<K>(a, w, mine, t, W, lane);
       }
+    }
+    __syncthreads();
+  }
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) c += __shfl_xor_sync(0xffffffffu, c, o);
+  if (lane == 0 && c) atomicAdd(a.total, c);
+}
+
+// Stream programs, 33 <= d(v0) <= 256: a block takes the steps of a v0 from tables of its
+// two-hop vertices, a lane a step.  3.9 steps (d(v0) <= 128) and 5.7 share a v2's row on
+// R-MAT scale 12, so the lists may hold 1.5 entries a slot before a pass is cut; a step costs
+// no look-ups of its v2's whole list, and the queue leaves no lane without one.  P7 there:
+// 1.10 ms from k_bits_cta, 0.67 ms (blocks of 256 threads, three an SM with half the table
+// 0.98, one of 1,024 with twice the table 0.88).
+constexpr int kMapThreads = 512;
+constexpr int kMapBlocks = 2;    // an SM
+constexpr int kMapSlots = 4096;  // rows of four words; half with eight
+// Work of the class, an SM, from which a stream program takes k_bits_map: below, its few large
+// blocks leave SMs idle.  P7, k_bits_map against k_bits_cta, by R-MAT scale (work an SM):
+// 9 (1,569) 0.190 and 0.118 ms, 10 (4,035) 0.322 and 0.260, 11 (9,472) 0.534 and 0.551,
+// 12 (27,082) 1.32 and 1.78.
+constexpr int kMapWork = 8192;
+
+struct MapSmem {
+  uint32_t rows[kMidDeg * row_stride(kMidDeg / 32)];
+  int32_t key[4 * 2 * kMidDeg];
+  uint16_t pos[4 * 2 * kMidDeg];
+  int32_t n0[kMidDeg];
+  int32_t rel[kMidDeg], off[kMidDeg];
+  uint32_t live[kMidDeg / 32];
+  uint32_t queue[kMapThreads / 32][64];
+  long long sum[kMapThreads / 32], lists[kMapThreads / 32];
+  int64_t unit;
+  int next, probes, full, list, slot;
+  // tables (key, val), or the lanes' rows
+  __align__(16) uint32_t table[kMapSlots * 5];
+};
+static_assert(kMapBlocks * (sizeof(MapSmem) + 1024) <= 228 * 1024 &&
+                  kMapSlots * 5 >= kMapThreads * 8, "shared memory");
+
+template <int K, int NW>
+__device__ __forceinline__ unsigned long long map_steps(const BitArgs& a, const Local& w,
+                                                        MapSmem& m, const int4& unit,
+                                                        long long lists, int tid) {
+  const int lane = tid & 31, wib = tid >> 5;
+  constexpr int kSlots = NW == 4 ? kMapSlots : kMapSlots / 2;
+  const YTable t{(int32_t*)m.table + kSlots * NW, m.table, kSlots - 1, __clz(kSlots) + 1};
+  const int target = min(a.items, kSlots * 3 / 2);
+  // consecutive parts share a pass: about `target` entries of the lists each
+  const int passes = (int)((lists + target - 1) / target);
+  const int g = passes >= unit.z ? 1 : (unit.z + passes - 1) / passes;
+  if (unit.y % g) return 0;
+  const long long end = share(1LL << 32, min(unit.y + g, unit.z), unit.z);
+  long long lo = share(1LL << 32, unit.y, unit.z);
+  const int cut = max(1, (passes + unit.z - 1) / unit.z);
+  long long span = (end - lo + cut - 1) / cut;
+  unsigned long long c = 0;
+  while (lo < end) {
+    const long long hi = min(lo + span, end);
+    for (int k = tid; k < kSlots * NW / 4; k += kMapThreads)
+      ((int4*)t.val)[k] = make_int4(0, 0, 0, 0);
+    for (int k = tid; k < kSlots / 4; k += kMapThreads)
+      ((int4*)t.key)[k] = make_int4(-1, -1, -1, -1);
+    if (tid == 0) m.full = m.list = m.slot = 0;
+    __syncthreads();
+    bool fits = true;
+    for (;;) {
+      int i = 0;
+      if (lane == 0) i = atomicAdd(&m.list, 1);
+      i = __shfl_sync(0xffffffffu, i, 0);
+      if (i >= w.d0) break;
+      const int64_t b = a.rowptr[w.n0[i]];
+      const int n = (int)(a.rowptr[w.n0[i] + 1] - b);
+      const int32_t* l = a.col + b;
+      for (int at = lane; at < n; at += 32) {
+        const int y = l[at];
+        const uint32_t h = hash_part(y);
+        if (h >= lo && h < hi && look_up(w.t, w.probes, y) < 0) fits &= put<NW>(t, y, i);
+      }
+    }
+    if (!fits) m.full = 1;
+    __syncthreads();
+    if (m.full) {
+      span = (span + 1) / 2;
+      __syncthreads();
+      continue;
+    }
+    c += table_steps<K, NW>(a.p, w, t, m.live, m.queue[wib], &m.slot, lane);
+    __syncthreads();
+    lo = hi;
+  }
+  return c;
+}
+
+template <int K>
+__global__ void __launch_bounds__(kMapThreads, kMapBlocks) k_bits_map(BitArgs a) {
+  extern __shared__ __align__(16) unsigned char sm[];
+  MapSmem& m = *(MapSmem*)sm;
+  const int tid = threadIdx.x, lane = tid & 31, wib = tid >> 5;
+  Local w;
+  w.n0 = m.n0;
+  w.rows = m.rows;
+  w.t.key = m.key;
+  w.t.pos = m.pos;
+  const int64_t n_units = (int64_t)a.un[a.cls];
+  unsigned long long c = 0;
+  for (;;) {
+    if (tid == 0) {
+      m.unit = (int64_t)atomicAdd(a.head, 1ull);
+      m.next = 0;
+      m.probes = 1;
+    }
+    __syncthreads();
+    const int64_t u = m.unit;
+    if (u >= n_units) break;
+    const int4 unit = a.units[u];
+    const int W = load_v0<kMapThreads>(a, w, unit.x, m.n0, m.rows, 2 * kMidDeg, &m.probes, tid);
+    __syncthreads();
+    // a thread a task
+    int n = 0, d1 = 0;
+    if (tid < w.d0) {
+      n = task_size<K>(a, w, tid, W);
+      d1 = (int)(a.rowptr[w.n0[tid] + 1] - a.rowptr[w.n0[tid]]);
+    }
+    const unsigned on = __ballot_sync(0xffffffffu, n > 0);
+    if (lane == 0 && wib < kMidDeg / 32) m.live[wib] = on;
+    long long incl = n, lists = d1;
+#pragma unroll
+    for (int k = 1; k < 32; k <<= 1) {
+      const long long y = __shfl_up_sync(0xffffffffu, incl, k);
+      const long long z = __shfl_up_sync(0xffffffffu, lists, k);
+      if (lane >= k) incl += y, lists += z;
+    }
+    if (lane == 31) m.sum[wib] = incl, m.lists[wib] = lists;
+    __syncthreads();
+    w.probes = m.probes;
+    long long before = incl - n, all = 0;
+    lists = 0;
+    for (int k = 0; k < kMapThreads / 32; ++k) {
+      if (k < wib) before += m.sum[k];
+      all += m.sum[k];
+      lists += m.lists[k];
+    }
+    // (the rule of k_bits_warp)
+    if (2 * all >= lists && lists <= 16LL * a.items) {
+      c += W <= 4 ? map_steps<K, 4>(a, w, m, unit, lists, tid)
+                  : map_steps<K, 8>(a, w, m, unit, lists, tid);
+      __syncthreads();
+      continue;
+    }
+    const long long lo = share(all, unit.y, unit.z), hi = share(all, unit.y + 1, unit.z);
+    const int total = (int)(hi - lo);
+    if (tid < w.d0) {
+      m.rel[tid] = (int)max(0LL, min(before + n - lo, (long long)total));
+      m.off[tid] = before < hi && before + n > lo ? (int)(lo - before) : 0;
+    }
+    __syncthreads();
+    uint32_t* out = m.table + wib * 32 * 8;
+    for (;;) {
+      int base = 0;
+      if (lane == 0) base = atomicAdd(&m.next, 32);
+      base = __shfl_sync(0xffffffffu, base, 0);
+      if (base >= total) break;
+      c += W <= 4 ? lane_steps<K, 4>(a, w, m.rel, m.off, out, base, total, lane)
+                  : lane_steps<K, 8>(a, w, m.rel, m.off, out, base, total, lane);
     }
     __syncthreads();
   }
@@ -928,6 +1295,9 @@ cudaError_t build_index(const DevGraph& g, int num_sms, cudaStream_t s) {
     e = cudaGetLastError();
   }
   if (e != cudaSuccess) return e;
+  g.plan_items = (long long)h[1] < (long long)num_sms * kMapWork
+                     ? 0
+                     : (int)std::min<long long>(8192, std::max<long long>(2048, 8 * l.step[1]));
   g.plan_units = (int4*)units.p;
   g.plan_un = (unsigned long long*)un.p;
   units.p = un.p = nullptr;
@@ -971,13 +1341,29 @@ cudaError_t launch_k(const DevGraph& g, BitArgs a, unsigned long long* heads, in
   }
   // launched for graphs without such a degree too (one block that finds no unit), so that
   // a plan's launches do not depend on the degrees below the list form's
-  cudaError_t e =
-      launch_cta<K, kThreads>(g, a, 1, kMidDeg, g.max_deg > kWarpDeg, heads, num_sms, s);
+  const bool any = g.max_deg > kWarpDeg;
+  cudaError_t e;
+  if (a.p.stream && g.plan_items) {
+    a.cls = 1;
+    a.units = g.plan_units + g.plan_off[1];
+    a.head = heads + 1;
+    a.items = g.plan_items;
+    e = cudaFuncSetAttribute(k_bits_map<K>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                             (int)sizeof(MapSmem));
+    if (e != cudaSuccess) return e;
+    k_bits_map<K><<<any ? num_sms * kMapBlocks : 1, kMapThreads, sizeof(MapSmem), s>>>(a);
+    e = cudaGetLastError();
+  } else {
+    e = launch_cta<K, kThreads>(g, a, 1, kMidDeg, any, heads, num_sms, s);
+  }
   if (e != cudaSuccess) return e;
   a.cls = 0;
   a.units = g.plan_units + g.plan_off[0];
   a.head = heads;
-  k_bits_warp<K><<<num_sms * 5, kThreads, 0, s>>>(a);
+  const int bytes = kWarps * (int)(sizeof(SmallWarp) + (a.p.stream ? sizeof(SmallMap) : 0));
+  e = cudaFuncSetAttribute(k_bits_warp<K>, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
+  if (e != cudaSuccess) return e;
+  k_bits_warp<K><<<num_sms * 4, kThreads, bytes, s>>>(a);
   *launches += 2;
   return cudaGetLastError();
 }
