@@ -17,7 +17,7 @@
 //    thread, longer ones go to a table in shared memory, longest first, and are tested by
 //    eight lanes each, a 16-byte unit per lane and step.  A hub's in-neighbours are many
 //    units (u, chunk) that any CTA can take.
-//  - the other u: one lane per edge (v, u) merges the suffix with N+(u); both are short
+//  - the other u: one lane per edge (v, u) meets the suffix with N+(u) (merge_lists); both are short
 //    (deg v <= deg u <= kBigDeg).
 // Bitmaps are cleared by taking the inserted bits out again: a unit costs d+(u) stores,
 // not the bitmap's size.
@@ -28,14 +28,14 @@
 // matrix (k = 4 .. 7).
 //
 // Measured (GB300, a call before -> now):
-//  triangles  R-MAT s20 ef16 8.45 -> 1.48 ms; Barabasi-Albert, 3,312 vertices, 106 -> 28 us
+//  triangles  R-MAT s20 ef16 8.45 -> 1.42 ms; Barabasi-Albert, 3,312 vertices, 106 -> 26 us
 //             (13 launches -> 1: no task lists)
 //  4-cliques  R-MAT s22 65.6 -> 22.1 ms (rows 11.9, counting 9.6); s20 12.4 -> 3.5 ms
 //  5-cliques  R-MAT s20 140 -> 29 ms; 6-cliques R-MAT s16 96 -> 10.6 ms
-//  triangles per edge (diamonds), Chung-Lu 1.5 M vertices, degree 32: 9.9 -> 3.5 ms; R-MAT
+//  triangles per edge (diamonds), Chung-Lu 1.5 M vertices, degree 32: 9.9 -> 3.3 ms; R-MAT
 //             s19 3.76 -> 1.47 ms (the hits' rank look-ups and counters: the bare count of
 //             the same suffixes is 2.5 times faster)
-//  4,096 Barabasi-Albert graphs, triangles + 4-cliques + diamonds each: 3.44 -> 1.54 ms
+//  4,096 Barabasi-Albert graphs, triangles + 4-cliques + diamonds each: 3.44 -> 1.17 ms
 // The tests with a warp per suffix, a ballot per 32 elements: 1.86 ms (s20 triangles), 15.2
 // ms (s22 rows): 145 instructions a pair, of which a third for the pair itself.
 // Bound: R-MAT s22 rows, L2 and DRAM latency (2.2 G sectors, 12 GB of DRAM reads: the lists
@@ -124,20 +124,30 @@ struct RowWriter {
 };
 
 // Calls f(k, l) for every element the sorted ranges [a, ea) and [b, eb) of col have in common,
-// at col[k] and col[l].
+// at col[k] and col[l], k ascending.  Eight of b's elements at a time stay in registers and every
+// one of a's up to the last of them is compared with all: the loads do not wait for one another
+// as a merge's do, and lanes with lists of other lengths part less.  4,096 small graphs (5.5
+// out-neighbours a vertex), the owner kernel: 1.05 ms by a merge, 0.80 with four held, 0.69 with
+// six, 0.67 with eight.
+constexpr int kMergeHold = 8;
 template <class F>
 __device__ __forceinline__ void merge_lists(const int32_t* col, long long a, long long ea,
                                             long long b, long long eb, F f) {
-  if (a >= ea || b >= eb) return;
-  int32_t x = ldg_i32(col + a), y = ldg_i32(col + b);
-  for (;;) {
-    const bool le = x <= y, ge = x >= y;
-    if (le && ge) f(a, b);
-    a += le;
-    b += ge;
-    if (a >= ea || b >= eb) return;
-    if (le) x = ldg_i32(col + a);
-    if (ge) y = ldg_i32(col + b);
+  if (a >= ea) return;
+  for (; b < eb; b += kMergeHold) {
+    int32_t y[kMergeHold];
+#pragma unroll
+    for (int j = 0; j < kMergeHold; ++j) y[j] = b + j < eb ? ldg_i32(col + b + j) : INT32_MAX;
+    for (;;) {
+      const int32_t x = ldg_i32(col + a);
+      if (x > y[kMergeHold - 1]) break;
+      int at = -1;
+#pragma unroll
+      for (int j = 0; j < kMergeHold; ++j)
+        if (y[j] == x) at = j;
+      if (at >= 0) f(a, b + at);
+      if (++a >= ea) return;
+    }
   }
 }
 
@@ -152,10 +162,10 @@ __device__ __forceinline__ long long lower_at(const int32_t* col, long long lo, 
 
 // CTAs per SM the registers are cut for, measured per mode (the bitmap allows 5 at R-MAT s22):
 // triangles s20 1.52 / 1.49 / 1.43 ms with 4 / 5 / 6, rows s22 11.9 / 13.9 / 13.5,
-// participation of a 1.5 M vertex Chung-Lu graph 3.72 / 3.53 / 4.23, rows and participation
-// of 4,096 small graphs 1.26 / 1.13 / 1.04.
+// participation of a 1.5 M vertex Chung-Lu graph 3.47 / 3.30 / 3.95, rows and participation
+// of 4,096 small graphs 0.71 / 0.67 / 0.71.
 constexpr int own_ctas(int mode) {
-  return mode == kOwnRows ? 4 : (mode == kOwnPart ? 5 : 6);
+  return mode == kOwnRows ? 4 : (mode == kOwnCount ? 6 : 5);
 }
 
 template <int MODE>
