@@ -176,29 +176,37 @@ __global__ void k_rank_entry_keys(const int64_t* rowptr_o, const int32_t* col_o,
         src = rowptr_o[perm[r]];
       }
     }
-    int64_t incl = len;
+    int incl = (int)len;  // at most 32 * kLongRow
 #pragma unroll
     for (int o = 1; o < 32; o <<= 1) {
-      const int64_t y = __shfl_up_sync(0xffffffffu, incl, o);
+      const int y = __shfl_up_sync(0xffffffffu, incl, o);
       if (lane >= o) incl += y;
     }
-    const int64_t total = __shfl_sync(0xffffffffu, incl, 31);
-    const int64_t excl = incl - len;
-    for (int64_t b = 0; b < total; b += 32) {
-      const int64_t t = b + lane;
-      int k = 0;  // last row whose first flat index is <= t
+    const int total = __shfl_sync(0xffffffffu, incl, 31);
+    const int excl = incl - (int)len;
+    src -= excl;
+    dst -= excl;
+    // four entries a lane at a time: their column loads, then their rank loads, overlap
+    for (int b = 0; b < total; b += 128) {
+      int64_t at[4];
+      int32_t c[4], row[4];
 #pragma unroll
-      for (int step = 16; step > 0; step >>= 1) {
-        const int64_t ex = __shfl_sync(0xffffffffu, excl, k + step);
-        if (ex <= t) k += step;
+      for (int u = 0; u < 4; ++u) {
+        const int t = b + 32 * u + lane;
+        int k = 0;  // last row whose first flat index is <= t
+#pragma unroll
+        for (int step = 16; step > 0; step >>= 1) {
+          const int ex = __shfl_sync(0xffffffffu, excl, k + step);
+          if (ex <= t) k += step;
+        }
+        const int64_t ks = __shfl_sync(0xffffffffu, src, k);
+        at[u] = __shfl_sync(0xffffffffu, dst, k) + t;
+        row[u] = k;
+        c[u] = t < total ? col_o[ks + t] : -1;
       }
-      const int64_t ks = __shfl_sync(0xffffffffu, src, k);
-      const int64_t kd = __shfl_sync(0xffffffffu, dst, k);
-      const int64_t kx = __shfl_sync(0xffffffffu, excl, k);
-      if (t < total) {
-        const int64_t j = t - kx;
-        keys[kd + j] = ((uint64_t)rank[col_o[ks + j]] << vb) | (uint64_t)(r0 + k);
-      }
+#pragma unroll
+      for (int u = 0; u < 4; ++u)
+        if (c[u] >= 0) keys[at[u]] = ((uint64_t)rank[c[u]] << vb) | (uint64_t)(r0 + row[u]);
     }
   }
 }
@@ -219,13 +227,6 @@ __global__ void k_rank_entry_keys_long(const int64_t* rowptr_o, const int32_t* c
     for (int64_t j = lo + threadIdx.x; j < hi; j += blockDim.x)
       keys[dst + j] = ((uint64_t)rank[col_o[src + j]] << vb) | (uint64_t)r;
   }
-}
-
-__global__ void k_extract_col(const uint64_t* keys, int64_t ne, int vb, int32_t* col) {
-  const uint64_t vmask = (1ull << vb) - 1;
-  for (int64_t e = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; e < ne;
-       e += (int64_t)gridDim.x * blockDim.x)
-    col[e] = (int32_t)(keys[e] & vmask);
 }
 
 // dptr[r] = {first entry of row r with id > r, row end}; stats of the DAG.
@@ -475,12 +476,8 @@ cudaError_t finish_graph(DevGraph& g, const int32_t* group, int num_groups, cuda
     TRY(cudaGetLastError());
     cudaFreeAsync(longs, s);
   }
-  uint64_t* sorted = keys;
-  TRY(radix_sort_u64(keys, tmp, ne, vb, s, vb, &sorted));
-  if (ne > 0) {
-    k_extract_col<<<grid_for(ne), kThreads, 0, s>>>(sorted, ne, vb, g.col);
-    TRY(cudaGetLastError());
-  }
+  // the last pass writes the columns alone
+  TRY(radix_sort_u64(keys, tmp, ne, vb, s, vb, g.col, (uint32_t)((1ull << vb) - 1)));
   if (nv > 0) {
     k_dptr<<<grid_for(nv), kThreads, 0, s>>>(g.rowptr, g.col, nv, g.dptr, stats + 1, stats + 2,
                                              stats + 4, stats + 5);
