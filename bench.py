@@ -198,9 +198,9 @@ def measured_peaks() -> dict:
 
 
 def profile_summary(pattern: str, scale: int) -> dict:
-    """`key: value` lines of the committed ncu summary of the counting kernel
-    (profiles/k_clique<k>_rmat_s<scale>.md): DRAM traffic per launch and issue rate."""
-    name = {"4-clique": "k_clique4", "5-clique": "k_clique5", "triangle": "k_clique3"}[pattern]
+    """`key: value` lines of the committed ncu summary of the counting kernels
+    (profiles/rows<k>_rmat_s<scale>.md): DRAM traffic of a count, issue rate of its longest."""
+    name = {"4-clique": "rows4", "5-clique": "rows5", "triangle": "rows3"}[pattern]
     path = os.path.join(ROOT, "profiles", f"{name}_rmat_s{scale}.md")
     out = {"path": os.path.relpath(path, ROOT)}
     if not os.path.exists(path):
@@ -464,12 +464,12 @@ def engine_arm(args, dist: Dist) -> None:
         "frac": achieved / peaks["hbm_gbs"] if achieved else None,
         "traffic": int(traffic) if traffic else None,
         "traffic_source": (f"{prof['path']} (ncu dram__bytes_read.sum + dram__bytes_write.sum "
-                           "of this launch, committed capture; divided by this run's "
+                           "of a count's kernels, committed capture; divided by this run's "
                            "CUDA-event kernel time)") if traffic else "no committed capture",
         "peak_source": peaks["source"],
         # the reference plan's algorithmic bytes (4 B per list element it reads + 8 B per
-        # task): this kernel reads each list once per vertex task instead, so the plan's
-        # bytes over the launch time exceed the copy peak
+        # task): these kernels test each pair of a list once instead, so the plan's bytes
+        # over their time exceed the copy peak
         "plan_bytes_per_launch": plan,
         "plan_gbs": plan / (kern_ms / 1e3) / 1e9,
         "issue_active_pct": prof.get("issue_active_pct"),
