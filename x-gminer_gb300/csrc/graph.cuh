@@ -32,11 +32,11 @@ struct DevGraph {
   mutable uint16_t* bmask = nullptr;
   // set-operation programs (setbits.cu), built on first use: plan_deg is the largest
   // degree whose tasks run in the bitmap form (-1 none, 0 not built); its units {v0, part,
-  // parts} by class from plan_off[class], their numbers in plan_un; adjacency rows among
-  // N(v) for v of degree 33..1024, lut_off[v] words into lut_rows
+  // parts} by class from plan_off[class], at most plan_cap[class], their numbers in plan_un;
+  // adjacency rows among N(v) for v of degree 33..1024, lut_off[v] words into lut_rows
   mutable int plan_deg = 0;
   mutable int4* plan_units = nullptr;
-  mutable int64_t plan_off[3] = {0, 0, 0};
+  mutable int64_t plan_off[3] = {0, 0, 0}, plan_cap[3] = {0, 0, 0};
   mutable unsigned long long* plan_un = nullptr;
   mutable int plan_items = 0;  // list entries a block takes to a table at a time (0: no tables)
   mutable uint32_t* lut_rows = nullptr;

@@ -33,7 +33,7 @@
 // What bounds them: instruction issue (60-80 %, the integer pipe).  P7 on R-MAT scale 12
 // (5.9 M steps, 119 M v3 candidates): 6.40 ms when k_setlut and k_setprog interpreted the
 // operations with binary searches in lists, 1.97 ms with a look-up of every v2's list (400 M
-// look-ups), 1.32 ms with the tables; P15 on Erdos-Renyi 2^16 2.25, 1.25, 0.67 ms.
+// look-ups), 1.05 ms with the tables; P15 on Erdos-Renyi 2^16 2.25, 1.25, 0.67 ms.
 // R-MAT scale 9 P7 1.84 ms -> 0.12, where a few heavy tasks were the time; P10 on
 // Erdos-Renyi 2^16 0.83 -> 0.24 ms.
 #include <algorithm>
@@ -64,6 +64,17 @@ struct CtaLayout {
   int deg, buckets;
   int n0, key, pos, rel, off, warp, per_warp, bytes;
 };
+
+// The kernels of one count do not depend on one another: each may start as soon as every block
+// of the one before has, and ends after it (the stream's next operation follows the last).  P7
+// on R-MAT scale 11 0.54 -> 0.39 ms, on scale 12 1.32 -> 1.05: each kernel's tail is the next
+// one's beginning.
+__device__ __forceinline__ void let_next_start() {
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+}
+__device__ __forceinline__ void wait_for_previous() {
+  asm volatile("griddepcontrol.wait;" ::: "memory");
+}
 
 struct BitArgs {
   const int64_t* rowptr;
@@ -180,14 +191,6 @@ __device__ __forceinline__ int nth_bit(uint32_t m, int n) {
   }
   return at;
 }
-
-// Rows of v1 and v2 (NW words) and their places, for one step or one task.
-template <int NW>
-struct Step {
-  uint32_t r1[NW], r2[NW];
-  int i1, i2;      // index in N(v0); i2 = -1 outside it
-  int pre0, pre2;  // elements of N(v0) below v0, v2
-};
 
 // Word `wi` of a term over v1 (and v2 if `two`), of the words r1 and r2 of their rows; a
 // bound or exclusion by v3 is left out.
@@ -601,6 +604,7 @@ __device__ __forceinline__ unsigned long long small_map(const BitArgs& a, const 
 template <int K>
 __global__ void __launch_bounds__(kThreads, 4) k_bits_warp(BitArgs a) {
   extern __shared__ __align__(16) unsigned char sm[];
+  let_next_start();
   const int lane = threadIdx.x & 31;
   SmallWarp& w = ((SmallWarp*)sm)[threadIdx.x >> 5];
   // (a stream program's launch only)
@@ -683,6 +687,7 @@ __global__ void __launch_bounds__(kThreads, 4) k_bits_warp(BitArgs a) {
 #pragma unroll
   for (int o = 16; o > 0; o >>= 1) c += __shfl_xor_sync(0xffffffffu, c, o);
   if (lane == 0 && c) atomicAdd(a.total, c);
+  wait_for_previous();
 }
 
 // ------------------------------------------------------- 33 <= d(v0) <= 1,024
@@ -841,6 +846,7 @@ __device__ __forceinline__ int load_v0(const BitArgs& a, Local& w, int v0, int32
 template <int K, int NT>
 __global__ void __launch_bounds__(NT, NT == kThreads ? 4 : 1) k_bits_cta(BitArgs a) {
   extern __shared__ __align__(16) unsigned char sm[];
+  let_next_start();
   const CtaLayout& L = a.lay;
   __shared__ int64_t s_unit;
   __shared__ int s_next, s_probes;
@@ -930,6 +936,7 @@ __global__ void __launch_bounds__(NT, NT == kThreads ? 4 : 1) k_bits_cta(BitArgs
 #pragma unroll
   for (int o = 16; o > 0; o >>= 1) c += __shfl_xor_sync(0xffffffffu, c, o);
   if (lane == 0 && c) atomicAdd(a.total, c);
+  wait_for_previous();
 }
 
 // Stream programs, 33 <= d(v0) <= 256: a block takes the steps of a v0 from tables of its
@@ -1021,6 +1028,7 @@ __device__ __forceinline__ unsigned long long map_steps(const BitArgs& a, const 
 template <int K>
 __global__ void __launch_bounds__(kMapThreads, kMapBlocks) k_bits_map(BitArgs a) {
   extern __shared__ __align__(16) unsigned char sm[];
+  let_next_start();
   MapSmem& m = *(MapSmem*)sm;
   const int tid = threadIdx.x, lane = tid & 31, wib = tid >> 5;
   Local w;
@@ -1095,6 +1103,7 @@ __global__ void __launch_bounds__(kMapThreads, kMapBlocks) k_bits_map(BitArgs a)
 #pragma unroll
   for (int o = 16; o > 0; o >>= 1) c += __shfl_xor_sync(0xffffffffu, c, o);
   if (lane == 0 && c) atomicAdd(a.total, c);
+  wait_for_previous();
 }
 
 // --------------------------------------------------------------- per-graph index
@@ -1284,6 +1293,7 @@ cudaError_t build_index(const DevGraph& g, int num_sms, cudaStream_t s) {
   for (int k = 0; k < 3; ++k) {
     l.list[k] = cap[k] ? (int4*)units.p + at : nullptr;
     g.plan_off[k] = at;
+    g.plan_cap[k] = cap[k];
     at += cap[k];
   }
   k_bits_units<<<wblocks, kThreads, 0, s>>>(g.rowptr_o, (const int64_t*)work.p, nv, l,
@@ -1310,8 +1320,30 @@ cudaError_t build_index(const DevGraph& g, int num_sms, cudaStream_t s) {
   return cudaSuccess;
 }
 
+// No more blocks than there are units for: a small graph would only pay for starting them.
+unsigned blocks(int most, int64_t units) {
+  return (unsigned)std::max<int64_t>(1, std::min<int64_t>(most, units));
+}
+
+cudaError_t launch(void (*kern)(BitArgs), unsigned grid, int threads, int bytes, cudaStream_t s,
+                   const BitArgs& a, bool first) {
+  cudaLaunchConfig_t c{};
+  c.gridDim = dim3(grid);
+  c.blockDim = dim3((unsigned)threads);
+  c.dynamicSmemBytes = (size_t)bytes;
+  c.stream = s;
+  cudaLaunchAttribute at{};
+  at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  at.val.programmaticStreamSerializationAllowed = 1;
+  c.attrs = &at;
+  c.numAttrs = first ? 0 : 1;
+  cudaError_t e =
+      cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
+  return e == cudaSuccess ? cudaLaunchKernelEx(&c, kern, a) : e;
+}
+
 template <int K, int NT>
-cudaError_t launch_cta(const DevGraph& g, BitArgs a, int cls, int deg, bool any,
+cudaError_t launch_cta(const DevGraph& g, BitArgs a, int cls, int deg, bool any, bool first,
                        unsigned long long* heads, int num_sms, cudaStream_t s) {
   // the shared memory that the graph's own degrees need: more blocks an SM
   a.lay = cta_layout((int)std::min<int64_t>(deg, (std::max<int64_t>(g.max_deg, 1) + 127) / 128 * 128),
@@ -1319,25 +1351,27 @@ cudaError_t launch_cta(const DevGraph& g, BitArgs a, int cls, int deg, bool any,
   auto kern = k_bits_cta<K, NT>;
   cudaError_t e =
       cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, a.lay.bytes);
-  if (e != cudaSuccess) return e;
   int per_sm = 1;
-  if (any) e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, NT, a.lay.bytes);
+  if (e == cudaSuccess && any)
+    e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, NT, a.lay.bytes);
   if (e != cudaSuccess) return e;
   a.cls = cls;
   a.units = g.plan_units + g.plan_off[cls];
   a.head = heads + cls;
-  kern<<<any ? num_sms * std::max(per_sm, 1) : 1, NT, a.lay.bytes, s>>>(a);
-  return cudaGetLastError();
+  return launch(kern, blocks(num_sms * std::max(per_sm, 1), g.plan_cap[cls]), NT, a.lay.bytes, s, a,
+                first);
 }
 
 template <int K>
 cudaError_t launch_k(const DevGraph& g, BitArgs a, unsigned long long* heads, int num_sms,
                      cudaStream_t s, int* launches) {
   // the larger degrees first: a small unit fills what their last blocks leave
+  bool first = true;
   if (g.plan_deg > kMidDeg && g.max_deg > kMidDeg && g.lut_rows) {
-    cudaError_t e = launch_cta<K, kTopThreads>(g, a, 2, kTopDeg, true, heads, num_sms, s);
+    cudaError_t e = launch_cta<K, kTopThreads>(g, a, 2, kTopDeg, true, first, heads, num_sms, s);
     if (e != cudaSuccess) return e;
     ++*launches;
+    first = false;
   }
   // launched for graphs without such a degree too (one block that finds no unit), so that
   // a plan's launches do not depend on the degrees below the list form's
@@ -1348,24 +1382,21 @@ cudaError_t launch_k(const DevGraph& g, BitArgs a, unsigned long long* heads, in
     a.units = g.plan_units + g.plan_off[1];
     a.head = heads + 1;
     a.items = g.plan_items;
-    e = cudaFuncSetAttribute(k_bits_map<K>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                             (int)sizeof(MapSmem));
-    if (e != cudaSuccess) return e;
-    k_bits_map<K><<<any ? num_sms * kMapBlocks : 1, kMapThreads, sizeof(MapSmem), s>>>(a);
-    e = cudaGetLastError();
+    e = launch(k_bits_map<K>, blocks(num_sms * kMapBlocks, g.plan_cap[1]), kMapThreads,
+               (int)sizeof(MapSmem), s, a, first);
   } else {
-    e = launch_cta<K, kThreads>(g, a, 1, kMidDeg, any, heads, num_sms, s);
+    e = launch_cta<K, kThreads>(g, a, 1, kMidDeg, any, first, heads, num_sms, s);
   }
   if (e != cudaSuccess) return e;
   a.cls = 0;
   a.units = g.plan_units + g.plan_off[0];
   a.head = heads;
   const int bytes = kWarps * (int)(sizeof(SmallWarp) + (a.p.stream ? sizeof(SmallMap) : 0));
-  e = cudaFuncSetAttribute(k_bits_warp<K>, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
+  e = launch(k_bits_warp<K>, blocks(num_sms * 4, (g.plan_cap[0] + kWarps - 1) / kWarps), kThreads,
+             bytes, s, a, false);
   if (e != cudaSuccess) return e;
-  k_bits_warp<K><<<num_sms * 4, kThreads, bytes, s>>>(a);
   *launches += 2;
-  return cudaGetLastError();
+  return cudaSuccess;
 }
 
 }  // namespace
