@@ -54,6 +54,32 @@ __device__ __forceinline__ uint64_t warp_sum_u64(uint64_t v) {
   return v;
 }
 
+// Kernels of a call that do not depend on one another: each lets the next start as soon as all
+// of its own blocks have, and ends after the one before (so the stream's next operation follows
+// all of them).  The first is launched in stream order, the others by launch_next.
+__device__ __forceinline__ void let_next_start() {
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+}
+__device__ __forceinline__ void wait_for_previous() {
+  asm volatile("griddepcontrol.wait;" ::: "memory");
+}
+
+template <class... P, class... A>
+cudaError_t launch_next(bool first, void (*kern)(P...), int64_t grid, int threads, int smem,
+                        cudaStream_t s, A... args) {
+  cudaLaunchConfig_t c{};
+  c.gridDim = dim3((unsigned)grid);
+  c.blockDim = dim3((unsigned)threads);
+  c.dynamicSmemBytes = (size_t)smem;
+  c.stream = s;
+  cudaLaunchAttribute at{};
+  at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  at.val.programmaticStreamSerializationAllowed = 1;
+  c.attrs = &at;
+  c.numAttrs = first ? 0 : 1;
+  return cudaLaunchKernelEx(&c, kern, P(args)...);
+}
+
 // Row load that bypasses L1 allocation for streaming adjacency reads.
 __device__ __forceinline__ int32_t ldg_i32(const int32_t* p) { return __ldg(p); }
 __device__ __forceinline__ longlong2 ldg_ll2(const longlong2* p) { return __ldg(p); }

@@ -1085,6 +1085,7 @@ __global__ void __launch_bounds__(NT, team_ctas(K, NT)) k_rows_team(RowTasks t, 
   constexpr int kWarps = NT / 32, kTeams = kWarps / kTeam;
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   constexpr int kParts = team_parts(K, NT);
+  let_next_start();
   const long long nt = (long long)*t.n;
   uint64_t total = 0;
   if (tid == 0) task_s = (long long)atomicAdd(head, 1ull);
@@ -1186,6 +1187,7 @@ __global__ void __launch_bounds__(NT, team_ctas(K, NT)) k_rows_team(RowTasks t, 
   }
   total = warp_sum_u64(total);
   if (lane == 0 && total) atomicAdd(count, (unsigned long long)total);
+  wait_for_previous();
 }
 
 // Tasks of up to 32 out-neighbours, a warp each, lane i holding row i.  K = 4: one block on
@@ -1303,11 +1305,13 @@ __global__ void __launch_bounds__(kWordThreads, KIND == 3 ? 4 : 1)
     k_rows_narrow(RowTasks word, RowTasks group, OwnHeads* heads, unsigned long long* count,
                   GOut o) {
   __shared__ uint32_t rows_s[kWordThreads];
+  let_next_start();
   uint64_t acc = 0;
   if (KIND & 1) acc += word_tasks<K>(word, &heads->word, o, rows_s);
   if (KIND & 2) acc += group_tasks<K>(group, &heads->group, o, rows_s);
   acc = warp_sum_u64(acc);
   if ((threadIdx.x & 31) == 0 && acc) atomicAdd(count, (unsigned long long)acc);
+  wait_for_previous();
 }
 constexpr int64_t kOneNarrow = int64_t(1) << 17;  // tasks up to which both kinds share a launch
 
@@ -1324,7 +1328,8 @@ static_assert(4 * team_words<7, 16>(kRowsCap / 32) <= 226 * 1024, "wide tasks fi
 
 template <int K, int NT>
 cudaError_t launch_team(const DevGraph& g, RowTasks t, int cap, unsigned long long* head,
-                        unsigned long long* count, int num_sms, cudaStream_t s, const GOut& o) {
+                        unsigned long long* count, int num_sms, cudaStream_t s, const GOut& o,
+                        bool first) {
   t.wcap = (int)((std::min<int64_t>(g.max_out, cap) + 31) / 32);
   const int smem = 4 * team_words<K, NT / 32>(t.wcap);
   int grid = 0, dev = 0;
@@ -1340,8 +1345,7 @@ cudaError_t launch_team(const DevGraph& g, RowTasks t, int cap, unsigned long lo
   if (e == cudaSuccess) e = full_grid(k_rows_team<K, NT>, NT, smem, num_sms, &grid);
   if (e != cudaSuccess) return e;
   grid = (int)std::min<int64_t>(grid, g.nv * team_parts(K, NT));
-  k_rows_team<K, NT><<<grid, NT, smem, s>>>(t, head, count, o);
-  return cudaGetLastError();
+  return launch_next(first, k_rows_team<K, NT>, grid, NT, smem, s, t, head, count, o);
 }
 
 template <int K>
@@ -1349,13 +1353,15 @@ cudaError_t launch_rows_k(const DevGraph& g, const uint32_t* rows, OwnHeads* hea
                           unsigned long long* count, int num_sms, cudaStream_t s, const GOut& o) {
   const unsigned long long* rn = g.rn;
   cudaError_t e = cudaSuccess;
-  if (g.max_out > kRowsMid) {
+  bool first = g.max_out <= kRowsMid;
+  if (!first) {
     const RowTasks t{g.dptr, g.roff, rows, g.rtask + 2 * g.nv - 1, rn + 4, 1, 0};
-    e = launch_team<K, K == 4 ? 256 : 512>(g, t, kRowsCap, &heads->wide, count, num_sms, s, o);
+    e = launch_team<K, K == 4 ? 256 : 512>(g, t, kRowsCap, &heads->wide, count, num_sms, s, o, true);
   }
   if (e == cudaSuccess && g.max_out > 32) {
     const RowTasks t{g.dptr, g.roff, rows, g.rtask + g.nv, rn + 3, 0, 0};
-    e = launch_team<K, 128>(g, t, kRowsMid, &heads->team, count, num_sms, s, o);
+    e = launch_team<K, 128>(g, t, kRowsMid, &heads->team, count, num_sms, s, o, first);
+    first = false;
   }
   if (e != cudaSuccess) return e;
   // at most `roots` word and group tasks; claims small enough that every warp has a few
@@ -1370,8 +1376,9 @@ cudaError_t launch_rows_k(const DevGraph& g, const uint32_t* rows, OwnHeads* hea
     const RowTasks word{g.dptr, g.roff, rows, g.rtask + g.nv - 1, rn + 2, 1,
                         (int)std::max<int64_t>(claim, 1)};
     const RowTasks group{g.dptr, g.roff, rows, g.rtask, rn + 1, 0, (int)std::max<int64_t>(claim, 4)};
-    kernel<<<grid, kWordThreads, 0, s>>>(word, group, heads, count, o);
-    return cudaGetLastError();
+    const bool f = first;
+    first = false;
+    return launch_next(f, kernel, grid, kWordThreads, 0, s, word, group, heads, count, o);
   };
   if (g.max_out <= 8) return narrow(k_rows_narrow<K, 2>, 4);
   if (roots <= kOneNarrow) return narrow(k_rows_narrow<K, 3>, 1);

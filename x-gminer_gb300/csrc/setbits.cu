@@ -65,17 +65,6 @@ struct CtaLayout {
   int n0, key, pos, rel, off, warp, per_warp, bytes;
 };
 
-// The kernels of one count do not depend on one another: each may start as soon as every block
-// of the one before has, and ends after it (the stream's next operation follows the last).  P7
-// on R-MAT scale 11 0.54 -> 0.39 ms, on scale 12 1.32 -> 1.05: each kernel's tail is the next
-// one's beginning.
-__device__ __forceinline__ void let_next_start() {
-  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
-}
-__device__ __forceinline__ void wait_for_previous() {
-  asm volatile("griddepcontrol.wait;" ::: "memory");
-}
-
 struct BitArgs {
   const int64_t* rowptr;
   const int32_t* col;
@@ -1327,19 +1316,9 @@ unsigned blocks(int most, int64_t units) {
 
 cudaError_t launch(void (*kern)(BitArgs), unsigned grid, int threads, int bytes, cudaStream_t s,
                    const BitArgs& a, bool first) {
-  cudaLaunchConfig_t c{};
-  c.gridDim = dim3(grid);
-  c.blockDim = dim3((unsigned)threads);
-  c.dynamicSmemBytes = (size_t)bytes;
-  c.stream = s;
-  cudaLaunchAttribute at{};
-  at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
-  at.val.programmaticStreamSerializationAllowed = 1;
-  c.attrs = &at;
-  c.numAttrs = first ? 0 : 1;
-  cudaError_t e =
+  const cudaError_t e =
       cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
-  return e == cudaSuccess ? cudaLaunchKernelEx(&c, kern, a) : e;
+  return e == cudaSuccess ? launch_next(first, kern, grid, threads, bytes, s, a) : e;
 }
 
 template <int K, int NT>
@@ -1365,7 +1344,8 @@ cudaError_t launch_cta(const DevGraph& g, BitArgs a, int cls, int deg, bool any,
 template <int K>
 cudaError_t launch_k(const DevGraph& g, BitArgs a, unsigned long long* heads, int num_sms,
                      cudaStream_t s, int* launches) {
-  // the larger degrees first: a small unit fills what their last blocks leave
+  // the larger degrees first; each kernel's tail is the next one's beginning (P7 on R-MAT scale
+  // 11 0.54 -> 0.39 ms, on scale 12 1.32 -> 1.05, against one after the other)
   bool first = true;
   if (g.plan_deg > kMidDeg && g.max_deg > kMidDeg && g.lut_rows) {
     cudaError_t e = launch_cta<K, kTopThreads>(g, a, 2, kTopDeg, true, first, heads, num_sms, s);
