@@ -250,7 +250,7 @@ xgm_status batch_sequence(xgm_ctx* ctx, xgm_batch* b, const Slots& sl, int P,
     }
     if (part)
       XGM_CUDA_TRY(launch_graph_terms(view, g.gid, b->num_graphs, b->epart, b->sums, b->d_out, P,
-                                      sl.tri, sl.dia, sl.tail, s));
+                                      sl.tri, sl.dia, sl.tail, s, k));
   } else if (sl.tri >= 0 || sl.k4 >= 0 || sl.dia >= 0 || sl.tail >= 0) {
     const bool part = sl.dia >= 0 || sl.tail >= 0;
     if (part) {

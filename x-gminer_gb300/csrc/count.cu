@@ -480,12 +480,17 @@ xgm_status motif4_parts(xgm_ctx* ctx, const DevGraph& g, const xgm_sched& sp, bo
     XGM_CUDA_TRY(cudaMemsetAsync(ctx->epart, 0, sizeof(unsigned) * (g.ne > 0 ? g.ne : 1), s));
     XGM_CUDA_TRY(ctx_mark(ctx, 1));
     XGM_CUDA_TRY(launch_owner_multi(g, ctx->rows, ctx->epart, &sc->own, ctx->num_sms, s));
-    XGM_CUDA_TRY(launch_rows_count(4, g, ctx->rows, &sc->own, &sc->count, ctx->num_sms, s));
-    XGM_CUDA_TRY(launch_motif_terms(g.view(), ctx->epart, sc->terms, s));
+    // the 4-cycles depend on nothing before them, the others on the owner kernel alone: a
+    // kernel that starts in stream order after one that waits for it is past its end
+    bool next = false;
     if (need_c4) {
       const C4Lists lists{ctx->c4_lists, ctx->c4_lists + g.nv, ctx->c4_lists + 2 * g.nv};
-      XGM_CUDA_TRY(launch_cycle4(g, &sc->c4, lists, &sc->aux, ctx->num_sms, s));
+      XGM_CUDA_TRY(launch_cycle4(g, &sc->c4, lists, &sc->aux, ctx->num_sms, s, GOut{}, true));
+      next = cycle4_has_cta(g);
     }
+    XGM_CUDA_TRY(launch_rows_count(4, g, ctx->rows, &sc->own, &sc->count, ctx->num_sms, s, GOut{},
+                                   next));
+    XGM_CUDA_TRY(launch_motif_terms(g.view(), ctx->epart, sc->terms, s, true));
     XGM_CUDA_TRY(ctx_mark(ctx, 2));
     xgm_status q = ctx_sync_scalars(ctx);
     if (q != XGM_OK) return q;

@@ -163,6 +163,7 @@ __global__ void __launch_bounds__(kWarpThreads, 4) k_c4_warp(GView g, C4Queue* q
                                                              int step, unsigned long long* out,
                                                              GOut o) {
   extern __shared__ __align__(16) char sm[];
+  let_next_start();
   const int lane = threadIdx.x & 31;
   WarpTable& t = reinterpret_cast<WarpTable*>(sm)[threadIdx.x >> 5];
   unsigned long long acc = 0;
@@ -242,6 +243,7 @@ __global__ void __launch_bounds__(kWarpThreads, 4) k_c4_warp(GView g, C4Queue* q
   }
   acc = warp_sum_u64(acc);
   if (lane == 0 && acc) atomicAdd(out, acc);
+  wait_for_previous();
 }
 
 // The wedges of v0 whose v2 is in [a, a + tile), one tile of counters.  Every warp takes 32
@@ -320,6 +322,7 @@ __device__ unsigned long long tile_wedges(const GView& g, CtaTile& t, int* next,
 __global__ void __launch_bounds__(kCtaThreads4, 2) k_c4_cta(GView g, C4Queue* q, C4Lists l,
                                                             unsigned long long* out, GOut o) {
   extern __shared__ __align__(16) char sm[];
+  let_next_start();
   __shared__ long long task_s;
   constexpr int kWarps = kCtaThreads4 / 32;
   __shared__ int next, wsum[kWarps];
@@ -417,12 +420,19 @@ __global__ void __launch_bounds__(kCtaThreads4, 2) k_c4_cta(GView g, C4Queue* q,
   }
   acc = warp_sum_u64(acc);
   if (lane == 0 && acc) atomicAdd(out, acc);
+  wait_for_previous();
 }
 
 }  // namespace
 
+bool cycle4_has_cta(const DevGraph& g) {
+  // v0 has at most max_deg lower neighbours, with rows of at most max_deg
+  return g.max_deg * g.max_deg > kWarpWedges;
+}
+
 cudaError_t launch_cycle4(const DevGraph& g, C4Queue* q, const C4Lists& l,
-                          unsigned long long* out, int num_sms, cudaStream_t s, const GOut& o) {
+                          unsigned long long* out, int num_sms, cudaStream_t s, const GOut& o,
+                          bool next) {
   if (g.nv == 0) return cudaSuccess;
   constexpr int kWarps = kWarpThreads / 32;
   constexpr int smem = kWarps * (int)sizeof(WarpTable);
@@ -440,10 +450,8 @@ cudaError_t launch_cycle4(const DevGraph& g, C4Queue* q, const C4Lists& l,
   if (e != cudaSuccess) return e;
   const int64_t grid = std::min<int64_t>(4 * num_sms, (g.nv + kWarps - 1) / kWarps);
   const int step = (int)std::max<int64_t>(1, std::min<int64_t>(32, g.nv / (4 * kWarps * grid)));
-  k_c4_warp<<<(unsigned)grid, kWarpThreads, smem, s>>>(g.view(), q, l, step, out, o);
-  e = cudaGetLastError();
-  // v0 has at most max_deg lower neighbours, with rows of at most max_deg
-  if (e != cudaSuccess || g.max_deg * g.max_deg <= kWarpWedges) return e;
+  e = launch_next(!next, k_c4_warp, grid, kWarpThreads, smem, s, g.view(), q, l, step, out, o);
+  if (e != cudaSuccess || !cycle4_has_cta(g)) return e;
   k_c4_cta<<<2 * num_sms, kCtaThreads4, kCtaSmem4, s>>>(g.view(), q, l, out, o);
   return cudaGetLastError();
 }

@@ -69,6 +69,7 @@ __device__ __forceinline__ unsigned long long choose3(unsigned long long d) {
 __global__ void __launch_bounds__(kThreads) k_motif_terms(GView g, const unsigned* epart,
                                                           unsigned long long* out) {
   const int lane = threadIdx.x & 31;
+  let_next_start();
   unsigned long long acc[7] = {0, 0, 0, 0, 0, 0, 0};
   const int64_t nwarps = (int64_t)gridDim.x * (kThreads / 32);
   for (int64_t r = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) >> 5; r < g.nv; r += nwarps) {
@@ -99,6 +100,7 @@ __global__ void __launch_bounds__(kThreads) k_motif_terms(GView g, const unsigne
     const unsigned long long w = warp_sum_u64(acc[i]);
     if (lane == 0 && w) atomicAdd(out + i, w);
   }
+  wait_for_previous();
 }
 
 // Entries of row v1 below v0: col[rowptr[v1] .. first index with col >= v0).
@@ -177,6 +179,7 @@ __global__ void __launch_bounds__(kThreads) k_graph_terms(GView g, const int32_t
                                                           unsigned long long* out, int stride,
                                                           int slot_d, unsigned long long* sums) {
   __shared__ int64_t row_s[kThreads / 32][33];
+  let_next_start();
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   int64_t* row = row_s[warp];
   const int64_t nwarps = (int64_t)gridDim.x * (kThreads / 32);
@@ -244,6 +247,7 @@ __global__ void __launch_bounds__(kThreads) k_graph_terms(GView g, const int32_t
       }
     }
   }
+  wait_for_previous();
 }
 
 // Triangles and tailed triangles per graph from the sums (a slot < 0 is skipped).
@@ -275,10 +279,10 @@ cudaError_t launch_diamond_reduce(const unsigned* epart, int64_t ne, unsigned lo
 }
 
 cudaError_t launch_motif_terms(const GView& g, const unsigned* epart, unsigned long long* out,
-                               cudaStream_t s) {
+                               cudaStream_t s, bool next) {
   if (g.nv == 0) return cudaSuccess;
-  k_motif_terms<<<std::min(grid_for(g.nv * 32), kReduceBlocks), kThreads, 0, s>>>(g, epart, out);
-  return cudaGetLastError();
+  return launch_next(!next, k_motif_terms, std::min(grid_for(g.nv * 32), kReduceBlocks), kThreads,
+                     0, s, g, epart, out);
 }
 
 uint64_t tailed_from_terms(const unsigned long long* terms) {
@@ -295,13 +299,12 @@ cudaError_t launch_wedge_count(const GView& g, long long* wedges, cudaStream_t s
 cudaError_t launch_graph_terms(const GView& g, const int32_t* gid, int graphs,
                                const unsigned* epart, unsigned long long* sums,
                                unsigned long long* out, int stride, int slot_tri, int slot_d,
-                               int slot_t, cudaStream_t s) {
+                               int slot_t, cudaStream_t s, bool next) {
   if (g.nv == 0) return cudaSuccess;
   const unsigned grid = std::min(grid_for(g.nv), kReduceBlocks);
-  if (slot_t >= 0)
-    k_graph_terms<true><<<grid, kThreads, 0, s>>>(g, gid, epart, out, stride, slot_d, sums);
-  else
-    k_graph_terms<false><<<grid, kThreads, 0, s>>>(g, gid, epart, out, stride, slot_d, sums);
+  const cudaError_t e = launch_next(!next, slot_t >= 0 ? k_graph_terms<true> : k_graph_terms<false>,
+                                    grid, kThreads, 0, s, g, gid, epart, out, stride, slot_d, sums);
+  if (e != cudaSuccess) return e;
   k_graph_finish<<<grid_for(graphs), kThreads, 0, s>>>(sums, graphs, out, stride, slot_tri, slot_t);
   return cudaGetLastError();
 }

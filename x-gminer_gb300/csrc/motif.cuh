@@ -12,9 +12,10 @@ cudaError_t launch_diamond_reduce(const unsigned* epart, int64_t ne, unsigned lo
                                   cudaStream_t s);
 
 // out[0..6] += the wedge / 3-star / 3-walk / tailed-triangle / diamond / 3 x triangle sums
-// (edge-induced; see motif.cu; epart null for the 3-vertex census).
+// (edge-induced; see motif.cu; epart null for the 3-vertex census).  next, here and below: the
+// kernel may start before the one launched before it has ended (launch_next).
 cudaError_t launch_motif_terms(const GView& g, const unsigned* epart, unsigned long long* out,
-                               cudaStream_t s);
+                               cudaStream_t s, bool next = false);
 // Edge-induced tailed triangles from the seven sums.
 uint64_t tailed_from_terms(const unsigned long long* terms);
 
@@ -33,7 +34,9 @@ struct C4Lists {
 };
 cudaError_t launch_cycle4(const DevGraph& g, C4Queue* q, const C4Lists& l,
                           unsigned long long* out, int num_sms, cudaStream_t s,
-                          const GOut& o = GOut{});
+                          const GOut& o = GOut{}, bool next = false);
+// Whether launch_cycle4 launches k_c4_cta, which depends on its first kernel.
+bool cycle4_has_cta(const DevGraph& g);
 
 // Batched graphs: per-graph diamond (slot_d) and tailed-triangle (slot_t) totals from the
 // participation counters; a slot < 0 is skipped.
@@ -47,6 +50,6 @@ cudaError_t launch_part_reduce_graphs(const GView& g, const int32_t* gid,
 cudaError_t launch_graph_terms(const GView& g, const int32_t* gid, int graphs,
                                const unsigned* epart, unsigned long long* sums,
                                unsigned long long* out, int stride, int slot_tri, int slot_d,
-                               int slot_t, cudaStream_t s);
+                               int slot_t, cudaStream_t s, bool next = false);
 
 }  // namespace xgm

@@ -173,6 +173,7 @@ __global__ void __launch_bounds__(kOwnThreads, own_ctas(MODE)) k_owner(OwnArgs a
                                                        unsigned long long* count) {
   constexpr bool ROWS = (MODE & kOwnRows) != 0, PART = (MODE & kOwnPart) != 0;
   extern __shared__ uint32_t bm[];
+  let_next_start();
   // participation mode: counters per rank in N+(u), members before each bitmap word
   uint32_t* rcnt = bm + a.wmask + 1;
   uint16_t* wpre = reinterpret_cast<uint16_t*>(rcnt + a.ranks);
@@ -514,6 +515,7 @@ __global__ void __launch_bounds__(kOwnThreads, own_ctas(MODE)) k_owner(OwnArgs a
     acc = warp_sum_u64(acc);
     if (lane == 0 && acc) atomicAdd(count, acc);
   }
+  wait_for_previous();
 }
 
 template <int MODE>
@@ -1350,13 +1352,14 @@ cudaError_t launch_team(const DevGraph& g, RowTasks t, int cap, unsigned long lo
 
 template <int K>
 cudaError_t launch_rows_k(const DevGraph& g, const uint32_t* rows, OwnHeads* heads,
-                          unsigned long long* count, int num_sms, cudaStream_t s, const GOut& o) {
+                          unsigned long long* count, int num_sms, cudaStream_t s, const GOut& o,
+                          bool first) {
   const unsigned long long* rn = g.rn;
   cudaError_t e = cudaSuccess;
-  bool first = g.max_out <= kRowsMid;
-  if (!first) {
+  if (g.max_out > kRowsMid) {
     const RowTasks t{g.dptr, g.roff, rows, g.rtask + 2 * g.nv - 1, rn + 4, 1, 0};
-    e = launch_team<K, K == 4 ? 256 : 512>(g, t, kRowsCap, &heads->wide, count, num_sms, s, o, true);
+    e = launch_team<K, K == 4 ? 256 : 512>(g, t, kRowsCap, &heads->wide, count, num_sms, s, o, first);
+    first = false;
   }
   if (e == cudaSuccess && g.max_out > 32) {
     const RowTasks t{g.dptr, g.roff, rows, g.rtask + g.nv, rn + 3, 0, 0};
@@ -1445,13 +1448,13 @@ cudaError_t launch_owner_rows(const DevGraph& g, uint32_t* rows, OwnHeads* heads
 
 cudaError_t launch_rows_count(int k, const DevGraph& g, const uint32_t* rows, OwnHeads* heads,
                               unsigned long long* count, int num_sms, cudaStream_t s,
-                              const GOut& o) {
+                              const GOut& o, bool next) {
   if (g.nv == 0) return cudaSuccess;
   switch (k) {
-    case 4: return launch_rows_k<4>(g, rows, heads, count, num_sms, s, o);
-    case 5: return launch_rows_k<5>(g, rows, heads, count, num_sms, s, o);
-    case 6: return launch_rows_k<6>(g, rows, heads, count, num_sms, s, o);
-    case 7: return launch_rows_k<7>(g, rows, heads, count, num_sms, s, o);
+    case 4: return launch_rows_k<4>(g, rows, heads, count, num_sms, s, o, !next);
+    case 5: return launch_rows_k<5>(g, rows, heads, count, num_sms, s, o, !next);
+    case 6: return launch_rows_k<6>(g, rows, heads, count, num_sms, s, o, !next);
+    case 7: return launch_rows_k<7>(g, rows, heads, count, num_sms, s, o, !next);
     default: return cudaErrorInvalidValue;
   }
 }

@@ -52,9 +52,10 @@ cudaError_t launch_owner_rows(const DevGraph& g, uint32_t* rows, OwnHeads* heads
 //  launch_owner_multi: fills the row store and credits epart (launch_owner_part) in one pass.
 cudaError_t launch_owner_multi(const DevGraph& g, uint32_t* rows, unsigned* epart,
                                OwnHeads* heads, int num_sms, cudaStream_t s);
-//  (o: per-graph totals of batched graphs instead)
+//  (o: per-graph totals of batched graphs instead; next: it may start before the kernel launched
+//  before it has ended, launch_next)
 cudaError_t launch_rows_count(int k, const DevGraph& g, const uint32_t* rows, OwnHeads* heads,
                               unsigned long long* count, int num_sms, cudaStream_t s,
-                              const GOut& o = GOut{});
+                              const GOut& o = GOut{}, bool next = false);
 
 }  // namespace xgm
