@@ -96,3 +96,18 @@ def test_participation_oracle_and_task_tiers(xgm, orc, ctx, gen, args):
         assert ctx.count(g, pattern) == want
         assert ctx.count(g, pattern, policy=xgm.SCHED_FIXED, variant=xgm.VAR_WARP) == want
     g.close()
+
+
+@pytest.mark.parametrize("core", [24, 25, 26, 27])
+def test_short_lists_with_hubs(xgm, orc, ctx, core):
+    # largest out-degree 23 to 26, around the line below which no edge takes a bitmap unit,
+    # with hubs of degree above 64 either side of it
+    nv, src, dst = _join(core, 300, core - 4)
+    rowptr, col = orc.build_csr(nv, src, dst)
+    g = ctx.graph_from_edges(nv, src, dst)
+    assert g.info()["max_out_degree"] == core - 1
+    assert ctx.count(g, "triangle") == math.comb(core, 3) + 300 * math.comb(core - 4, 2)
+    assert ctx.count(g, "4-clique") == math.comb(core, 4) + 300 * math.comb(core - 4, 3)
+    assert ctx.count(g, "diamond") == orc.count("diamond", rowptr, col)
+    assert xgm.MotifSolver(g, 4) == [int(c) for c in orc.motif(4, rowptr, col)]
+    g.close()

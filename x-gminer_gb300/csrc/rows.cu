@@ -11,14 +11,14 @@
 // sum_(v,u) d+(u): at R-MAT scale 22 7.2 G against 29 G elements, because the
 // out-neighbours u of a low vertex are hubs with long lists.
 //
-//  - big u (degree > kBigDeg): a CTA holds N+(u) as a bitmap over [u + 1, V) and takes up
+//  - big u (degree > kBigDeg, in graphs with out-lists above kShortLists): a CTA holds N+(u) as a bitmap over [u + 1, V) and takes up
 //    to kOwnChunk in-neighbours v of u.  A thread finds u's place in N+(v) by binary
 //    search (N+(v) is sorted); suffixes of up to kOwnShort elements are tested by that
 //    thread, longer ones go to a table in shared memory, longest first, and are tested by
 //    eight lanes each, a 16-byte unit per lane and step.  A hub's in-neighbours are many
 //    units (u, chunk) that any CTA can take.
 //  - the other u: one lane per edge (v, u) meets the suffix with N+(u) (merge_lists); both are short
-//    (deg v <= deg u <= kBigDeg).
+//    (deg v <= deg u <= kBigDeg, or no list above kShortLists).
 // Bitmaps are cleared by taking the inserted bits out again: a unit costs d+(u) stores,
 // not the bitmap's size.
 //
@@ -28,7 +28,7 @@
 // matrix (k = 4 .. 7).
 //
 // Measured (GB300, a call before -> now):
-//  triangles  R-MAT s20 ef16 8.45 -> 1.42 ms; Barabasi-Albert, 3,312 vertices, 106 -> 26 us
+//  triangles  R-MAT s20 ef16 8.45 -> 1.42 ms; Barabasi-Albert, 3,312 vertices, 106 -> 20 us
 //             (13 launches -> 1: no task lists)
 //  4-cliques  R-MAT s22 65.6 -> 22.1 ms (rows 11.9, counting 9.6); s20 12.4 -> 3.5 ms
 //  5-cliques  R-MAT s20 140 -> 29 ms; 6-cliques R-MAT s16 96 -> 10.6 ms
@@ -55,6 +55,11 @@ constexpr int kOwnThreads = 256;
 constexpr int kOwnWarps = kOwnThreads / 32;
 constexpr int kOwnChunk = 512;   // in-neighbours of one unit (two per thread)
 constexpr int kOwnShort = 12;    // longest suffix one thread tests by itself
+// Largest out-degree of a graph whose edges are all joined by lanes: a bitmap unit costs its
+// phases' latency however short its lists.  Barabasi-Albert, 3,312 vertices (at most 7) triangles
+// 25.7 -> 20.2 us; 200,001 vertices of degree 16 (17) triangles 75 -> 54 us, 4-cliques 109 -> 91;
+// R-MAT s10 ef5 (26) diamonds 42 -> 50 us, 4-cliques 37.5 -> 39.9.
+constexpr int kShortLists = 24;
 constexpr int kOwnLevels = 512;  // most units of one owner (host: raises the chunk above it)
 constexpr int kSmallStep = 128;  // most vertices per claim of the small phase
 
@@ -523,7 +528,7 @@ cudaError_t launch_owner(const DevGraph& g, OwnArgs a, OwnHeads* heads, unsigned
                          int num_sms, cudaStream_t s) {
   if (g.nv == 0) return cudaSuccess;
   a.g = g.view();
-  const int64_t nbig = std::min<int64_t>(g.n_big, kOwnBits);
+  const int64_t nbig = g.max_out <= kShortLists ? 0 : std::min<int64_t>(g.n_big, kOwnBits);
   a.big0 = g.nv - nbig;
   const int64_t per = (g.max_deg + kOwnLevels - 1) / kOwnLevels;
   a.chunk = std::max<int64_t>(kOwnChunk, (per + kOwnChunk - 1) / kOwnChunk * kOwnChunk);
