@@ -1,6 +1,6 @@
 """Counting from the later endpoint of each DAG edge (csrc/rows.cu), the default route of
-the triangle plan: bitmaps of the out-lists of vertices of degree > 64, merges for the
-others.  Sizes sit at the edges of its tiers: degrees around 64, in-neighbour counts
+the triangle plan: bitmaps of the out-lists of vertices of degree > 112, merges for the
+others.  Sizes sit at the edges of its tiers: degrees around 112, in-neighbour counts
 around the 512 of one unit and several units, suffixes around the longest that one thread
 tests (12) and the 128 elements of one warp pass.  Counts equal closed forms, the oracle
 and the task tiers (forced by a fixed schedule)."""
@@ -28,7 +28,7 @@ def _join(core, leaves, per_leaf):
     return core + leaves, np.concatenate([s, ls]), np.concatenate([d, ld])
 
 
-@pytest.mark.parametrize("n", [2, 3, 14, 15, 33, 64, 65, 66, 67, 128, 129, 130, 195, 300])
+@pytest.mark.parametrize("n", [2, 3, 14, 15, 33, 64, 65, 66, 67, 112, 113, 114, 115, 128, 129, 130, 195, 300])
 def test_complete_graphs(ctx, n):
     g = ctx.graph_from_edges(*_complete(n))
     assert ctx.count(g, "triangle") == math.comb(n, 3)
@@ -101,7 +101,7 @@ def test_participation_oracle_and_task_tiers(xgm, orc, ctx, gen, args):
 @pytest.mark.parametrize("core", [24, 25, 26, 27])
 def test_short_lists_with_hubs(xgm, orc, ctx, core):
     # largest out-degree 23 to 26, around the line below which no edge takes a bitmap unit,
-    # with hubs of degree above 64 either side of it
+    # with hubs of degree above 112 either side of it
     nv, src, dst = _join(core, 300, core - 4)
     rowptr, col = orc.build_csr(nv, src, dst)
     g = ctx.graph_from_edges(nv, src, dst)

@@ -11,8 +11,8 @@
 // sum_(v,u) d+(u): at R-MAT scale 22 7.2 G against 29 G elements, because the
 // out-neighbours u of a low vertex are hubs with long lists.
 //
-//  - big u (degree > kBigDeg, in graphs with out-lists above kShortLists): a CTA holds N+(u) as a bitmap over [u + 1, V) and takes up
-//    to kOwnChunk in-neighbours v of u.  A thread finds u's place in N+(v) by binary
+//  - big u (degree > kBigDeg, in graphs with out-lists above kShortLists): a CTA holds N+(u)
+//    as a bitmap over [u + 1, V) and takes up to kOwnChunk in-neighbours v of u.  A thread finds u's place in N+(v) by binary
 //    search (N+(v) is sorted); suffixes of up to kOwnShort elements are tested by that
 //    thread, longer ones go to a table in shared memory, longest first, and are tested by
 //    eight lanes each, a 16-byte unit per lane and step.  A hub's in-neighbours are many
@@ -30,9 +30,9 @@
 // Measured (GB300, a call before -> now):
 //  triangles  R-MAT s20 ef16 8.45 -> 1.42 ms; Barabasi-Albert, 3,312 vertices, 106 -> 20 us
 //             (13 launches -> 1: no task lists)
-//  4-cliques  R-MAT s22 65.6 -> 22.1 ms (rows 11.9, counting 9.6); s20 12.4 -> 3.5 ms
-//  5-cliques  R-MAT s20 140 -> 29 ms; 6-cliques R-MAT s16 96 -> 10.6 ms
-//  triangles per edge (diamonds), Chung-Lu 1.5 M vertices, degree 32: 9.9 -> 3.3 ms; R-MAT
+//  4-cliques  R-MAT s22 65.6 -> 20.0 ms (rows 10.4, counting 9.0); s20 12.4 -> 3.5 ms
+//  5-cliques  R-MAT s20 140 -> 28.6 ms; 6-cliques R-MAT s16 96 -> 10.5 ms
+//  triangles per edge (diamonds), Chung-Lu 1.5 M vertices, degree 32: 9.9 -> 2.8 ms; R-MAT
 //             s19 3.76 -> 1.47 ms (the hits' rank look-ups and counters: the bare count of
 //             the same suffixes is 2.5 times faster)
 //  4,096 Barabasi-Albert graphs, triangles + 4-cliques + diamonds each: 3.44 -> 1.17 ms
@@ -528,7 +528,7 @@ cudaError_t launch_owner(const DevGraph& g, OwnArgs a, OwnHeads* heads, unsigned
                          int num_sms, cudaStream_t s) {
   if (g.nv == 0) return cudaSuccess;
   a.g = g.view();
-  const int64_t nbig = g.max_out <= kShortLists ? 0 : std::min<int64_t>(g.n_big, kOwnBits);
+  const int64_t nbig = g.max_out <= kShortLists ? 0 : std::min<int64_t>(g.n_big, own_bits((MODE & kOwnPart) != 0));
   a.big0 = g.nv - nbig;
   const int64_t per = (g.max_deg + kOwnLevels - 1) / kOwnLevels;
   a.chunk = std::max<int64_t>(kOwnChunk, (per + kOwnChunk - 1) / kOwnChunk * kOwnChunk);

@@ -6,11 +6,17 @@
 namespace xgm {
 
 // Vertices of degree above kBigDeg are "big": their out-list becomes a shared-memory
-// bitmap that the suffixes of their in-neighbours' lists are tested against.  Ranks are
-// sorted by degree, so the big vertices are the top DevGraph::n_big ranks; at most
-// kOwnBits of them are treated so (the bitmap of one CTA: 32 KB).
-constexpr int kBigDeg = 64;
+// bitmap and their in-neighbours' suffixes are tested against it; at most the top
+// own_bits of them are treated so.  kBigDeg 48 / 64 / 96 / 112 / 128 / 192: triangles R-MAT
+// s20 1.49 / 1.41 / 1.41 / 1.41 / 1.47 / 1.69 ms, triangles per edge of a 1.5 M vertex
+// Chung-Lu graph 3.71 / 3.29 / 2.80 / 2.75 / 2.72 / 2.82, rows R-MAT s20 2.13 / 2.02 / 2.03 /
+// 2.03 / 2.13 / 2.60.
+constexpr int kBigDeg = 112;
 constexpr int64_t kOwnBits = int64_t(1) << 18;
+// 2^17 bits (16 KB a CTA, so that L1 keeps the lists) where hits need no rank look-ups: rows
+// R-MAT s22 10.4 ms (2^16 bits 16.0, 2^18 11.7), triangles s23 20.6 ms (2^18 28.9); with them
+// 2^18, triangles per edge s23 48.0 ms (2^17 49.5).
+constexpr int64_t own_bits(bool part) { return part ? kOwnBits : kOwnBits / 2; }
 
 // Row store up to 16 GB (R-MAT scale 22: 0.6 GB); larger graphs, and a device without that
 // much memory left, count with the task kernel.
