@@ -12,13 +12,13 @@
 // out-neighbours u of a low vertex are hubs with long lists.
 //
 //  - big u (degree > kBigDeg, in graphs with out-lists above kShortLists): a CTA holds N+(u)
-//    as a bitmap over [u + 1, V) and takes up to kOwnChunk in-neighbours v of u.  A thread finds u's place in N+(v) by binary
-//    search (N+(v) is sorted); suffixes of up to kOwnShort elements are tested by that
-//    thread, longer ones go to a table in shared memory, longest first, and are tested by
-//    eight lanes each, a 16-byte unit per lane and step.  A hub's in-neighbours are many
-//    units (u, chunk) that any CTA can take.
-//  - the other u: one lane per edge (v, u) meets the suffix with N+(u) (merge_lists); both are short
-//    (deg v <= deg u <= kBigDeg, or no list above kShortLists).
+//    as a bitmap over [u + 1, V) and takes up to kOwnChunk in-neighbours v of u.  A thread
+//    finds u's place in N+(v) by binary search (N+(v) is sorted); suffixes of up to kOwnShort
+//    elements are tested by that thread, longer ones go to a table in shared memory, longest
+//    first, and are tested by eight lanes each, a 16-byte unit per lane and step.  A hub's
+//    in-neighbours are many units (u, chunk) that any CTA can take.
+//  - the other u: one lane per edge (v, u) meets the suffix with N+(u) (merge_lists); both
+//    are short (deg v <= deg u <= kBigDeg, or no list above kShortLists).
 // Bitmaps are cleared by taking the inserted bits out again: a unit costs d+(u) stores,
 // not the bitmap's size.
 //

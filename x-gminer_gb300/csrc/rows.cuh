@@ -18,7 +18,7 @@ constexpr int64_t kOwnBits = int64_t(1) << 18;
 // 2^18, triangles per edge s23 48.0 ms (2^17 49.5).
 constexpr int64_t own_bits(bool part) { return part ? kOwnBits : kOwnBits / 2; }
 
-// Row store up to 16 GB (R-MAT scale 22: 0.6 GB); larger graphs, and a device without that
+// Row store up to 16 GB (R-MAT scale 22: 1.9 GB); larger graphs, and a device without that
 // much memory left, count with the task kernel.
 constexpr int64_t kRowStoreMax = int64_t(1) << 32;  // words
 constexpr int kRowsCap = 1024;  // largest out-degree whose rows are stored
