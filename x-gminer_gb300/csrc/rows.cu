@@ -168,7 +168,7 @@ __device__ __forceinline__ long long lower_at(const int32_t* col, long long lo, 
 // CTAs per SM the registers are cut for, measured per mode (the bitmap allows 5 at R-MAT s22):
 // triangles s20 1.52 / 1.49 / 1.43 ms with 4 / 5 / 6, rows s22 11.9 / 13.9 / 13.5,
 // participation of a 1.5 M vertex Chung-Lu graph 3.47 / 3.30 / 3.95, rows and participation
-// of 4,096 small graphs 0.71 / 0.67 / 0.71.
+// of 4,096 small graphs 0.71 / 0.67 / 0.71 (all with 2^18-bit bitmaps from degree 65 on).
 constexpr int own_ctas(int mode) {
   return mode == kOwnRows ? 4 : (mode == kOwnCount ? 6 : 5);
 }
