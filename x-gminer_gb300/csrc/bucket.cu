@@ -65,10 +65,7 @@ __global__ void __launch_bounds__(kThreads) k_bucket_index(GView g, int32_t* bco
   }
 }
 
-}  // namespace
-
-cudaError_t ensure_bucket_index(const DevGraph& g, cudaStream_t s) {
-  if (g.bcol || g.nv == 0) return cudaSuccess;
+cudaError_t build_bucket_index(const DevGraph& g, cudaStream_t s) {
   int32_t* bcol = nullptr;
   uint32_t* boff = nullptr;
   uint16_t* bmask = nullptr;
@@ -94,6 +91,13 @@ cudaError_t ensure_bucket_index(const DevGraph& g, cudaStream_t s) {
   g.boff = boff;
   g.bmask = bmask;
   return cudaSuccess;
+}
+
+}  // namespace
+
+cudaError_t ensure_bucket_index(const DevGraph& g, cudaStream_t s) {
+  return build_once(
+      g, s, [&] { return g.bcol || g.nv == 0; }, [&] { return build_bucket_index(g, s); });
 }
 
 }  // namespace xgm

@@ -169,6 +169,8 @@ xgm_status clique_route(xgm_ctx* ctx, const DevGraph& g, int k, const xgm_sched&
   if (*route == CliqueRoute::kTasks || (*route == CliqueRoute::kRows && g.max_out > kRowsCap))
     XGM_CUDA_TRY(taskbuf_reserve(ctx->tb, g.nv, s));
   if (*route == CliqueRoute::kTasks && sched_may_bucket(sp)) XGM_CUDA_TRY(ensure_bucket_index(g, s));
+  if (*route == CliqueRoute::kTasks && sp.policy == XGM_SCHED_LEARNED)
+    XGM_CUDA_TRY(ensure_task_stats(g, s));
   return XGM_OK;
 }
 

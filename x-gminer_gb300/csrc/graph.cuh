@@ -1,5 +1,8 @@
 // Device graph storage and the GPU CSR build (csr_build.cu).
 #pragma once
+#include <memory>
+#include <mutex>
+
 #include "common.cuh"
 
 namespace xgm {
@@ -26,6 +29,9 @@ struct DevGraph {
   int32_t* col = nullptr;    // [ne] rank space, sorted rows
   longlong2* dptr = nullptr; // [nv] {first out-neighbour, row end}
   int32_t* gid = nullptr;    // [nv] rank -> graph id (batched graphs only)
+  // Held while an index below is looked for and built: any context, on its own stream and
+  // host thread, may be the first to need it (build_once).
+  std::shared_ptr<std::recursive_mutex> index_lock = std::make_shared<std::recursive_mutex>();
   // bucket index (GView), built on first use by a schedule that can pick BUCKET
   mutable int32_t* bcol = nullptr;
   mutable uint32_t* boff = nullptr;
@@ -54,8 +60,22 @@ struct DevGraph {
   mutable int64_t* tsum = nullptr;
   mutable int32_t* tmax = nullptr;
 
-  GView view() const { return GView{col, rowptr, dptr, nv, bcol, boff, bmask, tsum, tmax}; }
+  GView view() const {
+    std::lock_guard<std::recursive_mutex> hold(*index_lock);
+    return GView{col, rowptr, dptr, nv, bcol, boff, bmask, tsum, tmax};
+  }
 };
+
+// Builds one of g's indexes on stream s unless it is there.  Nobody else sees it before its
+// kernels have run: the lock is held until the stream is through (once per graph and index).
+// Not inside stream capture, but for an index that is there.
+template <class Built, class Build>
+cudaError_t build_once(const DevGraph& g, cudaStream_t s, Built built, Build build) {
+  std::lock_guard<std::recursive_mutex> hold(*g.index_lock);
+  if (built()) return cudaSuccess;
+  const cudaError_t e = build();
+  return e == cudaSuccess ? cudaStreamSynchronize(s) : e;
+}
 
 void free_graph(DevGraph& g, cudaStream_t s);
 

@@ -301,8 +301,7 @@ __global__ void k_task_stats(GView g, int64_t* tsum, int32_t* tmax) {
   }
 }
 
-cudaError_t ensure_task_stats(const DevGraph& g, cudaStream_t s) {
-  if (g.tsum || g.nv == 0) return cudaSuccess;
+static cudaError_t build_task_stats(const DevGraph& g, cudaStream_t s) {
   int64_t* tsum = nullptr;
   int32_t* tmax = nullptr;
   cudaError_t e = cudaMallocAsync((void**)&tsum, sizeof(int64_t) * (size_t)g.nv, s);
@@ -323,6 +322,11 @@ cudaError_t ensure_task_stats(const DevGraph& g, cudaStream_t s) {
   g.tsum = tsum;
   g.tmax = tmax;
   return cudaSuccess;
+}
+
+cudaError_t ensure_task_stats(const DevGraph& g, cudaStream_t s) {
+  return build_once(
+      g, s, [&] { return g.tsum || g.nv == 0; }, [&] { return build_task_stats(g, s); });
 }
 
 cudaError_t classify_learned(const DevGraph& g, int k, const xgm_model& m, TaskBuf& tb,

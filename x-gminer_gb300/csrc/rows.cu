@@ -1394,6 +1394,31 @@ cudaError_t launch_rows_k(const DevGraph& g, const uint32_t* rows, OwnHeads* hea
   return e == cudaSuccess ? narrow(k_rows_narrow<K, 2>, 4) : e;
 }
 
+cudaError_t build_rows_index(const DevGraph& g, cudaStream_t s) {
+  int64_t* roff = nullptr;
+  int32_t* rtask = nullptr;
+  unsigned long long* rn = nullptr;
+  cudaError_t e = cudaMallocAsync((void**)&roff, sizeof(int64_t) * (size_t)g.nv, s);
+  if (e == cudaSuccess) e = cudaMallocAsync((void**)&rtask, sizeof(int32_t) * 2 * (size_t)g.nv, s);
+  if (e == cudaSuccess) e = cudaMallocAsync((void**)&rn, sizeof(*rn) * 5, s);
+  if (e == cudaSuccess) e = cudaMemsetAsync(rn, 0, sizeof(*rn) * 5, s);
+  if (e == cudaSuccess) {
+    const int64_t blocks = std::min<int64_t>((g.nv + 255) / 256, 65536);
+    k_rows_index<<<(unsigned)blocks, 256, 0, s>>>(g.dptr, g.nv, roff, rtask, rtask + g.nv, rn);
+    e = cudaGetLastError();
+  }
+  if (e != cudaSuccess) {
+    if (roff) cudaFreeAsync(roff, s);
+    if (rtask) cudaFreeAsync(rtask, s);
+    if (rn) cudaFreeAsync(rn, s);
+    return e;
+  }
+  g.roff = roff;
+  g.rtask = rtask;
+  g.rn = rn;
+  return cudaSuccess;
+}
+
 }  // namespace
 
 cudaError_t launch_owner_count(const DevGraph& g, OwnHeads* heads, unsigned long long* count,
@@ -1418,29 +1443,8 @@ cudaError_t launch_owner_part(const DevGraph& g, OwnHeads* heads, unsigned* epar
 }
 
 cudaError_t ensure_rows_index(const DevGraph& g, cudaStream_t s) {
-  if (g.roff || g.nv == 0) return cudaSuccess;
-  int64_t* roff = nullptr;
-  int32_t* rtask = nullptr;
-  unsigned long long* rn = nullptr;
-  cudaError_t e = cudaMallocAsync((void**)&roff, sizeof(int64_t) * (size_t)g.nv, s);
-  if (e == cudaSuccess) e = cudaMallocAsync((void**)&rtask, sizeof(int32_t) * 2 * (size_t)g.nv, s);
-  if (e == cudaSuccess) e = cudaMallocAsync((void**)&rn, sizeof(*rn) * 5, s);
-  if (e == cudaSuccess) e = cudaMemsetAsync(rn, 0, sizeof(*rn) * 5, s);
-  if (e == cudaSuccess) {
-    const int64_t blocks = std::min<int64_t>((g.nv + 255) / 256, 65536);
-    k_rows_index<<<(unsigned)blocks, 256, 0, s>>>(g.dptr, g.nv, roff, rtask, rtask + g.nv, rn);
-    e = cudaGetLastError();
-  }
-  if (e != cudaSuccess) {
-    if (roff) cudaFreeAsync(roff, s);
-    if (rtask) cudaFreeAsync(rtask, s);
-    if (rn) cudaFreeAsync(rn, s);
-    return e;
-  }
-  g.roff = roff;
-  g.rtask = rtask;
-  g.rn = rn;
-  return cudaSuccess;
+  return build_once(
+      g, s, [&] { return g.roff || g.nv == 0; }, [&] { return build_rows_index(g, s); });
 }
 
 cudaError_t launch_owner_rows(const DevGraph& g, uint32_t* rows, OwnHeads* heads, int num_sms,

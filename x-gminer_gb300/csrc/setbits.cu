@@ -1382,16 +1382,19 @@ cudaError_t launch_k(const DevGraph& g, BitArgs a, unsigned long long* heads, in
 }  // namespace
 
 cudaError_t ensure_plan_index(const DevGraph& g, int num_sms, cudaStream_t s) {
-  if (g.plan_deg != 0) return cudaSuccess;
-  g.plan_deg = -1;
-  if (g.nv == 0 || g.ne == 0) return cudaSuccess;
-  const cudaError_t e = build_index(g, num_sms, s);
-  if (e == cudaErrorMemoryAllocation) {  // no room: every task stays on the list form
-    cudaGetLastError();
-    return cudaSuccess;
-  }
-  if (e != cudaSuccess) g.plan_deg = 0;
-  return e;
+  auto build = [&] {
+    g.plan_deg = -1;
+    if (g.nv == 0 || g.ne == 0) return cudaSuccess;
+    const cudaError_t e = build_index(g, num_sms, s);
+    if (e == cudaErrorMemoryAllocation) {  // no room: every task stays on the list form
+      cudaGetLastError();
+      return cudaSuccess;
+    }
+    if (e != cudaSuccess) g.plan_deg = 0;
+    return e;
+  };
+  return build_once(
+      g, s, [&] { return g.plan_deg != 0; }, build);
 }
 
 int bits_launches(const DevGraph& g) {
