@@ -85,3 +85,34 @@ def test_kernel_count_before_the_first_learned_count(xgm, contexts):
     assert c.count(g, "triangle", policy=xgm.SCHED_LEARNED, model=m, hub_max=-1) == want
     g.close()
     assert np.uint64(want) > 0
+
+
+def _hub(n, leaves):
+    """A complete graph on n vertices, the first of which has `leaves` neighbours more."""
+    iu = np.triu_indices(n, 1)
+    l = np.arange(n, n + leaves, dtype=np.int32)
+    return (n + leaves, np.concatenate([iu[0].astype(np.int32), np.zeros(leaves, np.int32)]),
+            np.concatenate([iu[1].astype(np.int32), l]))
+
+
+def test_plans_on_graphs_of_other_degrees_at_once(xgm, contexts):
+    """A bitmap-form kernel's shared memory follows the graph's largest degree, and the warp
+    kernel's the program: calls of other sizes at the same time must not limit one another."""
+    graphs = [_hub(12, 20), _hub(12, 180), _hub(12, 300), _hub(12, 900)]
+    jobs = []  # per context: its own graphs and plans
+    for c in contexts:
+        gs = [c.graph_from_edges(*x) for x in graphs]
+        ps = [c.plan(p) for p in ("P7", "P10", "P6", "P15")]
+        jobs.append((gs, ps, [[c.count(g, p) for p in ps] for g in gs]))
+
+    def work(i, c):
+        gs, ps, want = jobs[i]
+        rng = np.random.default_rng(i)
+        for a, b in zip(rng.integers(0, len(gs), 1500), rng.integers(0, len(ps), 1500)):
+            assert c.count(gs[a], ps[b]) == want[a][b]
+
+    assert _all(contexts, work) == []
+    assert jobs[0][2] == jobs[1][2] == jobs[2][2]
+    for gs, _, _ in jobs:
+        for g in gs:
+            g.close()

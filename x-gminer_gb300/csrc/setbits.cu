@@ -37,6 +37,7 @@
 // R-MAT scale 9 P7 1.84 ms -> 0.12, where a few heavy tasks were the time; P10 on
 // Erdos-Renyi 2^16 0.83 -> 0.24 ms.
 #include <algorithm>
+#include <atomic>
 
 #include "api_internal.h"
 #include "graph.cuh"
@@ -1314,31 +1315,47 @@ unsigned blocks(int most, int64_t units) {
   return (unsigned)std::max<int64_t>(1, std::min<int64_t>(most, units));
 }
 
-cudaError_t launch(void (*kern)(BitArgs), unsigned grid, int threads, int bytes, cudaStream_t s,
+// The shared-memory opt-in of a kernel, `most` bytes, once per device.  The attribute is the
+// process's: set to what each call needs, one context's launch met the smaller limit that
+// another's had just set.
+template <void (*KERN)(BitArgs)>
+cudaError_t opt_in(int most) {
+  static std::atomic<unsigned long long> opted{0};
+  int dev = 0;
+  cudaError_t e = cudaGetDevice(&dev);
+  const unsigned long long bit = dev < 64 ? 1ull << dev : 0ull;
+  if (e == cudaSuccess && !(opted.load(std::memory_order_acquire) & bit)) {
+    e = cudaFuncSetAttribute(KERN, cudaFuncAttributeMaxDynamicSharedMemorySize, most);
+    if (e == cudaSuccess) opted.fetch_or(bit, std::memory_order_acq_rel);
+  }
+  return e;
+}
+
+template <void (*KERN)(BitArgs)>
+cudaError_t launch(unsigned grid, int threads, int bytes, int most, cudaStream_t s,
                    const BitArgs& a, bool first) {
-  const cudaError_t e =
-      cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
-  return e == cudaSuccess ? launch_next(first, kern, grid, threads, bytes, s, a) : e;
+  const cudaError_t e = opt_in<KERN>(most);
+  return e == cudaSuccess ? launch_next(first, KERN, grid, threads, bytes, s, a) : e;
 }
 
 template <int K, int NT>
-cudaError_t launch_cta(const DevGraph& g, BitArgs a, int cls, int deg, bool any, bool first,
+cudaError_t launch_cta(const DevGraph& g, BitArgs a, int cls, bool any, bool first,
                        unsigned long long* heads, int num_sms, cudaStream_t s) {
+  constexpr int deg = NT == kThreads ? kMidDeg : kTopDeg;
+  constexpr int most = cta_layout(deg, NT / 32).bytes;
   // the shared memory that the graph's own degrees need: more blocks an SM
   a.lay = cta_layout((int)std::min<int64_t>(deg, (std::max<int64_t>(g.max_deg, 1) + 127) / 128 * 128),
                      NT / 32);
-  auto kern = k_bits_cta<K, NT>;
-  cudaError_t e =
-      cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, a.lay.bytes);
+  cudaError_t e = opt_in<k_bits_cta<K, NT>>(most);
   int per_sm = 1;
   if (e == cudaSuccess && any)
-    e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, NT, a.lay.bytes);
+    e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_bits_cta<K, NT>, NT, a.lay.bytes);
   if (e != cudaSuccess) return e;
   a.cls = cls;
   a.units = g.plan_units + g.plan_off[cls];
   a.head = heads + cls;
-  return launch(kern, blocks(num_sms * std::max(per_sm, 1), g.plan_cap[cls]), NT, a.lay.bytes, s, a,
-                first);
+  return launch<k_bits_cta<K, NT>>(blocks(num_sms * std::max(per_sm, 1), g.plan_cap[cls]), NT,
+                                   a.lay.bytes, most, s, a, first);
 }
 
 template <int K>
@@ -1348,7 +1365,7 @@ cudaError_t launch_k(const DevGraph& g, BitArgs a, unsigned long long* heads, in
   // 11 0.54 -> 0.39 ms, on scale 12 1.32 -> 1.05, against one after the other)
   bool first = true;
   if (g.plan_deg > kMidDeg && g.max_deg > kMidDeg && g.lut_rows) {
-    cudaError_t e = launch_cta<K, kTopThreads>(g, a, 2, kTopDeg, true, first, heads, num_sms, s);
+    cudaError_t e = launch_cta<K, kTopThreads>(g, a, 2, true, first, heads, num_sms, s);
     if (e != cudaSuccess) return e;
     ++*launches;
     first = false;
@@ -1362,18 +1379,19 @@ cudaError_t launch_k(const DevGraph& g, BitArgs a, unsigned long long* heads, in
     a.units = g.plan_units + g.plan_off[1];
     a.head = heads + 1;
     a.items = g.plan_items;
-    e = launch(k_bits_map<K>, blocks(num_sms * kMapBlocks, g.plan_cap[1]), kMapThreads,
-               (int)sizeof(MapSmem), s, a, first);
+    e = launch<k_bits_map<K>>(blocks(num_sms * kMapBlocks, g.plan_cap[1]), kMapThreads,
+                              (int)sizeof(MapSmem), (int)sizeof(MapSmem), s, a, first);
   } else {
-    e = launch_cta<K, kThreads>(g, a, 1, kMidDeg, any, first, heads, num_sms, s);
+    e = launch_cta<K, kThreads>(g, a, 1, any, first, heads, num_sms, s);
   }
   if (e != cudaSuccess) return e;
   a.cls = 0;
   a.units = g.plan_units + g.plan_off[0];
   a.head = heads;
-  const int bytes = kWarps * (int)(sizeof(SmallWarp) + (a.p.stream ? sizeof(SmallMap) : 0));
-  e = launch(k_bits_warp<K>, blocks(num_sms * 4, (g.plan_cap[0] + kWarps - 1) / kWarps), kThreads,
-             bytes, s, a, false);
+  constexpr int most = kWarps * (int)(sizeof(SmallWarp) + sizeof(SmallMap));
+  const int bytes = a.p.stream ? most : kWarps * (int)sizeof(SmallWarp);
+  e = launch<k_bits_warp<K>>(blocks(num_sms * 4, (g.plan_cap[0] + kWarps - 1) / kWarps), kThreads,
+                             bytes, most, s, a, false);
   if (e != cudaSuccess) return e;
   *launches += 2;
   return cudaSuccess;
