@@ -207,7 +207,8 @@ xgm_status batch_prepare(xgm_ctx* ctx, xgm_batch* b, const Slots& sl, int P,
     XGM_CUDA_TRY(ensure_rows_index(g, s));
     XGM_CUDA_TRY(alloc_once(&b->rows, g.row_store_words + 4, s));
   }
-  if (!rows && (sl.dia >= 0 || sl.tail >= 0)) {
+  // the multi-pattern launch credits participation whichever of its plans are asked for
+  if (!rows && (sl.tri >= 0 || sl.k4 >= 0 || sl.dia >= 0 || sl.tail >= 0)) {
     XGM_CUDA_TRY(alloc_once(&b->vpart, g.nv, s));
     XGM_CUDA_TRY(alloc_once(&b->epart, g.ne + 3, s));
   }
@@ -261,12 +262,6 @@ xgm_status batch_sequence(xgm_ctx* ctx, xgm_batch* b, const Slots& sl, int P,
     // tasks of this multi-pattern launch (kFeatMulti)
     xgm_status r = schedule_into(b->tb, g, 3, sp, s, kFeatMulti);
     if (r != XGM_OK) return r;
-    // without a participation plan the counters go to a dummy-free path: the multi
-    // kernel always credits participation, so give it real buffers
-    if (!part) {
-      XGM_CUDA_TRY(alloc_once(&b->vpart, g.nv, s));
-      XGM_CUDA_TRY(alloc_once(&b->epart, g.ne + 3, s));
-    }
     GOut o{g.gid, b->d_out, P, sl.tri, sl.k4};
     XGM_CUDA_TRY(launch_multi(view, b->tb.lists(false), &b->d_sc->q, b->vpart, b->epart,
                               &b->d_sc->err, grid, s, o));
