@@ -48,6 +48,7 @@ struct xgm_batch {
   unsigned* epart = nullptr;
   int32_t* c4_lists = nullptr;  // task lists of the 4-cycle kernels
   uint32_t* rows = nullptr;     // row store (rows.cu)
+  int64_t rows_cap = 0;
   unsigned long long* sums = nullptr;  // per-graph sums of launch_graph_terms
   std::vector<xgm::CachedExec> cache;
 };
@@ -87,11 +88,15 @@ inline unsigned grid_for(int64_t n) {
   return (unsigned)std::max<int64_t>(1, std::min<int64_t>(b, 65536));
 }
 
-void batch_free(xgm_batch* b) {
-  cudaStream_t s = b->ctx->stream;
+void batch_drop_graphs(xgm_batch* b) {
   for (auto& c : b->cache)
     if (c.exec) cudaGraphExecDestroy(c.exec);
   b->cache.clear();
+}
+
+void batch_free(xgm_batch* b) {
+  cudaStream_t s = b->ctx->stream;
+  batch_drop_graphs(b);
   taskbuf_free(b->tb, s);
   void* ps[] = {b->d_out, b->vpart, b->epart, b->c4_lists, b->rows, b->sums};
   for (void* p : ps)
@@ -180,9 +185,11 @@ bool batch_from_rows(const DevGraph& g, const xgm_sched& sp) {
   return sched_is_open(sp) && g.max_out <= kRowsCap && g.row_store_words <= kRowStoreMax;
 }
 
-// Allocations a sequence needs, made before any capture.
-xgm_status batch_prepare(xgm_ctx* ctx, xgm_batch* b, const Slots& sl, int P,
-                         const xgm_sched& sp) {
+// Allocations a sequence needs, made before any capture; *rows: the owner and row kernels
+// run it.  The row store comes last but for the few words per graph: without room for it the
+// batch is the task kernel's, whose buffers do not have to fit beside it.
+xgm_status batch_prepare(xgm_ctx* ctx, xgm_batch* b, const Slots& sl, int P, const xgm_sched& sp,
+                         bool* rows_out) {
   cudaStream_t s = ctx->stream;
   const DevGraph& g = b->graph.g;
   const int64_t need = (int64_t)b->num_graphs * P;
@@ -194,25 +201,36 @@ xgm_status batch_prepare(xgm_ctx* ctx, xgm_batch* b, const Slots& sl, int P,
     XGM_CUDA_TRY(cudaMallocAsync(&b->d_out, sizeof(unsigned long long) * need, s));
     XGM_CUDA_TRY(cudaMallocHost(&b->h_out, sizeof(unsigned long long) * need));
     b->out_cap = need;
-    for (auto& c : b->cache)
-      if (c.exec) cudaGraphExecDestroy(c.exec);
-    b->cache.clear();
+    batch_drop_graphs(b);
   }
-  const bool rows = batch_from_rows(g, sp);
-  if (rows && (sl.tri >= 0 || sl.dia >= 0 || sl.tail >= 0)) {
-    XGM_CUDA_TRY(alloc_once(&b->epart, g.ne + 3, s));  // whole 16-byte units
-    XGM_CUDA_TRY(alloc_once(&b->sums, 3 * (int64_t)b->num_graphs, s));
+  const bool part = sl.tri >= 0 || sl.dia >= 0 || sl.tail >= 0;
+  bool rows = batch_from_rows(g, sp);
+  auto buffers = [&]() -> cudaError_t {
+    cudaError_t e = cudaSuccess;
+    if (sl.c4 >= 0) e = alloc_once(&b->c4_lists, 3 * g.nv, s);
+    // (whole 16-byte units; the task kernel's multi-pattern launch credits participation
+    // whichever of its plans are asked for)
+    if (e == cudaSuccess && (part || (!rows && sl.k4 >= 0))) e = alloc_once(&b->epart, g.ne + 3, s);
+    if (e == cudaSuccess && !rows && (part || sl.k4 >= 0)) e = alloc_once(&b->vpart, g.nv, s);
+    if (e == cudaSuccess && rows && part) e = alloc_once(&b->sums, 3 * (int64_t)b->num_graphs, s);
+    return e;
+  };
+  cudaError_t e = buffers();
+  if (e == cudaErrorMemoryAllocation && b->rows) {  // once more without an earlier call's store
+    cudaGetLastError();
+    batch_drop_graphs(b);  // they hold its address
+    cudaFreeAsync(b->rows, s);
+    b->rows = nullptr;
+    b->rows_cap = 0;
+    XGM_CUDA_TRY(cudaStreamSynchronize(s));
+    e = buffers();
   }
+  XGM_CUDA_TRY(e);
   if (rows && (sl.k4 >= 0 || sl.k5 >= 0)) {
-    XGM_CUDA_TRY(ensure_rows_index(g, s));
-    XGM_CUDA_TRY(alloc_once(&b->rows, g.row_store_words + 4, s));
+    XGM_CUDA_TRY(reserve_rows(g, &b->rows, &b->rows_cap, &rows, s));
+    if (!rows) XGM_CUDA_TRY(buffers());
   }
-  // the multi-pattern launch credits participation whichever of its plans are asked for
-  if (!rows && (sl.tri >= 0 || sl.k4 >= 0 || sl.dia >= 0 || sl.tail >= 0)) {
-    XGM_CUDA_TRY(alloc_once(&b->vpart, g.nv, s));
-    XGM_CUDA_TRY(alloc_once(&b->epart, g.ne + 3, s));
-  }
-  if (sl.c4 >= 0) XGM_CUDA_TRY(alloc_once(&b->c4_lists, 3 * g.nv, s));
+  *rows_out = rows;
   ensure_clique_grid(ctx);
   if (!rows && sched_may_bucket(sp)) XGM_CUDA_TRY(ensure_bucket_index(g, s));  // before any capture
   if (!rows && sp.policy == XGM_SCHED_LEARNED) XGM_CUDA_TRY(ensure_task_stats(g, s));
@@ -222,7 +240,7 @@ xgm_status batch_prepare(xgm_ctx* ctx, xgm_batch* b, const Slots& sl, int P,
 
 // The device work of one batched count: stream operations only.
 xgm_status batch_sequence(xgm_ctx* ctx, xgm_batch* b, const Slots& sl, int P,
-                          const xgm_sched& sp) {
+                          const xgm_sched& sp, bool rows) {
   cudaStream_t s = ctx->stream;
   const DevGraph& g = b->graph.g;
   const GView view = g.view();
@@ -230,7 +248,6 @@ xgm_status batch_sequence(xgm_ctx* ctx, xgm_batch* b, const Slots& sl, int P,
   const int grid = ensure_clique_grid(ctx);
   XGM_CUDA_TRY(cudaMemsetAsync(b->d_out, 0, sizeof(unsigned long long) * nout, s));
   XGM_CUDA_TRY(cudaMemsetAsync(b->d_sc, 0, sizeof(Scalars), s));
-  const bool rows = batch_from_rows(g, sp);
   if (rows) {
     const bool part = sl.tri >= 0 || sl.dia >= 0 || sl.tail >= 0, k = sl.k4 >= 0 || sl.k5 >= 0;
     OwnHeads* heads = &b->d_sc->own;
@@ -312,12 +329,13 @@ xgm_status count_batched_impl(xgm_ctx* ctx, xgm_batch* b, const xgm_plan* const*
   Slots sl;
   xgm_status r = slots_of(plans, P, sl);
   if (r != XGM_OK) return r;
-  r = batch_prepare(ctx, b, sl, P, sp);
+  bool rows = false;
+  r = batch_prepare(ctx, b, sl, P, sp, &rows);
   if (r != XGM_OK) return r;
   const bool use_graph = !(sp.flags & XGM_SCHED_NO_GRAPH);
   XGM_CUDA_TRY(ctx_mark(ctx, 0));
   if (use_graph) {
-    const std::string key = sched_key(sl, sp);
+    const std::string key = sched_key(sl, sp) + (rows ? 'r' : 't');
     cudaGraphExec_t exec = nullptr;
     for (auto& c : b->cache)
       if (c.key == key) {
@@ -326,7 +344,7 @@ xgm_status count_batched_impl(xgm_ctx* ctx, xgm_batch* b, const xgm_plan* const*
       }
     if (!exec) {
       XGM_CUDA_TRY(cudaStreamBeginCapture(s, cudaStreamCaptureModeThreadLocal));
-      r = batch_sequence(ctx, b, sl, P, sp);
+      r = batch_sequence(ctx, b, sl, P, sp, rows);
       cudaGraph_t graph = nullptr;
       const cudaError_t e = cudaStreamEndCapture(s, &graph);
       if (r != XGM_OK) {
@@ -354,7 +372,7 @@ xgm_status count_batched_impl(xgm_ctx* ctx, xgm_batch* b, const xgm_plan* const*
     }
     XGM_CUDA_TRY(cudaGraphLaunch(exec, s));
   } else {
-    r = batch_sequence(ctx, b, sl, P, sp);
+    r = batch_sequence(ctx, b, sl, P, sp, rows);
     if (r != XGM_OK) return r;
   }
   XGM_CUDA_TRY(ctx_mark(ctx, 1));

@@ -25,6 +25,20 @@ cudaError_t grow(T** p, int64_t* cap, int64_t n, cudaStream_t s) {
   return e;
 }
 
+// An allocation that fails while the context keeps an earlier call's row store: once more
+// without it.
+template <class F>
+cudaError_t with_room(xgm_ctx* ctx, F alloc) {
+  cudaError_t e = alloc();
+  if (e != cudaErrorMemoryAllocation || !ctx->rows) return e;
+  cudaGetLastError();
+  cudaFreeAsync(ctx->rows, ctx->stream);
+  ctx->rows = nullptr;
+  ctx->rows_cap = 0;
+  e = cudaStreamSynchronize(ctx->stream);
+  return e == cudaSuccess ? alloc() : e;
+}
+
 int clique_kind(int pattern) {
   switch (pattern) {
     case XGM_PATTERN_TRIANGLE: return 3;
@@ -150,7 +164,9 @@ xgm_status schedule_tasks(xgm_ctx* ctx, const DevGraph& g, int k, const xgm_sche
 // task kernel then only runs the vertices above their capacity), or the task kernel.
 enum class CliqueRoute { kOwner, kRows, kTasks };
 
-// Chooses the route and gets its buffers and per-graph indexes (outside stream capture).
+// Chooses the route and gets its buffers and per-graph indexes (outside stream capture).  The
+// row store comes last: what else the call needs is there (nothing else fails for it), and
+// without room for the store the call is the task kernel's.
 xgm_status clique_route(xgm_ctx* ctx, const DevGraph& g, int k, const xgm_sched& sp,
                         CliqueRoute* route) {
   cudaStream_t s = ctx->stream;
@@ -159,15 +175,15 @@ xgm_status clique_route(xgm_ctx* ctx, const DevGraph& g, int k, const xgm_sched&
     if (k == 3) {
       *route = CliqueRoute::kOwner;
     } else if (g.nv > 0 && g.row_store_words <= kRowStoreMax) {
-      XGM_CUDA_TRY(ensure_rows_index(g, s));
-      const cudaError_t e = grow(&ctx->rows, &ctx->rows_cap, g.row_store_words + 4, s);
-      if (e == cudaSuccess) *route = CliqueRoute::kRows;
-      else if (e != cudaErrorMemoryAllocation) XGM_CUDA_TRY(e);
-      else cudaGetLastError();
+      if (g.max_out > kRowsCap)
+        XGM_CUDA_TRY(with_room(ctx, [&] { return taskbuf_reserve(ctx->tb, g.nv, s); }));
+      bool fits = false;
+      XGM_CUDA_TRY(reserve_rows(g, &ctx->rows, &ctx->rows_cap, &fits, s));
+      if (fits) *route = CliqueRoute::kRows;
     }
   }
-  if (*route == CliqueRoute::kTasks || (*route == CliqueRoute::kRows && g.max_out > kRowsCap))
-    XGM_CUDA_TRY(taskbuf_reserve(ctx->tb, g.nv, s));
+  if (*route == CliqueRoute::kTasks)
+    XGM_CUDA_TRY(with_room(ctx, [&] { return taskbuf_reserve(ctx->tb, g.nv, s); }));
   if (*route == CliqueRoute::kTasks && sched_may_bucket(sp)) XGM_CUDA_TRY(ensure_bucket_index(g, s));
   if (*route == CliqueRoute::kTasks && sp.policy == XGM_SCHED_LEARNED)
     XGM_CUDA_TRY(ensure_task_stats(g, s));
@@ -210,17 +226,17 @@ xgm_status launch_participation(xgm_ctx* ctx, const DevGraph& g, const xgm_sched
   xgm_sched tri = sp;
   if (tri.policy == XGM_SCHED_LEARNED && !tri.model) tri.policy = XGM_SCHED_HEURISTIC;
   *tasks = !sched_is_open(tri) || g.max_out > kOwnPartMaxOut;
-  XGM_CUDA_TRY(grow(&ctx->epart, &ctx->epart_cap, g.ne, s));
+  XGM_CUDA_TRY(with_room(ctx, [&] { return grow(&ctx->epart, &ctx->epart_cap, g.ne, s); }));
   XGM_CUDA_TRY(cudaMemsetAsync(ctx->epart, 0, sizeof(unsigned) * (g.ne > 0 ? g.ne : 1), s));
   if (!*tasks) {
     XGM_CUDA_TRY(ctx_mark(ctx, 1));
     XGM_CUDA_TRY(launch_owner_part(g, &ctx->d_sc->own, ctx->epart, ctx->num_sms, s));
     return XGM_OK;
   }
-  XGM_CUDA_TRY(taskbuf_reserve(ctx->tb, g.nv, s));
+  XGM_CUDA_TRY(with_room(ctx, [&] { return taskbuf_reserve(ctx->tb, g.nv, s); }));
   xgm_status r = schedule_tasks(ctx, g, 3, tri);
   if (r != XGM_OK) return r;
-  XGM_CUDA_TRY(grow(&ctx->vpart, &ctx->vpart_cap, g.nv, s));
+  XGM_CUDA_TRY(with_room(ctx, [&] { return grow(&ctx->vpart, &ctx->vpart_cap, g.nv, s); }));
   XGM_CUDA_TRY(cudaMemsetAsync(ctx->vpart, 0, sizeof(unsigned long long) * (g.nv > 0 ? g.nv : 1), s));
   XGM_CUDA_TRY(ctx_mark(ctx, 1));
   XGM_CUDA_TRY(launch_triangle_participation(g.view(), ctx->tb.lists(false), &ctx->d_sc->q,
@@ -265,7 +281,9 @@ xgm_status count_dispatch(xgm_ctx* ctx, const DevGraph& g, int pattern, const xg
       XGM_CUDA_TRY(launch_motif_terms(view, ctx->epart, ctx->d_sc->terms, s));
     launches = 2;
   } else if (pattern == XGM_PATTERN_CYCLE4) {
-    XGM_CUDA_TRY(grow(&ctx->c4_lists, &ctx->c4_lists_cap, 3 * g.nv, s));
+    XGM_CUDA_TRY(with_room(ctx, [&] {
+      return grow(&ctx->c4_lists, &ctx->c4_lists_cap, 3 * g.nv, s);
+    }));
     XGM_CUDA_TRY(ctx_mark(ctx, 1));
     const C4Lists lists{ctx->c4_lists, ctx->c4_lists + g.nv, ctx->c4_lists + 2 * g.nv};
     XGM_CUDA_TRY(launch_cycle4(g, &ctx->d_sc->c4, lists, &ctx->d_sc->count, ctx->num_sms, s));
@@ -468,15 +486,19 @@ xgm_status motif4_parts(xgm_ctx* ctx, const DevGraph& g, const xgm_sched& sp, bo
   // one owner pass, all parts behind one read-back
   CliqueRoute route = CliqueRoute::kTasks;
   if (sched_is_open(sp) && g.max_out <= kRowsCap) {
+    cudaStream_t s = ctx->stream;
     XGM_CUDA_TRY(cudaSetDevice(ctx->device));
+    XGM_CUDA_TRY(with_room(ctx, [&] {
+      cudaError_t e = grow(&ctx->epart, &ctx->epart_cap, g.ne, s);
+      if (e == cudaSuccess && need_c4) e = grow(&ctx->c4_lists, &ctx->c4_lists_cap, 3 * g.nv, s);
+      return e;
+    }));
     xgm_status q = clique_route(ctx, g, 4, sp, &route);
     if (q != XGM_OK) return q;
   }
   if (route == CliqueRoute::kRows) {
     cudaStream_t s = ctx->stream;
     Scalars* sc = ctx->d_sc;
-    XGM_CUDA_TRY(grow(&ctx->epart, &ctx->epart_cap, g.ne, s));
-    if (need_c4) XGM_CUDA_TRY(grow(&ctx->c4_lists, &ctx->c4_lists_cap, 3 * g.nv, s));
     XGM_CUDA_TRY(cudaMemsetAsync(sc, 0, sizeof(Scalars), s));
     XGM_CUDA_TRY(ctx_mark(ctx, 0));
     XGM_CUDA_TRY(cudaMemsetAsync(ctx->epart, 0, sizeof(unsigned) * (g.ne > 0 ? g.ne : 1), s));

@@ -43,6 +43,7 @@
 // 29 ms of the s20 5-clique) and the shifts and ANDs that feed it at 16 warps per SM.
 #include <algorithm>
 #include <atomic>
+#include <cstdlib>
 #include <type_traits>
 
 #include "rows.cuh"
@@ -1445,6 +1446,26 @@ cudaError_t launch_owner_part(const DevGraph& g, OwnHeads* heads, unsigned* epar
 cudaError_t ensure_rows_index(const DevGraph& g, cudaStream_t s) {
   return build_once(
       g, s, [&] { return g.roff || g.nv == 0; }, [&] { return build_rows_index(g, s); });
+}
+
+cudaError_t reserve_rows(const DevGraph& g, uint32_t** rows, int64_t* cap, bool* fits,
+                         cudaStream_t s) {
+  const int64_t words = g.row_store_words + 4;
+  cudaError_t e = ensure_rows_index(g, s);
+  if (e == cudaSuccess && (!*rows || *cap < words)) {
+    if (*rows) cudaFreeAsync(*rows, s);
+    *rows = nullptr;
+    *cap = 0;
+    // test hook: XGM_ROW_STORE_CAP is the number of words from which there is no room
+    const char* room = std::getenv("XGM_ROW_STORE_CAP");
+    e = room && words > std::atoll(room) ? cudaErrorMemoryAllocation
+                                         : cudaMallocAsync((void**)rows, sizeof(uint32_t) * words, s);
+    if (e == cudaSuccess) *cap = words;
+  }
+  *fits = e == cudaSuccess;
+  if (e != cudaErrorMemoryAllocation) return e;
+  cudaGetLastError();
+  return cudaSuccess;
 }
 
 cudaError_t launch_owner_rows(const DevGraph& g, uint32_t* rows, OwnHeads* heads, int num_sms,

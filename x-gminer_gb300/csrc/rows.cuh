@@ -53,6 +53,11 @@ cudaError_t launch_owner_part(const DevGraph& g, OwnHeads* heads, unsigned* epar
 //  launch_owner_rows: fills the row store.
 //  launch_rows_count: adds the k-cliques (k = 4 .. 7) of all stored tasks to *count.
 cudaError_t ensure_rows_index(const DevGraph& g, cudaStream_t s);
+// The index and a row store of g's size, grown where it has fewer words than *cap; *fits:
+// whether there was room (no error where there was not: *rows is null then, and the caller
+// counts with the task kernel).
+cudaError_t reserve_rows(const DevGraph& g, uint32_t** rows, int64_t* cap, bool* fits,
+                         cudaStream_t s);
 cudaError_t launch_owner_rows(const DevGraph& g, uint32_t* rows, OwnHeads* heads, int num_sms,
                               cudaStream_t s);
 //  launch_owner_multi: fills the row store and credits epart (launch_owner_part) in one pass.
