@@ -12,8 +12,10 @@
 //    the task (clearing it costs as much as filling it); larger tasks go to the lists of
 //  - k_c4_cta, two CTAs per SM: up to kHashWedges wedges in one hash table; more are counted
 //    a tile of v2 ids at a time in an array of 16-bit counters, read back and cleared once
-//    per tile.  Rows are sorted, so a row's part in a tile is one run: tasks
-//    of up to kCursors lower neighbours keep a cursor per row and go tile by tile; hubs are
+//    per tile, or, where few of them fall in a tile, a range of ids at a time in the hash table
+//    (hash_passes).  Rows are sorted, so a row's part in a tile is one run: tasks
+//    of up to kCursors lower neighbours keep a cursor per row and go tile by tile, from their
+//    smallest v2 on (a batch's graphs begin at other ids); hubs are
 //    one unit per tile (any CTA can take it) and find the run by binary search.
 // Measured (GB300): Erdos-Renyi 2^20, degree 32 (331 M wedges) 14.6 -> 4.6 ms; R-MAT s19
 // ef16 (2.2 G wedges) 29.4 -> 10.2 ms.  (Before: a 4096-slot table cleared by a 256-thread
@@ -42,6 +44,13 @@ constexpr int kHashWedges = 8192;
 constexpr int kTileWords = 23552;     // counter words: 47,104 counters of 16 bits
 constexpr int kSegs = 512;            // most lower neighbours of a task that may be hashed
 constexpr int kCursors = 2048;        // largest lower degree that keeps cursors
+constexpr int kPassWedges = 6144;     // wedges a hash pass aims at
+// Tiles (of 2 kTileWords ids) that cost as much as a pass; a task of no more passes than
+// tiles / kPassTiles is counted in passes.  1 / 2 / 4 / 8 / 16: R-MAT s19 9.5 / 9.1 / 9.9 / 9.9 /
+// 9.9 ms, s21 107 / 107 / 107 / 109 / 126, Chung-Lu 2^21 103 / 100 / 98 / 101 / 106, Erdos-Renyi
+// 2^20 degree 128 98 / 98 / 98 / 163 / 224, Barabasi-Albert 1 M degree 64 33 / 32 / 32 / 36 / 43.
+constexpr int kPassTiles = 2;
+constexpr int kRowCap = 1 << 20;      // row lengths are summed up to here
 
 struct WarpTable {
   uint32_t key[kWarpSlots];
@@ -319,16 +328,204 @@ __device__ unsigned long long tile_wedges(const GView& g, CtaTile& t, int* next,
   return acc;
 }
 
+// Exclusive prefix of v over the CTA's threads in `before`, their sum returned.
+__device__ __forceinline__ int block_scan(int v, int* wsum, int& before) {
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  int inc = v;
+#pragma unroll
+  for (int d = 1; d < 32; d <<= 1) {
+    const int y = __shfl_up_sync(kFull, inc, d);
+    if (lane >= d) inc += y;
+  }
+  __syncthreads();  // (every warp has read the sums of the scan before)
+  if (lane == 31) wsum[warp] = inc;
+  __syncthreads();
+  const int ws = lane < kCtaThreads4 / 32 ? wsum[lane] : 0;
+  before = (int)__reduce_add_sync(kFull, (unsigned)(lane < warp ? ws : 0)) + inc - v;
+  return (int)__reduce_add_sync(kFull, (unsigned)ws);
+}
+
+// A thread's rows of a task: rows tid, tid + kCtaThreads4, ..
+constexpr int kRowsPerThread = kCursors / kCtaThreads4;
+
+// Wedges of v0 (rows beyond kRowCap counted as that many), and the smallest v2 (v0: none).
+__device__ __forceinline__ int task_wedges(const GView& g, int32_t v0, long long a0, int dl,
+                                           int* wsum, int* least) {
+  int sum = 0, low = v0, before;
+  for (int i = threadIdx.x; i < dl; i += kCtaThreads4) {
+    const int32_t v1 = ldg_i32(g.col + a0 + i);
+    const long long b = g.rowptr[v1], e = first_ge(g.col, b, g.dptr[v1].y, v0);
+    sum += (int)(e - b < kRowCap - 1 ? e - b : kRowCap - 1);
+    if (b < e) low = min(low, ldg_i32(g.col + b));
+  }
+  if (threadIdx.x == 0) *least = v0;
+  const int w = block_scan(sum, wsum, before);
+  low = __reduce_min_sync(kFull, low);
+  if ((threadIdx.x & 31) == 0 && low < v0) atomicMin(least, low);
+  __syncthreads();
+  return w;
+}
+
+// The wedges of v0 whose v2 is in [lo, end), a range of ids at a time, each range's wedges in
+// the hash table; the first range is `step` long, each next one as long as its wedges fit by the
+// density of the last.  For tasks whose wedges are few for the ids they are spread over: a tile
+// of counters costs its scan however few it holds.  Erdos-Renyi 2^22, degree 128 (89 tiles for
+// about 10,000 wedges): 2.66 s in tiles, 0.43 s in passes (1.75 s with counters in global
+// memory).  CURSOR: up to kCursors rows, their places in registers; else searched for.
+template <bool CURSOR>
+__device__ __noinline__ unsigned long long hash_passes(const GView& g, CtaTable& h, int* wsum,
+                                                       int32_t v0, long long a0, int dl,
+                                                       int64_t lo, int64_t end, int64_t step) {
+  const int tid = threadIdx.x;
+  int cur[kRowsPerThread] = {}, len[kRowsPerThread] = {};
+  unsigned long long acc = 0;
+  // row i's place at id a (with CURSOR cur, its chunk's, says it)
+  auto place = [&](int i, int64_t a, int at, long long* e) {
+    const int32_t v1 = ldg_i32(g.col + a0 + i);
+    const long long b = g.rowptr[v1];
+    *e = g.dptr[v1].y;
+    return CURSOR ? b + at : first_ge(g.col, b, *e, (int32_t)a);
+  };
+  for (int64_t a = lo; a < end;) {
+    int64_t limit = min(a + step, end);
+    int total, before;
+    for (;;) {  // (a range of one id has at most a wedge per row)
+      int sum = 0;
+      long long e;
+      if constexpr (CURSOR) {
+#pragma unroll
+        for (int c = 0; c < kRowsPerThread; ++c) {
+          const int i = tid + c * kCtaThreads4;
+          if (i < dl) {
+            const long long p = place(i, a, cur[c], &e);
+            len[c] = (int)(first_ge(g.col, p, e, (int32_t)limit) - p);
+          }
+          sum += min(len[c], kHashWedges + 1);
+        }
+      } else {
+        for (int i = tid; i < dl; i += kCtaThreads4) {
+          const long long p = place(i, a, 0, &e);
+          sum += (int)min(first_ge(g.col, p, e, (int32_t)limit) - p, (long long)kHashWedges);
+          sum = min(sum, kHashWedges + 1);
+        }
+      }
+      total = block_scan(sum, wsum, before);
+      if (total <= kHashWedges || limit - a <= 1) break;
+      limit = a + (limit - a) / 2;
+    }
+    // one id in more rows than the table takes
+    if (total > kHashWedges && tid == 0) acc += (unsigned long long)total * (total - 1) / 2;
+    if (total > 1 && total <= kHashWedges) {
+      const int slots = slots_for(total, kHashSlots);
+      clear_table(h, slots, tid, kCtaThreads4);
+      unsigned part = 0;
+      auto walk = [&](long long p, int n) {  // the chunk's runs, one a thread
+        const int all = block_scan(n, wsum, before);
+        h.base[tid] = p;
+        h.pre[tid] = before;
+        if (tid == 0) h.pre[kSegs] = all;
+        __syncthreads();
+        int r = 0;
+        if (tid < all) {  // the run of wedge tid: largest r with pre[r] <= tid
+          int hi = kSegs;
+          while (hi - r > 1) {
+            const int mid = (r + hi) >> 1;
+            if (h.pre[mid] <= tid) r = mid; else hi = mid;
+          }
+        }
+        walk_runs(g.col, h.base, h.pre, r, tid, kCtaThreads4, all, [&](int32_t (&x)[4]) {
+          part += table_add4(h.key, h.cnt, (uint32_t)slots - 1u, x);
+        });
+      };
+      long long e;
+      if constexpr (CURSOR) {
+#pragma unroll
+        for (int c = 0; c < kRowsPerThread; ++c) {
+          if (c * kCtaThreads4 >= dl) break;
+          walk(len[c] ? place(tid + c * kCtaThreads4, a, cur[c], &e) : 0, len[c]);
+        }
+      } else {
+        for (int i0 = 0; i0 < dl; i0 += kCtaThreads4) {
+          long long p = 0;
+          int n = 0;
+          if (i0 + tid < dl) {
+            p = place(i0 + tid, a, 0, &e);
+            n = (int)(first_ge(g.col, p, e, (int32_t)limit) - p);
+          }
+          walk(p, n);
+        }
+      }
+      acc += part;
+    }
+    if constexpr (CURSOR) {
+#pragma unroll
+      for (int c = 0; c < kRowsPerThread; ++c) cur[c] += len[c];
+    }
+    const int64_t took = limit - a;
+    a = limit;
+    step = max((int64_t)1, min(4 * took, took * kPassWedges / max(total, 1)));
+  }
+  __syncthreads();
+  return acc;
+}
+
+// What k_c4_hubs says of hub h: tiles of kTileWords ids that one hash pass takes (1: tiles of
+// counters) and its smallest v2.  A vertex is in one list, so the other two lists' ends are free
+// for as many entries as there are hubs.
+__device__ __forceinline__ int32_t& hub_tiles(const C4Lists& l, int64_t nv, long long h) {
+  return l.mid[nv - 1 - h];
+}
+__device__ __forceinline__ int32_t& hub_least(const C4Lists& l, int64_t nv, long long h) {
+  return l.hash[nv - 1 - h];
+}
+
+// A CTA a hub: its wedges by its rows' lengths (most of a lower neighbour's row lies below v0).
+// R-MAT s24 ef8 (713 tiles): 2.47 s with tiles for every hub, 1.54 s.
+__global__ void __launch_bounds__(kCtaThreads4) k_c4_hubs(GView g, const C4Queue* q, C4Lists l) {
+  __shared__ unsigned long long sum_s;
+  __shared__ int low_s;
+  for (long long u = blockIdx.x; u < (long long)q->n_hub; u += gridDim.x) {
+    const int32_t v0 = l.hub[u];
+    const long long a0 = g.rowptr[v0], dl = g.dptr[v0].x - a0;
+    __syncthreads();
+    if (threadIdx.x == 0) sum_s = 0, low_s = v0;
+    __syncthreads();
+    unsigned long long sum = 0;
+    int low = v0;
+    for (long long i = threadIdx.x; i < dl; i += kCtaThreads4) {
+      const int32_t v1 = ldg_i32(g.col + a0 + i);
+      const long long b = g.rowptr[v1], e = g.dptr[v1].y;
+      sum += (unsigned long long)(e - b);
+      if (b < e) low = min(low, ldg_i32(g.col + b));
+    }
+    sum = warp_sum_u64(sum);
+    low = __reduce_min_sync(kFull, low);
+    if ((threadIdx.x & 31) == 0) {
+      atomicAdd(&sum_s, sum);
+      atomicMin(&low_s, low);
+    }
+    __syncthreads();
+    if (threadIdx.x == 0) {
+      const long long passes = (long long)(sum_s / kPassWedges) + 1;
+      const long long tiles = ((long long)v0 - low_s + kTileWords - 1) / kTileWords;
+      hub_tiles(l, g.nv, u) =
+          2 * kPassTiles * passes <= tiles ? (int32_t)max(2ll, tiles / passes) : 1;
+      hub_least(l, g.nv, u) = low_s;
+    }
+  }
+}
+
 __global__ void __launch_bounds__(kCtaThreads4, 2) k_c4_cta(GView g, C4Queue* q, C4Lists l,
+                                                            bool planned,
                                                             unsigned long long* out, GOut o) {
   extern __shared__ __align__(16) char sm[];
   let_next_start();
   __shared__ long long task_s;
   constexpr int kWarps = kCtaThreads4 / 32;
-  __shared__ int next, wsum[kWarps];
+  __shared__ int next, wsum[kWarps], least;
   CtaTile& t = *reinterpret_cast<CtaTile*>(sm);
   CtaTable& h = *reinterpret_cast<CtaTable*>(sm);
-  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const int tid = threadIdx.x, lane = tid & 31;
   unsigned long long acc = 0;
   const long long n_hub = (long long)q->n_hub, n_mid = (long long)q->n_mid,
                   n_hash = (long long)q->n_hash;
@@ -342,31 +539,66 @@ __global__ void __launch_bounds__(kCtaThreads4, 2) k_c4_cta(GView g, C4Queue* q,
     __syncthreads();
     return task_s;
   };
-  // a task tile by tile (counters zero), a cursor per row
-  auto all_tiles = [&](int32_t v0, long long a0, int dl) {
+  bool zero = n_hub + n_mid > 0;  // the tile counters are
+  auto clear_counters = [&] {
+    if (!zero)
+      for (int i = tid; i < kTileWords / 4; i += kCtaThreads4)
+        reinterpret_cast<uint4*>(t.ctr)[i] = make_uint4(0, 0, 0, 0);
+    zero = true;
+    __syncthreads();
+  };
+  // a task of w wedges from id lo on: tile by tile, a cursor per row, or in hash passes
+  auto ranges = [&](int32_t v0, long long a0, int dl, int lo, int w) {
+    const int tiles = ((int64_t)v0 - lo + 2 * kTileWords - 1) / (2 * kTileWords);
+    unsigned long long part = 0;
+    if (w >= 0 && w / kPassWedges + 1 <= tiles / kPassTiles) {
+      zero = false;
+      return hash_passes<true>(g, h, wsum, v0, a0, dl, lo, v0,
+                               max((int64_t)1, ((int64_t)v0 - lo) * kPassWedges / max(w, 1)));
+    }
+    clear_counters();
     for (int i = tid; i < dl; i += kCtaThreads4) t.cur[i] = 0;
     __syncthreads();
-    unsigned long long part = 0;
-    for (int64_t a = 0; a < v0; a += 2 * kTileWords)
+    for (int64_t a = lo; a < v0; a += 2 * kTileWords)
       part += tile_wedges<true>(g, t, &next, v0, a0, dl, a, false);
     return part;
   };
-  // hubs: unit = (hub, tile of kTileWords ids); a 16-bit tile takes two of them
+  // hubs: unit = (hub, tile of kTileWords ids); a 16-bit tile takes two of them, a hash pass as
+  // many as k_c4_hubs says
   const long long tiles = (g.nv + kTileWords - 1) / kTileWords;
   for (long long u = claim(&q->h_hub); u < n_hub * tiles; u = claim(&q->h_hub)) {
     const int32_t v0 = l.hub[u / tiles];
+    const long long tile = u % tiles, at = tile * kTileWords;
+    if (at >= v0) continue;
     const long long a0 = g.rowptr[v0];
     const int dl = (int)(g.dptr[v0].x - a0);
     const bool wide = dl > 0xFFFF;  // a counter may pass 16 bits
-    const long long tile = u % tiles;
-    if (tile * kTileWords >= v0 || (!wide && (tile & 1))) continue;
-    c4_emit(o, v0, tile_wedges<false>(g, t, &next, v0, a0, dl, tile * kTileWords, wide), acc);
+    const int most = planned ? hub_tiles(l, g.nv, u / tiles) : 1;
+    const int64_t lo = planned ? hub_least(l, g.nv, u / tiles) : 0;
+    if (most > 1) {
+      if (tile % most) continue;
+      const int64_t a = max((int64_t)at, lo), end = min((int64_t)at + (int64_t)most * kTileWords, (int64_t)v0);
+      if (a >= end) continue;
+      zero = false;
+      c4_emit(o, v0, hash_passes<false>(g, h, wsum, v0, a0, dl, a, end, end - a), acc);
+      continue;
+    }
+    if ((!wide && (tile & 1)) || at + (wide ? 1 : 2) * kTileWords <= lo) continue;
+    clear_counters();
+    c4_emit(o, v0, tile_wedges<false>(g, t, &next, v0, a0, dl, at, wide), acc);
   }
   for (long long u = claim(&q->h_mid); u < n_mid; u = claim(&q->h_mid)) {
     const int32_t v0 = l.mid[u];
     const long long a0 = g.rowptr[v0];
     const int dl = (int)(g.dptr[v0].x - a0);
-    c4_emit(o, v0, all_tiles(v0, a0, dl), acc);
+    // the wedges are looked up only where their number can matter: with enough tiles below v0,
+    // or in a batch, whose graphs begin at other ids
+    int lo = 0, w = -1;
+    if (o.gid || v0 >= 4 * kPassTiles * 2 * kTileWords) {
+      w = task_wedges(g, v0, a0, dl, wsum, &least);
+      lo = least;
+    }
+    c4_emit(o, v0, ranges(v0, a0, dl, lo, w), acc);
   }
   for (long long u = claim(&q->h_hash); u < n_hash; u = claim(&q->h_hash)) {
     const int32_t v0 = l.hash[u];
@@ -379,27 +611,20 @@ __global__ void __launch_bounds__(kCtaThreads4, 2) k_c4_cta(GView g, C4Queue* q,
       b = g.rowptr[v1];
       len = (int)(first_ge(g.col, b, g.dptr[v1].y, v0) - b);
     }
-    // (lengths are capped: a sum past the table's size only has to stay past it)
-    const int capped = min(len, kHashWedges + 1);
-    int inc = capped;
-#pragma unroll
-    for (int d = 1; d < 32; d <<= 1) {
-      const int y = __shfl_up_sync(kFull, inc, d);
-      if (lane >= d) inc += y;
-    }
-    if (lane == 31) wsum[warp] = inc;
-    __syncthreads();
-    const int ws = lane < kWarps ? wsum[lane] : 0;
-    const int before = (int)__reduce_add_sync(kFull, (unsigned)(lane < warp ? ws : 0));
-    const int total = (int)__reduce_add_sync(kFull, (unsigned)ws);
+    int before;
+    const int total = block_scan(min(len, kRowCap - 1), wsum, before);
     if (total > kHashWedges) {
-      for (int w = tid; w < kTileWords / 4; w += kCtaThreads4)
-        reinterpret_cast<uint4*>(t.ctr)[w] = make_uint4(0, 0, 0, 0);
-      c4_emit(o, v0, all_tiles(v0, a0, dl), acc);
+      if (tid == 0) least = v0;
+      __syncthreads();
+      const int low = __reduce_min_sync(kFull, len ? ldg_i32(g.col + b) : v0);
+      if (lane == 0 && low < v0) atomicMin(&least, low);
+      __syncthreads();
+      c4_emit(o, v0, ranges(v0, a0, dl, least, total), acc);
       continue;
     }
+    zero = false;
     h.base[tid] = b;
-    h.pre[tid] = before + inc - capped;
+    h.pre[tid] = before;
     if (tid == 0) h.pre[kSegs] = total;
     const int slots = slots_for(total, kHashSlots);
     clear_table(h, slots, tid, kCtaThreads4);
@@ -452,7 +677,14 @@ cudaError_t launch_cycle4(const DevGraph& g, C4Queue* q, const C4Lists& l,
   const int step = (int)std::max<int64_t>(1, std::min<int64_t>(32, g.nv / (4 * kWarps * grid)));
   e = launch_next(!next, k_c4_warp, grid, kWarpThreads, smem, s, g.view(), q, l, step, out, o);
   if (e != cudaSuccess || !cycle4_has_cta(g)) return e;
-  k_c4_cta<<<2 * num_sms, kCtaThreads4, kCtaSmem4, s>>>(g.view(), q, l, out, o);
+  // hubs are looked over where their tiles can be too many (as for the other lists)
+  const bool planned = g.max_deg > kCursors && (o.gid || g.nv >= 4 * kPassTiles * 2 * kTileWords);
+  if (planned) {
+    k_c4_hubs<<<2 * num_sms, kCtaThreads4, 0, s>>>(g.view(), q, l);
+    e = cudaGetLastError();
+    if (e != cudaSuccess) return e;
+  }
+  k_c4_cta<<<2 * num_sms, kCtaThreads4, kCtaSmem4, s>>>(g.view(), q, l, planned, out, o);
   return cudaGetLastError();
 }
 
