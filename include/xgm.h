@@ -254,8 +254,9 @@ typedef struct {
   double prep_ms;          /* device time of task generation / scheduling */
   int64_t tasks;           /* top-level tasks */
   int64_t variant_tasks[XGM_NUM_VARIANTS]; /* tasks of the task kernel; 0 where the owner and
-                              row kernels count (default and learned policies, triangles
-                              and cliques, no threshold, hub limit or hash test asked for) */
+                              row kernels count (default and learned policies with no
+                              threshold, hub limit or hash test asked for, but for even
+                              graphs of long lists) */
   uint64_t algo_bytes;     /* algorithmic adjacency bytes of the plan (0 unless requested) */
   uint32_t device_error;   /* raw device error flag */
   int launches;            /* counting passes: 1, + 1 where the hub kernel runs (the kernels

@@ -114,6 +114,10 @@ bool sched_may_bucket(const xgm_sched& sp);  // the policy can assign the BUCKET
 // The schedule leaves the choice of kernel to the engine: a default or learned policy with
 // no threshold, hub limit or membership test asked for.
 bool sched_is_open(const xgm_sched& sp);
+// What the engine then chooses, by the graph (count.cu).
+bool task_kernel_wins(const DevGraph& g, int k);
+bool task_kernel_wins_part(const DevGraph& g);
+bool task_kernel_wins_batch(const DevGraph& g, bool rows, bool part, bool five, bool tail);
 int ensure_clique_grid(xgm_ctx* ctx);
 int match_pattern(const xgm_plan_desc* d);  // builtin id, 0 unsupported, -1 malformed
 // Builtin id for a pattern name (0 if unknown); GLUMIN ids also set induced / scale.

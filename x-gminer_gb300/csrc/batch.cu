@@ -180,9 +180,12 @@ cudaError_t alloc_once(T** p, int64_t n, cudaStream_t s, bool zero = false) {
 }
 
 // Triangles, cliques and participation plans from the owner and row kernels; explicit
-// schedules, and graphs above the row capacity, run the task kernel.
-bool batch_from_rows(const DevGraph& g, const xgm_sched& sp) {
-  return sched_is_open(sp) && g.max_out <= kRowsCap && g.row_store_words <= kRowStoreMax;
+// schedules, graphs above the row capacity and graphs of long lists run the task kernel.
+bool batch_from_rows(const DevGraph& g, const Slots& sl, const xgm_sched& sp) {
+  return sched_is_open(sp) && g.max_out <= kRowsCap && g.row_store_words <= kRowStoreMax &&
+         !task_kernel_wins_batch(g, sl.k4 >= 0 || sl.k5 >= 0,
+                                 sl.tri >= 0 || sl.dia >= 0 || sl.tail >= 0, sl.k5 >= 0,
+                                 sl.tail >= 0);
 }
 
 // Allocations a sequence needs, made before any capture; *rows: the owner and row kernels
@@ -204,7 +207,7 @@ xgm_status batch_prepare(xgm_ctx* ctx, xgm_batch* b, const Slots& sl, int P, con
     batch_drop_graphs(b);
   }
   const bool part = sl.tri >= 0 || sl.dia >= 0 || sl.tail >= 0;
-  bool rows = batch_from_rows(g, sp);
+  bool rows = batch_from_rows(g, sl, sp);
   auto buffers = [&]() -> cudaError_t {
     cudaError_t e = cudaSuccess;
     if (sl.c4 >= 0) e = alloc_once(&b->c4_lists, 3 * g.nv, s);

@@ -1,7 +1,8 @@
 // Triangle and k-clique counting on the degree-oriented DAG, hand-written for sm_103a: the task
-// kernel.  It runs under explicit schedules, for roots of out-degree above 1,024 and for graphs
-// whose row store does not fit; the owner and row kernels (rows.cu) count everything else
-// (4-cliques R-MAT s22 20.0 ms against 65.6 here).
+// kernel.  It runs under explicit schedules, for roots of out-degree above 1,024, for graphs
+// whose row store does not fit and for even graphs of long lists (task_kernel_wins, count.cu);
+// the owner and row kernels (rows.cu) count everything else (4-cliques R-MAT s22 20.0 ms against
+// 65.6 here).
 //
 // Reference kernels this replaces (same counts, different schedule):
 //  - warp_edge (TC): codes/GraphMiner/src/triangle/gpu_kernels/bs_warp_edge.cuh:1-20

@@ -94,6 +94,60 @@ bool sched_is_open(const xgm_sched& sp) {
   return sp.hub_max == 0 && !(sp.flags & XGM_SCHED_HASH_ONLY);
 }
 
+// Whether the task kernel is the faster one for an open schedule.  It streams N+(u) for every
+// edge (v, u); the owner kernel tests the part of N+(v) after u, coalesced against a bitmap
+// where u is of its top ranks, else a lane an edge.  In skewed graphs the streams are several
+// times the tests (R-MAT s14 and up 2.5 to 5 times, Chung-Lu 3 to 6) and mostly of bitmap
+// vertices, and the owner kernel wins by 2 to 20 times; in even ones (stream < 2 pairs:
+// Erdos-Renyi 1.05 to 1.2, geometric 1.3, Barabasi-Albert 2.0) it depends on how long the lists
+// are and whether the bitmaps cover them.  Unions of cliques (stream = pairs: every test hits)
+// keep the owner kernel.  Measured, task kernel against owner / row kernels in ms:
+//  triangles: Erdos-Renyi 2^20 degree 256 30.8 / 36.1; 2^20 degree 192 21.3 / 20.6
+//  4-cliques: Erdos-Renyi 2^20 degree 24 1.04 / 0.63, 48 2.41 / 2.75, 64 3.64 / 4.63, 128
+//    12.3 / 14.8; all bitmaps (2^17): degree 128 1.41 / 1.57, 192 2.62 / 2.21; small (2^14):
+//    degree 64 0.156 / 0.147, 96 0.208 / 0.282; Barabasi-Albert 1 M degree 64 4.03 / 4.68
+//  5-cliques: Erdos-Renyi 2^20 degree 24 1.02 / 0.53, 48 2.39 / 4.28; 2^17 degree 256 3.90 /
+//    4.26; 20,001 vertices of degree 300 1.06 / 0.88; geometric, degree 200 118 / 32.6
+//  7-cliques without bitmaps: a lane's recursion is as long as the longest of 32 rows; ring
+//    lattice 2^18 degree 80 956 / 2,044, cliques of 60 452 / 685, of 100 980 / 660
+bool task_kernel_wins(const DevGraph& g, int k) {
+  const double T = g.stream, P = g.pairs, E = (double)g.ne_dag, Tb = g.stream_big[0];
+  if (k == 3) return T < 2 * P && 2 * Tb < T && T > 80 * E;
+  if (g.max_out > kRowsCap || P < 12 * E) return false;
+  // (a task kernel's call is 13 launches: worth it from some work on)
+  if (P * (P / E) < (k == 4 ? 6e8 : 1.2e8)) return false;
+  if (k == 7 && T < 2.5 * P && 2 * Tb < T && P < 32 * E) return true;
+  if (T < 1.01 * P || T >= 2 * P) return false;
+  const bool covered = 5 * Tb >= 3 * T && T >= (k == 4 ? 48 : k == 5 ? 70 : 100) * E;
+  return !covered;
+}
+
+// The same for triangles per edge (diamonds, tailed triangles).  A bitmap owner's ranks cost a
+// scan of its bitmap, a thirty-second of the bitmap vertices above it: n^2 / 64 words in all.
+// Task kernel against owner kernel in ms, by n^2 / stream: Erdos-Renyi 2^17 degree 192 (21) 2.75
+// / 2.20, 2^18 degree 256 (24) 8.06 / 9.87, degree 128 (81) 3.24 / 5.80, ring lattice 2^18
+// degree 160 (41) 6.87 / 8.52, Barabasi-Albert 200,001 of degree 200 (13) 8.04 / 4.90.  Without
+// bitmaps, by pairs an edge: Erdos-Renyi 2^20 (14) 2.73 / 2.77, (19) 4.14 / 4.75, (29) 8.16 /
+// 9.93; Barabasi-Albert 1 M degree 64 (16) 4.56 / 4.07.
+bool task_kernel_wins_part(const DevGraph& g) {
+  const double T = g.stream, P = g.pairs, E = (double)g.ne_dag;
+  const double n = (double)std::min<int64_t>(g.n_big, own_bits(true));
+  if (g.max_out > kShortLists && n * n > 22 * T) return true;
+  return 2 * g.stream_big[1] < T && P >= 17 * E && T > 1.01 * P && T < 3 * P;
+}
+
+// And for a batch, whose ranks are sorted per graph: no bitmaps, a lane an edge joins both
+// lists.  rows, part: the plans need the row store, triangles per edge; five, tail: there are
+// 5-cliques, tailed triangles among them.  By (pairs + stream) an edge, task kernel / owner and
+// row kernels in ms: triangles + 4-cliques + diamonds 1,000
+// R-MAT s9 ef16 (23) 0.75 / 0.75, 200 s12 ef4 (20) 0.53 / 0.64, 200 s11 ef8 (26) 0.47 / 0.60,
+// 4,096 Barabasi-Albert (8) 5.5 / 1.16; 5-cliques 250 s10 ef16 (31) 0.61 / 0.78; 4-cliques alone
+// 0.45 / 0.37 there, 100 s12 ef8 (33) 0.49 / 0.51; triangles + diamonds 0.49 / 0.41 and 0.52 /
+// 0.61; tailed triangles 200 s11 ef8 0.45 / 0.50; 16 s16 ef16 (141) 6.3 / 22.9.
+bool task_kernel_wins_batch(const DevGraph& g, bool rows, bool part, bool five, bool tail) {
+  return g.pairs + g.stream >= ((rows && part) || five || tail ? 20.0 : 31.0) * (double)g.ne_dag;
+}
+
 // Fills tb from the schedule policy for a k-clique style launch (k = 3 for the
 // participation and multi-pattern launches).  Builds the graph's bucket index first
 // when the policy can pick BUCKET (outside stream capture: callers that capture call
@@ -171,7 +225,7 @@ xgm_status clique_route(xgm_ctx* ctx, const DevGraph& g, int k, const xgm_sched&
                         CliqueRoute* route) {
   cudaStream_t s = ctx->stream;
   *route = CliqueRoute::kTasks;
-  if (sched_is_open(sp)) {
+  if (sched_is_open(sp) && !task_kernel_wins(g, k)) {
     if (k == 3) {
       *route = CliqueRoute::kOwner;
     } else if (g.nv > 0 && g.row_store_words <= kRowStoreMax) {
@@ -225,7 +279,7 @@ xgm_status launch_participation(xgm_ctx* ctx, const DevGraph& g, const xgm_sched
   cudaStream_t s = ctx->stream;
   xgm_sched tri = sp;
   if (tri.policy == XGM_SCHED_LEARNED && !tri.model) tri.policy = XGM_SCHED_HEURISTIC;
-  *tasks = !sched_is_open(tri) || g.max_out > kOwnPartMaxOut;
+  *tasks = !sched_is_open(tri) || g.max_out > kOwnPartMaxOut || task_kernel_wins_part(g);
   XGM_CUDA_TRY(with_room(ctx, [&] { return grow(&ctx->epart, &ctx->epart_cap, g.ne, s); }));
   XGM_CUDA_TRY(cudaMemsetAsync(ctx->epart, 0, sizeof(unsigned) * (g.ne > 0 ? g.ne : 1), s));
   if (!*tasks) {
@@ -277,6 +331,8 @@ xgm_status count_dispatch(xgm_ctx* ctx, const DevGraph& g, int pattern, const xg
     if (r != XGM_OK) return r;
     if (pattern == XGM_PATTERN_DIAMOND)
       XGM_CUDA_TRY(launch_diamond_reduce(ctx->epart, g.ne, &ctx->d_sc->count, s));
+    else if (tasks)  // one pass over the vertices (Erdos-Renyi 2^20 degree 256 33.0 -> 31.8 ms)
+      XGM_CUDA_TRY(launch_tailed_reduce(view, ctx->vpart, &ctx->d_sc->count, s));
     else
       XGM_CUDA_TRY(launch_motif_terms(view, ctx->epart, ctx->d_sc->terms, s));
     launches = 2;
@@ -316,8 +372,8 @@ xgm_status count_dispatch(xgm_ctx* ctx, const DevGraph& g, int pattern, const xg
   else if (!k && !tasks && pattern != XGM_PATTERN_CYCLE4) st.tasks = g.n_roots[0];
   r = check_device_flag(ctx, ctx->h_sc->err);
   if (r != XGM_OK) return r;
-  *out = pattern == XGM_PATTERN_TAILED_TRIANGLE ? tailed_from_terms(ctx->h_sc->terms)
-                                                : ctx->h_sc->count;
+  *out = pattern == XGM_PATTERN_TAILED_TRIANGLE && !tasks ? tailed_from_terms(ctx->h_sc->terms)
+                                                          : ctx->h_sc->count;
   return XGM_OK;
 }
 
@@ -483,9 +539,10 @@ xgm_status motif4_parts(xgm_ctx* ctx, const DevGraph& g, const xgm_sched& sp, bo
                         Motif4Parts& m, xgm_stats& st) {
   xgm_stats x;
   // open schedules, every vertex within the row capacity: rows and triangles per edge from
-  // one owner pass, all parts behind one read-back
-  CliqueRoute route = CliqueRoute::kTasks;
-  if (sched_is_open(sp) && g.max_out <= kRowsCap) {
+  // one owner pass, all parts behind one read-back (but where the task kernel wins both)
+  bool rows = false;
+  if (sched_is_open(sp) && g.nv > 0 && g.max_out <= kRowsCap && g.row_store_words <= kRowStoreMax &&
+      !(task_kernel_wins(g, 4) && task_kernel_wins_part(g))) {
     cudaStream_t s = ctx->stream;
     XGM_CUDA_TRY(cudaSetDevice(ctx->device));
     XGM_CUDA_TRY(with_room(ctx, [&] {
@@ -493,10 +550,9 @@ xgm_status motif4_parts(xgm_ctx* ctx, const DevGraph& g, const xgm_sched& sp, bo
       if (e == cudaSuccess && need_c4) e = grow(&ctx->c4_lists, &ctx->c4_lists_cap, 3 * g.nv, s);
       return e;
     }));
-    xgm_status q = clique_route(ctx, g, 4, sp, &route);
-    if (q != XGM_OK) return q;
+    XGM_CUDA_TRY(reserve_rows(g, &ctx->rows, &ctx->rows_cap, &rows, s));
   }
-  if (route == CliqueRoute::kRows) {
+  if (rows) {
     cudaStream_t s = ctx->stream;
     Scalars* sc = ctx->d_sc;
     XGM_CUDA_TRY(cudaMemsetAsync(sc, 0, sizeof(Scalars), s));
@@ -583,7 +639,7 @@ xgm_status count_motifs(xgm_ctx* ctx, const DevGraph& g, int k, const xgm_sched&
   if (k == 3) {
     uint64_t t[6], tri = 0;
     xgm_stats x;
-    if (sched_is_open(sp)) {  // both parts behind one read-back
+    if (sched_is_open(sp) && !task_kernel_wins(g, 3)) {  // both parts behind one read-back
       cudaStream_t s = ctx->stream;
       Scalars* sc = ctx->d_sc;
       XGM_CUDA_TRY(cudaSetDevice(ctx->device));

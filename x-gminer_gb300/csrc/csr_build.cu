@@ -229,14 +229,24 @@ __global__ void k_rank_entry_keys_long(const int64_t* rowptr_o, const int32_t* c
   }
 }
 
+// Statistics of finish_graph, one word each.
+enum {
+  kStMaxDeg, kStMaxOut, kStNeDag, kStLong, kStBig, kStRoots, kStWords = kStRoots + 5, kStPairs,
+  kStStream, kStStreamBig, kStEnd = kStStreamBig + 2
+};
+
 // dptr[r] = {first entry of row r with id > r, row end}; stats of the DAG.
-__global__ void k_dptr(const int64_t* rowptr, const int32_t* col, int64_t nv, longlong2* dptr,
-                       unsigned long long* max_out, unsigned long long* ne_dag,
-                       unsigned long long* n_big, unsigned long long* n_roots) {
-  int64_t mo = 0;
-  unsigned long long sum = 0;
+__global__ void __launch_bounds__(kThreads) k_dptr(const int64_t* rowptr, const int32_t* col,
+                                                   int64_t nv, longlong2* dptr,
+                                                   unsigned long long* stats) {
+  __shared__ unsigned long long blk[kStEnd];
+  if (threadIdx.x < kStEnd) blk[threadIdx.x] = 0;
+  __syncthreads();
+  unsigned mo = 0;
   unsigned cnt[6] = {0, 0, 0, 0, 0, 0};  // degree > kBigDeg; out-degree >= 2 .. 6
-  unsigned long long words = 0;       // of the row store
+  // entries, row store words, tests, streams (and of those the bitmap tier's, count and
+  // participation modes)
+  unsigned long long sum[6] = {0, 0, 0, 0, 0, 0};
   for (int64_t r = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; r < nv;
        r += (int64_t)gridDim.x * blockDim.x) {
     int64_t lo = rowptr[r], hi = rowptr[r + 1];
@@ -246,30 +256,39 @@ __global__ void k_dptr(const int64_t* rowptr, const int32_t* col, int64_t nv, lo
       if (col[mid] > r) b = mid; else a = mid + 1;
     }
     dptr[r] = make_longlong2(a, hi);
-    int64_t d = hi - a;
-    mo = d > mo ? d : mo;
-    sum += (unsigned long long)d;
-    words += row_words(d);
-    cnt[0] += hi - lo > kBigDeg;
+    const unsigned long long d = (unsigned long long)(hi - a);
+    const unsigned long long through = (unsigned long long)(a - lo) * d;
+    const bool big = hi - lo > kBigDeg;
+    mo = d > mo ? (unsigned)d : mo;
+    sum[0] += d;
+    sum[1] += row_words((int64_t)d);
+    sum[2] += d * (d - (d > 0)) / 2;
+    sum[3] += through;
+    if (big && r >= nv - own_bits(false)) sum[4] += through;
+    if (big && r >= nv - own_bits(true)) sum[5] += through;
+    cnt[0] += big;
 #pragma unroll
-    for (int t = 1; t < 6; ++t) cnt[t] += d > t;
+    for (int t = 1; t < 6; ++t) cnt[t] += d > (unsigned long long)t;
   }
+  const bool first = (threadIdx.x & 31) == 0;
 #pragma unroll
   for (int t = 0; t < 6; ++t) {
     const unsigned c = __reduce_add_sync(kFull, cnt[t]);
-    if ((threadIdx.x & 31) == 0 && c) atomicAdd(t ? n_roots + t - 1 : n_big, (unsigned long long)c);
+    if (first && c) atomicAdd(&blk[t ? kStRoots + t - 1 : kStBig], (unsigned long long)c);
   }
+  constexpr int kSums[6] = {kStNeDag, kStWords, kStPairs, kStStream, kStStreamBig, kStStreamBig + 1};
 #pragma unroll
-  for (int o = 16; o > 0; o >>= 1) {
-    int64_t y = __shfl_down_sync(kFull, mo, o);
-    mo = y > mo ? y : mo;
-    sum += __shfl_down_sync(kFull, sum, o);
-    words += __shfl_down_sync(kFull, words, o);
+  for (int t = 0; t < 6; ++t) {
+    const unsigned long long c = warp_sum_u64(sum[t]);
+    if (first && c) atomicAdd(&blk[kSums[t]], c);
   }
-  if ((threadIdx.x & 31) == 0) {
-    if (words) atomicAdd(n_roots + 5, words);
-    if (mo > 0) atomicMax(max_out, (unsigned long long)mo);
-    if (sum) atomicAdd(ne_dag, sum);
+  mo = __reduce_max_sync(kFull, mo);
+  if (first && mo) atomicMax(&blk[kStMaxOut], (unsigned long long)mo);
+  __syncthreads();
+  const int t = threadIdx.x;
+  if (t < kStEnd && blk[t]) {
+    if (t == kStMaxOut) atomicMax(stats + t, blk[t]);
+    else atomicAdd(stats + t, blk[t]);
   }
 }
 
@@ -417,21 +436,19 @@ cudaError_t finish_graph(DevGraph& g, const int32_t* group, int num_groups, cuda
   const int64_t nv = g.nv, ne = g.ne;
   const int vb = bits_for(nv);
   int32_t *deg = nullptr, *degp = nullptr;
-  // [0] max deg, [1] max out, [2] ne_dag, [3] long rows, [4] big vertices, [5..9] roots,
-  // [10] row store words
   unsigned long long* stats = nullptr;
   TRY(dalloc(&deg, nv, s));
   TRY(dalloc(&degp, nv, s));
-  TRY(dalloc(&stats, 11, s));
-  TRY(cudaMemsetAsync(stats, 0, 11 * sizeof(unsigned long long), s));
+  TRY(dalloc(&stats, kStEnd, s));
+  TRY(cudaMemsetAsync(stats, 0, kStEnd * sizeof(unsigned long long), s));
   if (nv > 0) {
-    k_degrees<<<grid_for(nv), kThreads, 0, s>>>(g.rowptr_o, nv, deg, stats);
+    k_degrees<<<grid_for(nv), kThreads, 0, s>>>(g.rowptr_o, nv, deg, stats + kStMaxDeg);
     TRY(cudaGetLastError());
   }
-  unsigned long long h[11] = {};
+  unsigned long long h[kStEnd] = {};
   TRY(cudaMemcpyAsync(h, stats, sizeof(h), cudaMemcpyDeviceToHost, s));
   TRY(cudaStreamSynchronize(s));
-  g.max_deg = (int64_t)h[0];
+  g.max_deg = (int64_t)h[kStMaxDeg];
   const int db = bits_for(g.max_deg + 1);
   const int gb = group ? bits_for(num_groups) : 0;
   if (vb + db + gb > 64) return cudaErrorInvalidValue;
@@ -466,30 +483,33 @@ cudaError_t finish_graph(DevGraph& g, const int32_t* group, int num_groups, cuda
     const int64_t cap = ne / kLongRow + 1;
     int32_t* longs = nullptr;
     TRY(dalloc(&longs, cap, s));
-    TRY(cudaMemsetAsync(stats + 3, 0, sizeof(unsigned long long), s));
+    TRY(cudaMemsetAsync(stats + kStLong, 0, sizeof(unsigned long long), s));
     k_rank_entry_keys<<<grid_for(nv), kThreads, 0, s>>>(g.rowptr_o, g.col_o, g.rank, g.perm,
-                                                        g.rowptr, nv, vb, keys, longs, stats + 3);
+                                                        g.rowptr, nv, vb, keys, longs,
+                                                        stats + kStLong);
     TRY(cudaGetLastError());
     const dim3 lg((unsigned)std::min<int64_t>(cap, 2048), kLongSplit);
     k_rank_entry_keys_long<<<lg, kThreads, 0, s>>>(g.rowptr_o, g.col_o, g.rank, g.perm, g.rowptr,
-                                                   longs, stats + 3, vb, keys);
+                                                   longs, stats + kStLong, vb, keys);
     TRY(cudaGetLastError());
     cudaFreeAsync(longs, s);
   }
   // the last pass writes the columns alone
   TRY(radix_sort_u64(keys, tmp, ne, vb, s, vb, g.col, (uint32_t)((1ull << vb) - 1)));
   if (nv > 0) {
-    k_dptr<<<grid_for(nv), kThreads, 0, s>>>(g.rowptr, g.col, nv, g.dptr, stats + 1, stats + 2,
-                                             stats + 4, stats + 5);
+    k_dptr<<<grid_for(nv), kThreads, 0, s>>>(g.rowptr, g.col, nv, g.dptr, stats);
     TRY(cudaGetLastError());
   }
   TRY(cudaMemcpyAsync(h, stats, sizeof(h), cudaMemcpyDeviceToHost, s));
   TRY(cudaStreamSynchronize(s));
-  g.max_out = (int64_t)h[1];
-  g.ne_dag = (int64_t)h[2];
-  g.n_big = group ? 0 : (int64_t)h[4];
-  for (int i = 0; i < 5; ++i) g.n_roots[i] = (int64_t)h[5 + i];
-  g.row_store_words = (int64_t)h[10];
+  g.max_out = (int64_t)h[kStMaxOut];
+  g.ne_dag = (int64_t)h[kStNeDag];
+  g.n_big = group ? 0 : (int64_t)h[kStBig];
+  for (int i = 0; i < 5; ++i) g.n_roots[i] = (int64_t)h[kStRoots + i];
+  g.row_store_words = (int64_t)h[kStWords];
+  g.pairs = (double)h[kStPairs];
+  g.stream = (double)h[kStStream];
+  for (int i = 0; i < 2; ++i) g.stream_big[i] = group ? 0.0 : (double)h[kStStreamBig + i];
   cudaFreeAsync(keys, s);
   cudaFreeAsync(tmp, s);
   cudaFreeAsync(deg, s);

@@ -21,6 +21,10 @@ struct DevGraph {
   int64_t n_big = 0;       // vertices of degree > kBigDeg: the top ranks (rows.cuh; 0 for
                            // batched graphs, whose ranks are sorted by degree per graph)
   int64_t n_roots[5] = {0, 0, 0, 0, 0};  // vertices of out-degree >= 2 .. 6
+  // elements that a count of triangles touches: sum of C(d+(v), 2) (the owner kernel's tests)
+  // and of d+(u) over edges (v, u) (the task kernel's streams); the latter over the u that the
+  // owner kernel holds as bitmaps, in its count and row modes and in its participation modes
+  double pairs = 0, stream = 0, stream_big[2] = {0, 0};
   int64_t* rowptr_o = nullptr;
   int32_t* col_o = nullptr;
   int32_t* rank = nullptr;   // [nv] original -> rank

@@ -46,6 +46,20 @@ __global__ void __launch_bounds__(kThreads) k_diamond_reduce(const unsigned* epa
   if ((threadIdx.x & 31) == 0 && acc) atomicAdd(out, acc);
 }
 
+// Sum of t(v) (deg(v) - 2), t(v) the triangles of v (the task kernel's; the owner kernel counts
+// them per edge, k_motif_terms).
+__global__ void __launch_bounds__(kThreads) k_tailed_reduce(GView g, const unsigned long long* vpart,
+                                                            unsigned long long* out) {
+  unsigned long long acc = 0;
+  for (int64_t r = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; r < g.nv;
+       r += (int64_t)gridDim.x * blockDim.x) {
+    const int64_t d = g.rowptr[r + 1] - g.rowptr[r];
+    if (d > 2) acc += vpart[r] * (unsigned long long)(d - 2);
+  }
+  acc = warp_sum_u64(acc);
+  if ((threadIdx.x & 31) == 0 && acc) atomicAdd(out, acc);
+}
+
 // C(d, 3) in wrapping uint64 arithmetic without an intermediate overflow for d < 2^32:
 // 3 divides one of d, d-1, d-2; when it does not divide x = d(d-1)/2 it divides d-2.
 __device__ __forceinline__ unsigned long long choose3(unsigned long long d) {
@@ -275,6 +289,13 @@ cudaError_t launch_diamond_reduce(const unsigned* epart, int64_t ne, unsigned lo
                                   cudaStream_t s) {
   k_diamond_reduce<<<std::min(grid_for((ne + 3) / 4), kReduceBlocks), kThreads, 0, s>>>(epart, ne,
                                                                                        out);
+  return cudaGetLastError();
+}
+
+cudaError_t launch_tailed_reduce(const GView& g, const unsigned long long* vpart,
+                                 unsigned long long* out, cudaStream_t s) {
+  if (g.nv == 0) return cudaSuccess;
+  k_tailed_reduce<<<std::min(grid_for(g.nv), kReduceBlocks), kThreads, 0, s>>>(g, vpart, out);
   return cudaGetLastError();
 }
 

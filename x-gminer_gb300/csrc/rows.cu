@@ -18,7 +18,9 @@
 //    first, and are tested by eight lanes each, a 16-byte unit per lane and step.  A hub's
 //    in-neighbours are many units (u, chunk) that any CTA can take.
 //  - the other u: one lane per edge (v, u) meets the suffix with N+(u) (merge_lists); both
-//    are short (deg v <= deg u <= kBigDeg, or no list above kShortLists).
+//    are short where deg v <= deg u <= kBigDeg or no list is above kShortLists.  Longer ones
+//    come here too where more vertices are above kBigDeg than the bitmap has bits, and in
+//    batches: a graph with many of them is the task kernel's (task_kernel_wins, count.cu).
 // Bitmaps are cleared by taking the inserted bits out again: a unit costs d+(u) stores,
 // not the bitmap's size.
 //
@@ -56,11 +58,6 @@ constexpr int kOwnThreads = 256;
 constexpr int kOwnWarps = kOwnThreads / 32;
 constexpr int kOwnChunk = 512;   // in-neighbours of one unit (two per thread)
 constexpr int kOwnShort = 12;    // longest suffix one thread tests by itself
-// Largest out-degree of a graph whose edges are all joined by lanes: a bitmap unit costs its
-// phases' latency however short its lists.  Barabasi-Albert, 3,312 vertices (at most 7) triangles
-// 25.7 -> 20.2 us; 200,001 vertices of degree 16 (17) triangles 75 -> 54 us, 4-cliques 109 -> 91;
-// R-MAT s10 ef5 (26) diamonds 42 -> 50 us, 4-cliques 37.5 -> 39.9.
-constexpr int kShortLists = 24;
 constexpr int kOwnLevels = 512;  // most units of one owner (host: raises the chunk above it)
 constexpr int kSmallStep = 128;  // most vertices per claim of the small phase
 

@@ -18,6 +18,12 @@ constexpr int64_t kOwnBits = int64_t(1) << 18;
 // 2^18, triangles per edge s23 48.0 ms (2^17 49.5).
 constexpr int64_t own_bits(bool part) { return part ? kOwnBits : kOwnBits / 2; }
 
+// Largest out-degree of a graph whose edges are all joined by lanes: a bitmap unit costs its
+// phases' latency however short its lists.  Barabasi-Albert, 3,312 vertices (at most 7) triangles
+// 25.7 -> 20.2 us; 200,001 vertices of degree 16 (17) triangles 75 -> 54 us, 4-cliques 109 -> 91;
+// R-MAT s10 ef5 (26) diamonds 42 -> 50 us, 4-cliques 37.5 -> 39.9.
+constexpr int kShortLists = 24;
+
 // Row store up to 16 GB (R-MAT scale 22: 1.9 GB); larger graphs, and a device without that
 // much memory left, count with the task kernel.
 constexpr int64_t kRowStoreMax = int64_t(1) << 32;  // words
