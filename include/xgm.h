@@ -216,8 +216,11 @@ typedef enum {
 
 /* Autotuned schedule: the variant for each out-degree bucket.  Bucket b holds
  * out-degrees s with floor(log2(s)) == b - 1 (bucket 0: s == 0), the last bucket
- * everything above.  A variant that cannot hold a task falls back by capacity. */
+ * everything above.  A variant that cannot hold a task falls back by capacity.  A table
+ * that is XGM_TUNE_ENGINE throughout leaves the choice to the engine, as the default
+ * schedule does: none of the variants was faster. */
 #define XGM_TUNE_BUCKETS 16
+enum { XGM_TUNE_ENGINE = 255 };
 typedef struct {
   uint8_t variant[XGM_TUNE_BUCKETS];
 } xgm_tune_table;
@@ -307,7 +310,8 @@ xgm_status xgm_algo_bytes(xgm_ctx* ctx, const xgm_graph* g, const xgm_plan* plan
 /* ----------------------------------------------------------------- autotuner */
 /* Empirical search of the per-bucket variant table for `plan` on g (or on a batch when
  * g is NULL and b is set): coordinate descent over buckets, each candidate timed as
- * the median of `reps` counts; the counts are checked equal to the first.  `best_ms` /
+ * the median of `reps` counts; the counts are checked equal to the first.  Where the default
+ * schedule is the fastest, the table is XGM_TUNE_ENGINE throughout.  `best_ms` /
  * `heuristic_ms` report the tuned and plain per-call times.  No counterpart in the
  * reference (its thresholds are compile-time constants, common.h:114-116). */
 typedef struct {

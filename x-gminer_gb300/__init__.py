@@ -56,6 +56,7 @@ SCHED_HEURISTIC, SCHED_LEARNED, SCHED_FIXED, SCHED_TUNED = 0, 1, 2, 3
 SCHED_NO_GRAPH = 1
 SCHED_HASH_ONLY = 2  # CTA tasks use the Bloom filter + hash, never the span bitmap
 TUNE_BUCKETS = 16
+TUNE_ENGINE = 255  # every entry of a table that leaves the choice to the engine
 VAR_WARP, VAR_CTA, VAR_SPLIT, VAR_WIDE, VAR_SEARCH, VAR_BUCKET, VAR_GROUP = 0, 1, 2, 3, 4, 5, 6
 NUM_VARIANTS = 7
 ALL_VARIANTS = (VAR_WARP, VAR_CTA, VAR_SPLIT, VAR_WIDE, VAR_SEARCH, VAR_BUCKET, VAR_GROUP)

@@ -474,7 +474,7 @@ xgm_status xgm_count(xgm_ctx* ctx, const xgm_graph* g, const xgm_plan* plan, con
   if (!ctx || !g || !plan || !out_count) return XGM_ERR_INVALID;
   xgm_sched def;
   std::memset(&def, 0, sizeof(def));
-  const xgm_sched& sp = sched ? *sched : def;
+  const xgm_sched sp = sched_resolved(sched ? *sched : def);
   xgm_stats st_local;
   xgm_stats& st = stats ? *stats : st_local;
   std::memset(&st, 0, sizeof(st));
@@ -499,7 +499,8 @@ xgm_status xgm_motif_count(xgm_ctx* ctx, const xgm_graph* g, int k, const xgm_sc
   xgm_stats& st = stats ? *stats : st_local;
   std::memset(&st, 0, sizeof(st));
   ctx->timed = stats != nullptr;
-  return finish_status(ctx, count_motifs(ctx, g->g, k, sched ? *sched : def, counts, st));
+  return finish_status(ctx, count_motifs(ctx, g->g, k, sched_resolved(sched ? *sched : def),
+                                         counts, st));
 }
 
 xgm_status xgm_count_kernels(xgm_ctx* ctx, const xgm_graph* g, const xgm_plan* plan,
@@ -509,7 +510,8 @@ xgm_status xgm_count_kernels(xgm_ctx* ctx, const xgm_graph* g, const xgm_plan* p
     return finish_status(ctx, program_kernels(ctx, g->g, plan->prog, n_kernels));
   xgm_sched def;
   std::memset(&def, 0, sizeof(def));
-  return finish_status(ctx, count_kernels(ctx, g->g, plan->pattern, sched ? *sched : def, n_kernels));
+  return finish_status(ctx, count_kernels(ctx, g->g, plan->pattern,
+                                          sched_resolved(sched ? *sched : def), n_kernels));
 }
 
 xgm_status xgm_tc_solver(xgm_ctx* ctx, const xgm_graph* g, uint64_t* total) {

@@ -111,6 +111,8 @@ void program_buffers_free(xgm_ctx* ctx);
 xgm_status schedule_into(TaskBuf& tb, const DevGraph& g, int k, const xgm_sched& sp,
                          cudaStream_t s, int k_feat = 0, bool hub = false);
 bool sched_may_bucket(const xgm_sched& sp);  // the policy can assign the BUCKET variant
+// The schedule to follow: a tuned one whose table leaves the choice to the engine is the default.
+xgm_sched sched_resolved(const xgm_sched& sp);
 // The schedule leaves the choice of kernel to the engine: a default or learned policy with
 // no threshold, hub limit or membership test asked for.
 bool sched_is_open(const xgm_sched& sp);

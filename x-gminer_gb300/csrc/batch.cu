@@ -517,7 +517,8 @@ xgm_status xgm_count_batched(xgm_ctx* ctx, xgm_batch* b, const xgm_plan* const* 
   xgm_stats& st = stats ? *stats : local;
   std::memset(&st, 0, sizeof(st));
   ctx->timed = stats != nullptr;
-  return finish_status(ctx, count_batched_impl(ctx, b, plans, n_plans, sched ? *sched : def, out, st));
+  return finish_status(
+      ctx, count_batched_impl(ctx, b, plans, n_plans, sched_resolved(sched ? *sched : def), out, st));
 }
 
 void xgm_batch_destroy(xgm_batch* b) {
@@ -605,6 +606,10 @@ xgm_status xgm_autotune(xgm_ctx* ctx, const xgm_graph* g, xgm_batch* b, const xg
       }
       tab.variant[k] = bestv;
     }
+  }
+  if (base_ms <= best) {  // no table is worth leaving the engine's choice for
+    std::memset(tab.variant, XGM_TUNE_ENGINE, sizeof(tab.variant));
+    best = base_ms;
   }
   out->table = tab;
   out->best_ms = best;

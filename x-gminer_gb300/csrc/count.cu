@@ -84,6 +84,17 @@ int whole_hub_max(int k, int asked) {
 
 }  // namespace
 
+xgm_sched sched_resolved(const xgm_sched& sp) {
+  if (sp.policy != XGM_SCHED_TUNED || !sp.table) return sp;
+  for (int b = 0; b < XGM_TUNE_BUCKETS; ++b)
+    if (sp.table->variant[b] != XGM_TUNE_ENGINE) return sp;
+  xgm_sched r;
+  std::memset(&r, 0, sizeof(r));
+  r.flags = sp.flags;
+  r.hub_max = sp.hub_max;
+  return r;
+}
+
 bool sched_is_open(const xgm_sched& sp) {
   if (sp.policy == XGM_SCHED_LEARNED) {
     if (!sp.model) return false;  // refused by schedule_into
