@@ -194,7 +194,10 @@ void xgm_plan_destroy(xgm_plan* p);
 /* ---------------------------------------------------------------- schedule */
 typedef enum {
   XGM_SCHED_HEURISTIC = 0, /* degree-threshold split (common.h:114-116 analogue) */
-  XGM_SCHED_LEARNED = 1,   /* MLP cost model picks variant + order; needs a model */
+  XGM_SCHED_LEARNED = 1,   /* MLP cost model picks variant + order of the task kernel's tasks;
+                              needs a model.  Where the owner and row kernels count (see
+                              xgm_stats.variant_tasks), as under the default policy, these are
+                              the roots of out-degree above 1024, whose variant is given */
   XGM_SCHED_FIXED = 2,     /* force `variant` for every task (tuning / logging) */
   XGM_SCHED_TUNED = 3      /* per out-degree bucket variant table from xgm_autotune */
 } xgm_sched_policy;

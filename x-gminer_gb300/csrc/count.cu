@@ -250,7 +250,8 @@ xgm_status clique_route(xgm_ctx* ctx, const DevGraph& g, int k, const xgm_sched&
   if (*route == CliqueRoute::kTasks)
     XGM_CUDA_TRY(with_room(ctx, [&] { return taskbuf_reserve(ctx->tb, g.nv, s); }));
   if (*route == CliqueRoute::kTasks && sched_may_bucket(sp)) XGM_CUDA_TRY(ensure_bucket_index(g, s));
-  if (*route == CliqueRoute::kTasks && sp.policy == XGM_SCHED_LEARNED)
+  if (sp.policy == XGM_SCHED_LEARNED &&
+      (*route == CliqueRoute::kTasks || (*route == CliqueRoute::kRows && g.max_out > kRowsCap)))
     XGM_CUDA_TRY(ensure_task_stats(g, s));
   return XGM_OK;
 }
@@ -264,9 +265,12 @@ xgm_status launch_route(xgm_ctx* ctx, const DevGraph& g, int k, const xgm_sched&
   if (route == CliqueRoute::kTasks) {
     xgm_status r = schedule_tasks(ctx, g, k, sp, true);
     if (r != XGM_OK) return r;
-  } else if (hubs) {  // only the vertices above the row capacity are tasks
-    XGM_CUDA_TRY(classify_heuristic(g, kRowsCap + 2, kWarpCap, kWideCap, kCtaCap, ctx->tb, s));
-    XGM_CUDA_TRY(build_lists(g, ctx->tb, false, s, whole_hub_max(k, 0)));
+  } else if (hubs) {  // only the vertices above the row capacity are tasks: all split or whole,
+                      // in the order of a learned schedule's model where it asks for one
+    const bool learned = sp.policy == XGM_SCHED_LEARNED, order = learned && sp.order_by_cost != 0;
+    XGM_CUDA_TRY(learned ? classify_learned(g, kRowsCap + 2, *sp.model, ctx->tb, order, sp.margin, s, k)
+                         : classify_heuristic(g, kRowsCap + 2, kWarpCap, kWideCap, kCtaCap, ctx->tb, s));
+    XGM_CUDA_TRY(build_lists(g, ctx->tb, order, s, whole_hub_max(k, 0)));
   }
   XGM_CUDA_TRY(ctx_mark(ctx, 1));
   if (launches) *launches = 1;
