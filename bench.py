@@ -766,13 +766,15 @@ def patterns5_arm(args, dist: Dist) -> None:
 
 
 def ablation_arm(args, dist: Dist) -> None:
-    """What the learned schedule gains, and from what: on the same kernels, (1) the plain
-    degree-threshold heuristic (WARP <= 32 < WIDE <= 128 < CTA <= 1024 < split), (2) that
-    heuristic extended with the per-task variants by thresholds alone (GROUP <= 8 <
-    BUCKET <= 32), (3) the autotuned per-out-degree-bucket variant table (no model), (4)
-    the trained MLP's per-task choice.  4-clique on R-MAT scale 22 seed 2 (a training
-    scale, other seed) and on the held-out R-MAT scale 23 seed 99; the 4096-graph BA batch
-    (triangle + 4-clique + diamond).  Counts must agree across the arms."""
+    """What the learned schedule gains, and from what.  On the task kernel (an explicit hub
+    limit, with its default value, leaves the count to it): (1) the plain degree-threshold
+    heuristic (WARP <= 32 < WIDE <= 128 < CTA <= 1024 < split), (2) that heuristic extended
+    with the per-task variants by thresholds alone (GROUP <= 8 < BUCKET <= 32), (3) the
+    trained MLP's per-task choice.  Beside them the engine's own choice of kernels: (4) the
+    default schedule, (5) the autotuned table (the engine's choice where no table of variants
+    is faster).  4-clique on R-MAT scale 22 seed 2 (a training scale, other seed) and on the
+    held-out R-MAT scale 23 seed 99; the 4096-graph BA batch (triangle + 4-clique + diamond).
+    Counts must agree across the arms."""
     import numpy as np
     import torch
 
@@ -780,6 +782,7 @@ def ablation_arm(args, dist: Dist) -> None:
     torch.cuda.set_device(dist.local)
     ctx = xgm.Context(dist.local)
     learned = xgm.trained_schedule(ctx)
+    tasks = {"hub_max": 1536}
     ext = {"group_max": 8, "bucket_max": 32}
 
     def best_ms(fn, reps):
@@ -797,10 +800,10 @@ def ablation_arm(args, dist: Dist) -> None:
         g = ctx.graph_from_edges(nv, src, dst)
         del src, dst
         tune = ctx.autotune(g, "4-clique", reps=2)
-        arms = {"heuristic": {}, "extended_heuristic": ext,
+        arms = {"heuristic": tasks, "extended_heuristic": ext, "default": {},
                 "autotuned": {"policy": xgm.SCHED_TUNED, "table": tune["table"]}}
         if learned:
-            arms["learned"] = learned
+            arms["learned"] = {**learned, **tasks}
         row, want = {}, None
         for name, kw in arms.items():
             def run(kw=kw):
@@ -816,10 +819,10 @@ def ablation_arm(args, dist: Dist) -> None:
     vo, eo, src, dst = xgm.gen_ba_batch(4096, 100, 5000, 3, 8, seed=5)
     b = ctx.batch_from_edges(vo, src, dst)
     tune = ctx.autotune(b, BATCH_PATTERNS, reps=3)
-    arms = {"heuristic": {}, "extended_heuristic": ext,
+    arms = {"heuristic": tasks, "extended_heuristic": ext, "default": {},
             "autotuned": {"policy": xgm.SCHED_TUNED, "table": tune["table"]}}
     if learned:
-        arms["learned"] = learned
+        arms["learned"] = {**learned, **tasks}
     row, want = {}, None
     for name, kw in arms.items():
         def run(kw=kw):
@@ -835,8 +838,9 @@ def ablation_arm(args, dist: Dist) -> None:
     line = {"workload": "schedule ablation (ms per count, best of the steps)", "results": res,
             "schedule_definitions": {"heuristic": "WARP <= 32 < WIDE <= 128 < CTA <= 1024 < split",
                                      "extended_heuristic": "GROUP <= 8 < BUCKET <= 32 < WIDE <= 128 < CTA <= 1024 < split",
-                                     "autotuned": "per out-degree bucket variant table (xgm_autotune)",
-                                     "learned": "MLP per task (costmodel.json)"},
+                                     "learned": "MLP per task (costmodel.json)",
+                                     "default": "owner and row kernels",
+                                     "autotuned": "xgm_autotune: the engine's choice or a variant table"},
             "clocks": clk}
     print(json.dumps(line), flush=True)
     ctx.close()

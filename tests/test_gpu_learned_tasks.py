@@ -124,3 +124,44 @@ def test_order_of_the_roots_above_the_row_capacity(xgm, ctx):
     assert kernels[0] == ctx.count_kernels(g, "4-clique")
     assert kernels[1] != kernels[0]
     g.close()
+
+
+def test_the_trainer_times_the_model(xgm, ctx):
+    """Validation and evaluation of a trained model are counts on the kernel that it schedules."""
+    import importlib
+
+    tr = importlib.import_module("x-gminer_gb300.train_costmodel")
+    nv, src, dst = xgm.gen_rmat(13, 16, seed=6)
+    g = ctx.graph_from_edges(nv, src, dst)
+    m = _favouring(xgm, ctx, xgm.VAR_CTA)
+    for pat in tr.PATTERNS + ["triangle"]:
+        n, ms, tasks = tr.timed_count(ctx, g, pat, 1)
+        assert n == ctx.count(g, pat) and ms > 0 and sum(tasks) > 0, pat
+        _, _, by_model = tr.timed_count(ctx, g, pat, 1, policy=xgm.SCHED_LEARNED, model=m, margin=0.2)
+        assert sum(by_model) == sum(tasks) and by_model[xgm.VAR_CTA] == sum(by_model), pat
+    g.close()
+
+
+def test_trained_model_gains_on_the_task_kernel(xgm, ctx):
+    """As test_gpu_learned.py's gain on a held-out graph (R-MAT scale 21, seed 77; 3 % for the
+    noise of the clock), on the kernel that the model schedules."""
+    learned = xgm.trained_schedule(ctx)
+    if not learned:
+        pytest.skip("costmodel.json absent")
+    nv, s, d = xgm.gen_rmat(21, 16, seed=77)
+    g = ctx.graph_from_edges(nv, s, d)
+
+    def best(kw):
+        ctx.count(g, "4-clique", hub_max=1536, **kw)
+        ms = []
+        for _ in range(5):
+            cnt, st = ctx.count(g, "4-clique", hub_max=1536, with_stats=True, **kw)
+            assert sum(st["variant_tasks"]) > 0
+            ms.append(st["kernel_ms"] + st["prep_ms"])
+        return cnt, min(ms)
+
+    c_h, t_h = best({})
+    c_l, t_l = best(learned)
+    assert c_l == c_h
+    assert t_l <= 1.03 * t_h, f"learned {t_l:.2f} ms vs plain heuristic {t_h:.2f} ms"
+    g.close()

@@ -5,8 +5,8 @@ Training data: per-task clock64 timings the engine logs (xgm_model_collect) for 
 kernel, whose tasks are the k = 3 tasks) on R-MAT graphs of scales 18-22, edge factor
 16, seeds 10-14, under every kernel variant.  The network (12 -> 32 -> 1, fp16
 weights) is trained by the engine's own forward/backward/Adam kernels.  Evaluation: a
-held-out R-MAT scale 23 (seed 99) graph, learned vs plain degree-threshold schedule,
-same counts.
+held-out R-MAT scale 23 (seed 99) graph, learned vs plain degree-threshold schedule of the
+task kernel, same counts.
 
     python x-gminer_gb300/train_costmodel.py [--scales 18 19 20 21 22] [--eval-scale 23]
 """
@@ -30,7 +30,15 @@ OUT = os.path.join(HERE, "costmodel.json")
 PATTERNS = ["4-clique", "5-clique", "diamond"]
 
 
+def on_tasks(pat=None):
+    """Arguments of a count that the task kernel makes, whose schedule the model is: an explicit
+    hub limit, with the value that the default schedule has.  (Left open, the default and the
+    learned schedule run the owner and row kernels, the same for both.)"""
+    return {"hub_max": -1 if pat == "5-clique" else 1536}
+
+
 def timed_count(ctx, g, pat, reps, **kw):
+    kw = {**on_tasks(pat), **kw}
     ctx.count(g, pat, **kw)  # warm
     best = None
     cnt = None
@@ -99,6 +107,7 @@ def main():
     pats_b = ["triangle", "4-clique", "diamond"]
 
     def time_batch(b, **kw):
+        kw = {**on_tasks(), **kw}
         for _ in range(3):
             ctx.count_batched(b, pats_b, **kw)
         best, out = None, None
