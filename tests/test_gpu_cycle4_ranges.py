@@ -83,3 +83,23 @@ def test_batches_of_heavy_vertices(xgm, orc, ctx):
     want = [orc.count("cycle4", *orc.build_csr(n, s, d)) for s, d, n in parts]
     assert got == want
     b.close()
+
+
+@pytest.mark.parametrize("spokes", [8192, 8193, 9001, 20000])
+def test_one_id_in_more_rows_than_a_table_takes(xgm, orc, ctx, spokes):
+    """Two hubs with the same spokes: one v2 has as many wedges as there are spokes, the others
+    one each, all over the ids."""
+    rng = np.random.default_rng(9)
+    sp = np.arange(RIMS, RIMS + spokes)
+    c, v0 = RIMS + spokes, RIMS + spokes + 1
+    parts = [(np.full(spokes, c), sp), (np.full(spokes, v0), sp),
+             (np.full(10, v0), rng.choice(RIMS, 10, replace=False)),
+             (sp, rng.integers(0, RIMS, spokes)), (np.arange(RIMS), rng.permutation(RIMS))]
+    nv = RIMS + spokes + 2
+    src = np.concatenate([p[0] for p in parts]).astype(np.int32)
+    dst = np.concatenate([p[1] for p in parts]).astype(np.int32)
+    want = orc.count("cycle4", *orc.build_csr(nv, src, dst))
+    assert want >= spokes * (spokes - 1) // 2
+    g = ctx.graph_from_edges(nv, src, dst)
+    assert ctx.count(g, "rectangle") == want
+    g.close()
