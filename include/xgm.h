@@ -265,8 +265,11 @@ typedef struct {
                               graphs of long lists) */
   uint64_t algo_bytes;     /* algorithmic adjacency bytes of the plan (0 unless requested) */
   uint32_t device_error;   /* raw device error flag */
-  int launches;            /* counting passes: 1, + 1 where the hub kernel runs (the kernels
-                              of a whole call: xgm_count_kernels) */
+  int launches;            /* set-operation programs and replayed batches: kernels launched.
+                              Other counts: counting passes, not kernels (a clique count 1,
+                              + 1 where the hub kernel runs; diamonds and tailed triangles 2;
+                              4-cycles 1; a census the sum of its parts); the kernels of a
+                              clique count: xgm_count_kernels */
 } xgm_stats;
 
 /* Counts `plan` on `g`.  out_count receives the exact uint64 total. */
