@@ -156,7 +156,7 @@ bool task_kernel_wins_part(const DevGraph& g) {
 // 0.45 / 0.37 there, 100 s12 ef8 (33) 0.49 / 0.51; triangles + diamonds 0.49 / 0.41 and 0.52 /
 // 0.61; tailed triangles 200 s11 ef8 0.45 / 0.50; 16 s16 ef16 (141) 6.3 / 22.9.
 bool task_kernel_wins_batch(const DevGraph& g, bool rows, bool part, bool five, bool tail) {
-  return g.pairs + g.stream >= ((rows && part) || five || tail ? 20.0 : 31.0) * (double)g.ne_dag;
+  return g.pairs + g.stream > ((rows && part) || five || tail ? 20.0 : 31.0) * (double)g.ne_dag;
 }
 
 // Fills tb from the schedule policy for a k-clique style launch (k = 3 for the
