@@ -161,3 +161,21 @@ def test_batches_of_both_routes(xgm, ctx, kind, tasks):
         if sub != ["5-clique"]:
             assert (sum(st["variant_tasks"]) > 0) == tasks, sub
     b.close()
+
+
+@pytest.mark.parametrize("core,leaves,per", [(30, 300001, 14), (40, 1000, 33), (3, 9, 2)])
+def test_tailed_triangles_of_hubs(xgm, ctx, core, leaves, per):
+    """The first has edges in 300,000 triangles between vertices of degree 300,000 (a term above
+    32 bits), the second 34 out-neighbours a vertex on average (a warp a vertex), the third 2."""
+    iu = np.triu_indices(core, 1)
+    ls = np.repeat(np.arange(core, core + leaves, dtype=np.int32), per)
+    ld = np.tile(np.arange(per, dtype=np.int32), leaves)
+    g = ctx.graph_from_edges(core + leaves, np.concatenate([iu[0].astype(np.int32), ls]),
+                             np.concatenate([iu[1].astype(np.int32), ld]))
+    t_in = math.comb(core - 1, 2) + leaves * (per - 1)  # triangles of a joined core vertex
+    want = per * t_in * (core - 1 + leaves - 2) + (core - per) * math.comb(core - 1, 2) * (core - 3)
+    want += leaves * math.comb(per, 2) * max(per - 2, 0)
+    n, st = ctx.count(g, "tailedtriangle", with_stats=True)
+    assert n == want and sum(st["variant_tasks"]) == 0
+    assert ctx.count(g, "tailedtriangle", policy=xgm.SCHED_FIXED, variant=xgm.VAR_WARP) == want
+    g.close()

@@ -349,7 +349,7 @@ xgm_status count_dispatch(xgm_ctx* ctx, const DevGraph& g, int pattern, const xg
     else if (tasks)  // one pass over the vertices (Erdos-Renyi 2^20 degree 256 33.0 -> 31.8 ms)
       XGM_CUDA_TRY(launch_tailed_reduce(view, ctx->vpart, &ctx->d_sc->count, s));
     else
-      XGM_CUDA_TRY(launch_motif_terms(view, ctx->epart, ctx->d_sc->terms, s));
+      XGM_CUDA_TRY(launch_tailed_edges(view, g.ne_dag, ctx->epart, ctx->d_sc->terms, s));
     launches = 2;
   } else if (pattern == XGM_PATTERN_CYCLE4) {
     XGM_CUDA_TRY(with_room(ctx, [&] {

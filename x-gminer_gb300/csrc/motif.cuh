@@ -14,6 +14,10 @@ cudaError_t launch_diamond_reduce(const unsigned* epart, int64_t ne, unsigned lo
 cudaError_t launch_tailed_reduce(const GView& g, const unsigned long long* vpart,
                                  unsigned long long* out, cudaStream_t s);
 
+// out[3], out[6] += the tailed-triangle sums of launch_motif_terms.
+cudaError_t launch_tailed_edges(const GView& g, int64_t ne_dag, const unsigned* epart,
+                                unsigned long long* out, cudaStream_t s);
+
 // out[0..6] += the wedge / 3-star / 3-walk / tailed-triangle / diamond / 3 x triangle sums
 // (edge-induced; see motif.cu; epart null for the 3-vertex census).  next, here and below: the
 // kernel may start before the one launched before it has ended (launch_next).
